@@ -246,6 +246,12 @@ struct Geom {
     DevView tile_tris;  // int [blocks][tile_maxt]
     DevView tile_nt;    // int [blocks]
     DevView tile_loc;   // uint8 [N][2]
+    // patch fill (fill_patch.cu): compact groups of 24 RWGs and their triangles
+    bool patch_ready = false;
+    bool patch_ok = false;  // every free vertex is a corner of its triangle
+    int patch_nb = 0;
+    DevBuf patch_block;  // one allocation holding the arrays below
+    DevView patch_rwg, patch_nt, patch_tri, patch_slot, patch_side, patch_sphere, patch_sc;
 };
 
 // the FP64 vertices on the device (uploaded on first use)

@@ -112,6 +112,18 @@ __host__ __device__ inline void gauss7(V3<T> a, V3<T> b, V3<T> c, V3<T>* p)
     }
 }
 
+// barycentric coordinates of point i of the rule
+__host__ __device__ inline void gauss7_bary(int i, double out[3])
+{
+    const double g[7][2] = {{0.333333333333333, 0.333333333333333}, {0.797426985353087, 0.101286507323456},
+                            {0.101286507323456, 0.797426985353087}, {0.101286507323456, 0.101286507323456},
+                            {0.470142064105115, 0.470142064105115}, {0.470142064105115, 0.059715871789770},
+                            {0.059715871789770, 0.470142064105115}};
+    out[0] = g[i][0];
+    out[1] = g[i][1];
+    out[2] = 1.0 - g[i][0] - g[i][1];
+}
+
 template <typename T>
 __host__ __device__ inline T gauss7_weight(int i)
 {

@@ -14,10 +14,12 @@
 // 16 x 16 block's triangle pairs staged once); the EFIE one, whose regular
 // part is symmetric, fills the upper triangle of tiles and mirrors it
 // (k_fill_tile_sym); the CFIE one fills a tile and its mirror from the same
-// staged values, the EFIE part once for both (k_fill_tile_cfie_sym).
+// staged values, the EFIE part once for both (k_fill_tile_cfie_sym).  The FP64
+// entries and the 7 x 7-point ones come from patches of RWGs (fill_patch.cu).
 #include "emfa_internal.cuh"
 #include "emfa_math.cuh"
 #include "fill_entry.cuh"
+#include "fill_patch.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -273,73 +275,113 @@ __device__ void potential_integrals(const V3<double>* v, V3<double> r, double* I
     *Irho_out = Ir;
 }
 
-// one configuration-table value (unsigned), FP64
-__device__ static Cx<double> efie_cfg_pair(const V3<double>* tf, const V3<double>* ts, V3<double> vf, V3<double> vs,
-                                           bool self, const SingConst& c)
+// table: per triangle t, 4 slots (0 the triangle itself, 1..3 its edge
+// neighbours in nbr order) x 9 (field corner, source corner).  A (triangle,
+// slot) pair's kernel values and potential integrals belong to its points, not
+// to its corners: 8 threads a pair, thread p < 7 taking field point p (its row
+// of 7 smooth kernel values, reduced to the three barycentric sums that the
+// corners share, and its potential integrals), then a thread per value adds
+// the 7 rows in order.  Bound by the FP64 pipe; with a thread per value, each
+// doing all 49 point pairs, T = 1280 took 1.05 ms, now 0.16 ms.
+constexpr int CT_PAIRS = 16;
+__global__ void __launch_bounds__(8 * CT_PAIRS) k_config_table(const double* __restrict__ vd,
+                                                               const int* __restrict__ tris,
+                                                               const int* __restrict__ nbr, int nt, SingConst c,
+                                                               double2* __restrict__ tab)
 {
-    V3<double> P[7], Q[7];
-    gauss7(tf[0], tf[1], tf[2], P);
-    gauss7(ts[0], ts[1], ts[2], Q);
-    const double As = tri_area(ts[0], ts[1], ts[2]);
-    const V3<double> ns = normalized(cross(ts[1] - ts[0], ts[2] - ts[0]));
-    double zr = 0.0, zi = 0.0, sing = 0.0;
-    for (int p = 0; p < 7; ++p) {
+    __shared__ double2 row[CT_PAIRS][7][9];
+    const int pl = threadIdx.x >> 3, p = threadIdx.x & 7;
+    const int pair = blockIdx.x * CT_PAIRS + pl;
+    const int t = pair >> 2, slot = pair & 3;
+    const int s = t >= nt ? -1 : slot == 0 ? t : nbr[3 * t + slot - 1];
+    if (s >= 0 && p < 7) {
+        V3<double> tf[3], ts[3], P[7], Q[7];
+        for (int j = 0; j < 3; ++j) {
+            const int a = tris[3 * t + j], b = tris[3 * s + j];
+            tf[j] = v3(vd[3 * a], vd[3 * a + 1], vd[3 * a + 2]);
+            ts[j] = v3(vd[3 * b], vd[3 * b + 1], vd[3 * b + 2]);
+        }
+        gauss7(tf[0], tf[1], tf[2], P);
+        gauss7(ts[0], ts[1], ts[2], Q);
+        V3<double> Pp = P[0];
+#pragma unroll
+        for (int i = 1; i < 7; ++i)
+            if (i == p) Pp = P[i];
         const double wp = gauss7_weight<double>(p);
-        const V3<double> rf = P[p] - vf;
+        // g_j = sum_q w_q lambda_j(q) Gs(R_pq)
+        double gr[3] = {0, 0, 0}, gi[3] = {0, 0, 0};
+#pragma unroll
         for (int q = 0; q < 7; ++q) {
-            const double wq = gauss7_weight<double>(q);
-            const double R = norm(P[p] - Q[q]);
-            const double e = wp * wq * (0.25 * dot(rf, Q[q] - vs) - c.inv_k2);
+            const double R = norm(Pp - Q[q]);
+            double sr = 0.0, si = -c.k;
             if (R > 0) {
                 double sn, cs;
                 sincos(0.5 * c.k * R, &sn, &cs);
-                zr += e * (-2.0 * sn * sn / R);
-                zi += e * (-2.0 * sn * cs / R);
-            } else {
-                zi += e * (-c.k);
+                const double f = -2.0 * sn / R;
+                sr = f * sn;
+                si = f * cs;
+            }
+            double bary[3];
+            gauss7_bary(q, bary);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const double w = gauss7_weight<double>(q) * bary[j];
+                gr[j] += w * sr;
+                gi[j] += w * si;
             }
         }
+        const double g0r = gr[0] + gr[1] + gr[2], g0i = gi[0] + gi[1] + gi[2];
+        const double iA = 1.0 / tri_area(ts[0], ts[1], ts[2]);
+        const V3<double> ns = normalized(cross(ts[1] - ts[0], ts[2] - ts[0]));
         double I1;
         V3<double> Ir;
-        potential_integrals(ts, P[p], &I1, &Ir);
-        const V3<double> rho = P[p] - ns * dot(P[p] - ts[0], ns);
-        sing += wp * (0.25 * dot(rf, Ir + (rho - vs) * I1) - I1 * c.inv_k2);
+        potential_integrals(ts, Pp, &I1, &Ir);
+        const V3<double> rho = Pp - ns * dot(Pp - ts[0], ns);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const int b1 = (b + 1) % 3, b2 = (b + 2) % 3;
+            const V3<double> e1 = ts[b1] - ts[b], e2 = ts[b2] - ts[b];
+            // source vector of the row: smooth part and potential integrals
+            const V3<double> vr = e1 * gr[b1] + e2 * gr[b2] + (Ir + (rho - ts[b]) * I1) * iA;
+            const V3<double> vi = e1 * gi[b1] + e2 * gi[b2];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const V3<double> rf = Pp - tf[a];
+                row[pl][p][3 * a + b] = make_double2(wp * (0.25 * dot(rf, vr) - (g0r + I1 * iA) * c.inv_k2),
+                                                     wp * (0.25 * dot(rf, vi) - g0i * c.inv_k2));
+            }
+        }
     }
-    zr += sing / As;
-    if (self && sqrt(c.sig_re * c.sig_re + c.sig_im * c.sig_im) > 1e-8) {
-        // surface-impedance term (EFIE.cpp:297-306) with the 7-point rule
-        double acc = 0.0;
-        for (int i = 0; i < 7; ++i) acc += gauss7_weight<double>(i) * dot(P[i] - vf, P[i] - vs);
-        const double den = As * c.k * c.z0;
-        zr += c.pi * c.sig_im / den * acc;
-        zi -= c.pi * c.sig_re / den * acc;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 9 * CT_PAIRS; i += blockDim.x) {
+        const int l = i / 9, combo = i - 9 * l;
+        const int pr = blockIdx.x * CT_PAIRS + l, tt = pr >> 2, sl = pr & 3;
+        if (tt >= nt) continue;
+        const int so = sl == 0 ? tt : nbr[3 * tt + sl - 1];
+        double2 z = make_double2(0.0, 0.0);
+        if (so >= 0) {
+            for (int q = 0; q < 7; ++q) {
+                z.x += row[l][q][combo].x;
+                z.y += row[l][q][combo].y;
+            }
+            if (sl == 0 && sqrt(c.sig_re * c.sig_re + c.sig_im * c.sig_im) > 1e-8) {
+                // surface-impedance term (EFIE.cpp:297-306) with the 7-point rule
+                V3<double> v[3], P[7];
+                for (int j = 0; j < 3; ++j) {
+                    const int a = tris[3 * tt + j];
+                    v[j] = v3(vd[3 * a], vd[3 * a + 1], vd[3 * a + 2]);
+                }
+                gauss7(v[0], v[1], v[2], P);
+                double acc = 0.0;
+                for (int q = 0; q < 7; ++q)
+                    acc += gauss7_weight<double>(q) * dot(P[q] - v[combo / 3], P[q] - v[combo % 3]);
+                const double den = tri_area(v[0], v[1], v[2]) * c.k * c.z0;
+                z.x += c.pi * c.sig_im / den * acc;
+                z.y -= c.pi * c.sig_re / den * acc;
+            }
+        }
+        tab[(size_t)9 * pr + combo] = z;
     }
-    return cx(zr, zi);
-}
-
-// table: per triangle t, 4 slots (0 the triangle itself, 1..3 its edge
-// neighbours in nbr order) x 9 (field corner, source corner); a thread per
-// value
-__global__ void __launch_bounds__(144) k_config_table(const double* __restrict__ vd, const int* __restrict__ tris,
-                                                      const int* __restrict__ nbr, int nt, SingConst c,
-                                                      double2* __restrict__ tab)
-{
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= 36 * nt) return;
-    const int t = id / 36, slot = (id / 9) % 4, ef = (id / 3) % 3, es = id % 3;
-    const int s = slot == 0 ? t : nbr[3 * t + slot - 1];
-    if (s < 0) {
-        tab[id] = make_double2(0.0, 0.0);
-        return;
-    }
-    V3<double> tf[3], ts[3];
-    for (int j = 0; j < 3; ++j) {
-        int a = tris[3 * t + j], b = tris[3 * s + j];
-        tf[j] = v3(vd[3 * a], vd[3 * a + 1], vd[3 * a + 2]);
-        ts[j] = v3(vd[3 * b], vd[3 * b + 1], vd[3 * b + 2]);
-    }
-    const Cx<double> z = efie_cfg_pair(tf, ts, tf[ef], ts[es], slot == 0, c);
-    tab[id] = make_double2(z.re, z.im);
 }
 
 // one entry in the configuration's discretisation (EFIE): the far-pair
@@ -366,10 +408,7 @@ __device__ __forceinline__ Cx<T> z_entry_cfg(const RwgPack<T>& F, const RwgPack<
         for (int b = 0; b < 2; ++b) {
             const T sgn = (a == b) ? T(1) : T(-1);
             const int ts = S.tri[b];
-            const int slot = ts == tf ? 0
-                             : nbr[3 * tf] == ts ? 1
-                             : nbr[3 * tf + 1] == ts ? 2
-                             : nbr[3 * tf + 2] == ts ? 3 : -1;
+            const int slot = table_slot(nbr, tf, ts);
             if (slot >= 0) {
                 const double2 v = tab[(size_t)36 * tf + 9 * slot + 3 * F.e[a] + S.e[b]];
                 sr += (double)sgn * v.x;
@@ -418,7 +457,9 @@ __global__ void __launch_bounds__(256) k_fill_z_cfg(const RwgPack<T>* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// entry kernel: one thread per Z(f, s); a warp runs 32 consecutive s of one f
+// entry kernel: one thread per Z(f, s); a warp runs 32 consecutive s of one f.
+// For RWG tables whose free vertices are not corners of their triangles, which
+// the patch fill (fill_patch.cu) does not take; likewise k_fill_z_cfg above.
 // ---------------------------------------------------------------------------
 template <typename T, bool CFIE>
 __global__ void __launch_bounds__(256) k_fill_z(const RwgPack<T>* __restrict__ rw, int n, FillConst<T> c,
@@ -1085,20 +1126,22 @@ static emfa_status_t fill_z_cfg(Ctx* c, Geom* g, GeomDev<T>& d, const emfa_fill_
     void* tab = nullptr;
     EMFA_TRY(ctx_workspace(c, WS_FILL, sizeof(double2) * (size_t)g->nt * 36, &tab));
     const SingConst sc = sing_const(p);
-    k_config_table<<<(36 * g->nt + 143) / 144, 144, 0, st>>>(dptr<double>(g->vd), dptr<int>(d.tris),
-                                                             dptr<int>(g->nbr), g->nt, sc, (double2*)tab);
+    k_config_table<<<(4 * g->nt + CT_PAIRS - 1) / CT_PAIRS, 8 * CT_PAIRS, 0, st>>>(
+        dptr<double>(g->vd), dptr<int>(d.tris), dptr<int>(g->nbr), g->nt, sc, (double2*)tab);
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
     FillConst<T> fc = make_fill_const<T>(p);
-    dim3 blk(32, 8);
-    dim3 grd((g->n + 31) / 32, (g->n + 7) / 8);
-    {
+    bool done = false;
+    EMFA_TRY(launch_fill_patch<T>(c, g, d, p, fc, (const double2*)tab, Z, ldz, st, &done));
+    if (!done) {
+        dim3 blk(32, 8);
+        dim3 grd((g->n + 31) / 32, (g->n + 7) / 8);
         TimedLaunch tl(c, KT_FILL_Z, st, (double)g->n * g->n);
         k_fill_z_cfg<T><<<grd, blk, 0, st>>>(dptr<RwgPack<T>>(d.rwg), g->n, fc, (const double2*)tab,
                                              dptr<int>(g->nbr), dptr<T>(d.tri_q7), reinterpret_cast<Cx<T>*>(Z), ldz);
+        c->kernel_launches += 1;
+        EMFA_CUDA(c, cudaGetLastError());
     }
-    c->kernel_launches += 1;
-    EMFA_CUDA(c, cudaGetLastError());
     EMFA_CUDA(c, cudaStreamSynchronize(st));
     return EMFA_OK;
 }
@@ -1150,9 +1193,11 @@ static emfa_status_t fill_z_t(Ctx* c, Geom* g, GeomDev<T>& d, const emfa_fill_pa
         EMFA_CUDA(c, cudaStreamSynchronize(st));
         return EMFA_OK;
     }
-    dim3 blk(32, 8);
-    dim3 grd((g->n + 31) / 32, (g->n + 7) / 8);
-    {
+    bool done = false;
+    EMFA_TRY(launch_fill_patch<T>(c, g, d, p, fc, (const double2*)tab, Z, ldz, st, &done));
+    if (!done) {
+        dim3 blk(32, 8);
+        dim3 grd((g->n + 31) / 32, (g->n + 7) / 8);
         TimedLaunch tl(c, KT_FILL_Z, st, (double)g->n * g->n);
         if (cfie)
             k_fill_z<T, true><<<grd, blk, 0, st>>>(dptr<RwgPack<T>>(d.rwg), g->n, fc, (const double2*)tab,
@@ -1160,9 +1205,9 @@ static emfa_status_t fill_z_t(Ctx* c, Geom* g, GeomDev<T>& d, const emfa_fill_pa
         else
             k_fill_z<T, false><<<grd, blk, 0, st>>>(dptr<RwgPack<T>>(d.rwg), g->n, fc, (const double2*)tab,
                                                     reinterpret_cast<Cx<T>*>(Z), ldz);
+        c->kernel_launches += 1;
+        EMFA_CUDA(c, cudaGetLastError());
     }
-    c->kernel_launches += 1;
-    EMFA_CUDA(c, cudaGetLastError());
     EMFA_CUDA(c, cudaStreamSynchronize(st));
     return EMFA_OK;
 }
