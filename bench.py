@@ -247,7 +247,7 @@ def plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, X_mixed, r_mixed):
     import torch
     from emfa_gb300 import api
     fp64 = api.fill_params("cfie", "f64", freq, alpha)
-    sp64 = api.solver_params("gmres", restart=30, max_iter=900, tol=1e-6)
+    sp64 = api.solver_params("gmres", restart=30, max_iter=900, tol=1e-6, matvec="f64")
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     Z = api.fill_z(geo, fp64)
@@ -357,12 +357,12 @@ def run_c1(args):
     dirs = api.bistatic_dirs(0.0, 180.0, 1.0, 0.0, ring=True)
     out = {"workload": "c1_efie_sphere_1920", "n_rwg": geo.n, "directions": int(dirs.shape[0])}
     for name, prec, sp, disc in (
-            ("plain_fp64", "f64", api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000), "reference"),
+            ("plain_fp64", "f64", api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000, matvec="f64"), "reference"),
             ("mixed", "f32", api.solver_params("lu", tol=1e-6, max_iter=50), "reference"),
             # the discretisation the configuration states: 7-point rule,
             # extraction on self and edge-adjacent pairs (no reference run)
             ("plain_fp64_config_discretisation", "f64",
-             api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000), "config"),
+             api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000, matvec="f64"), "config"),
             ("mixed_config_discretisation", "f32", api.solver_params("lu", tol=1e-6, max_iter=50), "config")):
         fp = api.fill_params("efie", prec, 3e8, 1.0, discretisation=disc)
         times = []
@@ -580,7 +580,7 @@ def run_batch(args):
         geo = api.Geometry(ctx, m)
         fp = api.fill_params("efie", "f64", f, 1.0)
         fp.edm_mode = 2
-        sp = api.solver_params("gmres", restart=250, tol=1e-5, max_iter=5000)
+        sp = api.solver_params("gmres", restart=250, tol=1e-5, max_iter=5000, matvec="f64")
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         Z = api.fill_z(geo, fp)

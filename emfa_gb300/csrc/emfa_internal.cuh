@@ -89,6 +89,8 @@ enum WorkspaceSlot {
     WS_GEMM_B = 0, WS_GEMM_ERR, WS_KRYLOV, WS_FILL, WS_RCS, WS_ZPLANES, WS_HGEMM,
     WS_DENSE_Z, WS_DENSE_V, WS_DENSE_X,  // emfa_dense_rcs: the job's matrix, excitation and currents
     WS_LU_WAVE,                          // tickets and flags of the LU's triangular solves
+    WS_SLICE_Z, WS_SLICE_B,              // a solve's digit planes and product scratch (gemm_slice.cu)
+    WS_SLICE_MV, WS_SLICE_MV_B,          // the same of single products, which may come between a solve's
     WS_COUNT
 };
 
@@ -114,6 +116,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     std::string last_error;
     std::mutex mu;
+    std::mutex slice_mu;  // launches of one digit-plane product (its workspaces are the context's)
     int sm_count = 0;
     long long kernel_launches = 0;  // kernels launched through this context
     bool stream_ordered = false;  // allocations on `stream` (cudaMallocAsync), for lanes of the server

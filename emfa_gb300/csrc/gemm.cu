@@ -4,8 +4,8 @@
 // for many right-hand sides at once.
 //
 // 64 (f) x 64 (r) CTA tile, 16-wide K slices staged through shared memory,
-// 4 x 4 complex outputs per thread; up to 16 right-hand sides a warp-per-row
-// GEMV instead.  ACC selects the accumulation:
+// 4 x 4 complex outputs per thread; up to 16 right-hand sides, and in FP64
+// always, a warp-per-row GEMV instead.  ACC selects the accumulation:
 //   float / double : plain accumulation in that type
 //   CHUNKED        : FP32 products and sums over 64-wide K chunks, chunk sums
 //                    accumulated in FP64 (the refinement residual of the
@@ -115,6 +115,10 @@ __global__ void __launch_bounds__(256) k_cgemv(const Cx<T>* __restrict__ Z, size
     const int warp = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int f0 = warp * RPW;
     if (f0 >= n) return;
+    // block blockIdx.y of RB right-hand sides
+    X += (size_t)blockIdx.y * RB * n;
+    Y += (size_t)blockIdx.y * RB * n;
+    nrhs = min(RB, nrhs - (int)blockIdx.y * RB);
     T ar[RPW][RB], ai[RPW][RB];
 #pragma unroll
     for (int i = 0; i < RPW; ++i)
@@ -152,35 +156,32 @@ __global__ void __launch_bounds__(256) k_cgemv(const Cx<T>* __restrict__ Z, size
         }
 }
 
-// up to 16 right-hand sides: GEMV launches of 8; more: the tiled kernel
+// blocks of up to 8 right-hand sides, grid y
 template <typename T>
-static emfa_status_t cgemv_chunks(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+static emfa_status_t cgemv_blocks(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
                                   cudaStream_t st)
 {
     constexpr int RPW = sizeof(T) == 8 ? 1 : 4;
     const int warps = (n + RPW - 1) / RPW;
-    for (int r0 = 0; r0 < nrhs; r0 += 8) {
-        const int nr = std::min(8, nrhs - r0);
-        const Cx<T>* x = (const Cx<T>*)X + (size_t)r0 * n;
-        Cx<T>* y = (Cx<T>*)Y + (size_t)r0 * n;
-        const int grd = (warps + 7) / 8;
-        if (nr == 1)
-            k_cgemv<T, 1, RPW><<<grd, 256, 0, st>>>((const Cx<T>*)Z, ldz, x, n, nr, y);
-        else if (nr <= 2)
-            k_cgemv<T, 2, RPW><<<grd, 256, 0, st>>>((const Cx<T>*)Z, ldz, x, n, nr, y);
-        else if (nr <= 4)
-            k_cgemv<T, 4, RPW><<<grd, 256, 0, st>>>((const Cx<T>*)Z, ldz, x, n, nr, y);
-        else
-            k_cgemv<T, 8, RPW><<<grd, 256, 0, st>>>((const Cx<T>*)Z, ldz, x, n, nr, y);
-        c->kernel_launches += 1;
-        EMFA_CUDA(c, cudaGetLastError());
-    }
+    const Cx<T>*z = (const Cx<T>*)Z, *x = (const Cx<T>*)X;
+    Cx<T>* y = (Cx<T>*)Y;
+    const dim3 grd((warps + 7) / 8, (nrhs + 7) / 8);
+    if (nrhs == 1)
+        k_cgemv<T, 1, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
+    else if (nrhs <= 2)
+        k_cgemv<T, 2, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
+    else if (nrhs <= 4)
+        k_cgemv<T, 4, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
+    else
+        k_cgemv<T, 8, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
+    c->kernel_launches += 1;
+    EMFA_CUDA(c, cudaGetLastError());
     return EMFA_OK;
 }
 
 emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)
 {
-    if (nrhs <= 16) return cgemv_chunks<float>(c, Z, ldz, X, n, nrhs, Y, st);
+    if (nrhs <= 16) return cgemv_blocks<float>(c, Z, ldz, X, n, nrhs, Y, st);
     dim3 grd((n + 63) / 64, (nrhs + 63) / 64);
     k_cgemm<float, false><<<grd, 256, 0, st>>>((const Cx<float>*)Z, ldz, (const Cx<float>*)X, n, nrhs, (Cx<float>*)Y,
                                                nullptr, nullptr);
@@ -189,15 +190,14 @@ emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n,
     return EMFA_OK;
 }
 
+// FP64: the GEMV for any number of right-hand sides.  Both are bound by the
+// FP64 pipe, but the 64 x 64 tiles, for which this was once chosen above 16
+// right-hand sides, leave most SMs idle at these sizes (n = 1080 has 17 tiles
+// of rows): n = 1080 x 91, 4456 us with the tiles, 859 us; 2430 x 181, 9.9 ms
+// against 7.3 ms; 5070 x 360, 81 ms against 61 ms.
 emfa_status_t cgemm_f64(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)
 {
-    if (nrhs <= 16) return cgemv_chunks<double>(c, Z, ldz, X, n, nrhs, Y, st);
-    dim3 grd((n + 63) / 64, (nrhs + 63) / 64);
-    k_cgemm<double, false><<<grd, 256, 0, st>>>((const Cx<double>*)Z, ldz, (const Cx<double>*)X, n, nrhs,
-                                                (Cx<double>*)Y, nullptr, nullptr);
-    c->kernel_launches += 1;
-    EMFA_CUDA(c, cudaGetLastError());
-    return EMFA_OK;
+    return cgemv_blocks<double>(c, Z, ldz, X, n, nrhs, Y, st);
 }
 
 emfa_status_t cgemm_f32_chunked(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, const void* Bsub,

@@ -1,0 +1,717 @@
+// Y = Z X in FP64 accuracy on the 5th-generation tensor cores.
+//
+// GB300's FP64 pipe runs at 1/64 of the FP32 one, so the CUDA-core FP64 product
+// (gemm.cu) is bound by it from a few right-hand sides on.  Here both operands
+// are cut into eight signed 8-bit digits,
+//     z = 2^(e-62) sum_s d_s 2^(8 (7 - s)),   |d_s| <= 128,
+// with one power of two per row of Z and per right-hand side (the fixed-point
+// form of an FP64 significand: a row's largest entries keep all 53 bits, 62
+// below the row's maximum for the others), and the digits' products run as
+// FP16 MMAs (integers up to 128 are exact in FP16, their products in FP32).
+// Digit pairs (i, j) of one level i + j share an accumulator; levels 0..7 are
+// kept (36 of the 64 pairs: the next level is 2^-70 of the product of the
+// maxima).  128 columns of at most eight pairs add up to at most 2^24, so every
+// FP32 accumulator holds an exact integer, and the sums across those groups are
+// exact in 64-bit integers: the result is one rounding of the sum, whatever the
+// order, so K can be split over CTAs freely.
+//
+// Accuracy: relative to (row maximum) x (right-hand side's maximum) x sqrt(n) the
+// error is about 2^-68 before the final rounding, so a row's result is as good
+// as an FP64 sum's or better (measured against extended precision at n = 2430,
+// impedance-like with a dominant diagonal: 9e-17, the CUDA-core sums 3e-15); as with any blockwise scaling,
+// entries of a row below 2^-62 of its largest one count as zero.  A row or a
+// right-hand side with an infinity or NaN takes FP64 arithmetic in k_combine.
+//
+// Kernel k_slice<BN>: one 128 x BN tile and one range of K per CTA, 18 warps:
+//   warp 0      TMA producer, K in blocks of 64 columns (128-byte rows): the
+//               eight B planes of a block in one 3-D copy into one of two
+//               buffers, the A planes one by one through a ring
+//   warp 1      tensor memory, MMAs (M = 128, N = BN, K = 16): per block, plane
+//               i of A with planes 0..7-i of B, the k-steps outside, so that
+//               consecutive MMAs add to different levels (each level has its
+//               own BN columns).  After two blocks level i is complete once
+//               plane i of A is done, and is committed for the drain
+//   warps 2..17 drain: a level's columns to integers (FP32 arithmetic only:
+//               conversions share the slow pipe), added to a 64-bit sum per
+//               output; warps 2..9 levels 0-3, warps 10..17 levels 4-7
+// The MMAs are bound by shared-memory operand reads (4 KB + BN 32 B a MMA at
+// 128 B/cycle).  A first form staged 32 columns of all planes at a time, in
+// 64-byte rows: the copies (1536 rows a stage, four cycles each) set its pace,
+// 416 us at n = 2430 x 181 right-hand sides with the tensor pipe 32 % active,
+// whatever the drain did.  A single thread issuing MMAs with descriptors from
+// its own registers bounded the second (382 us, 86 cycles a MMA); now 301 us,
+// 45 %.
+// On GB300, a product of n unknowns and R right-hand sides, its split of Z
+// included, against the CUDA-core products:
+// 1080 x 91: 4456 -> 100 us;  2430 x 181: 9928 -> 428 us;  5070 x 360: 80.9 -> 2.93 ms
+#include "emfa_internal.cuh"
+#include "emfa_math.cuh"
+#include "gemm_slice.cuh"
+#include "tcgen05.cuh"
+
+#include <algorithm>
+#include <climits>
+
+namespace emfa {
+
+namespace sl {
+
+constexpr int NS = 8;        // digits
+constexpr int BM = 128;
+constexpr int BK = 64;       // halves of K per block: 128-byte rows
+constexpr int GROUP = 2;     // blocks per drain: 128 columns
+constexpr int RING = 4;      // A planes in flight
+constexpr int EPI = 8;       // drain warps of each half of the levels
+constexpr int THREADS = 32 * (2 + 2 * EPI);
+constexpr int SLICE_NONFINITE = INT_MAX;
+
+template <int BN>
+struct Smem {
+    static constexpr int A_BYTES = BM * BK * 2;  // one plane
+    static constexpr int B_SLICE = BN * BK * 2;
+    static constexpr int B_BYTES = NS * B_SLICE;
+    static constexpr int TMEM_COLS = NS * BN < 32 ? 32 : NS * BN;
+    static constexpr int TOTAL = RING * A_BYTES + 2 * B_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+};
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(tc::smem_u32(dst)), "l"((uint64_t)map), "r"(tc::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
+// CW consecutive columns (32 lanes x 32 bit) of tensor memory in one round trip
+template <int CW>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v)
+{
+    static_assert(CW == 8 || CW == 16, "");
+    if constexpr (CW == 16) {
+        tc::tmem_ld16(taddr, v);
+    } else {
+        uint32_t r[8];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr));
+        asm volatile("tcgen05.wait::ld.sync.aligned;"
+                     : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                     :
+                     : "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    }
+}
+
+// an integer |v| <= 2^24 held in FP32, plus INT_BIAS, as int: v = 4096 h + l
+// with both halves read off the mantissa of a sum with 1.5 * 2^23 (whose bits
+// are INT_BIAS; 4096 times them vanish modulo 2^32)
+constexpr int INT_BIAS = 0x4B400000;
+__device__ __forceinline__ int biased_int(float v)
+{
+    const float big = 12582912.0f;
+    const float h = fmaf(v, 1.0f / 4096.0f, big);
+    const float l = fmaf(h - big, -4096.0f, v) + big;
+    return (int)(((unsigned)__float_as_int(h) << 12) + (unsigned)__float_as_int(l));
+}
+
+// acc += x w, one multiply-add, w = 256^i from a kernel argument (w8): a power
+// of two known to the compiler becomes four shifts and additions on the ALU pipe, and the drain (30 cycles a
+// value of that pipe) then set the kernel's pace
+__device__ __forceinline__ void mad_wide(unsigned long long& acc, int x, int w)
+{
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(x), "r"(w));
+}
+
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code)
+{
+    return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, err, code));
+}
+// the four K = 16 steps of a block (32 bytes apart in both operands): the first
+// one adds to the columns where accum is not 0, the others always
+__device__ __forceinline__ void mma_f16_block(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
+{
+    asm volatile(
+        "{\n .reg .pred p, q;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        " elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+        " add.s64 a1, %1, 2;\n add.s64 a2, %1, 4;\n add.s64 a3, %1, 6;\n"
+        " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n}\n"
+        ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void commit_elect(uint64_t* bar)
+{
+    asm volatile(
+        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(tc::smem_u32(bar))
+        : "memory");
+}
+
+template <int BN>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_slice(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int C,
+            int kblocks, int per_split, int4 w8, long long* __restrict__ part, int* __restrict__ err)
+{
+    using S = Smem<BN>;
+    using namespace tc;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sA = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [RING]
+    uint8_t* sB = sA + RING * S::A_BYTES;                                       // [2][plane]
+    uint64_t* a_full = (uint64_t*)(sB + 2 * S::B_BYTES);
+    uint64_t* a_empty = a_full + RING;
+    uint64_t* b_full = a_empty + RING;
+    uint64_t* b_empty = b_full + 2;
+    uint64_t* acc_full = b_empty + 2;
+    uint64_t* acc_empty = acc_full + NS;
+    uint64_t* done = acc_empty + NS;
+    uint32_t* tmem_slot = (uint32_t*)(done + 1);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int f0 = blockIdx.y * BM, c0 = blockIdx.x * BN;
+    const int k0 = blockIdx.z * per_split, nk = min(per_split, kblocks - k0);  // blocks; nk >= 1
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < RING; ++i) {
+            mbar_init(a_full + i, 1);
+            mbar_init(a_empty + i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(b_full + i, 1);
+            mbar_init(b_empty + i, 1);
+        }
+        for (int l = 0; l < NS; ++l) {
+            mbar_init(acc_full + l, 1);
+            mbar_init(acc_empty + l, EPI);
+        }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(S::TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int na = 0, nb = 0;  // A planes and B blocks issued
+            bool ok = true;
+            auto load_b = [&](int kb) {
+                const int s = kb & 1;
+                if (kb >= 2 && !mbar_wait(b_empty + s, ((kb >> 1) - 1) & 1, err, 21)) return false;
+                mbar_expect_tx(b_full + s, S::B_BYTES);
+                tma_load_3d(sB + s * S::B_BYTES, &tmB, b_full + s, (k0 + kb) * BK, c0, 0);
+                nb = kb + 1;
+                return true;
+            };
+            ok = load_b(0);
+            for (int kb = 0; kb < nk && ok; ++kb)
+                for (int i = 0; i < NS && ok; ++i) {
+                    const int s = na % RING;
+                    if (na >= RING && !mbar_wait(a_empty + s, ((na / RING) - 1) & 1, err, 22)) {
+                        ok = false;
+                        break;
+                    }
+                    if (*(volatile int*)err) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(a_full + s, S::A_BYTES);
+                    tma_load_3d(sA + s * S::A_BYTES, &tmA, a_full + s, (k0 + kb) * BK, f0, i);
+                    ++na;
+                    if (i == 1 && kb + 1 < nk) ok = load_b(kb + 1);  // its buffer was free a block ago
+                }
+            // every copy issued must have landed before the CTA exits
+            for (int i = na - RING > 0 ? na - RING : 0; i < na; ++i) mbar_wait(a_full + (i % RING), (i / RING) & 1, err, 23);
+            for (int i = nb - 2 > 0 ? nb - 2 : 0; i < nb; ++i) mbar_wait(b_full + (i & 1), (i >> 1) & 1, err, 23);
+        }
+    } else if (warp == 1) {
+        // the whole warp walks the loop and one elected lane issues: the
+        // descriptors then are warp-uniform values, in uniform registers
+        constexpr uint32_t idesc = idesc_f16(BM, BN);
+        const uint32_t dhi = (uint32_t)(sw128_desc(0) >> 32);
+        const uint32_t a_lo = (uint32_t)sw128_desc(smem_u32(sA)), b_lo = (uint32_t)sw128_desc(smem_u32(sB));
+        bool ok = true;
+        for (int kb = 0; kb < nk && ok; ++kb) {
+            const int g = kb / GROUP;
+            const bool first = kb % GROUP == 0, last = kb % GROUP == GROUP - 1 || kb == nk - 1;
+            ok = warp_wait(b_full + (kb & 1), (kb >> 1) & 1, err, 24);
+            if (first && g > 0)
+                for (int l = 0; l < NS && ok; ++l) ok = warp_wait(acc_empty + l, (g - 1) & 1, err, 26);
+            if (!ok) break;
+            const uint32_t lb = b_lo + (kb & 1) * (S::B_BYTES >> 4);
+            const uint32_t add0 = first ? 0u : 1u;
+#pragma unroll
+            for (int i = 0; i < NS; ++i) {
+                const int s = (kb * NS + i) % RING;
+                if (!warp_wait(a_full + s, ((kb * NS + i) / RING) & 1, err, 25)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t la = a_lo + s * (S::A_BYTES >> 4);
+#pragma unroll
+                for (int j = 0; j < NS - i; ++j)
+                    mma_f16_block(tmem + (uint32_t)((i + j) * BN), ((uint64_t)dhi << 32) | la,
+                                  ((uint64_t)dhi << 32) | (lb + j * (S::B_SLICE >> 4)), idesc, i == 0 ? add0 : 1u);
+                commit_elect(a_empty + s);
+                if (last) commit_elect(acc_full + i);
+            }
+            commit_elect(b_empty + (kb & 1));
+        }
+        commit_elect(done);
+        warp_wait(done, 0, err, 27);
+    } else {
+        // drain warps: lane quadrant warp % 4, column half, half of the levels
+        constexpr int CW = BN / 2, LW = CW < 16 ? CW : 16;
+        const int q = warp & 3, half = ((warp - 2) >> 2) & 1, set = (warp - 2) >> 3;
+        const uint32_t tw = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * CW);
+        unsigned long long sum[CW];
+        const int weight[4] = {w8.x, w8.y, w8.z, w8.w};
+#pragma unroll
+        for (int i = 0; i < CW; ++i) sum[i] = 0;
+        const int groups = (nk + GROUP - 1) / GROUP;
+        bool ok = true;
+        for (int g = 0; g < groups && ok; ++g) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int l = 4 * set + j;
+                int w = lane == 0 ? (int)mbar_wait(acc_full + l, g & 1, err, 28) : 0;
+                w = __shfl_sync(0xffffffffu, w, 0);
+                if (!w) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < CW; c += LW) {
+                    float v[LW];
+                    tmem_ld<LW>(tw + (uint32_t)(l * BN + c), v);
+                    if (c + LW == CW) {  // all read: the level may be written again
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(acc_empty + l);
+                    }
+#pragma unroll
+                    for (int i = 0; i < LW; ++i) mad_wide(sum[c + i], biased_int(v[i]), weight[3 - j]);
+                }
+            }
+        }
+        // the bias of every drain and level; modulo 2^64, so the sums may have wrapped
+        const unsigned long long bias = (unsigned long long)groups * INT_BIAS * 0x01010101ull;
+        const int f = f0 + 32 * q + lane;
+        if (ok && f < M) {
+            long long* o = part + ((size_t)blockIdx.z * 2 + set) * C * M;
+#pragma unroll
+            for (int i = 0; i < CW; ++i) {
+                const int col = c0 + half * CW + i;
+                if (col < C) o[(size_t)col * M + f] = (long long)(sum[i] - bias);
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------
+// operand preparation, integers only
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int exponent_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// biased digits of x at scale eb (the row's largest exponent field, at least
+// 1): byte s of the result is d_(7-s) + 128
+__device__ __forceinline__ unsigned long long digits(double x, int eb)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int ef = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+    if (ef) m |= 1ull << 52;
+    const int s = (ef ? ef : 1) - eb + 9;  // 0..9 for the largest
+    long long v;
+    if (s >= 0)
+        v = (long long)(m << s);
+    else
+        v = s < -54 ? 0 : (long long)((m + (1ull << (-s - 1))) >> -s);
+    if ((long long)b < 0) v = -v;
+    return ((unsigned long long)v + 0x0080808080808080ull) ^ (0x80ull << 56);
+}
+
+// digit s of a complex pair as two FP16 integers: the byte under the exponent
+// of 1024 is 1024 + d + 128
+__device__ __forceinline__ unsigned pair_digit(unsigned long long a, unsigned long long b, int s)
+{
+    const int byte = 7 - s;
+    const unsigned wa = (unsigned)(a >> (byte & 4 ? 32 : 0)), wb = (unsigned)(b >> (byte & 4 ? 32 : 0));
+    const unsigned x = (__byte_perm(wa, wb, (byte & 3) | ((4 + (byte & 3)) << 8)) & 0x00ff00ffu) | 0x64006400u;
+    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2half2(__float2half_rn(1152.f)));
+    return *reinterpret_cast<const unsigned*>(&r);
+}
+
+__device__ __forceinline__ int block_max_int(int m, int* red)
+{
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) red[w] = m;
+    __syncthreads();
+    if (w == 0) {
+        m = l < (int)(blockDim.x >> 5) ? red[l] : 0;
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (l == 0) red[0] = m;
+    }
+    __syncthreads();
+    return red[0];
+}
+
+// CTA per row of Z: its scale, then its digits (the row is read twice, the
+// second time from L2)
+__global__ void __launch_bounds__(256) k_slice_rows(const double2* __restrict__ Z, size_t ldz, int n, size_t ldk,
+                                                    __half* __restrict__ D, int* __restrict__ ex)
+{
+    __shared__ int red[32];
+    const int i = blockIdx.x;
+    const double2* z = Z + (size_t)i * ldz;
+    int m = 1;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const double2 v = z[k];
+        m = max(m, max(exponent_field(v.x), exponent_field(v.y)));
+    }
+    m = block_max_int(m, red);
+    const bool bad = m == 0x7ff;
+    if (threadIdx.x == 0) ex[i] = bad ? SLICE_NONFINITE : m;
+    const size_t plane = (size_t)n * ldk / 2;
+    unsigned* o = reinterpret_cast<unsigned*>(D) + (size_t)i * (ldk / 2);
+#pragma unroll 2
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const double2 v = z[k];
+        const unsigned long long a = bad ? 0x8080808080808080ull : digits(v.x, m),
+                                 b = bad ? 0x8080808080808080ull : digits(v.y, m);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) o[s * plane + k] = pair_digit(a, b, s);
+    }
+}
+
+// CTA per right-hand side: B rows 2r = (Re, -Im) and 2r + 1 = (Im, Re)
+__global__ void __launch_bounds__(256) k_slice_rhs(const double2* __restrict__ X, int n, int nrhs, size_t ldk,
+                                                   __half* __restrict__ D, int* __restrict__ ex)
+{
+    __shared__ int red[32];
+    const int r = blockIdx.x;
+    const double2* x = X + (size_t)r * n;
+    int m = 1;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const double2 v = x[k];
+        m = max(m, max(exponent_field(v.x), exponent_field(v.y)));
+    }
+    m = block_max_int(m, red);
+    const bool bad = m == 0x7ff;
+    if (threadIdx.x == 0) ex[r] = bad ? SLICE_NONFINITE : m;
+    const size_t plane = (size_t)2 * nrhs * ldk / 2;
+    unsigned* o0 = reinterpret_cast<unsigned*>(D) + (size_t)(2 * r) * (ldk / 2);
+    unsigned* o1 = o0 + ldk / 2;
+#pragma unroll 2
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const double2 v = x[k];
+        const unsigned long long zero = 0x8080808080808080ull;
+        const unsigned long long a = bad ? zero : digits(v.x, m), b = bad ? zero : digits(v.y, m),
+                                 nb = bad ? zero : digits(-v.y, m);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            o0[s * plane + k] = pair_digit(a, nb, s);
+            o1[s * plane + k] = pair_digit(b, a, s);
+        }
+    }
+}
+
+// (hi 2^32 + lo) 2^ex, rounded to nearest even once (twice below the normal range)
+__device__ __forceinline__ double to_double(long long hi, long long lo, int ex)
+{
+    // 128-bit two's complement t1:t0
+    unsigned long long t0 = ((unsigned long long)hi << 32), t1 = (unsigned long long)(hi >> 32);
+    const unsigned long long s0 = t0 + (unsigned long long)lo;
+    t1 += (unsigned long long)(lo >> 63) + (s0 < t0 ? 1ull : 0ull);
+    t0 = s0;
+    const bool neg = (long long)t1 < 0;
+    if (neg) {
+        t0 = ~t0 + 1ull;
+        t1 = ~t1 + (t0 == 0 ? 1ull : 0ull);
+    }
+    if (!(t0 | t1)) return 0.0;
+    // top 64 significant bits, the rest as a sticky bit
+    int lz;
+    unsigned long long m;
+    if (t1) {
+        lz = __clzll((long long)t1);
+        m = lz ? (t1 << lz) | (t0 >> (64 - lz)) : t1;
+        if (lz ? (t0 << lz) : t0) m |= 1ull;
+    } else {
+        lz = 64 + __clzll((long long)t0);
+        m = t0 << (lz - 64);
+    }
+    unsigned long long q = m >> 11;
+    const unsigned rest = (unsigned)m & 0x7ffu;
+    q += (rest > 0x400u || (rest == 0x400u && (q & 1ull))) ? 1ull : 0ull;  // [2^52, 2^53]
+    const int e = 127 - lz - 52 + ex;  // value = q 2^e
+    double v;
+    if (e + 1075 >= 1 && e + 1075 <= 2045)
+        v = __longlong_as_double((long long)(((unsigned long long)(e + 1074) << 52) + q));
+    else
+        v = scalbn((double)q, e);
+    return neg ? -v : v;
+}
+
+// Y from the partial sums of all splits.  A row or a right-hand side with an
+// infinity or NaN is summed in FP64 as gemm.cu does; a pipeline that gave up
+// (err) leaves NaN.
+__global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ part, int splits, int n, int nrhs,
+                                                 const int* __restrict__ exz, const int* __restrict__ exx,
+                                                 const double2* __restrict__ Z, size_t ldz,
+                                                 const double2* __restrict__ X, const int* __restrict__ err,
+                                                 double2* __restrict__ Y)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+    if (f >= n) return;
+    const int ez = exz[f], ex = exx[r];
+    double2 y;
+    if (*err) {
+        y.x = y.y = __longlong_as_double(0x7ff8000000000000ll);
+    } else if (ez == SLICE_NONFINITE || ex == SLICE_NONFINITE) {
+        const double2* z = Z + (size_t)f * ldz;
+        const double2* x = X + (size_t)r * n;
+        double re = 0.0, im = 0.0;
+        for (int k = 0; k < n; ++k) {
+            const double2 a = z[k], b = x[k];
+            re = fma(a.x, b.x, re);
+            re = fma(-a.y, b.y, re);
+            im = fma(a.x, b.y, im);
+            im = fma(a.y, b.x, im);
+        }
+        y = make_double2(re, im);
+    } else {
+        const size_t plane = (size_t)2 * nrhs * n;
+        const long long* p0 = part + (size_t)(2 * r) * n + f;
+        long long h0 = 0, l0 = 0, h1 = 0, l1 = 0;
+        for (int s = 0; s < splits; ++s, p0 += 2 * plane) {
+            h0 += p0[0];
+            h1 += p0[n];
+            l0 += p0[plane];
+            l1 += p0[plane + n];
+        }
+        // z = V 2^(e-62), e = field - 1022; the lowest kept level weighs 2^56
+        const int e = (ez - 1022) + (ex - 1022) - 124 + 56;
+        y = make_double2(to_double(h0, l0, e), to_double(h1, l1, e));
+    }
+    Y[(size_t)r * n + f] = y;
+}
+
+}  // namespace sl
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+static size_t slice_ld(int n) { return ((size_t)2 * n + 7) & ~(size_t)7; }  // 16-byte rows
+
+static size_t slice_plane_bytes(int n)
+{
+    return Carver::round(sizeof(__half) * sl::NS * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
+}
+
+static emfa_status_t slice_map(Ctx* c, CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, size_t ld,
+                               uint32_t box_rows, uint32_t box_planes)
+{
+    auto fn = tensor_map_encoder();
+    if (!fn) {
+        set_error(c, "cuTensorMapEncodeTiled unavailable");
+        return EMFA_ERR_CUDA;
+    }
+    cuuint64_t dims[3] = {inner, rows, (cuuint64_t)sl::NS};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)ld * 2 * rows};
+    cuuint32_t box[3] = {(cuuint32_t)sl::BK, box_rows, box_planes};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error(c, "cuTensorMapEncodeTiled (digit planes) failed (" + std::to_string((int)r) + ")");
+        return EMFA_ERR_CUDA;
+    }
+    return EMFA_OK;
+}
+
+// error word of the sliced product: int 8 of the context's GEMM error slot
+static emfa_status_t slice_err(Ctx* c, int** err)
+{
+    void* ep = nullptr;
+    EMFA_TRY(ctx_workspace(c, WS_GEMM_ERR, 64, &ep));
+    *err = (int*)ep + 8;
+    return EMFA_OK;
+}
+
+bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st)
+{
+    // The planes take twice the matrix's memory, in workspaces of the context
+    // that calls on its own stream share: a context with an HBM budget, a
+    // caller's stream (its calls may overlap others of the context, and may be
+    // captured) and planes above 16 GB keep the CUDA-core product, which needs
+    // no memory.
+    if (c->budget || c->stream_ordered || st != c->stream || slice_plane_bytes(n) > ((size_t)16 << 30)) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    // Measured (us, a call with its one split of Z | the CUDA-core GEMV): n = 256, 8 right-hand sides 55 | 48,
+    // 16: 59 | 75; 480, 8: 58 | 63; 1080, 4: 81 | 68, 8: 80 | 106; 2430, 4: 182 | 191; 5070, 2: 646 | 438, 4: 647 | 847.
+    // With Z split already, n = 2430, 2: 125 | 110; 5070, 2: 400 | 438.
+    if (built) return n >= 128 && nrhs >= (n >= 2000 ? 3 : n >= 1000 ? 4 : n >= 480 ? 8 : 10);
+    return n >= 128 && nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
+}
+
+emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
+{
+    const size_t ldk = slice_ld(n);
+    void* wp = nullptr;
+    EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(n) + 512, &wp));
+    Carver cv{(char*)wp};
+    __half* d = cv.take<__half>(sl::NS * (size_t)n * ldk);
+    int* ex = cv.take<int>(n);
+    int* err = nullptr;
+    EMFA_TRY(slice_err(c, &err));
+    EMFA_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), st));
+    sl::k_slice_rows<<<n, 256, 0, st>>>((const double2*)Z, ldz, n, ldk, d, ex);
+    c->kernel_launches += 1;
+    EMFA_CUDA(c, cudaGetLastError());
+    *out = SlicePlanes{d, ex, (const double2*)Z, ldz, n, ldk};
+    return EMFA_OK;
+}
+
+// Column tile, and over how many CTAs a tile's K is split: the split with the
+// fewest K blocks in the longest chain of CTAs an SM runs, a CTA's fixed cost
+// (pipeline fill, last drain, 131 KB of partial sums written and read again)
+// counted as two and a half blocks.
+static void slice_shape(Ctx* c, int n, int nrhs, int* bn, int* splits, int* per_split)
+{
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    *bn = 2 * nrhs <= 16 ? 16 : 64;
+    const int blocks = (2 * n + sl::BK - 1) / sl::BK, groups = (blocks + sl::GROUP - 1) / sl::GROUP;
+    const long tiles = (long)((n + sl::BM - 1) / sl::BM) * ((2 * nrhs + *bn - 1) / *bn);
+    long best = -1;
+    for (int s = 1; s <= std::min(groups, 16); ++s) {
+        const int g = (groups + s - 1) / s, used = (groups + g - 1) / g;
+        const long waves = (tiles * used + sms - 1) / sms;
+        const long cost = waves * (2 * g * sl::GROUP + 5);
+        if (best < 0 || cost < best) {
+            best = cost;
+            *splits = used;
+            *per_split = g * sl::GROUP;
+        }
+    }
+}
+
+template <int BN>
+static emfa_status_t launch_slice(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int n, int nrhs, int splits,
+                                  int per_split, long long* part, int* err, cudaStream_t st)
+{
+    using S = sl::Smem<BN>;
+    EMFA_TRY(ensure_smem(c, sl::k_slice<BN>, S::TOTAL));
+    const dim3 grd((2 * nrhs + BN - 1) / BN, (n + sl::BM - 1) / sl::BM, splits);
+    sl::k_slice<BN><<<grd, sl::THREADS, S::TOTAL, st>>>(ta, tb, n, 2 * nrhs, (2 * n + sl::BK - 1) / sl::BK, per_split,
+                                                        make_int4(1, 1 << 8, 1 << 16, 1 << 24), part, err);
+    c->kernel_launches += 1;
+    EMFA_CUDA(c, cudaGetLastError());
+    return EMFA_OK;
+}
+
+emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
+{
+    const int n = p.n;
+    // blocks of right-hand sides bound the scratch (digits and partial sums)
+    constexpr int RB = 512;
+    const int rmax = std::min(nrhs, RB);
+    int bn, splits, per_split;
+    slice_shape(c, n, rmax, &bn, &splits, &per_split);
+    const size_t brow = (size_t)2 * rmax * p.ldk;
+    int smax = splits;
+    if (nrhs % RB) {
+        int b2, s2, p2;
+        slice_shape(c, n, nrhs % RB, &b2, &s2, &p2);
+        // scratch of the last block: fewer columns, perhaps more splits
+        smax = std::max(splits, (int)(((long)s2 * (nrhs % RB) + rmax - 1) / rmax));
+    }
+    void* wp = nullptr;
+    EMFA_TRY(ctx_workspace(c, slot,
+                           Carver::round(sizeof(__half) * sl::NS * brow) + Carver::round(sizeof(int) * (size_t)rmax) +
+                               Carver::round(sizeof(long long) * (size_t)smax * 4 * rmax * n) + 1024,
+                           &wp));
+    Carver cv{(char*)wp};
+    __half* b = cv.take<__half>(sl::NS * brow);
+    int* ex = cv.take<int>(rmax);
+    long long* part = cv.take<long long>((size_t)smax * 4 * rmax * n);
+    int* err = nullptr;
+    EMFA_TRY(slice_err(c, &err));
+    CUtensorMap ta, tb;
+    EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)n, p.ldk, sl::BM, 1));
+    for (int r0 = 0; r0 < nrhs; r0 += RB) {
+        const int nr = std::min(RB, nrhs - r0);
+        const double2* x = (const double2*)X + (size_t)r0 * n;
+        slice_shape(c, n, nr, &bn, &splits, &per_split);
+        EMFA_TRY(slice_map(c, &tb, b, 2 * (uint64_t)n, 2 * (uint64_t)nr, p.ldk, (uint32_t)bn, sl::NS));
+        sl::k_slice_rhs<<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex);
+        c->kernel_launches += 1;
+        EMFA_CUDA(c, cudaGetLastError());
+        EMFA_TRY(bn == 16 ? launch_slice<16>(c, ta, tb, n, nr, splits, per_split, part, err, st)
+                          : launch_slice<64>(c, ta, tb, n, nr, splits, per_split, part, err, st));
+        sl::k_combine<<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, p.Z, p.ldz, x, err,
+                                                                 (double2*)Y + (size_t)r0 * n);
+        c->kernel_launches += 1;
+        EMFA_CUDA(c, cudaGetLastError());
+    }
+    return EMFA_OK;
+}
+
+emfa_status_t slice_check(Ctx* c, cudaStream_t st)
+{
+    int* err = nullptr;
+    EMFA_TRY(slice_err(c, &err));
+    int h = 0;
+    EMFA_CUDA(c, cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    EMFA_CUDA(c, cudaStreamSynchronize(st));
+    if (h) {
+        set_error(c, "FP64 tensor-core product: a pipeline wait timed out (stage " + std::to_string(h) + ")");
+        return EMFA_ERR_TIMEOUT;
+    }
+    return EMFA_OK;
+}
+
+emfa_status_t slice_matvec(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                           cudaStream_t st, bool* done)
+{
+    *done = false;
+    if (!slice_worthwhile(c, n, nrhs, false, st)) return EMFA_OK;
+    // the whole sequence of launches at once: another thread's product on this
+    // context's stream uses the same workspaces before or after it
+    std::lock_guard<std::mutex> lk(c->slice_mu);
+    SlicePlanes p;
+    emfa_status_t s = slice_prepare(c, WS_SLICE_MV, Z, ldz, n, &p, st);
+    if (s == EMFA_OK) s = slice_apply(c, WS_SLICE_MV_B, p, X, nrhs, Y, st);
+    if (s == EMFA_ERR_OOM) {
+        cudaGetLastError();  // no room: the caller's CUDA-core product
+        return EMFA_OK;
+    }
+    EMFA_TRY(s);
+    *done = true;
+    return EMFA_OK;
+}
+
+}  // namespace emfa

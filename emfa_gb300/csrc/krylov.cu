@@ -17,6 +17,7 @@
 #include "emfa_internal.cuh"
 #include "emfa_math.cuh"
 #include "gemm.cuh"
+#include "gemm_slice.cuh"
 #include "krylov.cuh"
 #include "lu.cuh"
 
@@ -2149,9 +2150,30 @@ struct DenseOp : LinOp {
     const void* Z = nullptr;
     int mode = SIMT;
     HPlanes hp;  // F16X: planes of Z, split by prepare()
-    emfa_status_t prepare(Ctx* c, cudaStream_t st)
+    bool plain = false;   // FP64 on the CUDA cores asked for (EMFA_MV_F64)
+    bool sliced = false;  // FP64 by digit planes of Z, split by prepare()
+    SlicePlanes sp;
+    // a solve of nrhs right-hand sides
+    emfa_status_t prepare(Ctx* c, int nrhs, cudaStream_t st)
     {
-        return mode == F16X ? hsplit_prepare(c, Z, n, n, &hp, st) : EMFA_OK;
+        if (mode == F16X) return hsplit_prepare(c, Z, n, n, &hp, st);
+        if (prec == EMFA_F64 && !plain && slice_worthwhile(c, n, nrhs, true, st)) {
+            const emfa_status_t s = slice_prepare(c, WS_SLICE_Z, Z, n, n, &sp, st);
+            if (s == EMFA_OK) sliced = true;
+            if (s == EMFA_ERR_OOM) cudaGetLastError();  // no room for the planes: CUDA cores
+            else EMFA_TRY(s);
+        }
+        return EMFA_OK;
+    }
+    emfa_status_t product_f64(Ctx* c, const void* X, void* Y, int nrhs, cudaStream_t st)
+    {
+        if (sliced) {
+            const emfa_status_t s = slice_apply(c, WS_SLICE_B, sp, X, nrhs, Y, st);
+            if (s != EMFA_ERR_OOM) return s;
+            cudaGetLastError();
+            sliced = false;
+        }
+        return cgemm_f64(c, Z, n, X, n, nrhs, Y, st);
     }
     // tensor-core inner products (FP16 significands or TF32) against an
     // FP32/FP64-accurate residual: half the target, and a restart from the
@@ -2160,7 +2182,7 @@ struct DenseOp : LinOp {
     double inner_reduction() const override { return prec == EMFA_F32 && mode != SIMT ? kInnerReduction : 0.0; }
     emfa_status_t apply(Ctx* c, const void* X, void* Y, int nrhs, cudaStream_t st) override
     {
-        if (prec == EMFA_F64) return cgemm_f64(c, Z, n, X, n, nrhs, Y, st);
+        if (prec == EMFA_F64) return product_f64(c, X, Y, nrhs, st);
         if (mode == F16X) return hgemm_apply(c, hp, X, Y, nrhs, st);
         if (mode == TF32) return cgemm_tf32(c, Z, n, X, n, nrhs, Y, st);
         return cgemm_f32(c, Z, n, X, n, nrhs, Y, st);
@@ -2171,7 +2193,7 @@ struct DenseOp : LinOp {
         const size_t vec = (size_t)n * nrhs;
         if (prec == EMFA_F32 && mode == F16X) return hgemm_residual(c, hp, X, B, true, R, nrhs, st);
         if (prec == EMFA_F64) {
-            EMFA_TRY(cgemm_f64(c, Z, n, X, n, nrhs, R, st));  // R = Z X
+            EMFA_TRY(product_f64(c, X, R, nrhs, st));  // R = Z X
             k_residual<double2><<<grid1(vec), 256, 0, st>>>((const double2*)B, R, R, vec);
             c->kernel_launches += 1;
             return EMFA_OK;
@@ -2203,6 +2225,7 @@ struct DenseOp : LinOp {
     emfa_status_t check(Ctx* c, cudaStream_t st) override
     {
         if (mode == F16X) return hgemm_check_error(c, st);
+        if (sp.d) return slice_check(c, st);
         return mode == TF32 ? gemm_check_error(c, st) : EMFA_OK;
     }
 };
@@ -2322,7 +2345,8 @@ emfa_status_t solve_dense(Ctx* c, int prec, const void* Z, int n, const void* B,
     A.prec = prec;
     A.Z = Z;
     A.mode = dense_mode(prec, sp->matvec, Z, n);
-    EMFA_TRY(A.prepare(c, st));
+    A.plain = sp->matvec == EMFA_MV_F64;
+    EMFA_TRY(A.prepare(c, nrhs, st));
     if (sp->method == EMFA_LU) return lu_refined(c, A, Z, B, nrhs, (double2*)X, sp, info, st);
     return solve_op(c, A, B, nrhs, X, sp, info, st);
 }
@@ -2356,7 +2380,11 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
     }
     EMFA_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    if (prec == EMFA_F64) return cgemm_f64(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    if (prec == EMFA_F64) {
+        bool done = false;
+        if (matvec != EMFA_MV_F64) EMFA_TRY(slice_matvec(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
+        return done ? EMFA_OK : cgemm_f64(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    }
     if (prec != EMFA_F32) {
         set_error(ctx, "emfa_matvec: precision");
         return EMFA_ERR_INVALID;
@@ -2389,7 +2417,9 @@ emfa_status_t emfa_residual(emfa_ctx_t* ctx, int prec, int matvec, const void* Z
     A.prec = prec;
     A.Z = Z_dev;
     A.mode = dense_mode(prec, matvec, Z_dev, n);
-    EMFA_TRY(A.prepare(ctx, st));
+    // one product: planes of their own do not pay unless the block is wide
+    A.plain = matvec == EMFA_MV_F64 || !slice_worthwhile(ctx, n, n_rhs, false, st);
+    EMFA_TRY(A.prepare(ctx, n_rhs, st));
     DevBuf xt;
     if (A.mode != DenseOp::F16X) EMFA_TRY(xt.alloc(ctx, sizeof(float2) * (size_t)n * n_rhs));
     EMFA_TRY(A.residual(ctx, (const double2*)X_dev, B_dev, (double2*)R_dev, n_rhs, dptr<float2>(xt), st));

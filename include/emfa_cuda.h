@@ -47,8 +47,11 @@ typedef enum { EMFA_EFIE = 0, EMFA_CFIE = 1 } emfa_kind_t;
  * (EMSolver/EFIE.cpp:89 has a commented-out Eigen LU). */
 typedef enum { EMFA_GMRES = 0, EMFA_BICGSTAB = 1, EMFA_LU = 2 } emfa_method_t;
 typedef enum {
-    EMFA_MV_AUTO = 0,  /* F64: FP64 SIMT; F32: EMFA_MV_F16X                          */
-    EMFA_MV_F64 = 1,   /* FP64 complex GEMM on CUDA cores (plain path)               */
+    EMFA_MV_AUTO = 0,  /* F64: FP64 accuracy on the tensor cores for blocks of right- */
+                       /* hand sides (operands as 8-bit digit planes, exact sums; an */
+                       /* error no larger than an FP64 sum's relative to the row and */
+                       /* vector maxima), else FP64 SIMT; F32: EMFA_MV_F16X          */
+    EMFA_MV_F64 = 1,   /* FP64 complex product on CUDA cores (plain path)            */
     EMFA_MV_F32 = 2,   /* FP32 complex GEMM on CUDA cores; residual FP32 products    */
                        /* with FP64 chunk sums                                       */
     EMFA_MV_TF32 = 3,  /* tcgen05 TF32 complex GEMM, FP32 accumulation; residual as  */
