@@ -18,9 +18,12 @@
 //     k_agg_finest    finest-level aggregation
 //     k_upward        interpolation + shift, child -> parent: the 3 x 3 Lagrange stencil as two
 //                     1-D passes (theta into shared memory, then phi)
-//     k_downward      translation from far boxes + anterpolation from the parent (transposed
-//                     stencil as two 1-D passes), by chunks of phi rows
-//     k_disagg_near   disaggregation at the finest level fused with the near-field product
+//     k_translate     translation of every level at once, by sibling groups: each source pattern read
+//                     once for the up to eight boxes of a parent
+//     k_downward      anterpolation from the parent (transposed stencil as two 1-D passes), by chunks
+//                     of phi rows, added to the translated pattern
+//     k_finish        the finest level: anterpolation, disaggregation and near-field product (or
+//                     k_downward and k_disagg_near, for boxes too large for shared memory)
 #include "emfa_internal.cuh"
 #include "emfa_math.cuh"
 #include "fill_entry.cuh"
@@ -64,7 +67,7 @@ struct Box {
     int oct = 0;      // child index (x*2+y)*2+z within the parent
     int offset = 0;   // first unknown (box order)
     std::vector<int> unk;
-    std::vector<int> child, near, far;
+    std::vector<int> child, near;
 };
 
 // Legendre value / derivative recurrence of GaussLegendre::Evaluation
@@ -148,7 +151,11 @@ struct MLevel {
     float len = 0;
     DevBuf parent, oct;                 // parent index and octant per box (int)
     DevBuf child_ptr, child_idx;        // CSR children (int)
-    DevBuf far_ptr, far;                // CSR far lists: int2 {source box, offset index}
+    // translation by sibling groups: the children of one box of the level
+    // above, at most four a group (TransGroup), and their source boxes, the
+    // children of the boxes near the parent
+    DevBuf grp, grp_src;
+    int ngrp = 0;
     DevBuf trans;                       // float2 [343][K]
     DevBuf up, down;                    // planar float2 [right-hand side][nbox][3][K]
     // interpolation to this level from the level below, separable: 3-point
@@ -184,7 +191,7 @@ struct emfa_mlfma {
     int rcap = 1;                  // right-hand sides the level patterns hold (one apply chunk)
     emfa::DevBuf perm_d, box_of;   // int [n]
     emfa::DevBuf rad, rec;         // C2f [n][Kf]: theta, phi components in each sample's basis
-    emfa::DevBuf tp;               // float [Kf][6]: theta_hat, phi_hat of the finest samples
+    emfa::DevBuf tp;               // float [6][Kf]: theta_hat, phi_hat of the finest samples
     emfa::DevBuf coeff;            // float [Kf]
     emfa::DevBuf box_off, box_cnt; // finest boxes: first unknown, count
     emfa::DevBuf near_ptr, near_box, near_col, row_cols;  // CSR near lists, column base per slot, C_b per box
@@ -192,6 +199,9 @@ struct emfa_mlfma {
     emfa::DevBuf near_val;         // float2 [nnz]
     emfa::DevBuf near_cbase, near_cidx;  // per finest box: first entry, column unknowns of its near rows
     size_t nnz = 0;
+    emfa::DevBuf trans_work;       // TransWork per CTA of the translation
+    int trans_ctas = 0;
+    int max_cols = 0;              // near columns of a box, most
     emfa::DevBuf tmp_in, tmp_out;  // complex64 scratch for residuals
     // SAI preconditioner P (CSR over box-order rows), built when p.precond
     bool precond = false;
@@ -255,7 +265,8 @@ __global__ void k_radrec(const RwgPack<float>* __restrict__ rw, const int* __res
     float2 hz = make_float2(kh.x * rh[1].x - kh.y * rh[0].x, kh.x * rh[1].y - kh.y * rh[0].y);
     const float h = R.len / 2;
     const float b = 1.0f - alpha;
-    const float* e = tp + 6 * kk;  // theta_hat, phi_hat
+    const float e[6] = {tp[kk],         tp[K + kk],     tp[2 * K + kk],
+                        tp[3 * K + kk], tp[4 * K + kk], tp[5 * K + kk]};  // theta_hat, phi_hat
     C3f o, q;
     o.x = cscalef(ra[0], h);
     o.y = cscalef(ra[1], h);
@@ -311,6 +322,8 @@ __global__ void k_agg_finest(const float2* __restrict__ x, int n, int nr, const 
 {
     const int b = blockIdx.x;
     const int o = box_off[b], cnt = box_cnt[b];
+    x += (size_t)blockIdx.y * n;  // RB = 1: a right-hand side a grid row
+    out += blockIdx.y * ostride;
     for (int kk = threadIdx.x; kk < K; kk += blockDim.x) {
         float2 at[RB], ap[RB];
 #pragma unroll
@@ -325,7 +338,7 @@ __global__ void k_agg_finest(const float2* __restrict__ x, int n, int nr, const 
                     ap[r] = caddf(ap[r], cmulf(xv, rv.p));
                 }
         }
-        const float* e = tp + 6 * kk;
+        const float e[6] = {tp[kk], tp[K + kk], tp[2 * K + kk], tp[3 * K + kk], tp[4 * K + kk], tp[5 * K + kk]};
 #pragma unroll
         for (int r = 0; r < RB; ++r)
             if (RB == 1 || r < nr) {
@@ -417,105 +430,329 @@ __global__ void k_upward(const float2* __restrict__ child, int Lc, const int* __
     }
 }
 
-// translation from far boxes + anterpolation from the parent: CTA per (box,
-// chunk of phi rows [pc0, pc0 + R)), i.e. the contiguous samples
-// [pc0 L, (pc0 + R) L) of the box (samples k = pc L + tc, phi-major).
-//   1. theta pass (boxes below the top level): for the parent phi rows
-//      pp in [win.x, win.y) that the chunk's phi stencils read, and every theta
-//      column tc: h[comp][pp - win.x][tc] = sum over the transposed theta
-//      stencil of w * conj(phase_oct(pp, t)) * parent(pp, t), into shared memory;
-//   2. per pair of samples (16-byte loads of the planar patterns and of the
-//      translation table): the far boxes' translated patterns in far-list
-//      order, then the transposed phi stencil over h.
-__device__ __forceinline__ void cfma2(float4& acc, float4 t, float4 v)
+// Translation, all levels in one launch: down(b) = sum over far boxes f of
+// T[offset(b, f)] up(f), sample by sample.  The far boxes of the siblings under
+// one parent are nearly the same: all are children of the boxes near the
+// parent, and the operator depends on the offset alone.  A warp takes up to
+// four siblings and 32 samples (a lane each) and reads each source pattern once
+// for all of them, the siblings' sums in registers; near offsets have T = 0 in
+// the table, so the siblings need no lists of their own.  The table of the
+// CTA's 32 samples (343 offsets, 88 KB) is staged in shared memory, and a
+// child's octant shifts its offset by a constant.  Four patterns are in flight
+// at a time (lists are padded to fours with an offset that is near for every
+// octant); warps take groups from a counter.
+// Per (source, sibling): one 8-byte shared load and 12 FMA, against an 8-byte
+// table and a 24-byte pattern load through L1 when a thread took one box's far
+// list (5-wavelength sphere, 122,880 unknowns: 518 us for the five levels with
+// the anterpolation, the L1 data path 80 % busy).  Now 290 us,
+// and 107 for the anterpolation above the finest level; still bound by L1
+// wavefronts (71 %), half of them the siblings' table values.  Eight siblings a
+// warp, or two patterns in flight, were no faster (spills; latency).
+constexpr int TRANS_LEVELS = 24;  // octree levels a launch takes
+constexpr int TRANS_WARPS = 12, TRANS_K = 32, TRANS_OFF = 343, TRANS_NC = 4, TRANS_BATCH = 4;
+constexpr size_t TRANS_SMEM = sizeof(float2) * TRANS_OFF * TRANS_K;
+struct TransGroup {
+    int s0, s1, nc, pad;      // sources [s0, s1), multiples of TRANS_BATCH; siblings
+    int2 child[TRANS_NC];     // box, its octant's shift in table rows x 32
+};
+struct TransWork {  // one CTA: a level's groups [g0, g1), samples [k0, k0 + 32)
+    int level, k0, g0, g1;
+};
+struct TransLevel {
+    const float2* up;
+    float2* down;
+    const float2* trans;
+    const int4* src;          // per two sources: first element of the pattern, row x 32 of its offset
+    const TransGroup* grp;
+    int K;
+    size_t stride;            // complex64 from one right-hand side to the next
+};
+struct TransLevels {
+    TransLevel l[TRANS_LEVELS];
+};
+
+template <int NC>
+__device__ __forceinline__ void translate_group(const TransGroup& G, const int4* __restrict__ src,
+                                                const float2* __restrict__ tab, const float2* __restrict__ u, int K,
+                                                int k, bool store, float2* __restrict__ down)
 {
-    acc.x += t.x * v.x - t.y * v.y;
-    acc.y += t.x * v.y + t.y * v.x;
-    acc.z += t.z * v.z - t.w * v.w;
-    acc.w += t.z * v.w + t.w * v.z;
+    C3f acc[NC];
+    const float2* t0[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        acc[c] = c3zero();
+        t0[c] = tab + G.child[c].y;
+    }
+    const float2 *u1 = u + K, *u2 = u1 + K;
+    const int s1 = G.s1;
+#pragma unroll 1
+    for (int s = G.s0; s < s1; s += TRANS_BATCH) {
+        unsigned at[TRANS_BATCH];
+        int row[TRANS_BATCH];
+#pragma unroll
+        for (int j = 0; j < TRANS_BATCH; j += 2) {
+            const int4 e = src[(s + j) >> 1];
+            at[j] = (unsigned)e.x;
+            row[j] = e.y;
+            at[j + 1] = (unsigned)e.z;
+            row[j + 1] = e.w;
+        }
+        C3f v[TRANS_BATCH];
+#pragma unroll
+        for (int j = 0; j < TRANS_BATCH; ++j) v[j] = C3f{u[at[j]], u1[at[j]], u2[at[j]]};
+#pragma unroll
+        for (int j = 0; j < TRANS_BATCH; ++j) {
+            const C3f w = v[j];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float2 t = t0[c][row[j]];
+                acc[c].x.x = fmaf(t.x, w.x.x, fmaf(-t.y, w.x.y, acc[c].x.x));
+                acc[c].x.y = fmaf(t.x, w.x.y, fmaf(t.y, w.x.x, acc[c].x.y));
+                acc[c].y.x = fmaf(t.x, w.y.x, fmaf(-t.y, w.y.y, acc[c].y.x));
+                acc[c].y.y = fmaf(t.x, w.y.y, fmaf(t.y, w.y.x, acc[c].y.y));
+                acc[c].z.x = fmaf(t.x, w.z.x, fmaf(-t.y, w.z.y, acc[c].z.x));
+                acc[c].z.y = fmaf(t.x, w.z.y, fmaf(t.y, w.z.x, acc[c].z.y));
+            }
+        }
+    }
+    if (store) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            float2* o = down + (size_t)3 * G.child[c].x * K + k;
+            o[0] = acc[c].x;
+            o[K] = acc[c].y;
+            o[2 * K] = acc[c].z;
+        }
+    }
 }
 
-__global__ void k_downward(const float4* __restrict__ up, const int* __restrict__ far_ptr,
-                           const int2* __restrict__ far, const float4* __restrict__ trans, int L, int R,
-                           const float2* __restrict__ pdown, int Lp, const int2* __restrict__ win,
+__global__ void __launch_bounds__(32 * TRANS_WARPS, 2) k_translate(const __grid_constant__ TransLevels lv,
+                                                                   const TransWork* __restrict__ work, int nr)
+{
+    extern __shared__ float2 s_tab[];  // [offset][32 samples]
+    __shared__ int s_next;
+    const TransWork w = work[blockIdx.x];
+    const TransLevel& L = lv.l[w.level];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = min(w.k0 + lane, L.K - 1);  // the last chunk's spare lanes repeat the last sample
+    if (threadIdx.x == 0) s_next = 0;
+    for (int o = warp; o < TRANS_OFF; o += TRANS_WARPS) s_tab[o * TRANS_K + lane] = L.trans[(size_t)o * L.K + k];
+    __syncthreads();
+    const int n = (w.g1 - w.g0) * nr;
+    const bool store = w.k0 + lane < L.K;
+    const float2* tab = s_tab + lane;
+    for (;;) {
+        int i = lane == 0 ? atomicAdd(&s_next, 1) : 0;
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= n) break;
+        const int r = nr == 1 ? 0 : i % nr;
+        const TransGroup& G = L.grp[w.g0 + (nr == 1 ? i : i / nr)];
+        const float2* u = L.up + r * L.stride + k;
+        float2* down = L.down + r * L.stride;
+        switch (G.nc) {
+        case 1: translate_group<1>(G, L.src, tab, u, L.K, k, store, down); break;
+        case 2: translate_group<2>(G, L.src, tab, u, L.K, k, store, down); break;
+        case 3: translate_group<3>(G, L.src, tab, u, L.K, k, store, down); break;
+        default: translate_group<4>(G, L.src, tab, u, L.K, k, store, down); break;
+        }
+    }
+}
+
+// Anterpolation from a parent pattern, theta pass: for the parent phi rows
+// [w2.x, w2.y) and every theta column tc of the child
+//   h[comp][pp - w2.x][tc] = sum over the transposed theta stencil of
+//                            w * conj(phase(pp, t)) * parent(pp, t)
+// into shared memory.  The parent's samples are shifted first (each serves
+// about three columns), into s_q, then summed.
+__device__ __forceinline__ void anterp_theta(const float2* __restrict__ src, const float2* __restrict__ ph, int2 w2,
+                                             int L, int Lp, const int* __restrict__ th_ptr,
+                                             const int* __restrict__ th_src, const float* __restrict__ th_w,
+                                             float2* s_q, float2* s_h)
+{
+    const int Kp = 2 * Lp * Lp, base = w2.x * Lp, qsz = (w2.y - w2.x) * Lp, hsz = (w2.y - w2.x) * L;
+    for (int i = threadIdx.x; i < qsz; i += blockDim.x) {
+        const float2 p = ph[base + i], c = make_float2(p.x, -p.y);  // exp(+j k k.(parent - child))
+        s_q[i] = cmulf(c, src[base + i]);
+        s_q[qsz + i] = cmulf(c, src[Kp + base + i]);
+        s_q[2 * qsz + i] = cmulf(c, src[2 * Kp + base + i]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < hsz; i += blockDim.x) {
+        const int r = i / L, tc = i - r * L;
+        const float2* q = s_q + r * Lp;
+        float2 sx = make_float2(0, 0), sy = sx, sz = sx;
+        for (int a = th_ptr[tc]; a < th_ptr[tc + 1]; ++a) {
+            const int t = th_src[a];
+            const float w = th_w[a];
+            sx = caddf(sx, cscalef(q[t], w));
+            sy = caddf(sy, cscalef(q[qsz + t], w));
+            sz = caddf(sz, cscalef(q[2 * qsz + t], w));
+        }
+        s_h[i] = sx;
+        s_h[hsz + i] = sy;
+        s_h[2 * hsz + i] = sz;
+    }
+    __syncthreads();
+}
+
+// phi pass: the transposed phi stencil of child sample k = pc L + tc over h
+__device__ __forceinline__ void anterp_phi(int pc, int tc, int w0, int L, int hsz, const int* __restrict__ ph_ptr,
+                                           const int* __restrict__ ph_src, const float* __restrict__ ph_w,
+                                           const float2* s_h, float2& sx, float2& sy, float2& sz)
+{
+    for (int a = ph_ptr[pc]; a < ph_ptr[pc + 1]; ++a) {
+        const int r = (ph_src[a] - w0) * L + tc;
+        const float w = ph_w[a];
+        sx = caddf(sx, cscalef(s_h[r], w));
+        sy = caddf(sy, cscalef(s_h[hsz + r], w));
+        sz = caddf(sz, cscalef(s_h[2 * hsz + r], w));
+    }
+}
+
+// a level's anterpolation, added to its translated pattern: CTA per (box, chunk
+// of phi rows [pc0, pc0 + R)), i.e. the contiguous samples [pc0 L, (pc0 + R) L)
+// of the box (samples k = pc L + tc, phi-major)
+__global__ void k_downward(int L, int R, const float2* __restrict__ pdown, int Lp, const int2* __restrict__ win,
                            const int* __restrict__ parent, const int* __restrict__ oct,
                            const float2* __restrict__ pphase, const int* __restrict__ th_ptr,
                            const int* __restrict__ th_src, const float* __restrict__ th_w,
                            const int* __restrict__ ph_ptr, const int* __restrict__ ph_src,
-                           const float* __restrict__ ph_w, float4* __restrict__ out, size_t ustride, size_t pstride)
+                           const float* __restrict__ ph_w, float2* __restrict__ out, size_t ustride, size_t pstride)
 {
-    extern __shared__ float2 s_h[];  // [3][rows of the window][L]
+    extern __shared__ float2 s_h[];  // [3][rows of the window][L], then the shifted rows [3][rows][Lp]
     // right-hand side blockIdx.z: strides in complex64 (this level, parent level)
-    up += blockIdx.z * (ustride / 2);
-    out += blockIdx.z * (ustride / 2);
-    if (pdown) pdown += blockIdx.z * pstride;
+    out += blockIdx.z * ustride;
+    pdown += blockIdx.z * pstride;
     const int b = blockIdx.x;
-    const int K = 2 * L * L, K2 = K >> 1;
+    const int K = 2 * L * L;
     const int pc0 = blockIdx.y * R;
-    const int npair = (min(R, 2 * L - pc0) * L) >> 1;
-    int2 w2 = make_int2(0, 0);
-    int hsz = 0;
-    if (pdown) {
-        w2 = win[blockIdx.y];
-        hsz = (w2.y - w2.x) * L;
-        const int Kp = 2 * Lp * Lp;
-        const float2* src = pdown + (size_t)3 * parent[b] * Kp;
-        const float2* ph0 = pphase + (size_t)oct[b] * Kp;
-        for (int i = threadIdx.x; i < hsz; i += blockDim.x) {
-            const int r = i / L, tc = i - r * L;
-            const int base = (w2.x + r) * Lp;
-            float2 sx = make_float2(0, 0), sy = sx, sz = sx;
-            for (int a = th_ptr[tc]; a < th_ptr[tc + 1]; ++a) {
-                const int kp = base + th_src[a];
-                const float w = th_w[a];
-                float2 ph = ph0[kp];
-                ph = make_float2(ph.x * w, -ph.y * w);  // conj: exp(+j k k.(parent - child))
-                sx = caddf(sx, cmulf(ph, src[kp]));
-                sy = caddf(sy, cmulf(ph, src[Kp + kp]));
-                sz = caddf(sz, cmulf(ph, src[2 * Kp + kp]));
-            }
-            s_h[i] = sx;
-            s_h[hsz + i] = sy;
-            s_h[2 * hsz + i] = sz;
-        }
-        __syncthreads();
+    const int ns = min(R, 2 * L - pc0) * L;
+    const int2 w2 = win[blockIdx.y];
+    const int hsz = (w2.y - w2.x) * L;
+    const int Kp = 2 * Lp * Lp;
+    anterp_theta(pdown + (size_t)3 * parent[b] * Kp, pphase + (size_t)oct[b] * Kp, w2, L, Lp, th_ptr, th_src, th_w,
+                 s_h + 3 * hsz, s_h);
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+        const int k = pc0 * L + i;
+        const int pc = k / L, tc = k - pc * L;
+        float2* ob = out + (size_t)3 * b * K + k;
+        float2 sx = ob[0], sy = ob[K], sz = ob[2 * K];
+        anterp_phi(pc, tc, w2.x, L, hsz, ph_ptr, ph_src, ph_w, s_h, sx, sy, sz);
+        ob[0] = sx;
+        ob[K] = sy;
+        ob[2 * K] = sz;
     }
-    const int f0 = far_ptr[b], f1 = far_ptr[b + 1];
-    for (int i = threadIdx.x; i < npair; i += blockDim.x) {
-        const int q = ((pc0 * L) >> 1) + i;  // pair index: samples 2q, 2q + 1
-        float4 ax = make_float4(0, 0, 0, 0), ay = ax, az = ax;
-        for (int f = f0; f < f1; ++f) {
-            const int2 e = far[f];
-            const float4 t = trans[(size_t)e.y * K2 + q];
-            const float4* sp = up + (size_t)3 * e.x * K2 + q;
-            cfma2(ax, t, sp[0]);
-            cfma2(ay, t, sp[K2]);
-            cfma2(az, t, sp[2 * K2]);
-        }
-        if (pdown) {
+}
+
+// The finest level's anterpolation, the disaggregation and the near field in
+// one pass, CTA per finest box, up to RB right-hand sides (nr of them):
+//   1. per right-hand side, the box's down pattern: translated part plus
+//      anterpolation, projected on theta_hat and phi_hat of each sample, times
+//      its quadrature coefficient, into shared memory; the x of the box's near
+//      columns beside it;
+//   2. a warp per unknown: receive pattern times down pattern, then the near row.
+// As two kernels (the anterpolation writing x, y, z patterns that each unknown
+// read and projected again, and gathered its near x itself) this took 252 us on
+// 122,880 unknowns, latency-bound; now 189.
+struct FinishArgs {
+    const float2* x;
+    int n, nr;
+    const C2f* rec;
+    const float* tp;
+    const float2* down;
+    size_t dstride;
+    const float* coeff;
+    int L, Lp;
+    const float2* pdown;  // parent level's patterns; null: the finest level is the top one
+    size_t pstride;
+    const int *parent, *oct;
+    const float2* pphase;
+    const int *th_ptr, *th_src;
+    const float* th_w;
+    const int *ph_ptr, *ph_src;
+    const float* ph_w;
+    const int *box_off, *box_cnt, *row_cols;
+    const size_t* row_base;
+    const int *near_cbase, *near_cidx;
+    const float2* val;
+    int parts;  // 0 near + far, 1 near, 2 far
+    float2* y;
+};
+constexpr int FINISH_WARPS = 4;
+
+template <int RB>
+__global__ void __launch_bounds__(32 * FINISH_WARPS) k_finish(const __grid_constant__ FinishArgs A)
+{
+    extern __shared__ float2 s_h[];  // [3][2 Lp][L], [3][2 Lp][Lp], down [RB][2][K], x [RB][near columns]
+    const int b = blockIdx.x, L = A.L, K = 2 * L * L, Lp = A.Lp, n = A.n;
+    const int r0 = blockIdx.y, nr = RB == 1 ? 1 : A.nr;  // RB = 1: a right-hand side a grid row
+    const float2* x = A.x + (size_t)r0 * n;
+    float2* y = A.y + (size_t)r0 * n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int hsz = A.pdown ? 2 * Lp * L : 0, qsz = A.pdown ? 2 * Lp * Lp : 0;
+    float2* s_q = s_h + 3 * hsz;
+    float2* s_d = s_q + 3 * qsz;
+    float2* s_x = s_d + (size_t)RB * 2 * K;
+    const int o = A.box_off[b], cnt = A.box_cnt[b], rc = A.parts == 2 ? 0 : A.row_cols[b];
+    const int* ci = A.near_cidx + A.near_cbase[b];
+    for (int j = threadIdx.x; j < rc; j += blockDim.x) {
+        const int cj = ci[j];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int kk = 2 * q + h;
-                const int pc = kk / L, tc = kk - pc * L;
-                float2 sx = make_float2(0, 0), sy = sx, sz = sx;
-                for (int a = ph_ptr[pc]; a < ph_ptr[pc + 1]; ++a) {
-                    const int r = (ph_src[a] - w2.x) * L + tc;
-                    const float w = ph_w[a];
-                    sx = caddf(sx, cscalef(s_h[r], w));
-                    sy = caddf(sy, cscalef(s_h[hsz + r], w));
-                    sz = caddf(sz, cscalef(s_h[2 * hsz + r], w));
+        for (int r = 0; r < RB; ++r)
+            if (RB == 1 || r < nr) s_x[r * rc + j] = x[(size_t)r * n + cj];
+    }
+    if (A.parts != 1)
+        for (int r = 0; r < nr; ++r) {
+            if (A.pdown)
+                anterp_theta(A.pdown + (r0 + r) * A.pstride + (size_t)3 * A.parent[b] * qsz, A.pphase + (size_t)A.oct[b] * qsz,
+                             make_int2(0, 2 * Lp), L, Lp, A.th_ptr, A.th_src, A.th_w, s_q, s_h);
+            const float2* d = A.down + (r0 + r) * A.dstride + (size_t)3 * b * K;
+            for (int k = threadIdx.x; k < K; k += blockDim.x) {
+                float2 sx = d[k], sy = d[K + k], sz = d[2 * K + k];
+                if (A.pdown) {
+                    const int pc = k / L;
+                    anterp_phi(pc, k - pc * L, 0, L, hsz, A.ph_ptr, A.ph_src, A.ph_w, s_h, sx, sy, sz);
                 }
-                if (h == 0) {
-                    ax.x += sx.x; ax.y += sx.y; ay.x += sy.x; ay.y += sy.y; az.x += sz.x; az.y += sz.y;
-                } else {
-                    ax.z += sx.x; ax.w += sx.y; ay.z += sy.x; ay.w += sy.y; az.z += sz.x; az.w += sz.y;
-                }
+                const float e[6] = {A.tp[k],         A.tp[K + k],     A.tp[2 * K + k],
+                                    A.tp[3 * K + k], A.tp[4 * K + k], A.tp[5 * K + k]};
+                const float cf = A.coeff[k];
+                s_d[(2 * r) * K + k] = cscalef(caddf(caddf(cscalef(sx, e[0]), cscalef(sy, e[1])), cscalef(sz, e[2])), cf);
+                s_d[(2 * r + 1) * K + k] = cscalef(caddf(caddf(cscalef(sx, e[3]), cscalef(sy, e[4])), cscalef(sz, e[5])), cf);
             }
         }
-        float4* ob = out + (size_t)3 * b * K2 + q;
-        ob[0] = ax;
-        ob[K2] = ay;
-        ob[2 * K2] = az;
+    __syncthreads();
+    const int kf = A.parts == 1 ? 0 : K;
+    for (int u = warp; u < cnt; u += FINISH_WARPS) {
+        float2 acc[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) acc[r] = make_float2(0, 0);
+        const C2f* rr = A.rec + (size_t)(o + u) * K;
+#pragma unroll 4
+        for (int k = lane; k < kf; k += 32) {
+            const C2f rv = rr[k];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+                if (RB == 1 || r < nr)
+                    acc[r] = caddf(acc[r], caddf(cmulf(rv.t, s_d[(2 * r) * K + k]), cmulf(rv.p, s_d[(2 * r + 1) * K + k])));
+        }
+        const float2* vrow = A.val + A.row_base[b] + (size_t)u * A.row_cols[b];
+#pragma unroll 4
+        for (int j = lane; j < rc; j += 32) {
+            const float2 v = vrow[j];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+                if (RB == 1 || r < nr) acc[r] = caddf(acc[r], cmulf(v, s_x[r * rc + j]));
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (RB > 1 && r >= nr) break;
+#pragma unroll
+            for (int q = 16; q > 0; q >>= 1) {
+                acc[r].x += __shfl_xor_sync(0xffffffffu, acc[r].x, q);
+                acc[r].y += __shfl_xor_sync(0xffffffffu, acc[r].y, q);
+            }
+            if (lane == 0) y[(size_t)r * n + o + u] = acc[r];
+        }
     }
 }
 
@@ -535,6 +772,9 @@ __global__ void k_disagg_near(const float2* __restrict__ x, int nr, const C2f* _
 {
     const int warp = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (warp >= n) return;
+    x += (size_t)blockIdx.y * n;  // RB = 1: a right-hand side a grid row
+    y += (size_t)blockIdx.y * n;
+    down += blockIdx.y * dstride;
     const int u = warp, b = box_of[u];
     float2 acc[RB];
 #pragma unroll
@@ -545,7 +785,7 @@ __global__ void k_disagg_near(const float2* __restrict__ x, int nr, const C2f* _
     for (int kk = lane; kk < K; kk += 32) {
         const C2f rv = rr[kk];
         const float cf = coeff[kk];
-        const float* e = tp + 6 * kk;
+        const float e[6] = {tp[kk], tp[K + kk], tp[2 * K + kk], tp[3 * K + kk], tp[4 * K + kk], tp[5 * K + kk]};
 #pragma unroll
         for (int r = 0; r < RB; ++r)
             if (RB == 1 || r < nr) {
@@ -942,7 +1182,7 @@ static bool build_plan(const std::vector<double>& verts, int nv, const std::vect
             for (int pn : lb[l - 1][b.parent].near)
                 for (int cidx : lb[l - 1][pn].child) {
                     float dist = mh::fnorm3(lb[l][cidx].c, b.c);
-                    (dist < lim ? b.near : b.far).push_back(cidx);
+                    if (dist < lim) b.near.push_back(cidx);
                 }
         }
     }
@@ -1138,6 +1378,10 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     std::vector<int>& cnt_h = P.cnt;
     std::vector<float>& cen_h = P.cen;
     const int nl = L - 1;
+    if (nl > TRANS_LEVELS) {
+        set_error(c, "mlfma: more than " + std::to_string(TRANS_LEVELS + 1) + " octree levels (box threshold too small)");
+        return EMFA_ERR_UNSUPPORTED;
+    }
     M->lv.clear();
     M->lv.resize(nl);
     for (int l = 2; l <= L; ++l) {
@@ -1151,25 +1395,53 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     // the interpolation and anterpolation passes may use more than the default 48 KB of shared memory
     EMFA_TRY(ensure_smem(c, k_upward, 96 * 1024));
     EMFA_TRY(ensure_smem(c, k_downward, 200 * 1024));
+    EMFA_TRY(ensure_smem(c, k_translate, TRANS_SMEM));
     // per-level device tables
     for (int l = 2; l <= L; ++l) {
         const int i = l - 2;
         MLevel& ml = M->lv[i];
         const int K = ml.K;
-        std::vector<int> par, oc, cptr{0}, cidx, fptr{0}, fbox, foff;
+        std::vector<int> par, oc, cptr{0}, cidx;
         for (auto& b : lb[l]) {
             par.push_back(b.parent);
             oc.push_back(b.oct);
-            for (int f : b.far) {
-                const float* a = b.c;
-                const float* o = lb[l][f].c;
-                int dx = (int)std::lround((a[0] - o[0]) / ml.len), dy = (int)std::lround((a[1] - o[1]) / ml.len),
-                    dz = (int)std::lround((a[2] - o[2]) / ml.len);
-                fbox.push_back(f);
-                foff.push_back(((dx + 3) * 7 + (dy + 3)) * 7 + (dz + 3));
-            }
-            fptr.push_back((int)fbox.size());
         }
+        // sibling groups: the far boxes of a box are the children of the boxes
+        // near its parent that are not near itself (setBoxParameter), in that order
+        std::vector<TransGroup> grp;
+        std::vector<int2> gsrc;
+        if ((size_t)3 * ml.nbox * K > 0xffffffffull) {
+            set_error(c, "mlfma: level patterns exceed 2^32 values");
+            return EMFA_ERR_UNSUPPORTED;
+        }
+        for (auto& pb : lb[l - 1]) {
+            float o[3];  // centre of the parent's first octant
+            for (int d = 0; d < 3; ++d) o[d] = pb.c[d] - 0.5f * ml.len;
+            const int s0 = (int)gsrc.size();
+            const int self = (int)(&pb - lb[l - 1].data());
+            for (int pn : pb.near)
+                for (int f : lb[l - 1][pn].child) {
+                    if (pn == self) break;  // the siblings are near one another
+                    const float* a = lb[l][f].c;
+                    int off = 0;
+                    for (int d = 0; d < 3; ++d) off = 7 * off + (int)std::lround((o[d] - a[d]) / ml.len) + 3;
+                    gsrc.push_back(make_int2((int)(unsigned)((size_t)3 * f * K), off * TRANS_K));
+                }
+            // the offset (0, 0, 0) is near for every octant: T = 0
+            while (gsrc.size() % TRANS_BATCH) gsrc.push_back(make_int2(gsrc.back().x, 171 * TRANS_K));  // gsrc.size() > s0 here
+            const int nc = (int)pb.child.size(), parts = (nc + TRANS_NC - 1) / TRANS_NC;
+            for (int q = 0; q < parts; ++q) {
+                TransGroup g{};
+                g.s0 = s0;
+                g.s1 = (int)gsrc.size();
+                for (int j = nc * q / parts; j < nc * (q + 1) / parts; ++j) {
+                    const int oct = lb[l][pb.child[j]].oct;
+                    g.child[g.nc++] = make_int2(pb.child[j], (49 * (oct >> 2) + 7 * ((oct >> 1) & 1) + (oct & 1)) * TRANS_K);
+                }
+                grp.push_back(g);
+            }
+        }
+        ml.ngrp = (int)grp.size();
         if (l < L)
             for (auto& b : lb[l]) {
                 for (int ch : b.child) cidx.push_back(ch);
@@ -1177,12 +1449,8 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
             }
         EMFA_TRY(upload(c, ml.parent, par, st));
         EMFA_TRY(upload(c, ml.oct, oc, st));
-        {
-            std::vector<int2> fe(fbox.size());
-            for (size_t f = 0; f < fbox.size(); ++f) fe[f] = make_int2(fbox[f], foff[f]);
-            EMFA_TRY(upload(c, ml.far_ptr, fptr, st));
-            EMFA_TRY(upload(c, ml.far, fe, st));
-        }
+        EMFA_TRY(upload(c, ml.grp_src, gsrc, st));
+        EMFA_TRY(upload(c, ml.grp, grp, st));
         EMFA_TRY(upload(c, ml.child_ptr, cptr, st));
         EMFA_TRY(upload(c, ml.child_idx, cidx, st));
         // translation operators per offset: sum_l (2l+1)(-j)^l h_l^(2)(kD) P_l(k.D/|D|),
@@ -1226,6 +1494,26 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         }
         EMFA_TRY(ml.up.alloc(c, sizeof(float2) * 3 * (size_t)ml.nbox * K));
         EMFA_TRY(ml.down.alloc(c, sizeof(float2) * 3 * (size_t)ml.nbox * K));
+    }
+    // translation work: up to 24 groups a CTA (two a warp and right-hand side, so
+    // that the table's staging is a few percent), fewer where that leaves SMs idle
+    {
+        std::vector<TransWork> tw;
+        size_t tasks = 0;
+        for (const MLevel& ml : M->lv) tasks += (size_t)ml.ngrp * ((ml.K + TRANS_K - 1) / TRANS_K);
+        const size_t sms = c->sm_count > 0 ? c->sm_count : 148;
+        const int per = (int)std::min<size_t>(24, std::max<size_t>(6, tasks / (8 * sms)));
+        for (int i = nl - 1; i >= 0; --i) {
+            const MLevel& ml = M->lv[i];
+            const int parts = std::max(1, (ml.ngrp + per / 2) / per);
+            for (int k0 = 0; k0 < ml.K; k0 += TRANS_K)
+                for (int p = 0; p < parts; ++p)
+                    tw.push_back(TransWork{i, k0, (int)((long long)ml.ngrp * p / parts),
+                                           (int)((long long)ml.ngrp * (p + 1) / parts)});
+        }
+        M->trans_ctas = (int)tw.size();
+        EMFA_TRY(upload(c, M->trans_work, tw, st));
+        EMFA_CUDA(c, cudaStreamSynchronize(st));  // tw goes out of scope
     }
     // interpolation level i+1 (child, fewer samples) -> level i (parent), i = 0..nl-2
     for (int i = 0; i + 1 < nl; ++i) {
@@ -1327,7 +1615,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                 dw[ch] = make_int2(lo, hi);
                 most = std::max(most, hi - lo);
             }
-            cm.down_smem = sizeof(float2) * 3 * (size_t)most * Lc;
+            cm.down_smem = sizeof(float2) * 3 * (size_t)most * (Lc + Lp);
             if (cm.down_smem > 200 * 1024) {
                 set_error(c, "mlfma: anterpolation rows exceed shared memory (level too large)");
                 return EMFA_ERR_UNSUPPORTED;
@@ -1370,7 +1658,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
             const double px = -ky / rho, py = kx / rho;
             const double tx = py * kz, ty = -px * kz, tz = px * ky - py * kx;
             const double tv[6] = {tx, ty, tz, px, py, 0.0};
-            for (int j = 0; j < 6; ++j) tp[6 * (size_t)kk + j] = (float)tv[j];
+            for (int j = 0; j < 6; ++j) tp[(size_t)j * Kf + kk] = (float)tv[j];
         }
         EMFA_TRY(upload(c, M->tp, tp, st));
     }
@@ -1400,6 +1688,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         nptr.push_back((int)nbox.size());
         max_near = std::max(max_near, (int)fin[b].near.size());
         rcols.push_back(cols);
+        M->max_cols = std::max(M->max_cols, cols);
         rbase.push_back(nnz);
         nnz += (size_t)cols * fin[b].unk.size();
     }
@@ -1459,6 +1748,38 @@ static emfa_status_t reserve_rhs(emfa_mlfma* M, int nr)
     return EMFA_OK;
 }
 
+// shared bytes of k_finish<RB>
+static size_t finish_smem(emfa_mlfma* M, int rb)
+{
+    const int nl = M->levels - 1;
+    const MLevel& fl = M->lv[nl - 1];
+    const size_t Lp = nl > 1 ? M->lv[nl - 2].L : 0;
+    return sizeof(float2) * (6 * Lp * (fl.L + Lp) + (size_t)rb * (2 * fl.K + M->max_cols));
+}
+// k_finish where at least two of its CTAs fit an SM; larger finest boxes (many
+// samples or near columns) keep the anterpolation and the warp-per-unknown
+// disaggregation as two kernels
+constexpr size_t FINISH_SMEM_MAX = 100 * 1024;
+template <int RB>
+static emfa_status_t launch_finish(emfa_mlfma* M, const float2* x, int nr, float2* y, int parts, cudaStream_t st)
+{
+    const int nl = M->levels - 1;
+    MLevel& fl = M->lv[nl - 1];
+    MLevel& pm = M->lv[nl > 1 ? nl - 2 : 0];
+    const bool par = nl > 1;
+    const FinishArgs a{x, M->n, nr, dptr<C2f>(M->rec), dptr<float>(M->tp), dptr<float2>(fl.down),
+                       (size_t)3 * fl.nbox * fl.K, dptr<float>(M->coeff), fl.L, par ? pm.L : 0,
+                       par ? dptr<float2>(pm.down) : nullptr, (size_t)3 * pm.nbox * pm.K, dptr<int>(fl.parent),
+                       dptr<int>(fl.oct), dptr<float2>(pm.up_phase), dptr<int>(fl.th_ptr), dptr<int>(fl.th_src),
+                       dptr<float>(fl.th_w), dptr<int>(fl.ph_ptr), dptr<int>(fl.ph_src), dptr<float>(fl.ph_w),
+                       dptr<int>(M->box_off), dptr<int>(M->box_cnt), dptr<int>(M->row_cols), dptr<size_t>(M->row_base),
+                       dptr<int>(M->near_cbase), dptr<int>(M->near_cidx), dptr<float2>(M->near_val), parts, y};
+    const size_t sm = finish_smem(M, RB);
+    EMFA_TRY(ensure_smem(M->ctx, k_finish<RB>, sm));
+    k_finish<RB><<<dim3(fl.nbox, RB == 1 ? nr : 1), 32 * FINISH_WARPS, sm, st>>>(a);
+    return EMFA_OK;
+}
+
 template <int RB>
 static void launch_agg_disagg(emfa_mlfma* M, bool agg, const float2* x, int nr, float2* y, int parts, cudaStream_t st)
 {
@@ -1467,24 +1788,36 @@ static void launch_agg_disagg(emfa_mlfma* M, bool agg, const float2* x, int nr, 
     const int Kf = fl.K, n = M->n;
     const size_t lstride = (size_t)3 * fl.nbox * Kf;
     if (agg)
-        k_agg_finest<RB><<<fl.nbox, 128, 0, st>>>(x, n, nr, dptr<C2f>(M->rad), dptr<float>(M->tp),
+        k_agg_finest<RB><<<dim3(fl.nbox, RB == 1 ? nr : 1), 128, 0, st>>>(x, n, nr, dptr<C2f>(M->rad), dptr<float>(M->tp),
                                                   dptr<int>(M->box_off), dptr<int>(M->box_cnt), Kf,
                                                   dptr<float2>(fl.up), lstride);
     else
-        k_disagg_near<RB><<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, st>>>(
+        k_disagg_near<RB><<<dim3((unsigned)(((size_t)n * 32 + 255) / 256), RB == 1 ? nr : 1), 256, 0, st>>>(
             x, nr, dptr<C2f>(M->rec), dptr<float>(M->tp), dptr<float2>(fl.down), lstride, dptr<float>(M->coeff),
             parts == 1 ? 0 : Kf,
             dptr<int>(M->box_of), dptr<int>(M->box_off), dptr<int>(M->row_cols), dptr<size_t>(M->row_base),
             dptr<int>(M->near_cbase), dptr<int>(M->near_cidx), dptr<float2>(M->near_val), n, parts == 2 ? 1 : 0, y);
 }
 
-static void agg_disagg(emfa_mlfma* M, bool agg, const float2* x, int nr, float2* y, int parts, cudaStream_t st)
+// Right-hand sides a CTA of the finest level's kernels takes (1, 2, 4 or 8):
+// all of them, so that the radiation and receive patterns are read from HBM
+// once, unless they stay in L2 anyway; then one each, on its own grid row, which
+// fills the SMs at these sizes (10,830 unknowns, 4 right-hand sides:
+// k_finish 115 -> 74 us, a product 328 -> 274 us).
+static int finest_rhs(emfa_mlfma* M, int nr)
 {
-    if (nr <= 1)
+    const size_t pat = sizeof(C2f) * (size_t)M->n * M->lv[M->levels - 2].K;
+    if (nr <= 1 || pat <= ((size_t)64 << 20)) return 1;
+    return nr <= 2 ? 2 : nr <= 4 ? 4 : 8;
+}
+
+static void agg_disagg(emfa_mlfma* M, bool agg, const float2* x, int nr, int rb, float2* y, int parts, cudaStream_t st)
+{
+    if (rb == 1)
         launch_agg_disagg<1>(M, agg, x, nr, y, parts, st);
-    else if (nr <= 2)
+    else if (rb == 2)
         launch_agg_disagg<2>(M, agg, x, nr, y, parts, st);
-    else if (nr <= 4)
+    else if (rb == 4)
         launch_agg_disagg<4>(M, agg, x, nr, y, parts, st);
     else
         launch_agg_disagg<8>(M, agg, x, nr, y, parts, st);
@@ -1497,7 +1830,8 @@ static emfa_status_t mlfma_apply(emfa_mlfma* M, const float2* x, float2* y, int 
     Ctx* c = M->ctx;
     EMFA_TRY(reserve_rhs(M, nr));
     const int nl = M->levels - 1;
-    agg_disagg(M, true, x, nr, y, parts, st);
+    const int rb = finest_rhs(M, nr);
+    agg_disagg(M, true, x, nr, rb, y, parts, st);
     for (int i = nl - 2; i >= 0; --i) {
         MLevel& pm = M->lv[i];
         MLevel& cm = M->lv[i + 1];
@@ -1510,22 +1844,37 @@ static emfa_status_t mlfma_apply(emfa_mlfma* M, const float2* x, float2* y, int 
             dptr<int2>(pm.up_win), pm.up_batch, dptr<float2>(pm.up_phase), pm.L, R, dptr<float2>(pm.up),
             (size_t)3 * cm.nbox * cm.K, (size_t)3 * pm.nbox * pm.K);
     }
+    TransLevels lv;
     for (int i = 0; i < nl; ++i) {
         MLevel& ml = M->lv[i];
-        const bool top = i == 0;
-        MLevel& pm = M->lv[top ? 0 : i - 1];
-        const int R = down_rows(ml.L);
-        const int bs = std::min(256, 32 * ((R * ml.L / 2 + 31) / 32));
-        const dim3 grid((unsigned)ml.nbox, (unsigned)((2 * ml.L + R - 1) / R), (unsigned)nr);
-        k_downward<<<grid, bs, top ? 0 : ml.down_smem, st>>>(
-            dptr<float4>(ml.up), dptr<int>(ml.far_ptr), dptr<int2>(ml.far), dptr<float4>(ml.trans), ml.L, R,
-            top ? nullptr : dptr<float2>(pm.down), pm.L, dptr<int2>(ml.down_win), dptr<int>(ml.parent),
-            dptr<int>(ml.oct), dptr<float2>(pm.up_phase), dptr<int>(ml.th_ptr), dptr<int>(ml.th_src),
-            dptr<float>(ml.th_w), dptr<int>(ml.ph_ptr), dptr<int>(ml.ph_src), dptr<float>(ml.ph_w),
-            dptr<float4>(ml.down), (size_t)3 * ml.nbox * ml.K, (size_t)3 * pm.nbox * pm.K);
+        lv.l[i] = TransLevel{dptr<float2>(ml.up),     dptr<float2>(ml.down),      dptr<float2>(ml.trans),
+                             dptr<int4>(ml.grp_src), dptr<TransGroup>(ml.grp), ml.K, (size_t)3 * ml.nbox * ml.K};
     }
-    agg_disagg(M, false, x, nr, y, parts, st);
-    c->kernel_launches += 2 * nl + 1;
+    k_translate<<<M->trans_ctas, 32 * TRANS_WARPS, TRANS_SMEM, st>>>(lv, dptr<TransWork>(M->trans_work), nr);
+    const bool fused = finish_smem(M, rb) <= FINISH_SMEM_MAX;
+    for (int i = 1; i < (fused ? nl - 1 : nl); ++i) {
+        MLevel& ml = M->lv[i];
+        MLevel& pm = M->lv[i - 1];
+        const int R = down_rows(ml.L);
+        const int bs = std::min(256, 32 * ((R * ml.L + 31) / 32));
+        const dim3 grid((unsigned)ml.nbox, (unsigned)((2 * ml.L + R - 1) / R), (unsigned)nr);
+        k_downward<<<grid, bs, ml.down_smem, st>>>(
+            ml.L, R, dptr<float2>(pm.down), pm.L, dptr<int2>(ml.down_win), dptr<int>(ml.parent), dptr<int>(ml.oct),
+            dptr<float2>(pm.up_phase), dptr<int>(ml.th_ptr), dptr<int>(ml.th_src), dptr<float>(ml.th_w),
+            dptr<int>(ml.ph_ptr), dptr<int>(ml.ph_src), dptr<float>(ml.ph_w), dptr<float2>(ml.down),
+            (size_t)3 * ml.nbox * ml.K, (size_t)3 * pm.nbox * pm.K);
+    }
+    if (!fused)
+        agg_disagg(M, false, x, nr, rb, y, parts, st);
+    else if (rb == 1)
+        EMFA_TRY(launch_finish<1>(M, x, nr, y, parts, st));
+    else if (rb == 2)
+        EMFA_TRY(launch_finish<2>(M, x, nr, y, parts, st));
+    else if (rb == 4)
+        EMFA_TRY(launch_finish<4>(M, x, nr, y, parts, st));
+    else
+        EMFA_TRY(launch_finish<8>(M, x, nr, y, parts, st));
+    c->kernel_launches += (fused ? 0 : 1) + 2 * nl;
     EMFA_CUDA(c, cudaGetLastError());
     return EMFA_OK;
 }
