@@ -364,6 +364,147 @@ __global__ void __launch_bounds__(256) k_vupdate(const Cx<T>* __restrict__ V, si
     griddep_launch();
 }
 
+// ---------------------------------------------------------------------------
+// The same two passes on the FP64 basis, where the FP64 pipe (16 cycles a warp
+// instruction and SM) is the bound: four FMAs an element and vector, the warp
+// sums of two vectors' four values by a transposed butterfly (6 additions
+// instead of 20), and CTAs over CH = 256 elements where chunks of 1024 would
+// not fill the SMs (vchunk64).  GMRES(30) with CGS2, n = 1080 x 91 right-hand
+// sides: coefficients 68.8 -> 17.0 us a launch, updates 57 -> 17 us.
+// ---------------------------------------------------------------------------
+template <int CH>
+__global__ void __launch_bounds__(256) k_vdots64(const Cx<double>* __restrict__ V, size_t vstride, int nv,
+                                                 const Cx<double>* __restrict__ W, int n, int nrhs, int nblk,
+                                                 double2* __restrict__ partial, const int* __restrict__ active)
+{
+    const int blk = blockIdx.x, r = blockIdx.y;
+    if (!active[r]) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t base = (size_t)r * n;
+    const int k0 = blk * CH, k1 = min(n, k0 + CH);
+    // pairs of vectors (i, i + 1), a warp a pair; an odd basis pairs its last
+    // vector with itself and drops the second value
+    for (int i = 2 * warp; i < nv; i += 16) {
+        const Cx<double>* va = V + (size_t)i * vstride + base;
+        const Cx<double>* vb = V + (size_t)min(i + 1, nv - 1) * vstride + base;
+        double ar = 0, ai = 0, br = 0, bi = 0;
+#pragma unroll 2
+        for (int k = k0 + lane; k < k1; k += 128) {
+            Cx<double> a[4], b[4], w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int kk = k + 32 * u;
+                const bool in = kk < k1;
+                a[u] = in ? va[kk] : Cx<double>{0.0, 0.0};
+                b[u] = in ? vb[kk] : Cx<double>{0.0, 0.0};
+                w[u] = in ? W[base + kk] : Cx<double>{0.0, 0.0};
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                ar = fma(a[u].re, w[u].re, fma(a[u].im, w[u].im, ar));
+                ai = fma(a[u].re, w[u].im, fma(-a[u].im, w[u].re, ai));
+                br = fma(b[u].re, w[u].re, fma(b[u].im, w[u].im, br));
+                bi = fma(b[u].re, w[u].im, fma(-b[u].im, w[u].re, bi));
+            }
+        }
+        // lanes 0-15 keep a, 16-31 b; then lanes with bit 8 clear keep re; then
+        // the lanes that hold one value add up
+        const bool hi16 = lane & 16, hi8 = lane & 8;
+        double x = (hi16 ? br : ar) + __shfl_xor_sync(0xffffffffu, hi16 ? ar : br, 16);
+        double y = (hi16 ? bi : ai) + __shfl_xor_sync(0xffffffffu, hi16 ? ai : bi, 16);
+        double t = (hi8 ? y : x) + __shfl_xor_sync(0xffffffffu, hi8 ? x : y, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        const double im = __shfl_xor_sync(0xffffffffu, t, 8);
+        if ((lane & 15) == 0 && i + (hi16 ? 1 : 0) < nv)
+            partial[((size_t)(i + (hi16 ? 1 : 0)) * nrhs + r) * nblk + blk] = make_double2(t, im);
+    }
+}
+
+template <int CH, bool NORM>
+__global__ void __launch_bounds__(256) k_vupdate64(const Cx<double>* __restrict__ V, size_t vstride, int nv,
+                                                   double2* __restrict__ h, const double2* __restrict__ partial,
+                                                   Cx<double>* __restrict__ W, int n, int nrhs, int nblk,
+                                                   double2* __restrict__ pnorm, const int* __restrict__ active)
+{
+    const int blk = blockIdx.x, r = nrhs - 1 - (int)blockIdx.y;
+    if (!active[r]) return;
+    const size_t base = (size_t)r * n;
+    extern __shared__ unsigned char dyn_smem[];
+    double* hs0 = reinterpret_cast<double*>(dyn_smem);  // 2 nv values
+    double* hs1 = hs0 + nv;
+    __shared__ double red[8];
+    // re and im of a coefficient by a thread each
+    for (int t = threadIdx.x; t < 2 * nv; t += blockDim.x) {
+        const int i = t >> 1;
+        const double* p = reinterpret_cast<const double*>(partial + ((size_t)i * nrhs + r) * nblk) + (t & 1);
+        double s = 0;
+        for (int b = 0; b < nblk; ++b) s += p[2 * b];
+        (t & 1 ? hs1 : hs0)[i] = s;
+        if (blk == 0) reinterpret_cast<double*>(h + (size_t)i * nrhs + r)[t & 1] = s;
+    }
+    __syncthreads();
+    constexpr int EL = CH / 256, VG = 4;
+    const int k0 = blk * CH, k1 = min(n, k0 + CH);
+    int kc[EL];
+    Cx<double> w[EL];
+#pragma unroll
+    for (int e = 0; e < EL; ++e) {
+        kc[e] = min(k0 + (int)threadIdx.x + 256 * e, k1 - 1);
+        w[e] = W[base + kc[e]];
+    }
+    const Cx<double>* vb = V + base;
+    for (int i = 0; i < nv; i += VG) {
+        Cx<double> v[VG][EL];
+#pragma unroll
+        for (int u = 0; u < VG; ++u) {
+            const Cx<double>* vi = vb + (size_t)min(i + u, nv - 1) * vstride;
+#pragma unroll
+            for (int e = 0; e < EL; ++e) v[u][e] = vi[kc[e]];
+        }
+#pragma unroll
+        for (int u = 0; u < VG; ++u) {
+            if (i + u >= nv) break;
+            const double hr = hs0[i + u], hi = hs1[i + u];
+#pragma unroll
+            for (int e = 0; e < EL; ++e) {
+                w[e].re = fma(-hr, v[u][e].re, fma(hi, v[u][e].im, w[e].re));
+                w[e].im = fma(-hr, v[u][e].im, fma(-hi, v[u][e].re, w[e].im));
+            }
+        }
+    }
+    double nr = 0;
+#pragma unroll
+    for (int e = 0; e < EL; ++e) {
+        const int k = k0 + (int)threadIdx.x + 256 * e;
+        if (k >= k1) continue;
+        W[base + k] = w[e];
+        if (NORM) nr = fma(w[e].re, w[e].re, fma(w[e].im, w[e].im, nr));
+    }
+    if (NORM) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) nr += __shfl_xor_sync(0xffffffffu, nr, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = nr;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0;
+            for (int q = 0; q < 8; ++q) t += red[q];
+            // the maximum that the FP16 packing reads has no use here
+            pnorm[(size_t)r * nblk + blk] = make_double2(t, 0.0);
+        }
+    }
+}
+
+// Elements a CTA of the FP64 passes takes: 256 where chunks of 1024 give fewer
+// than four CTAs an SM, unless the context has a budget (the chunks' partial
+// sums take 1/256 of the basis more memory).
+static int vchunk64(const Ctx* c, int n, int nrhs)
+{
+    const long sms = c->sm_count > 0 ? c->sm_count : 148;
+    return !c->budget && (long)((n + VCHUNK - 1) / VCHUNK) * nrhs < 4 * sms ? 256 : VCHUNK;
+}
+
 // X[r][k] += sum_i y_i V_i[r][k]; the sum in the basis precision, added to
 // the FP64 iterate once
 template <typename T>
@@ -1519,7 +1660,8 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     const int nblk = std::max(1, std::min(std::max((2 * sms + nrhs - 1) / nrhs, (n + 2047) / 2048),
                                           (n + 4 * KB - 1) / (4 * KB)));
     const int chunk = (n + nblk - 1) / nblk;
-    const int vblk = (n + VCHUNK - 1) / VCHUNK;  // chunks of the Gram-Schmidt passes
+    const int vch = std::is_same<T, double>::value ? vchunk64(c, n, nrhs) : VCHUNK;
+    const int vblk = (n + vch - 1) / vch;  // chunks of the Gram-Schmidt passes
     // the FP32 inner solve of the refinement only has to gain a few digits per
     // cycle: one Gram-Schmidt pass; the plain FP64 path keeps two
     const bool two_pass = sp->orth == 2 || (sp->orth == 0 && prec == EMFA_F64);
@@ -1553,8 +1695,8 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                         Carver::round(sizeof(double) * (size_t)nrhs * m) +
                         Carver::round(sizeof(double2) * (size_t)nrhs * m) * 2 +
                         Carver::round(sizeof(double2) * (size_t)nrhs * (m + 1)) * 2 +
-                        Carver::round(sizeof(double2) * (size_t)nrhs * (m + 1) * std::max(nblk, (n + VCHUNK - 1) / VCHUNK)) +
-                        Carver::round(sizeof(double2) * (size_t)nrhs * std::max(nblk, (n + VCHUNK - 1) / VCHUNK)) +
+                        Carver::round(sizeof(double2) * (size_t)nrhs * (m + 1) * std::max(nblk, vblk)) +
+                        Carver::round(sizeof(double2) * (size_t)nrhs * std::max(nblk, vblk)) +
                         Carver::round(sizeof(double) * 5 * (size_t)nrhs) + Carver::round(sizeof(int) * 2 * (size_t)nrhs) +
                         Carver::round(sizeof(int) * 4) + 4096;
     void* wsp = nullptr;
@@ -1584,7 +1726,7 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     s.y = cv.take<double2>((size_t)nrhs * m);
     s.g = cv.take<double2>((size_t)nrhs * (m + 1));
     s.hcol = cv.take<double2>((size_t)nrhs * (m + 1));
-    const int pb = std::max(nblk, (n + VCHUNK - 1) / VCHUNK);
+    const int pb = std::max(nblk, vblk);
     double2* partial = cv.take<double2>((size_t)nrhs * (m + 1) * pb);
     double2* pnorm = cv.take<double2>((size_t)nrhs * pb);
     s.bnorm = cv.take<double>(5 * (size_t)nrhs);
@@ -1721,17 +1863,30 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                     }
                     c->kernel_launches += 3;
                 } else {
-                k_vdots<T><<<vg, 256, 0, st>>>(V, vec, nv, W, n, nrhs, vblk, partial, nullptr, s.active);
+                auto dots = [&] {
+                    if constexpr (std::is_same<T, double>::value)
+                        (vch == 256 ? k_vdots64<256> : k_vdots64<VCHUNK>)<<<vg, 256, 0, st>>>(
+                            V, vec, nv, W, n, nrhs, vblk, partial, s.active);
+                    else
+                        k_vdots<T><<<vg, 256, 0, st>>>(V, vec, nv, W, n, nrhs, vblk, partial, nullptr, s.active);
+                };
+                auto update = [&](bool norm, double2* h) {
+                    if constexpr (std::is_same<T, double>::value)
+                        (vch == 256 ? (norm ? k_vupdate64<256, true> : k_vupdate64<256, false>)
+                                    : (norm ? k_vupdate64<VCHUNK, true> : k_vupdate64<VCHUNK, false>))<<<vg, 256, hsm, st>>>(
+                            V, vec, nv, h, partial, W, n, nrhs, vblk, pnorm, s.active);
+                    else
+                        (norm ? k_vupdate<T, true> : k_vupdate<T, false>)<<<vg, 256, hsm, st>>>(
+                            V, vec, nv, h, partial, W, n, nrhs, vblk, pnorm, s.active);
+                };
+                dots();
                 if (two_pass) {
-                    k_vupdate<T, false><<<vg, 256, hsm, st>>>(V, vec, nv, s.hcol, partial, W, n, nrhs, vblk, pnorm,
-                                                              s.active);
-                    k_vdots<T><<<vg, 256, 0, st>>>(V, vec, nv, W, n, nrhs, vblk, partial, nullptr, s.active);
-                    k_vupdate<T, true><<<vg, 256, hsm, st>>>(V, vec, nv, s.y, partial, W, n, nrhs, vblk, pnorm,
-                                                             s.active);
+                    update(false, s.hcol);
+                    dots();
+                    update(true, s.y);
                     c->kernel_launches += 2;
                 } else {
-                    k_vupdate<T, true><<<vg, 256, hsm, st>>>(V, vec, nv, s.hcol, partial, W, n, nrhs, vblk, pnorm,
-                                                             s.active);
+                    update(true, s.hcol);
                 }
                 EMFA_CUDA(c, cudaMemsetAsync(s.step_cnt, 0, sizeof(int), st));
                 if (m <= 32)
