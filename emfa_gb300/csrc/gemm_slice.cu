@@ -1,4 +1,4 @@
-// Y = Z X in FP64 accuracy on the 5th-generation tensor cores.
+// Y = Z X in FP64 or FP32 accuracy on the 5th-generation tensor cores.
 //
 // GB300's FP64 pipe runs at 1/64 of the FP32 one, so the CUDA-core FP64 product
 // (gemm.cu) is bound by it from a few right-hand sides on.  Here both operands
@@ -44,6 +44,10 @@
 // On GB300, a product of n unknowns and R right-hand sides, its split of Z
 // included, against the CUDA-core products:
 // 1080 x 91: 4456 -> 100 us;  2430 x 181: 9928 -> 428 us;  5070 x 360: 80.9 -> 2.93 ms
+// FP32 (complex64) operands take four digits, 30 bits below the scale, of which
+// the ten pairs of levels 0..3 are kept (the next is 2^-31 of the product of the
+// maxima): one rounding to FP32 of a sum that is exact to that, against an FP32
+// sum's rounding at every term.
 #include "emfa_internal.cuh"
 #include "emfa_math.cuh"
 #include "gemm_slice.cuh"
@@ -56,17 +60,31 @@ namespace emfa {
 
 namespace sl {
 
-constexpr int NS = 8;        // digits
 constexpr int BM = 128;
 constexpr int BK = 64;       // halves of K per block: 128-byte rows
 constexpr int GROUP = 2;     // blocks per drain: 128 columns
 constexpr int RING = 4;      // A planes in flight
-constexpr int EPI = 8;       // drain warps of each half of the levels
-constexpr int THREADS = 32 * (2 + 2 * EPI);
+constexpr int THREADS = 32 * (2 + 16);
 constexpr int SLICE_NONFINITE = INT_MAX;
 
-template <int BN>
+// per element type: digits, bits of a scaled value, exponent field, and the
+// lowest kept level's weight in products of two scaled values
+template <typename T> struct Cut;
+template <> struct Cut<double> {
+    static constexpr int NS = 8, BITS = 62, FIELD_MAX = 0x7ff, EXP_ONE = 1022;
+    using Word = unsigned long long;
+};
+template <> struct Cut<float> {
+    static constexpr int NS = 4, BITS = 30, FIELD_MAX = 0xff, EXP_ONE = 126;
+    using Word = unsigned;
+};
+
+// NS digits; the drain's 16 warps: lane quadrant, column part, four levels each
+template <int NS, int BN>
 struct Smem {
+    static constexpr int SETS = NS / 4;        // of four levels
+    static constexpr int PARTS = 4 / SETS;     // of the columns
+    static constexpr int EPI = 4 * PARTS;      // warps that drain a level
     static constexpr int A_BYTES = BM * BK * 2;  // one plane
     static constexpr int B_SLICE = BN * BK * 2;
     static constexpr int B_BYTES = NS * B_SLICE;
@@ -151,12 +169,12 @@ __device__ __forceinline__ void commit_elect(uint64_t* bar)
         : "memory");
 }
 
-template <int BN>
+template <int NS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     k_slice(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int C,
             int kblocks, int per_split, int4 w8, long long* __restrict__ part, int* __restrict__ err)
 {
-    using S = Smem<BN>;
+    using S = Smem<NS, BN>;
     using namespace tc;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sA = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [RING]
@@ -185,7 +203,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         for (int l = 0; l < NS; ++l) {
             mbar_init(acc_full + l, 1);
-            mbar_init(acc_empty + l, EPI);
+            mbar_init(acc_empty + l, S::EPI);
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -272,10 +290,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         commit_elect(done);
         warp_wait(done, 0, err, 27);
     } else {
-        // drain warps: lane quadrant warp % 4, column half, half of the levels
-        constexpr int CW = BN / 2, LW = CW < 16 ? CW : 16;
-        const int q = warp & 3, half = ((warp - 2) >> 2) & 1, set = (warp - 2) >> 3;
-        const uint32_t tw = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * CW);
+        // drain warps: lane quadrant warp % 4, part of the columns, four levels
+        constexpr int CW = BN / S::PARTS, LW = CW < 16 ? CW : 16;
+        const int q = warp & 3, part_c = ((warp - 2) >> 2) % S::PARTS, set = ((warp - 2) >> 2) / S::PARTS;
+        const uint32_t tw = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(part_c * CW);
         unsigned long long sum[CW];
         const int weight[4] = {w8.x, w8.y, w8.z, w8.w};
 #pragma unroll
@@ -311,10 +329,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         const unsigned long long bias = (unsigned long long)groups * INT_BIAS * 0x01010101ull;
         const int f = f0 + 32 * q + lane;
         if (ok && f < M) {
-            long long* o = part + ((size_t)blockIdx.z * 2 + set) * C * M;
+            long long* o = part + ((size_t)blockIdx.z * S::SETS + set) * C * M;
 #pragma unroll
             for (int i = 0; i < CW; ++i) {
-                const int col = c0 + half * CW + i;
+                const int col = c0 + part_c * CW + i;
                 if (col < C) o[(size_t)col * M + f] = (long long)(sum[i] - bias);
             }
         }
@@ -330,9 +348,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 // operand preparation, integers only
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int exponent_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ int exponent_field(float x) { return (__float_as_int(x) >> 23) & 0xff; }
 
 // biased digits of x at scale eb (the row's largest exponent field, at least
-// 1): byte s of the result is d_(7-s) + 128
+// 1): byte s of the result is d_(NS-1-s) + 128
 __device__ __forceinline__ unsigned long long digits(double x, int eb)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
@@ -348,13 +367,30 @@ __device__ __forceinline__ unsigned long long digits(double x, int eb)
     if ((long long)b < 0) v = -v;
     return ((unsigned long long)v + 0x0080808080808080ull) ^ (0x80ull << 56);
 }
+__device__ __forceinline__ unsigned digits(float x, int eb)
+{
+    const unsigned b = (unsigned)__float_as_int(x);
+    const int ef = (int)((b >> 23) & 0xff);
+    unsigned m = b & 0x7fffffu;
+    if (ef) m |= 1u << 23;
+    const int s = (ef ? ef : 1) - eb + 6;  // 0..6 for the largest
+    int v;
+    if (s >= 0)
+        v = (int)(m << s);
+    else
+        v = s < -25 ? 0 : (int)((m + (1u << (-s - 1))) >> -s);
+    if ((int)b < 0) v = -v;
+    return ((unsigned)v + 0x00808080u) ^ 0x80000000u;
+}
 
 // digit s of a complex pair as two FP16 integers: the byte under the exponent
 // of 1024 is 1024 + d + 128
-__device__ __forceinline__ unsigned pair_digit(unsigned long long a, unsigned long long b, int s)
+template <typename Word>
+__device__ __forceinline__ unsigned pair_digit(Word a, Word b, int s)
 {
-    const int byte = 7 - s;
-    const unsigned wa = (unsigned)(a >> (byte & 4 ? 32 : 0)), wb = (unsigned)(b >> (byte & 4 ? 32 : 0));
+    const int byte = (int)sizeof(Word) - 1 - s;
+    const unsigned wa = (unsigned)(byte & 4 ? (unsigned long long)a >> 32 : a),
+                   wb = (unsigned)(byte & 4 ? (unsigned long long)b >> 32 : b);
     const unsigned x = (__byte_perm(wa, wb, (byte & 3) | ((4 + (byte & 3)) << 8)) & 0x00ff00ffu) | 0x64006400u;
     const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2half2(__float2half_rn(1152.f)));
     return *reinterpret_cast<const unsigned*>(&r);
@@ -377,60 +413,67 @@ __device__ __forceinline__ int block_max_int(int m, int* red)
 
 // CTA per row of Z: its scale, then its digits (the row is read twice, the
 // second time from L2)
-__global__ void __launch_bounds__(256) k_slice_rows(const double2* __restrict__ Z, size_t ldz, int n, size_t ldk,
+template <typename T>
+__global__ void __launch_bounds__(256) k_slice_rows(const Cx<T>* __restrict__ Z, size_t ldz, int n, size_t ldk,
                                                     __half* __restrict__ D, int* __restrict__ ex)
 {
+    using Word = typename Cut<T>::Word;
     __shared__ int red[32];
     const int i = blockIdx.x;
-    const double2* z = Z + (size_t)i * ldz;
+    const Cx<T>* z = Z + (size_t)i * ldz;
     int m = 1;
 #pragma unroll 4
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double2 v = z[k];
-        m = max(m, max(exponent_field(v.x), exponent_field(v.y)));
+        const Cx<T> v = z[k];
+        m = max(m, max(exponent_field(v.re), exponent_field(v.im)));
     }
     m = block_max_int(m, red);
-    const bool bad = m == 0x7ff;
+    const bool bad = m == Cut<T>::FIELD_MAX;
     if (threadIdx.x == 0) ex[i] = bad ? SLICE_NONFINITE : m;
     const size_t plane = (size_t)n * ldk / 2;
     unsigned* o = reinterpret_cast<unsigned*>(D) + (size_t)i * (ldk / 2);
-#pragma unroll 2
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double2 v = z[k];
-        const unsigned long long a = bad ? 0x8080808080808080ull : digits(v.x, m),
-                                 b = bad ? 0x8080808080808080ull : digits(v.y, m);
+    constexpr Word zero = (Word)0x8080808080808080ull;
+    // two elements a thread, one 8-byte store a plane (the rows of D are padded
+    // to 16 bytes: an odd row's last store ends in the padding)
+    for (int k = 2 * threadIdx.x; k < n; k += 2 * blockDim.x) {
+        const Cx<T> v = z[k], u = k + 1 < n ? z[k + 1] : cx(T(0), T(0));
+        const Word a = bad ? zero : digits(v.re, m), b = bad ? zero : digits(v.im, m);
+        const Word c = bad ? zero : digits(u.re, m), d = bad ? zero : digits(u.im, m);
 #pragma unroll
-        for (int s = 0; s < NS; ++s) o[s * plane + k] = pair_digit(a, b, s);
+        for (int s = 0; s < Cut<T>::NS; ++s)
+            *reinterpret_cast<uint2*>(o + s * plane + k) = make_uint2(pair_digit(a, b, s), pair_digit(c, d, s));
     }
 }
 
 // CTA per right-hand side: B rows 2r = (Re, -Im) and 2r + 1 = (Im, Re)
-__global__ void __launch_bounds__(256) k_slice_rhs(const double2* __restrict__ X, int n, int nrhs, size_t ldk,
+template <typename T>
+__global__ void __launch_bounds__(256) k_slice_rhs(const Cx<T>* __restrict__ X, int n, int nrhs, size_t ldk,
                                                    __half* __restrict__ D, int* __restrict__ ex)
 {
+    using Word = typename Cut<T>::Word;
     __shared__ int red[32];
     const int r = blockIdx.x;
-    const double2* x = X + (size_t)r * n;
+    const Cx<T>* x = X + (size_t)r * n;
     int m = 1;
 #pragma unroll 4
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double2 v = x[k];
-        m = max(m, max(exponent_field(v.x), exponent_field(v.y)));
+        const Cx<T> v = x[k];
+        m = max(m, max(exponent_field(v.re), exponent_field(v.im)));
     }
     m = block_max_int(m, red);
-    const bool bad = m == 0x7ff;
+    const bool bad = m == Cut<T>::FIELD_MAX;
     if (threadIdx.x == 0) ex[r] = bad ? SLICE_NONFINITE : m;
     const size_t plane = (size_t)2 * nrhs * ldk / 2;
     unsigned* o0 = reinterpret_cast<unsigned*>(D) + (size_t)(2 * r) * (ldk / 2);
     unsigned* o1 = o0 + ldk / 2;
+    constexpr Word zero = (Word)0x8080808080808080ull;
 #pragma unroll 2
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double2 v = x[k];
-        const unsigned long long zero = 0x8080808080808080ull;
-        const unsigned long long a = bad ? zero : digits(v.x, m), b = bad ? zero : digits(v.y, m),
-                                 nb = bad ? zero : digits(-v.y, m);
+        const Cx<T> v = x[k];
+        const Word a = bad ? zero : digits(v.re, m), b = bad ? zero : digits(v.im, m),
+                   nb = bad ? zero : digits(-v.im, m);
 #pragma unroll
-        for (int s = 0; s < NS; ++s) {
+        for (int s = 0; s < Cut<T>::NS; ++s) {
             o0[s * plane + k] = pair_digit(a, nb, s);
             o1[s * plane + k] = pair_digit(b, a, s);
         }
@@ -475,45 +518,55 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int ex)
 }
 
 // Y from the partial sums of all splits.  A row or a right-hand side with an
-// infinity or NaN is summed in FP64 as gemm.cu does; a pipeline that gave up
-// (err) leaves NaN.
+// infinity or NaN is summed in T as gemm.cu does; a pipeline that gave up (err)
+// leaves NaN.
+template <typename T>
 __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ part, int splits, int n, int nrhs,
                                                  const int* __restrict__ exz, const int* __restrict__ exx,
-                                                 const double2* __restrict__ Z, size_t ldz,
-                                                 const double2* __restrict__ X, const int* __restrict__ err,
-                                                 double2* __restrict__ Y)
+                                                 const Cx<T>* __restrict__ Z, size_t ldz,
+                                                 const Cx<T>* __restrict__ X, const int* __restrict__ err,
+                                                 Cx<T>* __restrict__ Y)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
     if (f >= n) return;
     const int ez = exz[f], ex = exx[r];
-    double2 y;
+    Cx<T> y;
     if (*err) {
-        y.x = y.y = __longlong_as_double(0x7ff8000000000000ll);
+        y.re = y.im = (T)__longlong_as_double(0x7ff8000000000000ll);
     } else if (ez == SLICE_NONFINITE || ex == SLICE_NONFINITE) {
-        const double2* z = Z + (size_t)f * ldz;
-        const double2* x = X + (size_t)r * n;
-        double re = 0.0, im = 0.0;
+        const Cx<T>* z = Z + (size_t)f * ldz;
+        const Cx<T>* x = X + (size_t)r * n;
+        T re = 0, im = 0;
         for (int k = 0; k < n; ++k) {
-            const double2 a = z[k], b = x[k];
-            re = fma(a.x, b.x, re);
-            re = fma(-a.y, b.y, re);
-            im = fma(a.x, b.y, im);
-            im = fma(a.y, b.x, im);
+            const Cx<T> a = z[k], b = x[k];
+            re = fma(a.re, b.re, re);
+            re = fma(-a.im, b.im, re);
+            im = fma(a.re, b.im, im);
+            im = fma(a.im, b.re, im);
         }
-        y = make_double2(re, im);
+        y = cx(re, im);
     } else {
         const size_t plane = (size_t)2 * nrhs * n;
         const long long* p0 = part + (size_t)(2 * r) * n + f;
-        long long h0 = 0, l0 = 0, h1 = 0, l1 = 0;
-        for (int s = 0; s < splits; ++s, p0 += 2 * plane) {
-            h0 += p0[0];
-            h1 += p0[n];
-            l0 += p0[plane];
-            l1 += p0[plane + n];
+        // z = V 2^(e - BITS), e = field - EXP_ONE; the lowest kept level, NS - 1, weighs 2^(8 (NS - 1)) in V V
+        const int e = ez + ex - 2 * (Cut<T>::EXP_ONE + Cut<T>::BITS) + 8 * (Cut<T>::NS - 1);
+        long long s0 = 0, s1 = 0;  // levels 0-3
+        if constexpr (Cut<T>::NS == 8) {
+            long long l0 = 0, l1 = 0;
+            for (int s = 0; s < splits; ++s, p0 += 2 * plane) {
+                s0 += p0[0];
+                s1 += p0[n];
+                l0 += p0[plane];
+                l1 += p0[plane + n];
+            }
+            y = cx((T)to_double(s0, l0, e), (T)to_double(s1, l1, e));
+        } else {
+            for (int s = 0; s < splits; ++s, p0 += plane) {
+                s0 += p0[0];
+                s1 += p0[n];
+            }
+            y = cx((T)to_double(s0 >> 32, s0 & 0xffffffffll, e), (T)to_double(s1 >> 32, s1 & 0xffffffffll, e));
         }
-        // z = V 2^(e-62), e = field - 1022; the lowest kept level weighs 2^56
-        const int e = (ez - 1022) + (ex - 1022) - 124 + 56;
-        y = make_double2(to_double(h0, l0, e), to_double(h1, l1, e));
     }
     Y[(size_t)r * n + f] = y;
 }
@@ -525,20 +578,20 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
 // ---------------------------------------------------------------------------
 static size_t slice_ld(int n) { return ((size_t)2 * n + 7) & ~(size_t)7; }  // 16-byte rows
 
-static size_t slice_plane_bytes(int n)
+static size_t slice_plane_bytes(int ns, int n)
 {
-    return Carver::round(sizeof(__half) * sl::NS * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
+    return Carver::round(sizeof(__half) * ns * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
 }
 
 static emfa_status_t slice_map(Ctx* c, CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, size_t ld,
-                               uint32_t box_rows, uint32_t box_planes)
+                               uint64_t planes, uint32_t box_rows, uint32_t box_planes)
 {
     auto fn = tensor_map_encoder();
     if (!fn) {
         set_error(c, "cuTensorMapEncodeTiled unavailable");
         return EMFA_ERR_CUDA;
     }
-    cuuint64_t dims[3] = {inner, rows, (cuuint64_t)sl::NS};
+    cuuint64_t dims[3] = {inner, rows, planes};
     cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)ld * 2 * rows};
     cuuint32_t box[3] = {(cuuint32_t)sl::BK, box_rows, box_planes};
     cuuint32_t estr[3] = {1, 1, 1};
@@ -561,49 +614,77 @@ static emfa_status_t slice_err(Ctx* c, int** err)
     return EMFA_OK;
 }
 
+// The planes take twice the matrix's memory, in workspaces of the context that
+// calls on its own stream share: a context with an HBM budget, a caller's
+// stream (its calls may overlap others of the context, and may be captured) and
+// planes above 16 GB keep the CUDA-core product, which needs no memory.
+static bool slice_allowed(Ctx* c, int ns, int n, cudaStream_t st)
+{
+    if (n < 128 || c->budget || c->stream_ordered || st != c->stream || slice_plane_bytes(ns, n) > ((size_t)16 << 30))
+        return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st)
 {
-    // The planes take twice the matrix's memory, in workspaces of the context
-    // that calls on its own stream share: a context with an HBM budget, a
-    // caller's stream (its calls may overlap others of the context, and may be
-    // captured) and planes above 16 GB keep the CUDA-core product, which needs
-    // no memory.
-    if (c->budget || c->stream_ordered || st != c->stream || slice_plane_bytes(n) > ((size_t)16 << 30)) return false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    if (!slice_allowed(c, sl::Cut<double>::NS, n, st)) return false;
     // Measured (us, a call with its one split of Z | the CUDA-core GEMV): n = 256, 8 right-hand sides 55 | 48,
     // 16: 59 | 75; 480, 8: 58 | 63; 1080, 4: 81 | 68, 8: 80 | 106; 2430, 4: 182 | 191; 5070, 2: 646 | 438, 4: 647 | 847.
     // With Z split already, n = 2430, 2: 125 | 110; 5070, 2: 400 | 438.
-    if (built) return n >= 128 && nrhs >= (n >= 2000 ? 3 : n >= 1000 ? 4 : n >= 480 ? 8 : 10);
-    return n >= 128 && nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
+    if (built) return nrhs >= (n >= 2000 ? 3 : n >= 1000 ? 4 : n >= 480 ? 8 : 10);
+    return nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
 }
 
-emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
+// One FP32 product with its split of Z, above the 16 right-hand sides of the
+// GEMV (against the 64 x 64 tiles: n = 480 x 17, 53 | 90 us; 1080 x 91, 72 | 193;
+// 2430 x 181, 194 | 380; 5067 x 37, 358 | 810).  Up to 16 the GEMV, whose lane
+// sums are shorter, can be the more exact one (n = 3000 x 3: 3.5e-7 against its
+// 2.5e-7; the tiles' error is 8.8e-7 to 1.8e-6 where this one's is 1.9e-7 to 3.6e-7).
+static bool slice_worthwhile_f32(Ctx* c, int n, int nrhs, cudaStream_t st)
 {
+    return slice_allowed(c, sl::Cut<float>::NS, n, st) && nrhs > 16;
+}
+
+template <typename T>
+static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
+{
+    constexpr int NS = sl::Cut<T>::NS;
     const size_t ldk = slice_ld(n);
     void* wp = nullptr;
-    EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(n) + 512, &wp));
+    EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(NS, n) + 512, &wp));
     Carver cv{(char*)wp};
-    __half* d = cv.take<__half>(sl::NS * (size_t)n * ldk);
+    __half* d = cv.take<__half>(NS * (size_t)n * ldk);
     int* ex = cv.take<int>(n);
     int* err = nullptr;
     EMFA_TRY(slice_err(c, &err));
     EMFA_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), st));
-    sl::k_slice_rows<<<n, 256, 0, st>>>((const double2*)Z, ldz, n, ldk, d, ex);
+    sl::k_slice_rows<T><<<n, 256, 0, st>>>((const Cx<T>*)Z, ldz, n, ldk, d, ex);
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
-    *out = SlicePlanes{d, ex, (const double2*)Z, ldz, n, ldk};
+    *out = SlicePlanes{d, ex, Z, ldz, n, ldk};
     return EMFA_OK;
 }
 
-// Column tile, and over how many CTAs a tile's K is split: the split with the
-// fewest K blocks in the longest chain of CTAs an SM runs, a CTA's fixed cost
-// (pipeline fill, last drain, 131 KB of partial sums written and read again)
-// counted as two and a half blocks.
+emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
+{
+    return prepare_t<double>(c, slot, Z, ldz, n, out, st);
+}
+
+// Column tile (narrow for few right-hand sides; the wide one fills tensor
+// memory with a level's sums each), and over how many CTAs a tile's K is split:
+// the split with the fewest K blocks in the longest chain of CTAs an SM runs, a
+// CTA's fixed cost (pipeline fill, last drain, partial sums written and read
+// again) counted as two and a half blocks.
+template <typename T> struct Tile;
+template <> struct Tile<double> { static constexpr int NARROW = 16, WIDE = 64; };
+template <> struct Tile<float> { static constexpr int NARROW = 32, WIDE = 128; };
+
+template <typename T>
 static void slice_shape(Ctx* c, int n, int nrhs, int* bn, int* splits, int* per_split)
 {
     const int sms = c->sm_count > 0 ? c->sm_count : 148;
-    *bn = 2 * nrhs <= 16 ? 16 : 64;
+    *bn = 2 * nrhs <= Tile<T>::NARROW ? Tile<T>::NARROW : Tile<T>::WIDE;
     const int blocks = (2 * n + sl::BK - 1) / sl::BK, groups = (blocks + sl::GROUP - 1) / sl::GROUP;
     const long tiles = (long)((n + sl::BM - 1) / sl::BM) * ((2 * nrhs + *bn - 1) / *bn);
     long best = -1;
@@ -619,65 +700,74 @@ static void slice_shape(Ctx* c, int n, int nrhs, int* bn, int* splits, int* per_
     }
 }
 
-template <int BN>
+template <int NS, int BN>
 static emfa_status_t launch_slice(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int n, int nrhs, int splits,
                                   int per_split, long long* part, int* err, cudaStream_t st)
 {
-    using S = sl::Smem<BN>;
-    EMFA_TRY(ensure_smem(c, sl::k_slice<BN>, S::TOTAL));
+    using S = sl::Smem<NS, BN>;
+    EMFA_TRY(ensure_smem(c, sl::k_slice<NS, BN>, S::TOTAL));
     const dim3 grd((2 * nrhs + BN - 1) / BN, (n + sl::BM - 1) / sl::BM, splits);
-    sl::k_slice<BN><<<grd, sl::THREADS, S::TOTAL, st>>>(ta, tb, n, 2 * nrhs, (2 * n + sl::BK - 1) / sl::BK, per_split,
-                                                        make_int4(1, 1 << 8, 1 << 16, 1 << 24), part, err);
+    sl::k_slice<NS, BN><<<grd, sl::THREADS, S::TOTAL, st>>>(ta, tb, n, 2 * nrhs, (2 * n + sl::BK - 1) / sl::BK,
+                                                            per_split, make_int4(1, 1 << 8, 1 << 16, 1 << 24), part,
+                                                            err);
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
     return EMFA_OK;
 }
 
-emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
+template <typename T>
+static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
 {
+    constexpr int NS = sl::Cut<T>::NS, SETS = NS / 4, NARROW = Tile<T>::NARROW, WIDE = Tile<T>::WIDE;
     const int n = p.n;
     // blocks of right-hand sides bound the scratch (digits and partial sums)
     constexpr int RB = 512;
     const int rmax = std::min(nrhs, RB);
     int bn, splits, per_split;
-    slice_shape(c, n, rmax, &bn, &splits, &per_split);
+    slice_shape<T>(c, n, rmax, &bn, &splits, &per_split);
     const size_t brow = (size_t)2 * rmax * p.ldk;
     int smax = splits;
     if (nrhs % RB) {
         int b2, s2, p2;
-        slice_shape(c, n, nrhs % RB, &b2, &s2, &p2);
+        slice_shape<T>(c, n, nrhs % RB, &b2, &s2, &p2);
         // scratch of the last block: fewer columns, perhaps more splits
         smax = std::max(splits, (int)(((long)s2 * (nrhs % RB) + rmax - 1) / rmax));
     }
+    const size_t parts = (size_t)smax * 2 * SETS * rmax * n;
     void* wp = nullptr;
     EMFA_TRY(ctx_workspace(c, slot,
-                           Carver::round(sizeof(__half) * sl::NS * brow) + Carver::round(sizeof(int) * (size_t)rmax) +
-                               Carver::round(sizeof(long long) * (size_t)smax * 4 * rmax * n) + 1024,
+                           Carver::round(sizeof(__half) * NS * brow) + Carver::round(sizeof(int) * (size_t)rmax) +
+                               Carver::round(sizeof(long long) * parts) + 1024,
                            &wp));
     Carver cv{(char*)wp};
-    __half* b = cv.take<__half>(sl::NS * brow);
+    __half* b = cv.take<__half>(NS * brow);
     int* ex = cv.take<int>(rmax);
-    long long* part = cv.take<long long>((size_t)smax * 4 * rmax * n);
+    long long* part = cv.take<long long>(parts);
     int* err = nullptr;
     EMFA_TRY(slice_err(c, &err));
     CUtensorMap ta, tb;
-    EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)n, p.ldk, sl::BM, 1));
+    EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)n, p.ldk, NS, sl::BM, 1));
     for (int r0 = 0; r0 < nrhs; r0 += RB) {
         const int nr = std::min(RB, nrhs - r0);
-        const double2* x = (const double2*)X + (size_t)r0 * n;
-        slice_shape(c, n, nr, &bn, &splits, &per_split);
-        EMFA_TRY(slice_map(c, &tb, b, 2 * (uint64_t)n, 2 * (uint64_t)nr, p.ldk, (uint32_t)bn, sl::NS));
-        sl::k_slice_rhs<<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex);
+        const Cx<T>* x = (const Cx<T>*)X + (size_t)r0 * n;
+        slice_shape<T>(c, n, nr, &bn, &splits, &per_split);
+        EMFA_TRY(slice_map(c, &tb, b, 2 * (uint64_t)n, 2 * (uint64_t)nr, p.ldk, NS, (uint32_t)bn, NS));
+        sl::k_slice_rhs<T><<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
-        EMFA_TRY(bn == 16 ? launch_slice<16>(c, ta, tb, n, nr, splits, per_split, part, err, st)
-                          : launch_slice<64>(c, ta, tb, n, nr, splits, per_split, part, err, st));
-        sl::k_combine<<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, p.Z, p.ldz, x, err,
-                                                                 (double2*)Y + (size_t)r0 * n);
+        EMFA_TRY((bn == NARROW ? launch_slice<NS, NARROW> : launch_slice<NS, WIDE>)(c, ta, tb, n, nr, splits, per_split,
+                                                                                  part, err, st));
+        sl::k_combine<T><<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, (const Cx<T>*)p.Z,
+                                                                    p.ldz, x, err, (Cx<T>*)Y + (size_t)r0 * n);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
     }
     return EMFA_OK;
+}
+
+emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
+{
+    return apply_t<double>(c, slot, p, X, nrhs, Y, st);
 }
 
 emfa_status_t slice_check(Ctx* c, cudaStream_t st)
@@ -688,23 +778,22 @@ emfa_status_t slice_check(Ctx* c, cudaStream_t st)
     EMFA_CUDA(c, cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     EMFA_CUDA(c, cudaStreamSynchronize(st));
     if (h) {
-        set_error(c, "FP64 tensor-core product: a pipeline wait timed out (stage " + std::to_string(h) + ")");
+        set_error(c, "digit-plane tensor-core product: a pipeline wait timed out (stage " + std::to_string(h) + ")");
         return EMFA_ERR_TIMEOUT;
     }
     return EMFA_OK;
 }
 
-emfa_status_t slice_matvec(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
-                           cudaStream_t st, bool* done)
+template <typename T>
+static emfa_status_t matvec_t(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                              cudaStream_t st, bool* done)
 {
-    *done = false;
-    if (!slice_worthwhile(c, n, nrhs, false, st)) return EMFA_OK;
     // the whole sequence of launches at once: another thread's product on this
     // context's stream uses the same workspaces before or after it
     std::lock_guard<std::mutex> lk(c->slice_mu);
     SlicePlanes p;
-    emfa_status_t s = slice_prepare(c, WS_SLICE_MV, Z, ldz, n, &p, st);
-    if (s == EMFA_OK) s = slice_apply(c, WS_SLICE_MV_B, p, X, nrhs, Y, st);
+    emfa_status_t s = prepare_t<T>(c, WS_SLICE_MV, Z, ldz, n, &p, st);
+    if (s == EMFA_OK) s = apply_t<T>(c, WS_SLICE_MV_B, p, X, nrhs, Y, st);
     if (s == EMFA_ERR_OOM) {
         cudaGetLastError();  // no room: the caller's CUDA-core product
         return EMFA_OK;
@@ -712,6 +801,15 @@ emfa_status_t slice_matvec(Ctx* c, const void* Z, size_t ldz, const void* X, int
     EMFA_TRY(s);
     *done = true;
     return EMFA_OK;
+}
+
+emfa_status_t slice_matvec(Ctx* c, int prec, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                           cudaStream_t st, bool* done)
+{
+    *done = false;
+    if (prec == EMFA_F64)
+        return slice_worthwhile(c, n, nrhs, false, st) ? matvec_t<double>(c, Z, ldz, X, n, nrhs, Y, st, done) : EMFA_OK;
+    return slice_worthwhile_f32(c, n, nrhs, st) ? matvec_t<float>(c, Z, ldz, X, n, nrhs, Y, st, done) : EMFA_OK;
 }
 
 }  // namespace emfa

@@ -1,22 +1,22 @@
-// FP64-accurate complex products on the tensor cores (gemm_slice.cu).
+// FP64- and FP32-accurate complex products on the tensor cores (gemm_slice.cu).
 #pragma once
 #include "gemm.cuh"
 
 namespace emfa {
 
-// Z (complex128, n x n) as eight planes of signed 8-bit digits held in FP16,
-// each n x 2n (re, im interleaved), rows ldk halves apart, and a power-of-two
-// scale per row.
+// Z (n x n) as planes of signed 8-bit digits held in FP16 (eight for complex128,
+// four for complex64), each n x 2n (re, im interleaved), rows ldk halves apart,
+// and a power-of-two scale per row.
 struct SlicePlanes {
-    const __half* d = nullptr;   // [8][n][ldk]
+    const __half* d = nullptr;   // [planes][n][ldk]
     const int* ex = nullptr;     // [n] row scales; SLICE_NONFINITE for a row with an infinity or NaN
-    const double2* Z = nullptr;  // the matrix itself
+    const void* Z = nullptr;     // the matrix itself
     size_t ldz = 0;
     int n = 0;
     size_t ldk = 0;
 };
 
-// Whether a block of nrhs products of n unknowns is worth the planes; built:
+// FP64: whether a block of nrhs products of n unknowns is worth the planes; built:
 // the planes exist already (a Krylov solve splits Z once).
 bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st);
 // Splits Z into workspace `slot` of the context.  EMFA_ERR_OOM: no room, the
@@ -26,9 +26,9 @@ emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, 
 // word of the pipeline's bounded waits turns Y into NaN (and slice_check tells)
 emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st);
 emfa_status_t slice_check(Ctx* c, cudaStream_t st);
-// one product: splits Z, multiplies; false in *done where the CUDA cores are
-// the better path or there is no room
-emfa_status_t slice_matvec(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+// one product in precision prec: splits Z, multiplies; false in *done where the
+// CUDA cores are the better path or there is no room
+emfa_status_t slice_matvec(Ctx* c, int prec, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
                            cudaStream_t st, bool* done);
 
 }  // namespace emfa

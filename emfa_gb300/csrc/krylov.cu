@@ -2537,7 +2537,7 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     if (prec == EMFA_F64) {
         bool done = false;
-        if (matvec != EMFA_MV_F64) EMFA_TRY(slice_matvec(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
+        if (matvec != EMFA_MV_F64) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
         return done ? EMFA_OK : cgemm_f64(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
     }
     if (prec != EMFA_F32) {
@@ -2554,7 +2554,9 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
         EMFA_TRY(hgemm_apply(ctx, hp, X_dev, Y_dev, n_rhs, st));
         return hgemm_check_error(ctx, st);
     }
-    return cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    bool done = false;
+    if (matvec != EMFA_MV_F32) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
+    return done ? EMFA_OK : cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
 }
 
 emfa_status_t emfa_residual(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_dev, int n, const void* X_dev,

@@ -4,7 +4,8 @@
 Bound: with z and x cut at 2^-63 of their scales (a power of two at most twice the largest entry of the row or vector)
 and the digit pairs of levels 8 and up dropped (at most 7 x 2^14 x 2^48 of 2^124, all pairs below it less), a real
 product is off by at most 2^-59 + 2 x 2^-63 < 2^-58 of the two scales, a complex entry's 2n products by 2n x 4 x 2^-58
-of the maxima, and the result by its own rounding."""
+of the maxima, and the result by its own rounding.  FP32: cut at 2^-31, levels 4 and up dropped (at most 3 x 2^14 x 2^16 of
+2^60 and less below it): 2^-28 of the two scales."""
 from fractions import Fraction
 
 import numpy as np
@@ -91,3 +92,45 @@ def test_slice_product_of_two_shapes_in_turn(ctx):
     first = [_run(ctx, z, x) for z, x in ops]
     for (z, x), y in list(zip(ops, first))[::-1]:
         assert np.array_equal(_run(ctx, z, x), y)
+
+
+@pytest.mark.parametrize("n,r", [(128, 17), (257, 18), (271, 17), (384, 64), (640, 65), (513, 130), (256, 520)])
+@pytest.mark.parametrize("kind", ["normal", "graded", "extreme"])
+def test_fp32_slice_product_against_exact_sums(ctx, n, r, kind):
+    rng = np.random.default_rng(n * 1000 + r + 7)
+    z, x = _cplx(rng, n, n), _cplx(rng, r, n)
+    if kind == "graded":
+        z *= 10.0 ** rng.uniform(-8, 8, (n, 1)) * 10.0 ** rng.uniform(-5, 0, (n, n))
+        x *= 10.0 ** rng.uniform(-8, 8, (r, 1))
+        z[np.arange(n), np.arange(n)] *= 1e3
+    if kind == "extreme":
+        z = np.full((n, n), 1 - 2.0 ** -24) * (1 + 1j)
+        x = np.full((r, n), -(1 - 2.0 ** -24)) * (1 - 1j)
+        z[1::3] *= 2.0 ** -60
+        x[1::2] *= 2.0 ** 50
+        z[2::5] *= 0.0
+    z, x = z.astype(np.complex64), x.astype(np.complex64)
+    y = _run(ctx, z, x)
+    zd, xd = z.astype(np.complex128), x.astype(np.complex128)
+    for f, s in [(0, 0), (n - 1, r - 1), (n // 2, r // 2), (127, 0), (min(128, n - 1), r - 1), (1, min(1, r - 1)), (n - 2, r // 3)]:
+        re, im = _exact(zd[f], xd[s])
+        big = max(abs(zd[f].real).max(), abs(zd[f].imag).max()), max(abs(xd[s].real).max(), abs(xd[s].imag).max())
+        tol = Fraction(2 * n * 4) * Fraction(big[0]) * Fraction(big[1]) / 2 ** 28
+        for got, want in ((y[s, f].real, re), (y[s, f].imag, im)):
+            assert abs(Fraction(float(got)) - want) <= tol + abs(want) / 2 ** 23 + Fraction(1, 2 ** 148), (f, s, got, float(want))
+
+
+def test_fp32_slice_product_keeps_infinities_and_nans(ctx):
+    rng = np.random.default_rng(8)
+    z, x = _cplx(rng, 300, 300).astype(np.complex64), _cplx(rng, 20, 300).astype(np.complex64)
+    z[7, 11] = np.inf
+    z[130, 0] = complex(0, np.nan)
+    x[3, 5] = complex(-np.inf, 0)
+    x[17, 299] = np.nan
+    a, b = _run(ctx, z, x), _run(ctx, z, x, "f32")
+    for p in (np.real, np.imag):
+        assert np.array_equal(np.isnan(p(a)), np.isnan(p(b)))
+        assert np.array_equal(np.isposinf(p(a)), np.isposinf(p(b))) and np.array_equal(np.isneginf(p(a)), np.isneginf(p(b)))
+    ok = np.isfinite(b)
+    assert ok.sum() > 290 * 17
+    assert np.abs(a[ok] - b[ok]).max() <= 1e-3
