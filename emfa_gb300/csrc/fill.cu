@@ -132,10 +132,28 @@ __device__ static Cx<double> efie_sigma(const V3<double>* v, V3<double> vf, V3<d
     return cx(c.pi * c.sig_im / den * acc, -c.pi * c.sig_re / den * acc);
 }
 
+// Edge term of the CFIE self pair at quadrature point p and edge i: the
+// distance P0 of the point from the edge and log((R+ + L+)/(R- + L-)), which
+// depend on neither RWG: one evaluation serves the triangle's 9 (test edge,
+// source edge) pairs.
+__device__ static double2 cfie_edge_term(const V3<double>* v, int p, int i)
+{
+    V3<double> g[3];
+    gauss3(v[0], v[1], v[2], g);
+    V3<double> a = v[(i + 1) % 3], b = v[i];
+    V3<double> L = normalized(a - b);
+    double Lp = dot(a - g[p], L), Lm = dot(b - g[p], L);
+    double Rp = norm(a - g[p]), Rm = norm(b - g[p]);
+    V3<double> sj0 = b + L * dot(g[p] - b, L);
+    double P0 = norm(sj0 - g[p]);
+    return make_double2(P0, P0 > 1e-10 ? log((Rp + Lp) / (Rm + Lm)) : 0.0);
+}
+
 // CFIE self term (Miscellaneous.cpp:32-77), unsigned, complete with the
 // alpha / (1 - alpha) combination.  The edge-log term reuses the source
 // rho of the last inner quadrature point, as the reference does.
-__device__ static Cx<double> cfie_self(const V3<double>* v, V3<double> vf, V3<double> vs, const SingConst& c)
+__device__ static Cx<double> cfie_self(const V3<double>* v, V3<double> vf, V3<double> vs, const SingConst& c,
+                                       const double2 (*edge)[3])
 {
     V3<double> g[3];
     gauss3(v[0], v[1], v[2], g);
@@ -153,13 +171,8 @@ __device__ static Cx<double> cfie_self(const V3<double>* v, V3<double> vf, V3<do
             ze1 = ze1 + coff * (c.w * c.w * (0.25 * dot(rf, rs) - c.inv_k2));
         }
         for (int i = 0; i < 3; ++i) {
-            V3<double> a = v[(i + 1) % 3], b = v[i];
-            V3<double> L = normalized(a - b);
-            double Lp = dot(a - g[p], L), Lm = dot(b - g[p], L);
-            double Rp = norm(a - g[p]), Rm = norm(b - g[p]);
-            V3<double> sj0 = b + L * dot(g[p] - b, L);
-            double P0 = norm(sj0 - g[p]);
-            if (P0 > 1e-10) ze2 += c.w * (0.25 * dot(rf, rs) - c.inv_k2) * P0 * log((Rp + Lp) / (Rm + Lm));
+            const double2 e = edge[p][i];
+            if (e.x > 1e-10) ze2 += c.w * (0.25 * dot(rf, rs) - c.inv_k2) * e.x * e.y;
         }
         zm += c.w * dot(g[p] - vf, g[p] - vs);
     }
@@ -173,13 +186,16 @@ __device__ static Cx<double> cfie_self(const V3<double>* v, V3<double> vf, V3<do
 
 // table layout per (t, ef, es): EFIE {A_direct, A_proj, B_sigma}, CFIE {S}.
 // A CTA of SING_TRIS triangles x 9 (ef, es) threads; for EFIE, 6 threads of
-// each triangle first evaluate its edge integrals (3 points x 2 variants).
+// each triangle first evaluate its edge integrals (3 points x 2 variants), for
+// CFIE its 9 threads the edge terms (3 points x 3 edges; each pair evaluating
+// all of them, 28,880 triangles took 0.67 ms, now 0.28).
 constexpr int SING_TRIS = 14;
 __global__ void __launch_bounds__(9 * SING_TRIS) k_singular_table(const double* __restrict__ vd,
                                                                   const int* __restrict__ tris, int nt,
                                                                   SingConst c, double2* __restrict__ tab)
 {
-    __shared__ double sIs[SING_TRIS][2][3][4];  // [triangle][variant][point][Is1 xyz, Is2]
+    __shared__ double sIs[SING_TRIS][2][3][4];  // EFIE [triangle][variant][point][Is1 xyz, Is2]
+    __shared__ double2 sEdge[SING_TRIS][3][3];  // CFIE [triangle][point][edge]
     const int tl = threadIdx.x / 9, combo = threadIdx.x % 9;
     const int t = blockIdx.x * SING_TRIS + tl;
     const bool valid = t < nt;
@@ -200,13 +216,15 @@ __global__ void __launch_bounds__(9 * SING_TRIS) k_singular_table(const double* 
             o[2] = Is1.z;
             o[3] = Is2;
         }
-        __syncthreads();
+    } else if (valid) {
+        sEdge[tl][combo / 3][combo % 3] = cfie_edge_term(v, combo / 3, combo % 3);
     }
+    __syncthreads();
     if (!valid) return;
     const int id = 9 * t + combo, ef = combo / 3, es = combo % 3;
     V3<double> vf = v[ef], vs = v[es];
     if (c.cfie) {
-        Cx<double> s = cfie_self(v, vf, vs, c);
+        Cx<double> s = cfie_self(v, vf, vs, c, sEdge[tl]);
         tab[id] = make_double2(s.re, s.im);
     } else {
         Cx<double> a = efie_self(v, vf, vs, c, sIs[tl][0]);

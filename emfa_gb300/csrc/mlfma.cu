@@ -281,29 +281,29 @@ __global__ void k_radrec(const RwgPack<float>* __restrict__ rw, const int* __res
     rec[id] = C2f{proj(q, e), proj(q, e + 3)};
 }
 
-// near-field blocks: thread per (field unknown, near-slot); values row-major
-// per field box over the concatenated near-box columns
-__global__ void k_near_fill(const RwgPack<float>* __restrict__ rw, const int* __restrict__ perm,
-                            const int* __restrict__ box_of, const int* __restrict__ box_off,
-                            const int* __restrict__ box_cnt, const int* __restrict__ near_ptr,
-                            const int* __restrict__ near_box, const int* __restrict__ near_col,
-                            const int* __restrict__ row_cols, const size_t* __restrict__ row_base, int n,
-                            int max_near, FillConst<float> fc, const double2* __restrict__ sing,
-                            float2* __restrict__ val)
+// near-field blocks, row-major per field box over the concatenated near-box
+// columns: a warp per field unknown, lanes over the columns (near_cidx), so that
+// the row is stored coalesced and the lanes share the work whatever the boxes'
+// sizes.  Bound by FP32 issue.  With a thread per (unknown, near box), idle
+// beyond a box's own near boxes and as slow as the largest one of its warp,
+// 43,320 unknowns took 1.59 ms; now 0.76.
+__global__ void __launch_bounds__(128) k_near_fill(const RwgPack<float>* __restrict__ rw, const int* __restrict__ perm,
+                                                   const int* __restrict__ box_of, const int* __restrict__ box_off,
+                                                   const int* __restrict__ row_cols,
+                                                   const size_t* __restrict__ row_base,
+                                                   const int* __restrict__ near_cbase,
+                                                   const int* __restrict__ near_cidx, int n, FillConst<float> fc,
+                                                   const double2* __restrict__ sing, float2* __restrict__ val)
 {
-    size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= (size_t)n * max_near) return;
-    const int u = (int)(id / max_near), j = (int)(id % max_near);
-    const int b = box_of[u];
-    const int slot = near_ptr[b] + j;
-    if (slot >= near_ptr[b + 1]) return;
-    const int nb = near_box[slot];
-    const int s0 = box_off[nb], ns = box_cnt[nb];
-    const RwgPack<float> F = rw[perm[u]];
-    float2* out = val + row_base[b] + (size_t)(u - box_off[b]) * row_cols[b] + near_col[slot];
-    for (int q = 0; q < ns; ++q) {
-        Cx<float> z = z_entry<float, true>(F, rw[perm[s0 + q]], fc, sing);
-        out[q] = make_float2(z.re, z.im);
+    const int u = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (u >= n) return;
+    const int b = box_of[u], rc = row_cols[b];
+    const int* ci = near_cidx + near_cbase[b];
+    const RwgPack<float>& F = rw[perm[u]];
+    float2* out = val + row_base[b] + (size_t)(u - box_off[b]) * rc;
+    for (int j = lane; j < rc; j += 32) {
+        const Cx<float> z = z_entry<float, true>(F, rw[perm[ci[j]]], fc, sing);
+        out[j] = make_float2(z.re, z.im);
     }
 }
 
@@ -997,10 +997,14 @@ __global__ void __launch_bounds__(128) k_sai(const int* __restrict__ rptr, const
 }
 
 // translation operator of every far-box offset at every sample (FP64, the
-// host recurrences of parallelLevelTrans, MLFMA.cpp:1191-1222): thread per
-// (offset, sample); hl holds each offset's spherical Hankel values
-__global__ void k_trans_table(const double2* __restrict__ hl, const int* __restrict__ minl, int lmax,
-                              const float* __restrict__ kd, int K, double len, float2* __restrict__ tr)
+// series of parallelLevelTrans, MLFMA.cpp:1191-1222): thread per (offset,
+// sample); cf holds each offset's (2q+1)(-j)^q h_q, rec the Legendre
+// recurrence's (2q-1)/q and (q-1)/q.  Bound by the FP64 pipe: five instructions
+// a term (with the division by q and the products in the loop, the levels of
+// 43,320 unknowns took 1.12 ms; now 0.34).
+__global__ void k_trans_table(const double2* __restrict__ cf, const double2* __restrict__ rec,
+                              const int* __restrict__ minl, int lmax, const float* __restrict__ kd, int K, double len,
+                              float2* __restrict__ tr)
 {
     const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= (size_t)343 * K) return;
@@ -1014,27 +1018,19 @@ __global__ void k_trans_table(const double2* __restrict__ hl, const int* __restr
     const double D0 = dx * len, D1 = dy * len, D2 = dz * len;
     const double Dn = sqrt(D0 * D0 + D1 * D1 + D2 * D2);
     const double ct = ((double)kd[3 * kk] * D0 + (double)kd[3 * kk + 1] * D1 + (double)kd[3 * kk + 2] * D2) / Dn;
-    const double2* h = hl + (size_t)off * (lmax + 1);
-    double vr = 0.0, vi = 0.0, p0 = 1.0, p1 = ct;
-    for (int q = 0; q <= ml; ++q) {
-        double Pq = q == 0 ? 1.0 : ct;
-        if (q >= 2) {
-            Pq = ((2 * q - 1) * ct * p1 - (q - 1) * p0) / q;
-            p0 = p1;
-            p1 = Pq;
-        }
-        // (2q+1) (-j)^q h_q P_q
-        const double2 hq = h[q];
-        double ar, ai;
-        switch (q & 3) {
-            case 0: ar = hq.x; ai = hq.y; break;
-            case 1: ar = hq.y; ai = -hq.x; break;
-            case 2: ar = -hq.x; ai = -hq.y; break;
-            default: ar = -hq.y; ai = hq.x; break;
-        }
-        const double w = (2.0 * q + 1) * Pq;
-        vr += w * ar;
-        vi += w * ai;
+    const double2* c = cf + (size_t)off * (lmax + 1);
+    double vr = c[0].x, vi = c[0].y, p0 = 1.0, p1 = ct;
+    if (ml >= 1) {
+        vr = fma(ct, c[1].x, vr);
+        vi = fma(ct, c[1].y, vi);
+    }
+    for (int q = 2; q <= ml; ++q) {
+        const double2 ab = rec[q], cq = c[q];
+        const double P = fma(ab.x, ct * p1, -(ab.y * p0));
+        p0 = p1;
+        p1 = P;
+        vr = fma(P, cq.x, vr);
+        vi = fma(P, cq.y, vi);
     }
     tr[id] = make_float2((float)vr, (float)vi);
 }
@@ -1475,17 +1471,27 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                         if (minL >= 1)
                             hl[1] = std::complex<double>(std::sin(x) / x - std::cos(x), std::cos(x) / x + std::sin(x)) / x;
                         for (int q = 2; q <= minL; ++q) hl[q] = ((2.0 * q - 1) / x) * hl[q - 1] - hl[q - 2];
-                        for (int q = 0; q <= minL; ++q)
-                            hlv[(size_t)off * (lmax + 1) + q] = make_double2(hl[q].real(), hl[q].imag());
+                        for (int q = 0; q <= minL; ++q) {
+                            // (2q+1) (-j)^q h_q
+                            const double w = 2.0 * q + 1, hr = w * hl[q].real(), hi = w * hl[q].imag();
+                            hlv[(size_t)off * (lmax + 1) + q] = (q & 3) == 0   ? make_double2(hr, hi)
+                                                                : (q & 3) == 1 ? make_double2(hi, -hr)
+                                                                : (q & 3) == 2 ? make_double2(-hr, -hi)
+                                                                               : make_double2(-hi, hr);
+                        }
                         minl[off] = minL;
                     }
-            DevBuf d_hl, d_minl, d_kd;
+            std::vector<double2> recv(lmax + 1, make_double2(0, 0));
+            for (int q = 1; q <= lmax; ++q) recv[q] = make_double2((2.0 * q - 1) / q, (q - 1.0) / q);
+            DevBuf d_hl, d_rec, d_minl, d_kd;
             EMFA_TRY(upload(c, d_hl, hlv, st));
+            EMFA_TRY(upload(c, d_rec, recv, st));
             EMFA_TRY(upload(c, d_minl, minl, st));
             EMFA_TRY(upload(c, d_kd, kd[i], st));
             EMFA_TRY(ml.trans.alloc(c, sizeof(float2) * (size_t)343 * K));
             const size_t tot = (size_t)343 * K;
-            k_trans_table<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(dptr<double2>(d_hl), dptr<int>(d_minl), lmax,
+            k_trans_table<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(dptr<double2>(d_hl), dptr<double2>(d_rec),
+                                                                         dptr<int>(d_minl), lmax,
                                                                          dptr<float>(d_kd), K, (double)ml.len,
                                                                          dptr<float2>(ml.trans));
             c->kernel_launches += 1;
@@ -1677,7 +1683,6 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     std::vector<int> nptr{0}, nbox, ncol, rcols;
     std::vector<size_t> rbase;
     size_t nnz = 0;
-    int max_near = 0;
     for (size_t b = 0; b < fin.size(); ++b) {
         int cols = 0;
         for (int nb : fin[b].near) {
@@ -1686,7 +1691,6 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
             cols += (int)fin[nb].unk.size();
         }
         nptr.push_back((int)nbox.size());
-        max_near = std::max(max_near, (int)fin[b].near.size());
         rcols.push_back(cols);
         M->max_cols = std::max(M->max_cols, cols);
         rbase.push_back(nnz);
@@ -1716,12 +1720,10 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         EMFA_TRY(tab.alloc(c, sizeof(double2) * (size_t)g->nt * 9));
         EMFA_TRY(build_singular_table(c, g, &fp, dptr<double2>(tab), st));
         FillConst<float> fc = make_fill_const<float>(&fp);
-        size_t tot = (size_t)n * max_near;
-        k_near_fill<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(
+        k_near_fill<<<(unsigned)(((size_t)n * 32 + 127) / 128), 128, 0, st>>>(
             dptr<RwgPack<float>>(g->g32.rwg), dptr<int>(M->perm_d), dptr<int>(M->box_of), dptr<int>(M->box_off),
-            dptr<int>(M->box_cnt), dptr<int>(M->near_ptr), dptr<int>(M->near_box), dptr<int>(M->near_col),
-            dptr<int>(M->row_cols), dptr<size_t>(M->row_base), n, max_near, fc, dptr<double2>(tab),
-            dptr<float2>(M->near_val));
+            dptr<int>(M->row_cols), dptr<size_t>(M->row_base), dptr<int>(M->near_cbase), dptr<int>(M->near_cidx), n,
+            fc, dptr<double2>(tab), dptr<float2>(M->near_val));
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
         EMFA_CUDA(c, cudaStreamSynchronize(st));
