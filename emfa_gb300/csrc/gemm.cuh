@@ -59,6 +59,7 @@ struct HPack {
     float* inv_t = nullptr;
     size_t ldh = 0;
     const int* skip = nullptr;  // optional: a device int; zero when the product starts skips it
+    int* seen = nullptr;        // optional, with skip: a page-locked host word that gets *skip
 };
 emfa_status_t hgemm_pack_target(Ctx* c, const HPlanes& h, int nrhs, HPack* out);
 emfa_status_t hgemm_apply_packed(Ctx* c, const HPlanes& h, const HPack& p, void* Y, int nrhs, cudaStream_t st);

@@ -69,20 +69,16 @@ template <int BN, int MS>
 __global__ void __launch_bounds__(THREADS, 1)
     k_hgemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             float2* __restrict__ Y, int M, int R, int kblocks, const float* __restrict__ inv_s,
-            const float* __restrict__ inv_t, int* __restrict__ err, const int* __restrict__ skip)
+            const float* __restrict__ inv_t, int* __restrict__ err, const int* __restrict__ skip,
+            int* __restrict__ seen)
 {
     using S = Smem<BN, MS>;
     using namespace tc;
     // one wave: every CTA is resident, so the next launch (the Gram-Schmidt
     // coefficients) may be scheduled beside it at once and wait for its end
     griddep_launch();
-    // launched as a dependent (the Krylov loop's products): the step that
-    // packed B and counted the active right-hand sides must have finished
-    griddep_wait();
-    // no right-hand side left active (the Krylov step queued after the last
-    // one): the same value in every thread, before any barrier or allocation
-    if (skip && *skip == 0) return;
     extern __shared__ uint8_t smem_raw[];
+    __shared__ float s_it[BN / 2];  // inv_s inv_t of the tile's right-hand sides
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sA = base;                               // [stage][row block]
     uint8_t* sB = base + S::STAGES * MS * S::A_BYTES;  // [stage]
@@ -116,13 +112,28 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
+    // Launched as a dependent (the Krylov loop's products), the step that
+    // packed B and counted the active right-hand sides must have finished:
+    // each role waits for it (griddep_wait) where it first needs its results.
+    // The barriers, the tensor memory and the first stages' tiles of the
+    // plane A, which no step writes, do not wait.  *skip == 0: no right-hand
+    // side is left active (the Krylov step queued after the last one).
     if (warp == 0) {
         if (lane == 0) {
-            int issued = 0;
-            for (int kb = 0; kb < kblocks; ++kb) {
+            const int pre = kblocks < S::STAGES ? kblocks : S::STAGES;
+            for (int kb = 0; kb < pre; ++kb) {
+                mbar_expect_tx(full + kb, S::STAGE_BYTES);
+#pragma unroll
+                for (int m = 0; m < MS; ++m)
+                    tma_load_2d(sA + (kb * MS + m) * S::A_BYTES, &tmA, full + kb, kb * BKH, f0 + m * BM);
+            }
+            griddep_wait();
+            for (int kb = 0; kb < pre; ++kb) tma_load_2d(sB + kb * S::B_BYTES, &tmB, full + kb, kb * BKH, c0);
+            const int kend = skip && *(volatile const int*)skip == 0 ? pre : kblocks;
+            int issued = pre;
+            for (int kb = pre; kb < kend; ++kb) {
                 const int s = kb % S::STAGES;
-                if (kb >= S::STAGES && !mbar_wait(empty + s, ((kb / S::STAGES) - 1) & 1, err, 1)) break;
-                if (*(volatile int*)err) break;
+                if (!mbar_wait(empty + s, ((kb / S::STAGES) - 1) & 1, err, 1)) break;
                 mbar_expect_tx(full + s, S::STAGE_BYTES);
 #pragma unroll
                 for (int m = 0; m < MS; ++m)
@@ -135,7 +146,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 mbar_wait(full + (kb % S::STAGES), (kb / S::STAGES) & 1, err, 2);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        griddep_wait();
+        if (lane == 0 && !(skip && *(volatile const int*)skip == 0)) {
             constexpr uint32_t idesc = idesc_f16(BM, BN);
             for (int kb = 0; kb < kblocks; ++kb) {
                 const int s = kb % S::STAGES;
@@ -160,19 +172,25 @@ __global__ void __launch_bounds__(THREADS, 1)
         __syncwarp();
     } else {
         // epilogue warps 2..5: lane quadrant (warp % 4) of tensor memory
-        const int q = warp & 3;
-        int ok = lane == 0 ? (int)mbar_wait(accum, 0, err, 5) : 0;
+        const int q = warp & 3, et = threadIdx.x - 64;
+        griddep_wait();
+        const int left = skip ? *(volatile const int*)skip : 1;
+        // the host follows the count of active right-hand sides from here, a
+        // step late, with no copy or event between the step and this product
+        if (seen && et == 0 && blockIdx.x == 0 && blockIdx.y == 0) *(volatile int*)seen = left;
+        if (et < BN / 2) s_it[et] = c0 / 2 + et < R ? *inv_s * inv_t[c0 / 2 + et] : 0.f;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        int ok = lane == 0 && left ? (int)mbar_wait(accum, 0, err, 5) : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float is = *inv_s;
             // 48 columns a round trip where BN allows (144 = 3 x 48), else 16
             constexpr int CW = BN % 48 == 0 ? 48 : 16;
 #pragma unroll 1
             for (int m = 0; m < MS; ++m) {
                 const int f = f0 + m * BM + 32 * q + lane;
 #pragma unroll 1
-                for (int c = 0; c < BN; c += CW) {
+                for (int c = 0; c < BN && c0 + c < 2 * R; c += CW) {
                     float v[CW];
                     if constexpr (CW == 48)
                         tmem_ld48(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(m * S::ACC + c), v);
@@ -183,7 +201,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         for (int i = 0; i < CW / 2; ++i) {
                             const int r = (c0 + c) / 2 + i;
                             if (r < R) {
-                                const float sc = is * inv_t[r];
+                                const float sc = s_it[c / 2 + i];
                                 Y[(size_t)r * M + f] = make_float2(v[2 * i] * sc, v[2 * i + 1] * sc);
                             }
                         }
@@ -467,7 +485,6 @@ __global__ void __launch_bounds__(RTHREADS, 1)
             for (int kb = 0; kb < kblocks; ++kb) {
                 const int s = kb % S::STAGES;
                 if (kb >= S::STAGES && !mbar_wait(empty + s, ((kb / S::STAGES) - 1) & 1, err, 11)) break;
-                if (*(volatile int*)err) break;
                 mbar_expect_tx(full + s, S::STAGE_BYTES);
                 tma_load_2d(sA + (2 * s) * S::A_BYTES, &tmA0, full + s, kb * BKH, f0);
                 tma_load_2d(sA + (2 * s + 1) * S::A_BYTES, &tmA1, full + s, kb * BKH, f0);
@@ -633,7 +650,7 @@ static emfa_status_t make_map_h(Ctx* c, CUtensorMap* m, const void* ptr, uint64_
 template <int BN, int MS>
 static emfa_status_t launch_h(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, float2* Y, int n, int nrhs,
                               const float* inv_s, const float* inv_t, int* err, cudaStream_t st, bool timed,
-                              const int* skip)
+                              const int* skip, int* seen)
 {
     using S = th::Smem<BN, MS>;
     EMFA_TRY(ensure_smem(c, th::k_hgemm<BN, MS>, S::TOTAL));
@@ -642,14 +659,15 @@ static emfa_status_t launch_h(Ctx* c, const CUtensorMap& ta, const CUtensorMap& 
     if (timed && !skip) {
         TimedLaunch tl(c, KT_GEMM, st, 8.0 * n * (double)n * nrhs);
         th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, n, nrhs, kblocks, inv_s, inv_t, err,
-                                                                  nullptr);
+                                                                  nullptr, nullptr);
     } else if (skip) {
         // the Krylov loop's product: scheduled while the step that packed its
         // operand drains (programmatic dependent launch)
         EMFA_CUDA(c, launch_dependent(th::k_hgemm<BN, MS>, grd, dim3(th::THREADS), (size_t)S::TOTAL, st, ta, tb, Y, n,
-                                      nrhs, kblocks, inv_s, inv_t, err, skip));
+                                      nrhs, kblocks, inv_s, inv_t, err, skip, seen));
     } else {
-        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, n, nrhs, kblocks, inv_s, inv_t, err, skip);
+        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, n, nrhs, kblocks, inv_s, inv_t, err, skip,
+                                                                  nullptr);
     }
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
@@ -737,13 +755,13 @@ static int fixed_variant(int n, int nrhs, int sms)
 
 static emfa_status_t launch_variant(Ctx* c, int v, const CUtensorMap& ta, const CUtensorMap* tb, float2* Y, int n,
                                     int nrhs, const float* inv_s, const float* inv_t, int* err, cudaStream_t st,
-                                    bool timed, const int* skip = nullptr)
+                                    bool timed, const int* skip = nullptr, int* seen = nullptr)
 {
     switch (v) {
-    case HV_64_1: return launch_h<64, 1>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip);
-    case HV_64_2: return launch_h<64, 2>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip);
-    case HV_144_1: return launch_h<144, 1>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip);
-    default: return launch_h<144, 2>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip);
+    case HV_64_1: return launch_h<64, 1>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    case HV_64_2: return launch_h<64, 2>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    case HV_144_1: return launch_h<144, 1>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    default: return launch_h<144, 2>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     }
 }
 
@@ -796,7 +814,7 @@ static emfa_status_t tune_variants(Ctx* c, const TuneKey& key, const CUtensorMap
 // the inner-product GEMM on an already packed B plane; skip (optional): an
 // int that, if zero when the product starts, skips it
 static emfa_status_t hgemm_run(Ctx* c, const HPlanes& h, const __half* bh, const float* inv_t, void* Y, int nrhs,
-                               int* err, cudaStream_t st, const int* skip = nullptr)
+                               int* err, cudaStream_t st, const int* skip = nullptr, int* seen = nullptr)
 {
     const int n = h.n;
     const size_t ldh = h.ldh;
@@ -818,7 +836,7 @@ static emfa_status_t hgemm_run(Ctx* c, const HPlanes& h, const __half* bh, const
         if (known < 0 && !skip) return tune_variants(c, key, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st);
         if (known >= 0) v = known;
     }
-    return launch_variant(c, v, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st, true, skip);
+    return launch_variant(c, v, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st, true, skip, seen);
 }
 
 emfa_status_t hgemm_tuned_shape(int device, int n, int nrhs, int* variant, float* ms)
@@ -889,7 +907,7 @@ emfa_status_t hgemm_apply_packed(Ctx* c, const HPlanes& h, const HPack& p, void*
 {
     int* err = nullptr;
     EMFA_TRY(herr(c, &err));
-    return hgemm_run(c, h, p.bh, p.inv_t, Y, nrhs, err, st, p.skip);
+    return hgemm_run(c, h, p.bh, p.inv_t, Y, nrhs, err, st, p.skip, p.seen);
 }
 
 emfa_status_t hgemm_pack(Ctx* c, const HPlanes& h, const void* X, const HPack& p, int nrhs, cudaStream_t st)

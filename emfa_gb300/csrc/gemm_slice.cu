@@ -240,10 +240,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                         ok = false;
                         break;
                     }
-                    if (*(volatile int*)err) {
-                        ok = false;
-                        break;
-                    }
                     mbar_expect_tx(a_full + s, S::A_BYTES);
                     tma_load_3d(sA + s * S::A_BYTES, &tmA, a_full + s, (k0 + kb) * BK, f0, i);
                     ++na;

@@ -91,7 +91,6 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int kb = 0; kb < kblocks; ++kb) {
                 const int s = kb % STAGES;
                 if (kb >= STAGES && !mbar_wait(empty + s, ((kb / STAGES) - 1) & 1, err, 1)) break;
-                if (*(volatile int*)err) break;
                 mbar_expect_tx(full + s, S::STAGE_BYTES);
                 tma_load_2d(sA + s * S::A_BYTES, &tmA, full + s, kb * BK, f0);
                 tma_load_2d(sB + s * S::B_BYTES, &tmB, full + s, kb * BK, c0);

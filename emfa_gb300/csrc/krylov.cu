@@ -1268,14 +1268,26 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
 
     const int r = blockIdx.y, rank = blockIdx.x, csize = gridDim.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (!s.active[r]) {  // the same branch in every CTA of the cluster: no barrier is left waiting
-        if (rank == 0 && tid == 0) s.scale[r] = 0.0;
-        return;
-    }
     const int nv = j + 1;
     const int k0 = rank * slice, len = min(n, k0 + slice) - k0;  // len >= 1 for every rank
     const float2* Vs = V + (size_t)r * n + k0;                    // this slice of basis vector 0
     const float2* Ws = W + (size_t)r * n + k0;
+
+    // Launched as a dependent of the product.  The product's CTAs start when
+    // every CTA of the last step is past its own wait, that is after the step
+    // before the last has finished: V_0 .. V_{j-1} may be read before the
+    // wait, V_j (the last step's) and W only after it.
+    const int ahead = min(j, sv);
+    for (int i = 0; i < ahead; ++i)
+        for (int k = tid; k < len; k += AS_THREADS) cp_async8(sV + (size_t)i * SW + k, Vs + (size_t)i * vstride + k);
+    griddep_wait();
+    griddep_launch();
+    if (rank == 0 && r == 0 && tid == 0) *s.step_next = 0;
+    if (!s.active[r]) {  // the same branch in every CTA of the cluster: no barrier is left waiting
+        if (rank == 0 && tid == 0) s.scale[r] = 0.0;
+        cp_async_wait_all();
+        return;
+    }
 
     // 1. partial coefficients.  Each round stages (asynchronous copies, all
     // in flight at once) up to sv basis slices, and w in the first; warp q
@@ -1287,7 +1299,7 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
         if (v0 > 0) __syncthreads();  // the previous round's reads are done
         if (v0 == 0)
             for (int k = tid; k < len; k += AS_THREADS) cp_async8(sW + k, Ws + k);
-        for (int i = v0; i < v1; ++i)
+        for (int i = v0 > 0 ? v0 : ahead; i < v1; ++i)
             for (int k = tid; k < len; k += AS_THREADS) cp_async8(sV + (size_t)(i - v0) * SW + k, Vs + (size_t)i * vstride + k);
         cp_async_wait_all();
         __syncthreads();
@@ -1625,13 +1637,15 @@ static emfa_status_t launch_step_e(Ctx* c, const StepShape& sh, int nrhs, cudaSt
     cfg.blockDim = dim3(AS_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = sh.cs;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     EMFA_CUDA(c, cudaLaunchKernelEx(&cfg, k_arnoldi_step<E>, s, j, V, vstride, W, n, sh.slice, sv, Vout, pk));
     return EMFA_OK;
 }
@@ -1698,7 +1712,7 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                         Carver::round(sizeof(double2) * (size_t)nrhs * (m + 1) * std::max(nblk, vblk)) +
                         Carver::round(sizeof(double2) * (size_t)nrhs * std::max(nblk, vblk)) +
                         Carver::round(sizeof(double) * 5 * (size_t)nrhs) + Carver::round(sizeof(int) * 2 * (size_t)nrhs) +
-                        Carver::round(sizeof(int) * 4) + 4096;
+                        Carver::round(sizeof(int) * 8) + 4096;
     void* wsp = nullptr;
     EMFA_TRY(ctx_workspace(c, WS_KRYLOV, need, &wsp));
     Carver cv{(char*)wsp};
@@ -1736,7 +1750,7 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     s.wmax = s.true_res + nrhs;
     s.jlen = cv.take<int>(2 * (size_t)nrhs);
     s.active = s.jlen + nrhs;
-    s.counters = cv.take<int>(4);
+    s.counters = cv.take<int>(8);
 
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -1749,10 +1763,14 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     int host_cnt[4];
     // Arnoldi steps are checked one step late: step j and the operator
     // application for step j + 1 are queued before the host reads step j-1's
-    // count of active right-hand sides (a page-locked word behind an event),
-    // so the device never waits for the host between steps.  The step queued
-    // after the last active one does nothing for converged right-hand sides
-    // (k_arnoldi_finish skips them).
+    // count of active right-hand sides, so the device never waits for the
+    // host between steps.  The count reaches the host in a page-locked word
+    // that the next product writes, or, for operators that cannot, by a copy
+    // on a side stream behind an event (an event and a memset between the
+    // launches of a step also kept them from overlapping: 22-27 us a step of
+    // one right-hand side at N = 480 that way, @STEP@ us now).  The step
+    // queued after the last active one does nothing for converged right-hand
+    // sides (k_arnoldi_finish skips them).
     struct StepEvents {
         cudaEvent_t e[2] = {nullptr, nullptr};     // the host's copy of a step's count has landed
         cudaEvent_t done[2] = {nullptr, nullptr};  // a step's kernels have finished (main stream)
@@ -1768,11 +1786,31 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             for (auto x : done)
                 if (x) cudaEventDestroy(x);
         }
+        cudaError_t create()
+        {
+            cudaError_t x = cudaSuccess;
+            for (auto* a : {e, done})
+                for (int i = 0; i < 2 && x == cudaSuccess; ++i)
+                    x = cudaEventCreateWithFlags(a + i, cudaEventDisableTiming);
+            return x == cudaSuccess ? cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) : x;
+        }
     } sev;
-    for (auto& x : sev.e) EMFA_CUDA(c, cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
-    for (auto& x : sev.done) EMFA_CUDA(c, cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
-    EMFA_CUDA(c, cudaStreamCreateWithFlags(&sev.side, cudaStreamNonBlocking));
     volatile int* slot = c->pinned;
+    // the word a product writes: -1 until it has run.  The stream is asked
+    // now and then, so that a failed launch ends the wait.
+    auto await_count = [&](volatile int* w) -> emfa_status_t {
+        for (long spin = 1; *w < 0; ++spin) {
+            if (spin & 0xfff) continue;
+            const cudaError_t q = cudaStreamQuery(st);
+            if (q == cudaErrorNotReady) continue;
+            EMFA_CUDA(c, q);
+            if (*w < 0) {
+                set_error(c, "the product left no count of active right-hand sides");
+                return EMFA_ERR_CUDA;
+            }
+        }
+        return EMFA_OK;
+    };
     for (int cyc = 0; cyc < max_cycles; ++cyc) {
         // true residual R = B - Z X (X = 0 on the first cycle: R = B)
         if (cyc == 0) {
@@ -1784,7 +1822,7 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             EMFA_TRY(A.residual(c, X, B, R, nrhs, Xt, st));
         }
         k_norm2<std::is_same<T, float>::value><<<dim3(nblk, nrhs), KB, 0, st>>>(R, n, nblk, chunk, pnorm);
-        EMFA_CUDA(c, cudaMemsetAsync(s.counters, 0, sizeof(int) * 4, st));
+        EMFA_CUDA(c, cudaMemsetAsync(s.counters, 0, sizeof(int) * 8, st));
         k_cycle_init<<<(nrhs + 127) / 128, 128, 0, st>>>(s, pnorm, nblk, cyc == 0);
         EMFA_CUDA(c, cudaMemcpyAsync(host_cnt, s.counters, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
         EMFA_CUDA(c, cudaStreamSynchronize(st));
@@ -1806,7 +1844,8 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             // (h2 = V^H W; W -= V h2) and H gets h + h2.
             const dim3 vg(vblk, nrhs);
             const int nv = j + 1;
-            s.step_cnt = s.counters + 2 + (j & 1);
+            s.step_cnt = s.counters + 2 + j % 3;
+            s.step_next = s.counters + 2 + (j + 1) % 3;
             HPack pk;
             bool packs = false;
             // the step normalises V_{j+1} itself (fused, or separate passes
@@ -1824,7 +1863,6 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             }
             if (fused) {
                 // V_{j+1} and the next product's operand come out of the step
-                EMFA_CUDA(c, cudaMemsetAsync(s.step_cnt, 0, sizeof(int), st));
                 EMFA_TRY(launch_arnoldi_step(c, sh, nrhs, st, s, j, (const float2*)V, vec, (const float2*)W, n,
                                              (float2*)(V + (size_t)(j + 1) * vec), pk));
                 c->kernel_launches += 1;
@@ -1896,16 +1934,26 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                 c->kernel_launches += 3;
                 }
             }
-            // the host reads the step's count on a side stream, so no copy sits
-            // between this step's last kernel and the next product
-            EMFA_CUDA(c, cudaEventRecord(sev.done[j & 1], st));
-            EMFA_CUDA(c, cudaStreamWaitEvent(sev.side, sev.done[j & 1], 0));
-            EMFA_CUDA(c, cudaMemcpyAsync((void*)(slot + (j & 1)), s.step_cnt, sizeof(int), cudaMemcpyDeviceToHost,
-                                         sev.side));
-            EMFA_CUDA(c, cudaEventRecord(sev.e[j & 1], sev.side));
+            const bool told = normalises && packs;
+            if (told) {
+                pk.seen = const_cast<int*>(slot + (j & 1));
+                slot[j & 1] = -1;
+            } else {
+                // the host reads the step's count on a side stream, so no copy sits
+                // between this step's last kernel and the next product
+                if (!sev.side) EMFA_CUDA(c, sev.create());
+                EMFA_CUDA(c, cudaEventRecord(sev.done[j & 1], st));
+                EMFA_CUDA(c, cudaStreamWaitEvent(sev.side, sev.done[j & 1], 0));
+                EMFA_CUDA(c, cudaMemcpyAsync((void*)(slot + (j & 1)), s.step_cnt, sizeof(int), cudaMemcpyDeviceToHost,
+                                             sev.side));
+                EMFA_CUDA(c, cudaEventRecord(sev.e[j & 1], sev.side));
+            }
             ++steps;
             if (j > 0) {
-                EMFA_CUDA(c, cudaEventSynchronize(sev.e[(j - 1) & 1]));
+                if (told)
+                    EMFA_TRY(await_count(slot + ((j - 1) & 1)));
+                else
+                    EMFA_CUDA(c, cudaEventSynchronize(sev.e[(j - 1) & 1]));
                 if (slot[(j - 1) & 1] == 0) {  // step j (queued) found nothing active
                     --steps;
                     break;

@@ -650,6 +650,7 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
     extern __shared__ uint8_t smem_raw[];
     __shared__ float rs[lutc::TN];  // 1 / s_i of the tile's rows
     __shared__ int eok;
+    __shared__ volatile int stopped;  // a wait of this CTA ran out
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sUh = base;
     uint8_t* sUl = sUh + lutc::U_BYTES;
@@ -666,6 +667,7 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
     const int cc0 = (blockIdx.x + ct0) * 64, r0 = blockIdx.y * lutc::TN;
 
     if (threadIdx.x == 0) {
+        stopped = 0;
         mbar_init(full, 1);
         mbar_init(empty, 1);
         mbar_init(accum, 1);
@@ -690,7 +692,6 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
             int issued = 0;
             for (int s = 0; s < nslices; ++s) {
                 if (s > 0 && !mbar_wait(empty, (s - 1) & 1, err, 11)) break;
-                if (*(volatile int*)err) break;
                 mbar_expect_tx(full, lutc::STAGE);
                 tma_load_2d(sUh, &tmU, full, 64 * s, 2 * cc0);
                 tma_load_2d(sUl, &tmU, full, 64 * s, 2 * n + 2 * cc0);
@@ -705,7 +706,11 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
         if (lane == 0) {
             constexpr uint32_t idesc = idesc_f16(lutc::TM, lutc::TN);
             for (int s = 0; s < nslices; ++s) {
-                if (!mbar_wait(full, s & 1, err, 13)) break;
+                if (!mbar_wait(full, s & 1, err, 13)) {
+                    stopped = 1;
+                    __threadfence_block();
+                    break;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t uh = sw128_desc(smem_u32(sUh)), ul = sw128_desc(smem_u32(sUl));
                 const uint64_t lh = sw128_desc(smem_u32(sLh)), ll = sw128_desc(smem_u32(sLl));
@@ -734,7 +739,7 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
         if (leader) {
             // the operand buffer is free once the MMAs are done
             int ok = (int)mbar_wait(accum, 0, err, 15);
-            if (ok) ok = *(volatile int*)err == 0;
+            if (ok) ok = stopped == 0;
             if (ok)
                 for (int c = 0; c < 3; ++c) {
                     mbar_expect_tx(cfull + c, lutc::C_BYTES);
@@ -750,7 +755,10 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
                 const int slot = c % 3;
                 float* cs = (float*)(base + slot * lutc::C_BYTES);  // [64][128] floats
                 int got = 0;
-                if (lane == 0) got = *(volatile int*)err == 0 && mbar_wait(cfull + slot, c / 3, err, 16);
+                if (lane == 0) {
+                    got = stopped == 0 && mbar_wait(cfull + slot, c / 3, err, 16);
+                    if (!got) stopped = 1;
+                }
                 got = __shfl_sync(0xffffffffu, got, 0);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -767,7 +775,7 @@ __global__ void __launch_bounds__(lutc::THREADS, 2)
                 }
                 fence_proxy_async();
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (leader && *(volatile int*)err == 0) {
+                if (leader && stopped == 0) {
                     tma_store_2d(&tmC, cs, xC, yC + 64 * c);
                     bulk_store_commit();
                     if (c == 0) {
