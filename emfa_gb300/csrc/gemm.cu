@@ -104,18 +104,23 @@ __global__ void __launch_bounds__(256) k_cgemm(const Cx<T>* __restrict__ Z, size
 }
 
 // Few right-hand sides (the 64-wide tile above would leave most of its RHS
-// columns empty): a warp per RPW rows of Z, lanes striding k, up to RB
-// right-hand sides per launch accumulated in registers, then reduced by
-// shuffles.  Each warp reads its rows once (coalesced 512-byte segments for
-// complex128) and the RHS entries from L1/L2; FP64 is bound by the FMA rate.
+// columns empty): a warp per RPW rows of Z, lanes striding k, RB right-hand
+// sides accumulated in registers, then reduced by shuffles.  Each warp reads
+// its rows once (coalesced 512-byte segments for complex128) and the RHS
+// entries from L1/L2.  FP64 is bound by the FMA rate.  FP32 is bound by the
+// latency of its loads, so U steps of k are loaded before any is used and
+// the rows of a warp are few where the warps would be (rpw_f32).  A sum's
+// terms and their order depend on none of RB, RPW and U.
 template <typename T, int RB, int RPW>
 __global__ void __launch_bounds__(256) k_cgemv(const Cx<T>* __restrict__ Z, size_t ldz, const Cx<T>* __restrict__ X,
                                                int n, int nrhs, Cx<T>* __restrict__ Y)
 {
+    constexpr int U = sizeof(T) == 8 ? 1 : RPW * RB >= 16 ? 2 : 4;
     const int warp = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int f0 = warp * RPW;
     if (f0 >= n) return;
-    // block blockIdx.y of RB right-hand sides
+    // block blockIdx.y of RB right-hand sides; the last may be short: its
+    // missing columns repeat the last one and are not stored
     X += (size_t)blockIdx.y * RB * n;
     Y += (size_t)blockIdx.y * RB * n;
     nrhs = min(RB, nrhs - (int)blockIdx.y * RB);
@@ -124,22 +129,45 @@ __global__ void __launch_bounds__(256) k_cgemv(const Cx<T>* __restrict__ Z, size
     for (int i = 0; i < RPW; ++i)
 #pragma unroll
         for (int r = 0; r < RB; ++r) ar[i][r] = ai[i][r] = T(0);
-    for (int k = lane; k < n; k += 32) {
+    const auto step = [&](const Cx<T> (&z)[RPW], int r, Cx<T> x) {
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) {
+            ar[i][r] = fma(z[i].re, x.re, ar[i][r]);
+            ar[i][r] = fma(-z[i].im, x.im, ar[i][r]);
+            ai[i][r] = fma(z[i].re, x.im, ai[i][r]);
+            ai[i][r] = fma(z[i].im, x.re, ai[i][r]);
+        }
+    };
+    int k = lane;
+    if constexpr (U > 1) {
+        const Cx<T>* zr[RPW];
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) zr[i] = Z + (size_t)min(f0 + i, n - 1) * ldz;
+        const Cx<T>* xr[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) xr[r] = X + (size_t)min(r, nrhs - 1) * n;
+        for (; k + 32 * (U - 1) < n; k += 32 * U) {
+            Cx<T> z[U][RPW], x[U][RB];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int i = 0; i < RPW; ++i) z[u][i] = zr[i][k + 32 * u];
+#pragma unroll
+                for (int r = 0; r < RB; ++r) x[u][r] = xr[r][k + 32 * u];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int r = 0; r < RB; ++r) step(z[u], r, x[u][r]);
+        }
+    }
+    for (; k < n; k += 32) {
         Cx<T> z[RPW];
 #pragma unroll
         for (int i = 0; i < RPW; ++i) z[i] = f0 + i < n ? Z[(size_t)(f0 + i) * ldz + k] : cx(T(0), T(0));
 #pragma unroll
         for (int r = 0; r < RB; ++r)
-            if (r < nrhs) {
-                const Cx<T> x = X[(size_t)r * n + k];
-#pragma unroll
-                for (int i = 0; i < RPW; ++i) {
-                    ar[i][r] = fma(z[i].re, x.re, ar[i][r]);
-                    ar[i][r] = fma(-z[i].im, x.im, ar[i][r]);
-                    ai[i][r] = fma(z[i].re, x.im, ai[i][r]);
-                    ai[i][r] = fma(z[i].im, x.re, ai[i][r]);
-                }
-            }
+            if (r < nrhs) step(z, r, X[(size_t)r * n + k]);
     }
 #pragma unroll
     for (int i = 0; i < RPW; ++i)
@@ -156,27 +184,63 @@ __global__ void __launch_bounds__(256) k_cgemv(const Cx<T>* __restrict__ Z, size
         }
 }
 
-// blocks of up to 8 right-hand sides, grid y
+template <typename T, int RPW>
+static void launch_gemv(const Cx<T>* z, size_t ldz, const Cx<T>* x, int n, int nrhs, Cx<T>* y, cudaStream_t st)
+{
+    // blocks of up to 8 right-hand sides of even size (grid y)
+    const int blocks = (nrhs + 7) / 8, rb = (nrhs + blocks - 1) / blocks;
+    const dim3 grd(((n + RPW - 1) / RPW + 7) / 8, blocks);
+    switch (rb) {
+    case 1: k_cgemv<T, 1, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 2: k_cgemv<T, 2, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 3: k_cgemv<T, 3, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 4: k_cgemv<T, 4, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 5: k_cgemv<T, 5, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 6: k_cgemv<T, 6, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    case 7: k_cgemv<T, 7, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    default: k_cgemv<T, 8, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y); break;
+    }
+}
+
+// Rows of a warp, FP32.  More rows read the right-hand sides fewer times
+// (they come from L1 and L2 once n x rb no longer fits L1), fewer rows make
+// more warps.  us at 1 | 2 | 4 rows: n = 480 x 8, 37 | 41 | 41; 2000 x 5,
+// 54 | 53 | 64; 2000 x 8, 57 | 73 | 60; 2000 x 12, 64 | 61 | 55; 3000 x 3,
+// 54 | 49 | 55; 3000 x 8, 78 | 97 | 72; 5067 x 1, 69 | 97 | 171; 5067 x 5,
+// 251 | 147 | 189; 5067 x 9, 338 | 233 | 307; 5067 x 16, 470 | 456 | 246.
+// Four rows a warp, one step of k at a time and blocks of 1, 2, 4 or 8 took
+// 60, 100, 138, 166, 194, 74 for 3 and 191, 217, 372, 751 and 1100.
+static int rpw_f32(int n, int rb)
+{
+    if (rb <= 2 || (long)n * rb < 9000) return 1;
+    return rb <= 5 ? 2 : 4;
+}
+
 template <typename T>
 static emfa_status_t cgemv_blocks(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
                                   cudaStream_t st)
 {
-    constexpr int RPW = sizeof(T) == 8 ? 1 : 4;
-    const int warps = (n + RPW - 1) / RPW;
     const Cx<T>*z = (const Cx<T>*)Z, *x = (const Cx<T>*)X;
     Cx<T>* y = (Cx<T>*)Y;
-    const dim3 grd((warps + 7) / 8, (nrhs + 7) / 8);
-    if (nrhs == 1)
-        k_cgemv<T, 1, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
-    else if (nrhs <= 2)
-        k_cgemv<T, 2, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
-    else if (nrhs <= 4)
-        k_cgemv<T, 4, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
-    else
-        k_cgemv<T, 8, RPW><<<grd, 256, 0, st>>>(z, ldz, x, n, nrhs, y);
+    if constexpr (sizeof(T) == 8) {
+        launch_gemv<T, 1>(z, ldz, x, n, nrhs, y, st);
+    } else {
+        const int blocks = (nrhs + 7) / 8, rpw = rpw_f32(n, (nrhs + blocks - 1) / blocks);
+        if (rpw == 1)
+            launch_gemv<T, 1>(z, ldz, x, n, nrhs, y, st);
+        else if (rpw == 2)
+            launch_gemv<T, 2>(z, ldz, x, n, nrhs, y, st);
+        else
+            launch_gemv<T, 4>(z, ldz, x, n, nrhs, y, st);
+    }
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
     return EMFA_OK;
+}
+
+emfa_status_t cgemv_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)
+{
+    return cgemv_blocks<float>(c, Z, ldz, X, n, nrhs, Y, st);
 }
 
 emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)

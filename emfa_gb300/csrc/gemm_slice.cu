@@ -632,14 +632,15 @@ bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st)
     return nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
 }
 
-// One FP32 product with its split of Z, above the 16 right-hand sides of the
-// GEMV (against the 64 x 64 tiles: n = 480 x 17, 53 | 90 us; 1080 x 91, 72 | 193;
-// 2430 x 181, 194 | 380; 5067 x 37, 358 | 810).  Up to 16 the GEMV, whose lane
-// sums are shorter, can be the more exact one (n = 3000 x 3: 3.5e-7 against its
-// 2.5e-7; the tiles' error is 8.8e-7 to 1.8e-6 where this one's is 1.9e-7 to 3.6e-7).
+// One FP32 product with its split of Z, above the right-hand sides up to which
+// the GEMV is faster or as fast (us, this | GEMV: n = 480 x 17, 56 | 35, x 33,
+// 56 | 39; 1033 x 33, 68 | 52; 2000 x 17, 97 | 64, x 33, 98 | 102; 3000 x 24, 150 | 98,
+// x 33, 153 | 158; 5067 x 17, 343 | 220, x 24, 346 | 265, x 33, 348 | 360).
+// Errors on normal entries, n = 480 to 5067: this 3e-8, the GEMV, whose lane
+// sums are short, 1.2e-7 to 3.3e-7, 64 x 64 tiles 5.5e-7 to 1.8e-6.
 static bool slice_worthwhile_f32(Ctx* c, int n, int nrhs, cudaStream_t st)
 {
-    return slice_allowed(c, sl::Cut<float>::NS, n, st) && nrhs > 16;
+    return slice_allowed(c, sl::Cut<float>::NS, n, st) && nrhs > SLICE_F32_MIN_RHS;
 }
 
 template <typename T>

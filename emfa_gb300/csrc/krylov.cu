@@ -1768,7 +1768,7 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     // that the next product writes, or, for operators that cannot, by a copy
     // on a side stream behind an event (an event and a memset between the
     // launches of a step also kept them from overlapping: 22-27 us a step of
-    // one right-hand side at N = 480 that way, @STEP@ us now).  The step
+    // one right-hand side at N = 480 that way, 16 us now).  The step
     // queued after the last active one does nothing for converged right-hand
     // sides (k_arnoldi_finish skips them).
     struct StepEvents {
@@ -2604,7 +2604,10 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
     }
     bool done = false;
     if (matvec != EMFA_MV_F32) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
-    return done ? EMFA_OK : cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    if (done) return EMFA_OK;
+    // above 16 the 64 x 64 tiles stay what an explicit FP32 product runs
+    if (matvec != EMFA_MV_F32 && n_rhs <= SLICE_F32_MIN_RHS) return cgemv_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    return cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
 }
 
 emfa_status_t emfa_residual(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_dev, int n, const void* X_dev,
