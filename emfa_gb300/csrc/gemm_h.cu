@@ -20,9 +20,9 @@
 // Kernel k_hgemm<BN, MS>: one (128 MS) x BN output tile per CTA, 6 warps:
 //   warp 0      TMA producer: MS blocks of A (128 x 64 halves each) and one
 //               B tile (BN x 64 halves), 128-byte swizzle, multi-stage ring
-//   warp 1      allocates tensor memory (one accumulator per row block); one
-//               lane issues tcgen05.mma (M = 128, N = BN, K = 16): 4 per stage
-//               and row block, and commits each stage free
+//   warp 1      allocates tensor memory (one accumulator per row block) and
+//               issues tcgen05.mma (M = 128, N = BN, K = 16): 4 per stage and
+//               row block, and commits each stage free
 //   warps 2..5  epilogue: tcgen05.ld 32 lanes x 16 columns, scaled complex64
 //               stores (consecutive lanes = consecutive rows: coalesced)
 // Every wait is bounded (clock64): on timeout the kernel records a code in
@@ -53,13 +53,17 @@ constexpr int SMEM_BUDGET = 216 * 1024;
 // Inner product: MS row blocks of 128 (M = 128 MMAs, one accumulator each)
 // share every B tile, so a 256-row tile reads 26% fewer operand bytes per
 // FLOP than a 128-row one; operand delivery from L2, not the tensor pipe,
-// bounds this skinny product (N = 2R = 720).
+// bounds this skinny product (N = 2R = 720: 64.6 bytes a cycle and SM arrive,
+// the port's width, with the tensor pipe 73 % active).  Up to 8 right-hand
+// sides take 16-column tiles: a quarter of the MMA cycles and more stages
+// ahead (one right-hand side, with its GMRES step: n = 7680, 64 -> 58 us).
 template <int BN, int MS>
 struct Smem {
     static constexpr int A_BYTES = BM * 128;  // one 128-row block
     static constexpr int B_BYTES = BN * 128;
     static constexpr int STAGE_BYTES = MS * A_BYTES + B_BYTES;
-    static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : SMEM_BUDGET / STAGE_BYTES;
+    static constexpr int MOST = BN < 64 ? 12 : 8;
+    static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > MOST ? MOST : SMEM_BUDGET / STAGE_BYTES;
     static constexpr int ACC = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;  // columns per accumulator
     static constexpr int TMEM_COLS = MS * ACC < 32 ? 32 : MS * ACC;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
@@ -147,29 +151,24 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     } else if (warp == 1) {
         griddep_wait();
-        if (lane == 0 && !(skip && *(volatile const int*)skip == 0)) {
+        if (!(skip && *(volatile const int*)skip == 0)) {
             constexpr uint32_t idesc = idesc_f16(BM, BN);
+            const uint64_t da0 = sw128_desc(smem_u32(sA)), db0 = sw128_desc(smem_u32(sB));
             for (int kb = 0; kb < kblocks; ++kb) {
                 const int s = kb % S::STAGES;
-                if (!mbar_wait(full + s, (kb / S::STAGES) & 1, err, 3)) break;
+                if (!warp_wait(full + s, (kb / S::STAGES) & 1, err, 3)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t db = sw128_desc(smem_u32(sB + s * S::B_BYTES));
 #pragma unroll
-                for (int m = 0; m < MS; ++m) {
-                    const uint64_t da = sw128_desc(smem_u32(sA + (s * MS + m) * S::A_BYTES));
-#pragma unroll
-                    for (int k = 0; k < BKH / 16; ++k)  // K = 16 halves = 32 bytes per instruction
-                        mma_f16(tmem + (uint32_t)(m * S::ACC), da + 2 * k, db + 2 * k, idesc,
-                                (kb > 0 || k > 0) ? 1u : 0u);
-                }
-                mma_commit(empty + s);
+                for (int m = 0; m < MS; ++m)
+                    mma_f16_block(tmem + (uint32_t)(m * S::ACC), da0 + (uint64_t)((s * MS + m) * (S::A_BYTES >> 4)),
+                                  db0 + (uint64_t)(s * (S::B_BYTES >> 4)), idesc, kb > 0 ? 1u : 0u);
+                commit_elect(empty + s);
             }
             // every MMA issued must be complete before the epilogue and before
             // tensor memory is released
-            mma_commit(accum);
-            mbar_wait(accum, 0, err, 4);
+            commit_elect(accum);
+            warp_wait(accum, 0, err, 4);
         }
-        __syncwarp();
     } else {
         // epilogue warps 2..5: lane quadrant (warp % 4) of tensor memory
         const int q = warp & 3, et = threadIdx.x - 64;
@@ -496,35 +495,26 @@ __global__ void __launch_bounds__(RTHREADS, 1)
                 mbar_wait(full + (kb % S::STAGES), (kb / S::STAGES) & 1, err, 12);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_f16(BM, RBN);
-            for (int kb = 0; kb < kblocks; ++kb) {
-                const int s = kb % S::STAGES;
-                const uint32_t acc = tmem + (uint32_t)((kb & 1) * S::ACC);
-                if (kb >= 2) {
-                    if (!mbar_wait(acc_empty + (kb & 1), ((kb >> 1) - 1) & 1, err, 16)) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                }
-                if (!mbar_wait(full + s, (kb / S::STAGES) & 1, err, 13)) break;
+        constexpr uint32_t idesc = idesc_f16(BM, RBN);
+        const uint64_t da0 = sw128_desc(smem_u32(sA)), db0 = sw128_desc(smem_u32(sB));
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const int s = kb % S::STAGES;
+            const uint32_t acc = tmem + (uint32_t)((kb & 1) * S::ACC);
+            if (kb >= 2) {
+                if (!warp_wait(acc_empty + (kb & 1), ((kb >> 1) - 1) & 1, err, 16)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dah = sw128_desc(smem_u32(sA + (2 * s) * S::A_BYTES));
-                const uint64_t dal = sw128_desc(smem_u32(sA + (2 * s + 1) * S::A_BYTES));
-                const uint64_t dbh = sw128_desc(smem_u32(sB + (2 * s) * S::B_BYTES));
-                const uint64_t dbl = sw128_desc(smem_u32(sB + (2 * s + 1) * S::B_BYTES));
-#pragma unroll
-                for (int k = 0; k < BKH / 16; ++k) {  // corrections: Zh Xl + Zl Xh
-                    mma_f16(acc, dah + 2 * k, dbl + 2 * k, idesc, k > 0 ? 1u : 0u);
-                    mma_f16(acc, dal + 2 * k, dbh + 2 * k, idesc, 1u);
-                }
-#pragma unroll
-                for (int k = 0; k < BKH / 16; ++k) mma_f16(acc, dah + 2 * k, dbh + 2 * k, idesc, 1u);
-                mma_commit(empty + s);
-                mma_commit(acc_full + (kb & 1));
             }
-            mma_commit(done);
-            mbar_wait(done, 0, err, 14);
+            if (!warp_wait(full + s, (kb / S::STAGES) & 1, err, 13)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t dah = da0 + (uint64_t)((2 * s) * (S::A_BYTES >> 4)), dal = dah + (S::A_BYTES >> 4);
+            const uint64_t dbh = db0 + (uint64_t)((2 * s) * (S::B_BYTES >> 4)), dbl = dbh + (S::B_BYTES >> 4);
+            mma_f16_block2(acc, dah, dbl, dal, dbh, idesc, 0u);  // corrections: Zh Xl + Zl Xh
+            mma_f16_block(acc, dah, dbh, idesc, 1u);
+            commit_elect(empty + s);
+            commit_elect(acc_full + (kb & 1));
         }
-        __syncwarp();
+        commit_elect(done);
+        warp_wait(done, 0, err, 14);
     } else {
         // epilogue warps 2..17: lane quadrant warp % 4, column quarter (warp - 2) / 4
         constexpr int CP = RCOLS / 2;  // column pairs (right-hand sides) per thread
@@ -758,8 +748,12 @@ static emfa_status_t launch_variant(Ctx* c, int v, const CUtensorMap& ta, const 
                                     bool timed, const int* skip = nullptr, int* seen = nullptr)
 {
     switch (v) {
-    case HV_64_1: return launch_h<64, 1>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
-    case HV_64_2: return launch_h<64, 2>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    case HV_64_1:
+        if (2 * nrhs <= 16) return launch_h<16, 1>(c, ta, tb[2], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        return launch_h<64, 1>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    case HV_64_2:
+        if (2 * nrhs <= 16) return launch_h<16, 2>(c, ta, tb[2], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        return launch_h<64, 2>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     case HV_144_1: return launch_h<144, 1>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     default: return launch_h<144, 2>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     }
@@ -818,10 +812,11 @@ static emfa_status_t hgemm_run(Ctx* c, const HPlanes& h, const __half* bh, const
 {
     const int n = h.n;
     const size_t ldh = h.ldh;
-    CUtensorMap ta, tb[2];  // tb[0]: 64-column boxes, tb[1]: 144-column boxes
+    CUtensorMap ta, tb[3];  // tb[0]: 64-column boxes, tb[1]: 144-column boxes, tb[2]: 16-column boxes
     const int sms = c->sm_count > 0 ? c->sm_count : 148;
     EMFA_TRY(make_map_h(c, &ta, h.zh, 2 * (uint64_t)n, (uint64_t)n, ldh, th::BM));
     EMFA_TRY(make_map_h(c, &tb[0], bh, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ldh, 64));
+    if (2 * nrhs <= 16) EMFA_TRY(make_map_h(c, &tb[2], bh, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ldh, 16));
     if (2 * nrhs > 64) EMFA_TRY(make_map_h(c, &tb[1], bh, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ldh, 144));
     int v = fixed_variant(n, nrhs, sms);
     if (autotune_enabled()) {

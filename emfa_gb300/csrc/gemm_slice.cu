@@ -141,34 +141,6 @@ __device__ __forceinline__ void mad_wide(unsigned long long& acc, int x, int w)
     asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(x), "r"(w));
 }
 
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code)
-{
-    return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, err, code));
-}
-// the four K = 16 steps of a block (32 bytes apart in both operands): the first
-// one adds to the columns where accum is not 0, the others always
-__device__ __forceinline__ void mma_f16_block(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
-{
-    asm volatile(
-        "{\n .reg .pred p, q;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
-        " elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
-        " add.s64 a1, %1, 2;\n add.s64 a2, %1, 4;\n add.s64 a3, %1, 6;\n"
-        " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n}\n"
-        ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accum)
-        : "memory");
-}
-__device__ __forceinline__ void commit_elect(uint64_t* bar)
-{
-    asm volatile(
-        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
-        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(tc::smem_u32(bar))
-        : "memory");
-}
-
 template <int NS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     k_slice(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int C,

@@ -1003,12 +1003,21 @@ __device__ __forceinline__ float2 shfl_f2(float2 v, int src)
     return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-__device__ void arnoldi_column_f32(const GmresDev& s, int r, int j, double2 hd, float beta)
+// In two parts: the earlier rotations need the column's coefficients only,
+// the new one needs beta as well.
+struct ColumnF32 {
+    float2 h, ph, gj;   // lane i: the rotated entry i; lane j: entry j over its modulus, and g[j]
+    float aa;           // lane j: the modulus of entry j
+    double thr, small;  // the step's residual target and breakdown bound
+};
+
+__device__ __forceinline__ ColumnF32 column_f32_begin(const GmresDev& s, int r, int j, double2 hd)
 {
     const int lane = threadIdx.x & 31, m = s.m;
-    double2* H = s.H + (size_t)r * (m + 1) * m;
-    double* cs = s.cs + (size_t)r * m;
-    double2* sn = s.sn + (size_t)r * m;
+    const double2 gjd = s.g[(size_t)r * (m + 1) + j];
+    const double bn = s.bnorm[r], tr = s.true_res[r];
+    const double* cs = s.cs + (size_t)r * m;
+    const double2* sn = s.sn + (size_t)r * m;
     float2 h = make_float2((float)hd.x, (float)hd.y);
     const float cl = lane < j ? (float)cs[lane] : 0.f;
     const double2 sld = lane < j ? sn[lane] : make_double2(0.0, 0.0);
@@ -1022,10 +1031,26 @@ __device__ void arnoldi_column_f32(const GmresDev& s, int r, int j, double2 hd, 
         else if (lane == i + 1)
             h = make_float2(-(sv.x * x.x + sv.y * x.y) + c * y.x, -(sv.x * x.y - sv.y * x.x) + c * y.y);
     }
+    ColumnF32 q;
+    q.h = h;
+    q.gj = make_float2((float)gjd.x, (float)gjd.y);
+    q.aa = hypotf(h.x, h.y);
+    q.ph = make_float2(h.x / q.aa, h.y / q.aa);
+    q.thr = fmax(s.inner * (s.tol_abs ? s.tol : s.tol * bn), s.red * tr * bn);
+    q.small = 1e-14 * bn;
+    return q;
+}
+
+// SCALE: the 1 / beta of a vector that another launch normalises
+template <bool SCALE>
+__device__ __forceinline__ void column_f32_end(const GmresDev& s, int r, int j, const ColumnF32& q, float beta)
+{
+    const int lane = threadIdx.x & 31, m = s.m;
+    double2* H = s.H + (size_t)r * (m + 1) * m;
+    float2 h = q.h;
     if (lane == j) {
-        const float2 a = h;
         const float b = beta;
-        const float aa = hypotf(a.x, a.y);
+        const float aa = q.aa;
         const float nu = hypotf(aa, b);
         float c;
         float2 sv;
@@ -1035,30 +1060,26 @@ __device__ void arnoldi_column_f32(const GmresDev& s, int r, int j, double2 hd, 
             h = make_float2(b, 0.f);
         } else {
             c = aa / nu;
-            const float2 ph = make_float2(a.x / aa, a.y / aa);
-            sv = make_float2(ph.x * b / nu, ph.y * b / nu);
-            h = make_float2(ph.x * nu, ph.y * nu);
+            sv = make_float2(q.ph.x * b / nu, q.ph.y * b / nu);
+            h = make_float2(q.ph.x * nu, q.ph.y * nu);
         }
         H[(j + 1) * m + j] = make_double2(0.0, 0.0);
-        cs[j] = c;
-        sn[j] = make_double2(sv.x, sv.y);
+        s.cs[(size_t)r * m + j] = c;
+        s.sn[(size_t)r * m + j] = make_double2(sv.x, sv.y);
         double2* g = s.g + (size_t)r * (m + 1);
-        const double2 gjd = g[j];
-        const float2 gj = make_float2((float)gjd.x, (float)gjd.y);
+        const float2 gj = q.gj;
         const float2 gn = make_float2(-(sv.x * gj.x + sv.y * gj.y), -(sv.x * gj.y - sv.y * gj.x));
         g[j + 1] = make_double2(gn.x, gn.y);
         g[j] = make_double2(c * gj.x, c * gj.y);
         const double res = hypotf(gn.x, gn.y);
         s.jlen[r] = j + 1;
         s.est[r] = res;
-        const double thr =
-            fmax(s.inner * (s.tol_abs ? s.tol : s.tol * s.bnorm[r]), s.red * s.true_res[r] * s.bnorm[r]);
-        const bool breakdown = (double)beta <= 1e-14 * s.bnorm[r];
-        if (res < thr || breakdown || j + 1 == m) {
+        const bool breakdown = (double)beta <= q.small;
+        if (res < q.thr || breakdown || j + 1 == m) {
             s.active[r] = 0;
             s.scale[r] = 0.0;
         } else {
-            s.scale[r] = 1.0 / (double)beta;
+            if constexpr (SCALE) s.scale[r] = 1.0 / (double)beta;
             atomicAdd(s.step_cnt, 1);
         }
     }
@@ -1151,7 +1172,7 @@ __global__ void __launch_bounds__(256) k_finish_pack(GmresDev s, int j, const do
     const bool column = chunk == 0;
     if (column && tid < 32) {
         const double2 h = lane <= j ? s.hcol[(size_t)lane * s.nrhs + r] : make_double2(0.0, 0.0);
-        arnoldi_column_f32(s, r, j, h, sbeta);
+        column_f32_end<true>(s, r, j, column_f32_begin(s, r, j, h), sbeta);
         return;
     }
     const float sc = nscale[0], t = nscale[1];
@@ -1206,26 +1227,39 @@ __global__ void __launch_bounds__(256) k_finish_pack(GmresDev s, int j, const do
 //   4. cluster barrier; beta = ||w||; v = w / beta goes to V_{j+1} and, for
 //      operators that pack their input, to the FP16 rows of the next product
 //      (the packing k_hpack_scale does: same scale, same rounding)
-//   5. the first CTA's warp 0 finishes the Arnoldi column (arnoldi_column)
+//   5. a warp of the first CTA's own does the Arnoldi column: the earlier
+//      rotations beside 3, the new one once beta is known, beside the stores
 // W is read once and never written: the next product reads the packed rows
 // (or V_{j+1}).  A right-hand side that is no longer active writes nothing
 // (its V_{j+1} is past its basis length; its rows in the product's operand
 // still hold its last, finite vector).  Replaces k_vdots, k_vupdate,
 // k_arnoldi_finish_warp and the normalisation pass: one launch instead of
 // four, the basis read once from HBM, W once.  Each CTA's work is a chain
-// (staging, two cluster barriers, FP64 sums on one thread, the Givens
-// column on the first CTA), so the step is faster where launches and
+// (staging, two barriers of the cluster, or of the CTA where it is alone,
+// sums by shuffles, the new rotation), which bounds it for few right-hand
+// sides: from the product's end 18.0k cycles of step 10 at N = 480 when the
+// column (6.8k, of it an FP64 division) and one thread's FP64 sums (3.5k)
+// were part of it, about 8k now; the basis of a restart stays in shared
+// memory where a CTA has an SM to itself (25 vectors of 512 else, 4k cycles
+// of the later ones).  GMRES(30) steps of one right-hand side, with the
+// product: N = 480, 16 -> 13 us; 7680, 69 -> 64.  So the step is faster where launches and
 // latency dominate (tens of right-hand sides) and the separate passes are
 // faster for hundreds; the solver picks by the grid size.
 // ---------------------------------------------------------------------------
 constexpr int AS_THREADS = 512;
 constexpr int AS_WARPS = AS_THREADS / 32;
+constexpr int AS_ALL = AS_THREADS + 32;  // and the column's warp
 constexpr int AS_MAXV = 32;     // restart lengths up to 32 (one coefficient per lane in arnoldi_column)
 constexpr int AS_MAX_CLUSTER = 8;
 constexpr int AS_STAGE_BYTES = 104 * 1024;  // staged slices a CTA: two CTAs an SM
+constexpr int AS_STAGE_ALONE = 208 * 1024;  // one CTA an SM
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// the barrier that only keeps a CTA's shared memory alive orders nothing
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // a double2 in the shared memory of CTA `rank` of the cluster, at the
 // address `local` has in this CTA
 __device__ __forceinline__ double2 ld_cluster_d2(const double2* local, int rank)
@@ -1250,7 +1284,7 @@ __device__ __forceinline__ void cp_async_wait_all()
 }
 
 template <int E>
-__global__ void __launch_bounds__(AS_THREADS, 2)
+__global__ void __launch_bounds__(AS_ALL, 2)
     k_arnoldi_step(GmresDev s, int j, const float2* __restrict__ V, size_t vstride, const float2* __restrict__ W,
                    int n, int slice, int sv, float2* __restrict__ Vout, HPack pk)
 {
@@ -1261,9 +1295,9 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
     __shared__ double2 hpart[AS_MAXV];  // this CTA's partial coefficients (read by the cluster)
     __shared__ double2 hs[AS_MAXV];     // the cluster's sums
     __shared__ float2 hf[AS_MAXV];
-    __shared__ double2 nred[AS_WARPS];
+    __shared__ float2 nred[AS_WARPS];   // a warp's |w|^2 and max |Re|, |Im|
     __shared__ double2 npart;           // this CTA's |w|^2 and max (read by the cluster)
-    __shared__ double2 ntot;            // beta and max |Re|, |Im| of w
+    __shared__ float nfin[2];           // beta and max |Re|, |Im| of w
     __shared__ float nscale[2];         // 1 / beta and the FP16 scale t
 
     const int r = blockIdx.y, rank = blockIdx.x, csize = gridDim.x;
@@ -1277,8 +1311,9 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
     // every CTA of the last step is past its own wait, that is after the step
     // before the last has finished: V_0 .. V_{j-1} may be read before the
     // wait, V_j (the last step's) and W only after it.
+    const bool colwarp = warp == AS_WARPS;  // copies, sums and updates nothing
     const int ahead = min(j, sv);
-    for (int i = 0; i < ahead; ++i)
+    for (int i = 0; i < ahead && !colwarp; ++i)
         for (int k = tid; k < len; k += AS_THREADS) cp_async8(sV + (size_t)i * SW + k, Vs + (size_t)i * vstride + k);
     griddep_wait();
     griddep_launch();
@@ -1297,13 +1332,13 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
         const int v1 = min(nv, v0 + sv);
         vlast = v0;
         if (v0 > 0) __syncthreads();  // the previous round's reads are done
-        if (v0 == 0)
+        if (v0 == 0 && !colwarp)
             for (int k = tid; k < len; k += AS_THREADS) cp_async8(sW + k, Ws + k);
-        for (int i = v0 > 0 ? v0 : ahead; i < v1; ++i)
+        for (int i = v0 > 0 ? v0 : ahead; i < v1 && !colwarp; ++i)
             for (int k = tid; k < len; k += AS_THREADS) cp_async8(sV + (size_t)(i - v0) * SW + k, Vs + (size_t)i * vstride + k);
         cp_async_wait_all();
         __syncthreads();
-        for (int i = v0 + warp; i < v1; i += AS_WARPS) {
+        for (int i = v0 + warp; i < v1 && !colwarp; i += AS_WARPS) {
             const float2* vi = sV + (size_t)(i - v0) * SW;
             float ar = 0.f, ai = 0.f;
 #pragma unroll 4
@@ -1321,21 +1356,48 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
         }
     }
     // 2. the cluster's sums (the barrier also orders this CTA's own writes)
-    cluster_arrive();
-    cluster_wait();
+    if (csize > 1) {
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
     if (tid < AS_MAXV) {
         double2 t = make_double2(0.0, 0.0);
-        if (tid < nv)
-            for (int c = 0; c < csize; ++c) {
-                const double2 p = ld_cluster_d2(&hpart[tid], c);
-                t.x += p.x;
-                t.y += p.y;
-            }
+        if (tid < nv) {
+            double2 p[AS_MAX_CLUSTER];
+#pragma unroll
+            for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+                if (c < csize) p[c] = ld_cluster_d2(&hpart[tid], c);
+#pragma unroll
+            for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+                if (c < csize) {
+                    t.x += p[c].x;
+                    t.y += p[c].y;
+                }
+        }
         hs[tid] = t;
         hf[tid] = make_float2((float)t.x, (float)t.y);
     }
     __syncthreads();
 
+    if (colwarp) {
+        // 5. the Arnoldi column, on the first CTA: its rotations beside the update
+        if (csize > 1) cluster_arrive();  // of 4: publishes nothing
+        ColumnF32 q;
+        if (rank == 0) q = column_f32_begin(s, r, j, lane <= j ? hs[lane] : make_double2(0.0, 0.0));
+        if (csize > 1) cluster_wait();
+        named_sync(2, AS_ALL);  // beta
+        if (rank == 0) {
+            if (lane == 0) s.wmax[r] = nfin[1];
+            column_f32_end<false>(s, r, j, q, nfin[0]);
+        }
+        if (csize > 1) {
+            cluster_arrive_relaxed();
+            cluster_wait();
+        }
+        return;
+    }
     // 3. w -= V h: the last round's slices from shared memory, earlier rounds'
     // (restarts longer than sv) again from global memory, where they were
     // read microseconds earlier
@@ -1371,41 +1433,52 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
         nr += __shfl_xor_sync(0xffffffffu, nr, o);
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
-    if (lane == 0) nred[warp] = make_double2((double)nr, (double)mx);
-    __syncthreads();
-    if (tid == 0) {
-        double t = 0.0, tm = 0.0;
-        for (int q = 0; q < AS_WARPS; ++q) {
-            t += nred[q].x;
-            tm = fmax(tm, nred[q].y);
+    if (lane == 0) nred[warp] = make_float2(nr, mx);
+    named_sync(1, AS_THREADS);
+    if (warp == 0) {
+        double t = lane < AS_WARPS ? (double)nred[lane].x : 0.0;
+        float tm = lane < AS_WARPS ? nred[lane].y : 0.f;
+#pragma unroll
+        for (int o = AS_WARPS / 2; o > 0; o >>= 1) {
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
         }
-        npart = make_double2(t, tm);
+        if (lane == 0) npart = make_double2(t, (double)tm);
     }
     // 4. beta and the normalised vector
-    cluster_arrive();
-    cluster_wait();
+    if (csize > 1) {
+        cluster_arrive();
+        cluster_wait();
+    }
     if (tid == 0) {
         // one thread, and FP32 for the root and the division (an FP64
         // instruction costs ~64 cycles of GB300's FP64 pipe)
-        double nr2 = 0.0, wm = 0.0;
-        for (int c = 0; c < csize; ++c) {
-            const double2 p = ld_cluster_d2(&npart, c);
-            nr2 += p.x;
-            wm = fmax(wm, p.y);
-        }
+        double2 p[AS_MAX_CLUSTER];
+#pragma unroll
+        for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+            if (c < csize) p[c] = ld_cluster_d2(&npart, c);
+        double nr2 = 0.0;
+        float wm = 0.f;
+#pragma unroll
+        for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+            if (c < csize) {
+                nr2 += p[c].x;
+                wm = fmaxf(wm, (float)p[c].y);
+            }
         const float beta = sqrtf((float)nr2);
         const float scale = beta > 0.f ? 1.f / beta : 0.f;
-        ntot = make_double2(beta, wm);
+        nfin[0] = beta;
+        nfin[1] = wm;
         nscale[0] = scale;
         nscale[1] = 1.f;
         if (pk.bh) {
-            const int ex = hpack_exponent_f((float)wm, scale);
+            const int ex = hpack_exponent_f(wm, scale);
             nscale[1] = ldexpf(1.f, 14 - ex);
             if (rank == 0) pk.inv_t[r] = ldexpf(1.f, ex - 14);
         }
     }
-    __syncthreads();
-    cluster_arrive();  // this CTA's reads of the others' shared memory are done
+    named_sync(1, AS_THREADS);
+    named_arrive(2, AS_ALL);
     const float sc = nscale[0], t = nscale[1];
     __half2* h0 = pk.bh ? reinterpret_cast<__half2*>(pk.bh + (size_t)(2 * r) * pk.ldh) + k0 : nullptr;
     __half2* h1 = pk.bh ? reinterpret_cast<__half2*>(pk.bh + (size_t)(2 * r + 1) * pk.ldh) + k0 : nullptr;
@@ -1422,12 +1495,11 @@ __global__ void __launch_bounds__(AS_THREADS, 2)
             h1[k] = __halves2half2(him, hre);
         }
     }
-    // 5. the Arnoldi column
-    if (rank == 0 && warp == 0) {
-        if (lane == 0) s.wmax[r] = ntot.y;
-        arnoldi_column_f32(s, r, j, lane <= j ? hs[lane] : make_double2(0.0, 0.0), (float)ntot.x);
+    if (csize > 1) {
+        // no CTA leaves while another may still read its shared memory
+        cluster_arrive_relaxed();
+        cluster_wait();
     }
-    cluster_wait();  // no CTA leaves while another may still read its shared memory
 }
 
 // out[r] = scale[r] W[r]: grid over (chunks of 1024, RHS).  An FP32 basis is
@@ -1629,12 +1701,15 @@ static emfa_status_t launch_step_e(Ctx* c, const StepShape& sh, int nrhs, cudaSt
                                    const HPack& pk)
 {
     const int sw = AS_THREADS * E;  // staged slice
-    const int sv = std::min(AS_MAXV, AS_STAGE_BYTES / (int)(sizeof(float2) * sw) - 1);
+    // one CTA an SM may hold every vector of a restart
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    const int budget = (long)nrhs * sh.cs <= sms ? AS_STAGE_ALONE : AS_STAGE_BYTES;
+    const int sv = std::min(AS_MAXV, budget / (int)(sizeof(float2) * sw) - 1);
     const size_t smem = sizeof(float2) * (size_t)sw * (sv + 1);
     EMFA_TRY(ensure_smem(c, k_arnoldi_step<E>, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sh.cs, nrhs);
-    cfg.blockDim = dim3(AS_THREADS);
+    cfg.blockDim = dim3(AS_ALL);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2];

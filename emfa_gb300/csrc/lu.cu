@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(256) k_lu_panels(float2* __restrict__ A, int n
 // one block's panels (K = 64 complex), 4 for two blocks'.
 //   warp 0      TMA producer: per K slice Uh, Ul (128 rows) and Lh, Ll (TN
 //               rows), 128-byte swizzle
-//   warp 1      allocates TN tensor-memory columns; one lane issues
+//   warp 1      allocates TN tensor-memory columns and issues
 //               tcgen05.mma M = 128, N = TN, K = 16: 12 per slice
 //   warps 2..9  epilogue, per 64-row chunk of the tile of A22 (TMA loads, 32
 //               KB): each warp takes a quadrant of the tensor-memory lanes
@@ -789,34 +789,26 @@ __global__ void __launch_bounds__(lutc::THREADS, TN == 256 ? 2 : 1)
             if (!S::WIDE) mbar_wait(cfull, 0, err, 12);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_f16(lutc::TM, TN);
-            for (int s = 0; s < nslices; ++s) {
-                if (!mbar_wait(full + s % NST, (s / NST) & 1, err, 13)) {
-                    stopped = 1;
-                    __threadfence_block();
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t* st = base + (s % NST) * S::STAGE;
-                const uint64_t uh = sw128_desc(smem_u32(st)), ul = sw128_desc(smem_u32(st + lutc::U_BYTES));
-                const uint64_t lh = sw128_desc(smem_u32(st + 2 * lutc::U_BYTES)),
-                               ll = sw128_desc(smem_u32(st + 2 * lutc::U_BYTES + S::L_BYTES));
-#pragma unroll
-                for (int k = 0; k < 4; ++k)  // K = 16 halves = 32 bytes per instruction
-                    mma_f16(tmem, uh + 2 * k, lh + 2 * k, idesc, (s > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) mma_f16(tmem, uh + 2 * k, ll + 2 * k, idesc, 1u);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) mma_f16(tmem, ul + 2 * k, lh + 2 * k, idesc, 1u);
-                if (s + NST < nslices) mma_commit(empty + s % NST);
+        constexpr uint32_t idesc = idesc_f16(lutc::TM, TN);
+        const uint64_t d0 = sw128_desc(smem_u32(base));
+        for (int s = 0; s < nslices; ++s) {
+            if (!warp_wait(full + s % NST, (s / NST) & 1, err, 13)) {
+                stopped = 1;
+                __threadfence_block();
+                break;
             }
-            // every MMA issued must be complete before the epilogue and before
-            // tensor memory is released
-            mma_commit(accum);
-            mbar_wait(accum, 0, err, 14);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t uh = d0 + (uint64_t)((s % NST) * (S::STAGE >> 4)), ul = uh + (lutc::U_BYTES >> 4);
+            const uint64_t lh = ul + (lutc::U_BYTES >> 4), ll = lh + (S::L_BYTES >> 4);
+            mma_f16_block(tmem, uh, lh, idesc, s > 0 ? 1u : 0u);
+            mma_f16_block(tmem, uh, ll, idesc, 1u);
+            mma_f16_block(tmem, ul, lh, idesc, 1u);
+            if (s + NST < nslices) commit_elect(empty + s % NST);
         }
-        __syncwarp();
+        // every MMA issued must be complete before the epilogue and before
+        // tensor memory is released
+        commit_elect(accum);
+        warp_wait(accum, 0, err, 14);
     } else {
         const int q = warp & 3, hf = (warp - 2) >> 2;
         const bool leader = threadIdx.x == 64;

@@ -135,12 +135,57 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n)
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
+// Issue by a whole warp that walks the loop, one elected lane at the
+// instruction: the descriptors are warp-uniform values in uniform registers.
+// From a single thread's branch they are not, and an MMA costs ~80 cycles of
+// issue.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
+}
+// the four K = 16 steps of a block (32 bytes apart in both operands): the first
+// one adds to the columns where accum is not 0, the others always
+__device__ __forceinline__ void mma_f16_block(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
 {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+        "{\n .reg .pred p, q;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        " elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+        " add.s64 a1, %1, 2;\n add.s64 a2, %1, 4;\n add.s64 a3, %1, 6;\n"
+        " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n}\n"
         ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+// two such products in turn, step by step: a0 b0, a1 b1
+__device__ __forceinline__ void mma_f16_block2(uint32_t tmem, uint64_t a0, uint64_t b0, uint64_t c0, uint64_t d0,
+                                               uint32_t idesc, uint32_t accum)
+{
+    asm volatile(
+        "{\n .reg .pred p, q;\n .reg .b64 a1, a2, a3, b1, b2, b3, c1, c2, c3, d1, d2, d3;\n"
+        " elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %6, 0;\n"
+        " add.s64 a1, %1, 2;\n add.s64 a2, %1, 4;\n add.s64 a3, %1, 6;\n"
+        " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
+        " add.s64 c1, %3, 2;\n add.s64 c2, %3, 4;\n add.s64 c3, %3, 6;\n"
+        " add.s64 d1, %4, 2;\n add.s64 d2, %4, 4;\n add.s64 d3, %4, 6;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %5, p;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %3, %4, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], c1, d1, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], c2, d2, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %5, 1;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], c3, d3, %5, 1;\n}\n"
+        ::"r"(tmem), "l"(a0), "l"(b0), "l"(c0), "l"(d0), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void commit_elect(uint64_t* bar)
+{
+    asm volatile(
+        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar))
         : "memory");
 }
 

@@ -1,0 +1,39 @@
+"""The split-FP16 product at the widths where its column tile changes (16, 64 and 144 real columns), the rows where a tile
+ends, and K shorter and longer than the stages loaded ahead; and GMRES steps whose basis fits the shared memory of a CTA
+that has an SM to itself, or of one of two.
+
+Each right-hand side is scaled by itself and its sums run over k in one order, so a column of a block is the product of that
+column alone, bit for bit.  Refined GMRES has to reach its tolerance on the true residual whatever the layout of a step."""
+import numpy as np
+import pytest
+
+from emfa_gb300 import api
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [33, 128, 129, 257, 385, 900])
+@pytest.mark.parametrize("r", [1, 7, 8, 9, 31, 32, 33, 73])
+def test_block_equals_its_columns(ctx, n, r):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + 1000 * r)
+    z = torch.randn(n, n, dtype=torch.complex64, device="cuda", generator=g)
+    x = torch.randn(r, n, dtype=torch.complex64, device="cuda", generator=g)
+    y = api.matvec(ctx, z, x, "f16x")
+    for c in sorted({0, r // 2, r - 1}):
+        assert torch.equal(y[c], api.matvec(ctx, z, x[c:c + 1].contiguous(), "f16x")[0])
+
+
+@pytest.mark.parametrize("n,r", [(31, 1), (512, 1), (513, 2), (1024, 160), (1025, 1), (2500, 40), (4100, 30), (8200, 2)])
+@pytest.mark.parametrize("restart", [2, 32])
+def test_gmres_step_layouts(ctx, n, r, restart):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + r)
+    z = torch.randn(n, n, dtype=torch.complex64, device="cuda", generator=g)
+    z.diagonal().add_(2.5 * n ** 0.5)
+    b = torch.randn(r, n, dtype=torch.complex64, device="cuda", generator=g)
+    x, info = api.solve(ctx, z, b, api.solver_params("gmres", restart=restart, tol=1e-6, orth="cgs1_fused"))
+    assert info.converged == r
+    res = b.to(torch.complex128) - x @ z.to(torch.complex128).T
+    # two roundings of the FP64 residual apart from the solver's own
+    assert float((res.norm(dim=1) / b.norm(dim=1)).max()) <= 1e-6 * (1 + 1e-6)
