@@ -65,24 +65,36 @@ struct Box {
     float c[3];
     int parent = -1;
     int oct = 0;      // child index (x*2+y)*2+z within the parent
-    int offset = 0;   // first unknown (box order)
-    std::vector<int> unk;
-    std::vector<int> child, near;
+    int ix[3] = {0, 0, 0};          // place on the level's grid
+    int offset = 0, count = 0;      // its unknowns in box order
+    int child0 = 0, nchild = 0;     // its children on the next level
 };
 
-// Legendre value / derivative recurrence of GaussLegendre::Evaluation
-static void gl_eval(float x, int n, float& v, float& d)
+// a level's boxes and their near lists (CSR)
+struct Level {
+    std::vector<Box> b;
+    std::vector<int> nptr{0}, near;
+};
+
+// Legendre value / derivative recurrence of GaussLegendre::Evaluation, for
+// GL roots side by side (one recurrence is a chain of divisions)
+constexpr int GL = 8;
+static void gl_eval(const float* x, int n, float* v, float* d)
 {
-    float vsub1 = x, vsub2 = 1;
-    float f = 1 / (x * x - 1);
-    v = 1;
-    d = 0;
-    for (int i = 2; i <= n; ++i) {
-        v = ((2 * i - 1) * x * vsub1 - (i - 1) * vsub2) / i;
-        d = i * f * (x * v - vsub1);
-        vsub2 = vsub1;
-        vsub1 = v;
+    float vsub1[GL], vsub2[GL];
+    for (int r = 0; r < GL; ++r) {
+        vsub1[r] = x[r];
+        vsub2[r] = 1;
+        v[r] = 1;
+        d[r] = 0;
     }
+    for (int i = 2; i <= n; ++i)
+        for (int r = 0; r < GL; ++r) {
+            v[r] = ((2 * i - 1) * x[r] * vsub1[r] - (i - 1) * vsub2[r]) / i;
+            if (i == n) d[r] = i * (1 / (x[r] * x[r] - 1)) * (x[r] * v[r] - vsub1[r]);
+            vsub2[r] = vsub1[r];
+            vsub1[r] = v[r];
+        }
 }
 
 // GaussLegendre::set (EMComponent/Quadrature.cpp:93-112): Newton from the
@@ -91,18 +103,34 @@ static void gauss_legendre(int n, std::vector<float>& r, std::vector<float>& w)
 {
     r.assign(n, 0);
     w.assign(n, 0);
-    for (int i = 0; i < n; ++i) {
-        float x = (float)std::cos((double)(PI * (i + 0.75f) / (n + 0.5f)));
-        float v, d, dr;
+    for (int i0 = 0; i0 < n; i0 += GL) {
+        float x[GL], v[GL], d[GL], xn[GL], vn[GL], dn[GL];
+        bool live[GL];
+        for (int q = 0; q < GL; ++q) {
+            const int i = std::min(i0 + q, n - 1);
+            x[q] = (float)std::cos((double)(PI * (i + 0.75f) / (n + 0.5f)));
+            live[q] = true;
+        }
         gl_eval(x, n, v, d);
         int guard = 0;
-        do {
-            dr = v / d;
-            x = x - dr;
-            gl_eval(x, n, v, d);
-        } while (std::fabs((double)dr) > 2e-7f && ++guard < 1000);
-        r[n - 1 - i] = x;
-        w[n - 1 - i] = 2 / ((1 - x * x) * d * d);
+        for (bool any = true; any;) {
+            for (int q = 0; q < GL; ++q) xn[q] = x[q] - v[q] / d[q];
+            gl_eval(xn, n, vn, dn);
+            const bool stop = ++guard >= 1000;
+            any = false;
+            for (int q = 0; q < GL; ++q)
+                if (live[q]) {  // a root that has converged keeps its last step
+                    live[q] = std::fabs((double)(v[q] / d[q])) > 2e-7f && !stop;
+                    any |= live[q];
+                    x[q] = xn[q];
+                    v[q] = vn[q];
+                    d[q] = dn[q];
+                }
+        }
+        for (int q = 0; q < GL && i0 + q < n; ++q) {
+            r[n - 1 - i0 - q] = x[q];
+            w[n - 1 - i0 - q] = 2 / ((1 - x[q] * x[q]) * d[q] * d[q]);
+        }
     }
 }
 
@@ -149,30 +177,30 @@ static float fnorm3(const float* a, const float* b)
 struct MLevel {
     int nbox = 0, L = 0, K = 0;
     float len = 0;
-    DevBuf parent, oct;                 // parent index and octant per box (int)
-    DevBuf child_ptr, child_idx;        // CSR children (int)
+    DevView parent, oct;                 // parent index and octant per box (int)
+    DevView child_ptr, child_idx;        // CSR children (int)
     // translation by sibling groups: the children of one box of the level
     // above, at most four a group (TransGroup), and their source boxes, the
     // children of the boxes near the parent
-    DevBuf grp, grp_src;
+    DevView grp, grp_src;
     int ngrp = 0;
-    DevBuf trans;                       // float2 [343][K]
-    DevBuf up, down;                    // planar float2 [right-hand side][nbox][3][K]
+    DevView trans;                       // float2 [343][K]
+    DevView up, down;                    // planar float2 [right-hand side][nbox][3][K]
     // interpolation to this level from the level below, separable: 3-point
     // Lagrange stencils in theta (per theta index of this level: child theta,
     // weight) and in phi (per phi index: child phi row, weight)
-    DevBuf ip_tl, ip_te, ip_pl, ip_pe;
+    DevView ip_tl, ip_te, ip_pl, ip_pe;
     // anterpolation from the level above, as two transposed 1-D Lagrange
     // stencils: theta (CSR over this level's theta index: parent theta, weight)
     // and phi (CSR over this level's phi index: parent phi, weight)
-    DevBuf th_ptr, th_src, th_w, ph_ptr, ph_src, ph_w;
+    DevView th_ptr, th_src, th_w, ph_ptr, ph_src, ph_w;
     size_t down_smem = 0;               // shared bytes per CTA (theta-pass rows)
-    DevBuf down_win;                    // int2 per chunk: parent phi rows its phi stencils read
-    DevBuf up_phase;                    // float2 [8][K]: exp(-j k k.(parent - child)) for the level below
+    DevView down_win;                    // int2 per chunk: parent phi rows its phi stencils read
+    DevView up_phase;                    // float2 [8][K]: exp(-j k k.(parent - child)) for the level below
     int up_rows = 0;                    // interpolation from the level below: phi rows per CTA,
     size_t up_child_bytes = 0;          //   shared bytes of one child's theta pass,
     int up_batch = 0;                   //   children per shared-memory pass,
-    DevBuf up_win;                      //   int2 per chunk: the child phi rows it reads
+    DevView up_win;                      //   int2 per chunk: the child phi rows it reads
 };
 
 }  // namespace emfa
@@ -189,17 +217,20 @@ struct emfa_mlfma {
     std::vector<int> poles;        // multipoles per level 2..L
     std::vector<emfa::MLevel> lv;  // index level - 2
     int rcap = 1;                  // right-hand sides the level patterns hold (one apply chunk)
-    emfa::DevBuf perm_d, box_of;   // int [n]
+    emfa::DevBuf fine_tables, level_tables;  // the lists and tables below and of every level
+    emfa::DevBuf trans_tables, patterns;     // translation operators, up and down patterns of every level
+    emfa::DevView perm_d, box_of;  // int [n]
     emfa::DevBuf rad, rec;         // C2f [n][Kf]: theta, phi components in each sample's basis
-    emfa::DevBuf tp;               // float [6][Kf]: theta_hat, phi_hat of the finest samples
-    emfa::DevBuf coeff;            // float [Kf]
-    emfa::DevBuf box_off, box_cnt; // finest boxes: first unknown, count
-    emfa::DevBuf near_ptr, near_box, near_col, row_cols;  // CSR near lists, column base per slot, C_b per box
-    emfa::DevBuf row_base;         // size_t per finest box: first value of the box's rows
+    emfa::DevView tp;               // float [6][Kf]: theta_hat, phi_hat of the finest samples
+    emfa::DevView coeff;            // float [Kf]
+    emfa::DevView box_off, box_cnt; // finest boxes: first unknown, count
+    emfa::DevView near_ptr, near_box, near_col, row_cols;  // CSR near lists, column base per slot, C_b per box
+    emfa::DevView row_base;         // size_t per finest box: first value of the box's rows
     emfa::DevBuf near_val;         // float2 [nnz]
-    emfa::DevBuf near_cbase, near_cidx;  // per finest box: first entry, column unknowns of its near rows
+    emfa::DevView near_cbase;      // per finest box: first entry of
+    emfa::DevBuf near_cidx;        //   the column unknowns of its near rows
     size_t nnz = 0;
-    emfa::DevBuf trans_work;       // TransWork per CTA of the translation
+    emfa::DevView trans_work;       // TransWork per CTA of the translation
     int trans_ctas = 0;
     int max_cols = 0;              // near columns of a box, most
     emfa::DevBuf tmp_in, tmp_out;  // complex64 scratch for residuals
@@ -1072,11 +1103,11 @@ struct Plan {
     int L = 0;
     float k = 0;
     std::vector<float> blen;
-    std::vector<std::vector<mh::Box>> lb;
+    std::vector<mh::Level> lev;
     std::vector<int> poles;
     std::vector<std::vector<float>> gt, gp, gw, kd;
     std::vector<std::vector<float>> wt1, wp1;  // 1-D Gauss weights in theta and phi (gw = wp1 x wt1)
-    std::vector<int> perm, box_of, off, cnt;
+    std::vector<int> perm, box_of, off, cnt;  // perm: box order -> RWG index
     std::vector<float> cen;
     std::vector<float> cp;  // RWG centres (v1 + v2) / 2, RWG order
 };
@@ -1124,15 +1155,21 @@ static bool build_plan(const std::vector<double>& verts, int nv, const std::vect
     cp.assign(3 * (size_t)n, 0.f);
     for (int u = 0; u < n; ++u)
         for (int d = 0; d < 3; ++d) cp[3 * u + d] = (vf[3 * rwg[6 * u] + d] + vf[3 * rwg[6 * u + 1] + d]) * 0.5f;
-    // octree (buildBox)
-    auto& lb = P.lb;
+    // octree (buildBox): the unknowns of every box are a range of one order,
+    // which each level refines by a stable counting sort within the boxes
+    auto& lev = P.lev;
     auto& blen = P.blen;
-    lb.assign(L + 1, {});
+    lev.assign(L + 1, mh::Level());
     blen.assign(L + 1, 0.f);
     mh::Box rb;
     std::copy(root, root + 3, rb.c);
-    for (int u = 0; u < n; ++u) rb.unk.push_back(u);
-    lb[0].push_back(rb);
+    rb.count = n;
+    lev[0].b.push_back(rb);
+    std::vector<int>& order = P.perm;
+    std::vector<int> next(n);
+    std::vector<unsigned char> oct(n);
+    order.resize(n);
+    for (int u = 0; u < n; ++u) order[u] = u;
     float cur = big / 2;
     blen[1] = cur;
     for (int l = 1; l <= L; ++l) {
@@ -1140,59 +1177,75 @@ static bool build_plan(const std::vector<double>& verts, int nv, const std::vect
             cur /= 2;
             blen[l] = cur;
         }
-        for (size_t pi = 0; pi < lb[l - 1].size(); ++pi) {
-            mh::Box& pb = lb[l - 1][pi];
-            mh::Box ch[8];
-            for (int x = 0; x < 2; ++x)
-                for (int y = 0; y < 2; ++y)
-                    for (int z = 0; z < 2; ++z) {
-                        int idx = (x * 2 + y) * 2 + z;
-                        ch[idx].c[0] = pb.c[0] + (x - 0.5f) * cur;
-                        ch[idx].c[1] = pb.c[1] + (y - 0.5f) * cur;
-                        ch[idx].c[2] = pb.c[2] + (z - 0.5f) * cur;
-                        ch[idx].parent = (int)pi;
-                        ch[idx].oct = idx;
-                    }
-            for (int u : pb.unk) {
-                int xf = cp[3 * u] < pb.c[0] ? 0 : 1, yf = cp[3 * u + 1] < pb.c[1] ? 0 : 1,
-                    zf = cp[3 * u + 2] < pb.c[2] ? 0 : 1;
-                ch[(xf * 2 + yf) * 2 + zf].unk.push_back(u);
+        auto& up = lev[l - 1].b;
+        auto& down = lev[l].b;
+        down.reserve(std::min<size_t>((size_t)n, 8 * up.size()));
+        for (size_t pi = 0; pi < up.size(); ++pi) {
+            mh::Box& pb = up[pi];
+            const int q0 = pb.offset, q1 = pb.offset + pb.count;
+            int pos[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            for (int q = q0; q < q1; ++q) {
+                const float* x = &cp[3 * (size_t)order[q]];
+                const int xf = x[0] < pb.c[0] ? 0 : 1, yf = x[1] < pb.c[1] ? 0 : 1, zf = x[2] < pb.c[2] ? 0 : 1;
+                oct[q] = (unsigned char)((xf * 2 + yf) * 2 + zf);
+                ++pos[oct[q]];
             }
-            int pos = pb.offset;
-            for (int ci = 0; ci < 8; ++ci) {
-                if (ch[ci].unk.empty()) continue;
-                ch[ci].offset = pos;
-                pos += (int)ch[ci].unk.size();
-                pb.child.push_back((int)lb[l].size());
-                lb[l].push_back(std::move(ch[ci]));
+            pb.child0 = (int)down.size();
+            int at = q0;
+            for (int idx = 0; idx < 8; ++idx) {
+                const int cnt = pos[idx], x = idx >> 2, y = (idx >> 1) & 1, z = idx & 1;
+                pos[idx] = at;
+                if (!cnt) continue;
+                mh::Box ch;
+                ch.c[0] = pb.c[0] + (x - 0.5f) * cur;
+                ch.c[1] = pb.c[1] + (y - 0.5f) * cur;
+                ch.c[2] = pb.c[2] + (z - 0.5f) * cur;
+                ch.parent = (int)pi;
+                ch.oct = idx;
+                ch.ix[0] = 2 * pb.ix[0] + x;
+                ch.ix[1] = 2 * pb.ix[1] + y;
+                ch.ix[2] = 2 * pb.ix[2] + z;
+                ch.offset = at;
+                ch.count = cnt;
+                at += cnt;
+                down.push_back(ch);
             }
+            pb.nchild = (int)down.size() - pb.child0;
+            for (int q = q0; q < q1; ++q) next[pos[oct[q]]++] = order[q];
         }
+        order.swap(next);
     }
-    // setBoxParameter: level 1 all near; level >= 2 near if centre distance < 1.75 box
-    for (size_t f = 0; f < lb[1].size(); ++f)
-        for (size_t s2 = 0; s2 < lb[1].size(); ++s2) lb[1][f].near.push_back((int)s2);
-    float clen = big / 4;
-    for (int l = 2; l <= L; ++l, clen /= 2) {
-        float lim = 1.75f * clen;
-        for (auto& b : lb[l]) {
-            for (int pn : lb[l - 1][b.parent].near)
-                for (int cidx : lb[l - 1][pn].child) {
-                    float dist = mh::fnorm3(lb[l][cidx].c, b.c);
-                    if (dist < lim) b.near.push_back(cidx);
+    // setBoxParameter: level 1 all near; level >= 2 near if the centres are
+    // less than 1.75 boxes apart, that is at most one box in each direction
+    // (sqrt(3) < 1.75 < 2)
+    for (size_t f = 0; f < lev[1].b.size(); ++f) {
+        for (size_t s2 = 0; s2 < lev[1].b.size(); ++s2) lev[1].near.push_back((int)s2);
+        lev[1].nptr.push_back((int)lev[1].near.size());
+    }
+    for (int l = 2; l <= L; ++l) {
+        const mh::Level& pl = lev[l - 1];
+        mh::Level& cl = lev[l];
+        cl.near.reserve(27 * cl.b.size());
+        for (const auto& b : cl.b) {
+            for (int s2 = pl.nptr[b.parent]; s2 < pl.nptr[b.parent + 1]; ++s2) {
+                const mh::Box& pn = pl.b[pl.near[s2]];
+                for (int cidx = pn.child0; cidx < pn.child0 + pn.nchild; ++cidx) {
+                    const int* x = cl.b[cidx].ix;
+                    if ((unsigned)(x[0] - b.ix[0] + 1) < 3u && (unsigned)(x[1] - b.ix[1] + 1) < 3u &&
+                        (unsigned)(x[2] - b.ix[2] + 1) < 3u)
+                        cl.near.push_back(cidx);
                 }
+            }
+            cl.nptr.push_back((int)cl.near.size());
         }
     }
     // box order of the unknowns
-    const auto& fin = lb[L];
-    P.perm.clear();
-    P.box_of.assign(n, 0);
+    const auto& fin = lev[L].b;
+    P.box_of.resize(n);
     for (size_t b = 0; b < fin.size(); ++b) {
         P.off.push_back(fin[b].offset);
-        P.cnt.push_back((int)fin[b].unk.size());
-        for (int u : fin[b].unk) {
-            P.box_of[P.perm.size()] = (int)b;
-            P.perm.push_back(u);
-        }
+        P.cnt.push_back(fin[b].count);
+        std::fill_n(P.box_of.begin() + fin[b].offset, fin[b].count, (int)b);
         P.cen.insert(P.cen.end(), fin[b].c, fin[b].c + 3);
     }
     // multipoles, samples, weights, directions
@@ -1256,7 +1309,8 @@ static emfa_status_t sai_build(emfa_mlfma* M, const Plan& P, cudaStream_t st)
                      "unknowns lie within sqrt(3)/2 box lengths of its centre)");
         return EMFA_ERR_INVALID;
     }
-    const auto& fin = P.lb[P.L];
+    const mh::Level& fl = P.lev[P.L];
+    const auto& fin = fl.b;
     const float bl = P.blen[P.L];
     const float thr_r = (float)M->p.row_threshold * bl, thr_c = (float)M->p.col_threshold * bl;
     const int nbox = (int)fin.size(), n = M->n;
@@ -1275,11 +1329,12 @@ static emfa_status_t sai_build(emfa_mlfma* M, const Plan& P, cudaStream_t st)
     int max_rows = 1, max_cols = 1;
     for (int b = 0; b < nbox; ++b) {
         int o = -1;
-        for (int nb : fin[b].near) {
+        for (int sl = fl.nptr[b]; sl < fl.nptr[b + 1]; ++sl) {
+            const int nb = fl.near[sl];
             if (nb == b) o = (int)(rows.size() - rptr.back());
-            for (size_t i = 0; i < fin[nb].unk.size(); ++i) {
-                const float dist = mh::fnorm3(&P.cp[3 * (size_t)fin[nb].unk[i]], fin[b].c);
-                const int idx = fin[nb].offset + (int)i;
+            for (int i = 0; i < fin[nb].count; ++i) {
+                const int idx = fin[nb].offset + i;
+                const float dist = mh::fnorm3(&P.cp[3 * (size_t)P.perm[idx]], fin[b].c);
                 if (dist <= thr_r) rows.push_back(idx);
                 if (dist <= thr_c) cols.push_back(idx);
             }
@@ -1291,23 +1346,23 @@ static emfa_status_t sai_build(emfa_mlfma* M, const Plan& P, cudaStream_t st)
         max_rows = std::max(max_rows, m);
         max_cols = std::max(max_cols, nc);
         ebase.push_back(nnz);
-        nnz += (size_t)nc * fin[b].unk.size();
+        nnz += (size_t)nc * fin[b].count;
     }
     // CSR of P over rows = cols[c], columns = the box's own unknowns, the
     // entries of a row in the order the boxes produce them
     std::vector<int> cnt(n + 1, 0), dest(std::max<size_t>(nnz, 1)), ccol(std::max<size_t>(nnz, 1));
     for (int b = 0; b < nbox; ++b)
-        for (size_t u = 0; u < fin[b].unk.size(); ++u)
+        for (int u = 0; u < fin[b].count; ++u)
             for (int k = cptr[b]; k < cptr[b + 1]; ++k) cnt[cols[k] + 1] += 1;
     for (int i = 0; i < n; ++i) cnt[i + 1] += cnt[i];
     std::vector<int> fillp(cnt.begin(), cnt.end() - 1);
     for (int b = 0; b < nbox; ++b)
-        for (size_t u = 0; u < fin[b].unk.size(); ++u)
+        for (int u = 0; u < fin[b].count; ++u)
             for (int k = cptr[b]; k < cptr[b + 1]; ++k) {
                 const size_t e = ebase[b] + u * (size_t)(cptr[b + 1] - cptr[b]) + (k - cptr[b]);
                 const int pos = fillp[cols[k]]++;
                 dest[e] = pos;
-                ccol[pos] = fin[b].offset + (int)u;
+                ccol[pos] = fin[b].offset + u;
             }
     const size_t smem = sizeof(float2) * ((size_t)max_rows * max_cols + max_cols) +
                         sizeof(float) * (max_cols + (max_cols & 1)) + sizeof(float2) * 4 * (size_t)(max_rows + max_cols);
@@ -1343,12 +1398,91 @@ static emfa_status_t sai_build(emfa_mlfma* M, const Plan& P, cudaStream_t st)
     return EMFA_OK;
 }
 
+// Host tables gathered for one device buffer and one copy; the views point
+// into it after upload().  The host copy must outlive the copy's stream order.
+struct Stage {
+    std::vector<char> host;
+    std::vector<std::pair<DevView*, size_t>> at;
+    template <typename T>
+    void put(DevView& v, const T* a, size_t n)
+    {
+        const size_t o = (host.size() + 255) & ~(size_t)255;
+        host.resize(o + sizeof(T) * std::max<size_t>(n, 1));
+        if (n) std::copy(a, a + n, reinterpret_cast<T*>(host.data() + o));
+        v.bytes = sizeof(T) * n;
+        at.push_back({&v, o});
+    }
+    template <typename T>
+    void put(DevView& v, const std::vector<T>& a)
+    {
+        put(v, a.data(), a.size());
+    }
+    emfa_status_t upload(Ctx* c, DevBuf& b, cudaStream_t st)
+    {
+        EMFA_TRY(b.alloc(c, std::max<size_t>(host.size(), 1)));
+        EMFA_CUDA(c, cudaMemcpyAsync(b.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+        for (auto& x : at) x.first->ptr = (char*)b.ptr + x.second;
+        return EMFA_OK;
+    }
+};
+
+// column unknowns of each finest box's near rows, in value order: a warp per box
+__global__ void k_near_cidx(int nbox, const int* __restrict__ near_ptr, const int* __restrict__ near_box,
+                            const int* __restrict__ near_col, const int* __restrict__ box_off,
+                            const int* __restrict__ box_cnt, const int* __restrict__ cbase, int* __restrict__ cidx)
+{
+    const int b = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (b >= nbox) return;
+    for (int sl = near_ptr[b]; sl < near_ptr[b + 1]; ++sl) {
+        const int nb = near_box[sl], off = box_off[nb], cnt = box_cnt[nb];
+        int* o = cidx + cbase[b] + near_col[sl];
+        for (int q = lane; q < cnt; q += 32) o[q] = off + q;
+    }
+}
+
+// The level patterns of nr right-hand sides, one buffer
+static emfa_status_t alloc_patterns(emfa_mlfma* M, int nr)
+{
+    size_t tot = 0;
+    for (auto& ml : M->lv) tot += 2 * Carver::round(sizeof(float2) * 3 * (size_t)ml.nbox * ml.K * nr);
+    M->rcap = 0;
+    EMFA_TRY(M->patterns.alloc(M->ctx, tot));
+    char* p = (char*)M->patterns.ptr;
+    for (auto& ml : M->lv) {
+        const size_t per = sizeof(float2) * 3 * (size_t)ml.nbox * ml.K * nr;
+        for (DevView* v : {&ml.up, &ml.down}) {
+            v->ptr = p;
+            v->bytes = per;
+            p += Carver::round(per);
+        }
+    }
+    M->rcap = nr;
+    return EMFA_OK;
+}
+
+// Set-up.  The device has about 1.3 ms of work at 43 k unknowns (singular
+// table, patterns, near field, translation series), the host about 3 ms
+// (tree and lists, series, stencils), and 120 allocations and as many copies
+// had cost 3 ms more with the first product and the release.  So the
+// singular table runs beside the tree, patterns and near field beside the
+// level tables, and the tables travel as two buffers: 10.6 -> 4.2 ms, with a
+// first product of four right-hand sides and the release 13.4 -> 6.1.
 static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
 {
     Ctx* c = M->ctx;
     Geom* g = M->geom;
     const int n = g->n;
     M->n = n;
+    emfa_fill_params_t fp{EMFA_CFIE, EMFA_F32, M->p.freq, M->p.alpha, 0, 0, 0};
+    Stage fine, tables, series;  // series: read by k_trans_table only
+    struct Landed {  // no return leaves a copy from the stages in flight
+        cudaStream_t s;
+        ~Landed() { cudaStreamSynchronize(s); }
+    } landed{st};
+    DevBuf tab;
+    EMFA_TRY(geom_prepare_f32(g, st));
+    EMFA_TRY(tab.alloc(c, sizeof(double2) * (size_t)g->nt * 9));
+    EMFA_TRY(build_singular_table(c, g, &fp, dptr<double2>(tab), st));
     Plan P;
     std::string err;
     if (!build_plan(g->verts, g->nv, g->rwg, n, M->p, P, err)) {
@@ -1359,20 +1493,16 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     const float k = P.k;
     M->k = k;
     M->levels = L;
-    auto& lb = P.lb;
+    auto& lev = P.lev;
     auto& gt = P.gt;
     auto& gp = P.gp;
     auto& gw = P.gw;
     auto& kd = P.kd;
-    const auto& fin = lb[L];
+    const auto& fin = lev[L].b;
     M->level_boxes.clear();
-    for (int l = 0; l <= L; ++l) M->level_boxes.push_back((int)lb[l].size());
+    for (int l = 0; l <= L; ++l) M->level_boxes.push_back((int)lev[l].b.size());
     M->perm = P.perm;
     M->poles = P.poles;
-    std::vector<int>& box_of_h = P.box_of;
-    std::vector<int>& off_h = P.off;
-    std::vector<int>& cnt_h = P.cnt;
-    std::vector<float>& cen_h = P.cen;
     const int nl = L - 1;
     if (nl > TRANS_LEVELS) {
         set_error(c, "mlfma: more than " + std::to_string(TRANS_LEVELS + 1) + " octree levels (box threshold too small)");
@@ -1383,22 +1513,118 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     for (int l = 2; l <= L; ++l) {
         const int i = l - 2;
         MLevel& ml = M->lv[i];
-        ml.nbox = (int)lb[l].size();
+        ml.nbox = (int)lev[l].b.size();
         ml.L = P.poles[i];
         ml.K = 2 * ml.L * ml.L;
         ml.len = P.blen[l];
+        if ((size_t)3 * ml.nbox * ml.K > 0xffffffffull) {
+            set_error(c, "mlfma: level patterns exceed 2^32 values");
+            return EMFA_ERR_UNSUPPORTED;
+        }
     }
     // the interpolation and anterpolation passes may use more than the default 48 KB of shared memory
     EMFA_TRY(ensure_smem(c, k_upward, 96 * 1024));
     EMFA_TRY(ensure_smem(c, k_downward, 200 * 1024));
     EMFA_TRY(ensure_smem(c, k_translate, TRANS_SMEM));
-    // per-level device tables
+    // finest-level lists and tables
+    MLevel& fl = M->lv[nl - 1];
+    const int Kf = fl.K;
+    DevView cen_d, kdir_d;
+    {
+        std::vector<float> coeff(Kf);
+        const float PIh = 0.5f * mh::PI;
+        size_t q = 0;
+        for (int pp = 0; pp < 2 * fl.L; ++pp)
+            for (int t = 0; t < fl.L; ++t, ++q)
+                coeff[q] = (float)(gw[nl - 1][q] * std::sin((double)(PIh * (gt[nl - 1][t] + 1))));
+        const float z0 = 120.0f * mh::PI;
+        const float cn = k * k * z0 / 32;
+        for (auto& v : coeff) v = cn * v;
+        fine.put(M->coeff, coeff);
+    }
+    fine.put(M->perm_d, M->perm);
+    fine.put(M->box_of, P.box_of);
+    fine.put(M->box_off, P.off);
+    fine.put(M->box_cnt, P.cnt);
+    fine.put(cen_d, P.cen);
+    fine.put(kdir_d, kd[nl - 1]);
+    // theta_hat, phi_hat of every finest sample direction (FP64 from the
+    // sample's float direction, stored in float): phi_hat = z x k / |z x k|,
+    // theta_hat = phi_hat x k (the Gauss-Legendre theta nodes avoid the poles)
+    {
+        std::vector<float> tp((size_t)6 * Kf);
+        const auto& kv = kd[nl - 1];
+        for (int kk = 0; kk < Kf; ++kk) {
+            const double kx = kv[3 * kk], ky = kv[3 * kk + 1], kz = kv[3 * kk + 2];
+            const double rho = std::sqrt(kx * kx + ky * ky);
+            const double px = -ky / rho, py = kx / rho;
+            const double tx = py * kz, ty = -px * kz, tz = px * ky - py * kx;
+            const double tv[6] = {tx, ty, tz, px, py, 0.0};
+            for (int j = 0; j < 6; ++j) tp[(size_t)j * Kf + kk] = (float)tv[j];
+        }
+        fine.put(M->tp, tp);
+    }
+    // near field: column bases, row bases
+    const int nfin = (int)fin.size();
+    std::vector<int> ncol, rcols, cbase{0};
+    std::vector<size_t> rbase;
+    size_t nnz = 0;
+    ncol.reserve(lev[L].near.size());
+    for (int b = 0; b < nfin; ++b) {
+        int cols = 0;
+        for (int sl = lev[L].nptr[b]; sl < lev[L].nptr[b + 1]; ++sl) {
+            ncol.push_back(cols);
+            cols += fin[lev[L].near[sl]].count;
+        }
+        rcols.push_back(cols);
+        cbase.push_back(cbase.back() + cols);
+        M->max_cols = std::max(M->max_cols, cols);
+        rbase.push_back(nnz);
+        nnz += (size_t)cols * fin[b].count;
+    }
+    M->nnz = nnz;
+    fine.put(M->near_ptr, lev[L].nptr);
+    fine.put(M->near_box, lev[L].near);
+    fine.put(M->near_col, ncol);
+    fine.put(M->row_cols, rcols);
+    fine.put(M->row_base, rbase);
+    fine.put(M->near_cbase, cbase);
+    EMFA_TRY(fine.upload(c, M->fine_tables, st));
+    EMFA_TRY(M->near_cidx.alloc(c, sizeof(int) * (size_t)std::max(cbase.back(), 1)));
+    EMFA_TRY(M->near_val.alloc(c, sizeof(float2) * std::max<size_t>(nnz, 1)));
+    EMFA_TRY(M->rad.alloc(c, sizeof(C2f) * (size_t)n * Kf));
+    EMFA_TRY(M->rec.alloc(c, sizeof(C2f) * (size_t)n * Kf));
+    {
+        k_near_cidx<<<(unsigned)((nfin + 3) / 4), 128, 0, st>>>(
+            nfin, dptr<int>(M->near_ptr), dptr<int>(M->near_box), dptr<int>(M->near_col), dptr<int>(M->box_off),
+            dptr<int>(M->box_cnt), dptr<int>(M->near_cbase), dptr<int>(M->near_cidx));
+        FillConst<float> fc = make_fill_const<float>(&fp);
+        k_near_fill<<<(unsigned)(((size_t)n * 32 + 127) / 128), 128, 0, st>>>(
+            dptr<RwgPack<float>>(g->g32.rwg), dptr<int>(M->perm_d), dptr<int>(M->box_of), dptr<int>(M->box_off),
+            dptr<int>(M->row_cols), dptr<size_t>(M->row_base), dptr<int>(M->near_cbase), dptr<int>(M->near_cidx), n,
+            fc, dptr<double2>(tab), dptr<float2>(M->near_val));
+        const size_t tot = (size_t)n * Kf;
+        k_radrec<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(dptr<RwgPack<float>>(g->g32.rwg), dptr<int>(M->perm_d),
+                                                               dptr<int>(M->box_of), dptr<float>(cen_d),
+                                                               dptr<float>(kdir_d), dptr<float>(M->tp), n, Kf, k,
+                                                               (float)M->p.alpha, dptr<C2f>(M->rad),
+                                                               dptr<C2f>(M->rec));
+        c->kernel_launches += 3;
+        EMFA_CUDA(c, cudaGetLastError());
+    }
+    // per-level tables
+    struct Series {
+        DevView hl, rec, minl, kd;
+    };
+    std::vector<Series> sv(nl);
     for (int l = 2; l <= L; ++l) {
         const int i = l - 2;
         MLevel& ml = M->lv[i];
         const int K = ml.K;
+        const auto& bx = lev[l].b;
+        const auto& up = lev[l - 1];
         std::vector<int> par, oc, cptr{0}, cidx;
-        for (auto& b : lb[l]) {
+        for (auto& b : bx) {
             par.push_back(b.parent);
             oc.push_back(b.oct);
         }
@@ -1406,56 +1632,54 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         // near its parent that are not near itself (setBoxParameter), in that order
         std::vector<TransGroup> grp;
         std::vector<int2> gsrc;
-        if ((size_t)3 * ml.nbox * K > 0xffffffffull) {
-            set_error(c, "mlfma: level patterns exceed 2^32 values");
-            return EMFA_ERR_UNSUPPORTED;
-        }
-        for (auto& pb : lb[l - 1]) {
-            float o[3];  // centre of the parent's first octant
-            for (int d = 0; d < 3; ++d) o[d] = pb.c[d] - 0.5f * ml.len;
+        for (int self = 0; self < (int)up.b.size(); ++self) {
+            const mh::Box& pb = up.b[self];
             const int s0 = (int)gsrc.size();
-            const int self = (int)(&pb - lb[l - 1].data());
-            for (int pn : pb.near)
-                for (int f : lb[l - 1][pn].child) {
-                    if (pn == self) break;  // the siblings are near one another
-                    const float* a = lb[l][f].c;
+            for (int sl = up.nptr[self]; sl < up.nptr[self + 1]; ++sl) {
+                const int pn = up.near[sl];
+                if (pn == self) continue;  // the siblings are near one another
+                const mh::Box& nbx = up.b[pn];
+                for (int f = nbx.child0; f < nbx.child0 + nbx.nchild; ++f) {
+                    // from the source box to the parent's first octant, in boxes
                     int off = 0;
-                    for (int d = 0; d < 3; ++d) off = 7 * off + (int)std::lround((o[d] - a[d]) / ml.len) + 3;
+                    for (int d = 0; d < 3; ++d) off = 7 * off + (2 * pb.ix[d] - bx[f].ix[d]) + 3;
                     gsrc.push_back(make_int2((int)(unsigned)((size_t)3 * f * K), off * TRANS_K));
                 }
+            }
             // the offset (0, 0, 0) is near for every octant: T = 0
             while (gsrc.size() % TRANS_BATCH) gsrc.push_back(make_int2(gsrc.back().x, 171 * TRANS_K));  // gsrc.size() > s0 here
-            const int nc = (int)pb.child.size(), parts = (nc + TRANS_NC - 1) / TRANS_NC;
+            const int nc = pb.nchild, parts = (nc + TRANS_NC - 1) / TRANS_NC;
             for (int q = 0; q < parts; ++q) {
-                TransGroup g{};
-                g.s0 = s0;
-                g.s1 = (int)gsrc.size();
+                TransGroup tg{};
+                tg.s0 = s0;
+                tg.s1 = (int)gsrc.size();
                 for (int j = nc * q / parts; j < nc * (q + 1) / parts; ++j) {
-                    const int oct = lb[l][pb.child[j]].oct;
-                    g.child[g.nc++] = make_int2(pb.child[j], (49 * (oct >> 2) + 7 * ((oct >> 1) & 1) + (oct & 1)) * TRANS_K);
+                    const int o = bx[pb.child0 + j].oct;
+                    tg.child[tg.nc++] = make_int2(pb.child0 + j, (49 * (o >> 2) + 7 * ((o >> 1) & 1) + (o & 1)) * TRANS_K);
                 }
-                grp.push_back(g);
+                grp.push_back(tg);
             }
         }
         ml.ngrp = (int)grp.size();
         if (l < L)
-            for (auto& b : lb[l]) {
-                for (int ch : b.child) cidx.push_back(ch);
+            for (auto& b : bx) {
+                for (int ch = b.child0; ch < b.child0 + b.nchild; ++ch) cidx.push_back(ch);
                 cptr.push_back((int)cidx.size());
             }
-        EMFA_TRY(upload(c, ml.parent, par, st));
-        EMFA_TRY(upload(c, ml.oct, oc, st));
-        EMFA_TRY(upload(c, ml.grp_src, gsrc, st));
-        EMFA_TRY(upload(c, ml.grp, grp, st));
-        EMFA_TRY(upload(c, ml.child_ptr, cptr, st));
-        EMFA_TRY(upload(c, ml.child_idx, cidx, st));
+        tables.put(ml.parent, par);
+        tables.put(ml.oct, oc);
+        tables.put(ml.grp_src, gsrc);
+        tables.put(ml.grp, grp);
+        tables.put(ml.child_ptr, cptr);
+        tables.put(ml.child_idx, cidx);
         // translation operators per offset: sum_l (2l+1)(-j)^l h_l^(2)(kD) P_l(k.D/|D|),
         // l <= min(poles, floor(kD)) (MLFMA.cpp:1203-1219), in FP64: the Hankel
-        // recurrence per offset here, the Legendre sums per sample on the device
+        // recurrence per distance here, the Legendre sums per sample on the device
         {
             const int lmax = ml.L;
             std::vector<double2> hlv((size_t)343 * (lmax + 1), make_double2(0, 0));
             std::vector<int> minl(343, -1);
+            std::vector<std::pair<double, int>> dist;  // distances so far and an offset of each
             for (int dx = -3; dx <= 3; ++dx)
                 for (int dy = -3; dy <= 3; ++dy)
                     for (int dz = -3; dz <= 3; ++dz) {
@@ -1466,6 +1690,16 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                         double x = (double)k * Dn;
                         int minL = (int)std::min((float)ml.L, (float)(k * (float)Dn));
                         minL = std::min(minL, lmax);
+                        minl[off] = minL;
+                        double2* out = &hlv[(size_t)off * (lmax + 1)];
+                        // offsets of one distance share the series
+                        size_t same = 0;
+                        while (same < dist.size() && dist[same].first != Dn) ++same;
+                        if (same < dist.size()) {
+                            std::copy_n(&hlv[(size_t)dist[same].second * (lmax + 1)], minL + 1, out);
+                            continue;
+                        }
+                        dist.push_back({Dn, off});
                         std::vector<std::complex<double>> hl(minL + 1);
                         hl[0] = std::complex<double>(std::sin(x), std::cos(x)) / x;
                         if (minL >= 1)
@@ -1474,32 +1708,19 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                         for (int q = 0; q <= minL; ++q) {
                             // (2q+1) (-j)^q h_q
                             const double w = 2.0 * q + 1, hr = w * hl[q].real(), hi = w * hl[q].imag();
-                            hlv[(size_t)off * (lmax + 1) + q] = (q & 3) == 0   ? make_double2(hr, hi)
-                                                                : (q & 3) == 1 ? make_double2(hi, -hr)
-                                                                : (q & 3) == 2 ? make_double2(-hr, -hi)
-                                                                               : make_double2(-hi, hr);
+                            out[q] = (q & 3) == 0   ? make_double2(hr, hi)
+                                     : (q & 3) == 1 ? make_double2(hi, -hr)
+                                     : (q & 3) == 2 ? make_double2(-hr, -hi)
+                                                    : make_double2(-hi, hr);
                         }
-                        minl[off] = minL;
                     }
             std::vector<double2> recv(lmax + 1, make_double2(0, 0));
             for (int q = 1; q <= lmax; ++q) recv[q] = make_double2((2.0 * q - 1) / q, (q - 1.0) / q);
-            DevBuf d_hl, d_rec, d_minl, d_kd;
-            EMFA_TRY(upload(c, d_hl, hlv, st));
-            EMFA_TRY(upload(c, d_rec, recv, st));
-            EMFA_TRY(upload(c, d_minl, minl, st));
-            EMFA_TRY(upload(c, d_kd, kd[i], st));
-            EMFA_TRY(ml.trans.alloc(c, sizeof(float2) * (size_t)343 * K));
-            const size_t tot = (size_t)343 * K;
-            k_trans_table<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(dptr<double2>(d_hl), dptr<double2>(d_rec),
-                                                                         dptr<int>(d_minl), lmax,
-                                                                         dptr<float>(d_kd), K, (double)ml.len,
-                                                                         dptr<float2>(ml.trans));
-            c->kernel_launches += 1;
-            EMFA_CUDA(c, cudaGetLastError());
-            EMFA_CUDA(c, cudaStreamSynchronize(st));  // host vectors and the small tables are released next
+            series.put(sv[i].hl, hlv);
+            series.put(sv[i].rec, recv);
+            series.put(sv[i].minl, minl);
+            series.put(sv[i].kd, kd[i]);
         }
-        EMFA_TRY(ml.up.alloc(c, sizeof(float2) * 3 * (size_t)ml.nbox * K));
-        EMFA_TRY(ml.down.alloc(c, sizeof(float2) * 3 * (size_t)ml.nbox * K));
     }
     // translation work: up to 24 groups a CTA (two a warp and right-hand side, so
     // that the table's staging is a few percent), fewer where that leaves SMs idle
@@ -1518,8 +1739,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                                            (int)((long long)ml.ngrp * (p + 1) / parts)});
         }
         M->trans_ctas = (int)tw.size();
-        EMFA_TRY(upload(c, M->trans_work, tw, st));
-        EMFA_CUDA(c, cudaStreamSynchronize(st));  // tw goes out of scope
+        tables.put(M->trans_work, tw);
     }
     // interpolation level i+1 (child, fewer samples) -> level i (parent), i = 0..nl-2
     for (int i = 0; i + 1 < nl; ++i) {
@@ -1530,10 +1750,10 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         mh::lagrange(gt[i + 1], gt[i], tloc, tel);
         mh::lagrange(gp[i + 1], gp[i], ploc, pel);
         const int Kp = pm.K, Lc = cm.L;
-        EMFA_TRY(upload(c, pm.ip_tl, tloc, st));
-        EMFA_TRY(upload(c, pm.ip_te, tel, st));
-        EMFA_TRY(upload(c, pm.ip_pl, ploc, st));
-        EMFA_TRY(upload(c, pm.ip_pe, pel, st));
+        tables.put(pm.ip_tl, tloc);
+        tables.put(pm.ip_te, tel);
+        tables.put(pm.ip_pl, ploc);
+        tables.put(pm.ip_pe, pel);
         {
             // phi-row chunks of about 256 parent samples and the child rows each reads
             pm.up_rows = down_rows(pm.L);
@@ -1556,7 +1776,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                 set_error(c, "mlfma: interpolation rows exceed shared memory (level too large)");
                 return EMFA_ERR_UNSUPPORTED;
             }
-            EMFA_TRY(upload(c, pm.up_win, win, st));
+            tables.put(pm.up_win, win);
         }
         // phases for the children of level i: exp(-j k kp . (parent - child)), per octant
         std::vector<float2> ph((size_t)8 * Kp);
@@ -1569,7 +1789,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                 ph[(size_t)o * Kp + kk] = make_float2((float)std::cos(a), (float)-std::sin(a));
             }
         }
-        EMFA_TRY(upload(c, pm.up_phase, ph, st));
+        tables.put(pm.up_phase, ph);
         // anterpolation into level i+1: the transposed theta and phi Lagrange
         // stencils, each weight scaled by w_parent / w_child of its own axis
         // (the 2-D weights are products: gw = wp x wt)
@@ -1599,12 +1819,12 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
             std::vector<float> tw, pw;
             transpose(tloc, tel, Lp, Lc, P.wt1[i], P.wt1[i + 1], tptr, tsrc, tw);
             transpose(ploc, pel, 2 * Lp, 2 * Lc, P.wp1[i], P.wp1[i + 1], pptr, psrc, pw);
-            EMFA_TRY(upload(c, cm.th_ptr, tptr, st));
-            EMFA_TRY(upload(c, cm.th_src, tsrc, st));
-            EMFA_TRY(upload(c, cm.th_w, tw, st));
-            EMFA_TRY(upload(c, cm.ph_ptr, pptr, st));
-            EMFA_TRY(upload(c, cm.ph_src, psrc, st));
-            EMFA_TRY(upload(c, cm.ph_w, pw, st));
+            tables.put(cm.th_ptr, tptr);
+            tables.put(cm.th_src, tsrc);
+            tables.put(cm.th_w, tw);
+            tables.put(cm.ph_ptr, pptr);
+            tables.put(cm.ph_src, psrc);
+            tables.put(cm.ph_w, pw);
             // phi-row chunks of about 256 samples, and the parent rows each reads
             const int rows = down_rows(Lc);
             const int nchunk = (2 * Lc + rows - 1) / rows;
@@ -1626,111 +1846,33 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                 set_error(c, "mlfma: anterpolation rows exceed shared memory (level too large)");
                 return EMFA_ERR_UNSUPPORTED;
             }
-            EMFA_TRY(upload(c, cm.down_win, dw, st));
+            tables.put(cm.down_win, dw);
         }
     }
-    // finest-level data
-    MLevel& fl = M->lv[nl - 1];
-    const int Kf = fl.K;
-    std::vector<float> coeff(Kf);
-    {
-        const float PIh = 0.5f * mh::PI;
-        size_t q = 0;
-        const int P = fl.L;
-        for (int pp = 0; pp < 2 * P; ++pp)
-            for (int t = 0; t < P; ++t, ++q) coeff[q] = (float)(gw[nl - 1][q] * std::sin((double)(PIh * (gt[nl - 1][t] + 1))));
-        const float z0 = 120.0f * mh::PI;
-        const float cn = k * k * z0 / 32;
-        for (auto& v : coeff) v = cn * v;
-    }
-    EMFA_TRY(upload(c, M->coeff, coeff, st));
-    EMFA_TRY(upload(c, M->perm_d, M->perm, st));
-    EMFA_TRY(upload(c, M->box_of, box_of_h, st));
-    EMFA_TRY(upload(c, M->box_off, off_h, st));
-    EMFA_TRY(upload(c, M->box_cnt, cnt_h, st));
-    DevBuf cen_d, kdir_d;
-    EMFA_TRY(upload(c, cen_d, cen_h, st));
-    EMFA_TRY(upload(c, kdir_d, kd[nl - 1], st));
-    EMFA_TRY(geom_prepare_f32(g, st));
-    // theta_hat, phi_hat of every finest sample direction (FP64 from the
-    // sample's float direction, stored in float): phi_hat = z x k / |z x k|,
-    // theta_hat = phi_hat x k (the Gauss-Legendre theta nodes avoid the poles)
-    {
-        std::vector<float> tp((size_t)6 * Kf);
-        const auto& kv = kd[nl - 1];
-        for (int kk = 0; kk < Kf; ++kk) {
-            const double kx = kv[3 * kk], ky = kv[3 * kk + 1], kz = kv[3 * kk + 2];
-            const double rho = std::sqrt(kx * kx + ky * ky);
-            const double px = -ky / rho, py = kx / rho;
-            const double tx = py * kz, ty = -px * kz, tz = px * ky - py * kx;
-            const double tv[6] = {tx, ty, tz, px, py, 0.0};
-            for (int j = 0; j < 6; ++j) tp[(size_t)j * Kf + kk] = (float)tv[j];
-        }
-        EMFA_TRY(upload(c, M->tp, tp, st));
-    }
-    EMFA_TRY(M->rad.alloc(c, sizeof(C2f) * (size_t)n * Kf));
-    EMFA_TRY(M->rec.alloc(c, sizeof(C2f) * (size_t)n * Kf));
-    {
-        size_t tot = (size_t)n * Kf;
-        k_radrec<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(dptr<RwgPack<float>>(g->g32.rwg), dptr<int>(M->perm_d),
-                                                               dptr<int>(M->box_of), dptr<float>(cen_d),
-                                                               dptr<float>(kdir_d), dptr<float>(M->tp), n, Kf, k,
-                                                               (float)M->p.alpha, dptr<C2f>(M->rad),
-                                                               dptr<C2f>(M->rec));
+    EMFA_TRY(tables.upload(c, M->level_tables, st));
+    DevBuf series_d;
+    EMFA_TRY(series.upload(c, series_d, st));
+    size_t tt = 0;
+    for (auto& ml : M->lv) tt += Carver::round(sizeof(float2) * (size_t)343 * ml.K);
+    EMFA_TRY(M->trans_tables.alloc(c, tt));
+    EMFA_TRY(alloc_patterns(M, 1));
+    tt = 0;
+    for (int i = 0; i < nl; ++i) {
+        MLevel& ml = M->lv[i];
+        const size_t tot = (size_t)343 * ml.K;
+        ml.trans.ptr = (char*)M->trans_tables.ptr + tt;
+        ml.trans.bytes = sizeof(float2) * tot;
+        tt += Carver::round(ml.trans.bytes);
+        k_trans_table<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(dptr<double2>(sv[i].hl), dptr<double2>(sv[i].rec),
+                                                                     dptr<int>(sv[i].minl), ml.L,
+                                                                     dptr<float>(sv[i].kd), ml.K, (double)ml.len,
+                                                                     dptr<float2>(ml.trans));
         c->kernel_launches += 1;
     }
-    // near field: CSR of near boxes, column bases, row bases
-    std::vector<int> nptr{0}, nbox, ncol, rcols;
-    std::vector<size_t> rbase;
-    size_t nnz = 0;
-    for (size_t b = 0; b < fin.size(); ++b) {
-        int cols = 0;
-        for (int nb : fin[b].near) {
-            nbox.push_back(nb);
-            ncol.push_back(cols);
-            cols += (int)fin[nb].unk.size();
-        }
-        nptr.push_back((int)nbox.size());
-        rcols.push_back(cols);
-        M->max_cols = std::max(M->max_cols, cols);
-        rbase.push_back(nnz);
-        nnz += (size_t)cols * fin[b].unk.size();
-    }
-    M->nnz = nnz;
-    {
-        // column unknowns of each box's near rows, in value order
-        std::vector<int> cbase{0}, cidx;
-        for (size_t b = 0; b < fin.size(); ++b) {
-            for (int nb : fin[b].near)
-                for (int q = 0; q < cnt_h[nb]; ++q) cidx.push_back(off_h[nb] + q);
-            cbase.push_back((int)cidx.size());
-        }
-        EMFA_TRY(upload(c, M->near_cbase, cbase, st));
-        EMFA_TRY(upload(c, M->near_cidx, cidx, st));
-    }
-    EMFA_TRY(upload(c, M->near_ptr, nptr, st));
-    EMFA_TRY(upload(c, M->near_box, nbox, st));
-    EMFA_TRY(upload(c, M->near_col, ncol, st));
-    EMFA_TRY(upload(c, M->row_cols, rcols, st));
-    EMFA_TRY(upload(c, M->row_base, rbase, st));
-    EMFA_TRY(M->near_val.alloc(c, sizeof(float2) * std::max<size_t>(nnz, 1)));
-    {
-        emfa_fill_params_t fp{EMFA_CFIE, EMFA_F32, M->p.freq, M->p.alpha, 0, 0, 0};
-        DevBuf tab;
-        EMFA_TRY(tab.alloc(c, sizeof(double2) * (size_t)g->nt * 9));
-        EMFA_TRY(build_singular_table(c, g, &fp, dptr<double2>(tab), st));
-        FillConst<float> fc = make_fill_const<float>(&fp);
-        k_near_fill<<<(unsigned)(((size_t)n * 32 + 127) / 128), 128, 0, st>>>(
-            dptr<RwgPack<float>>(g->g32.rwg), dptr<int>(M->perm_d), dptr<int>(M->box_of), dptr<int>(M->box_off),
-            dptr<int>(M->row_cols), dptr<size_t>(M->row_base), dptr<int>(M->near_cbase), dptr<int>(M->near_cidx), n,
-            fc, dptr<double2>(tab), dptr<float2>(M->near_val));
-        c->kernel_launches += 1;
-        EMFA_CUDA(c, cudaGetLastError());
-        EMFA_CUDA(c, cudaStreamSynchronize(st));
-    }
+    EMFA_CUDA(c, cudaGetLastError());
     if (M->p.precond) EMFA_TRY(sai_build(M, P, st));
     EMFA_CUDA(c, cudaGetLastError());
-    EMFA_CUDA(c, cudaStreamSynchronize(st));
+    EMFA_CUDA(c, cudaStreamSynchronize(st));  // the host tables and the temporary buffers are released on return
     return EMFA_OK;
 }
 
@@ -1738,17 +1880,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
 constexpr int RHS_CHUNK = 8;
 
 // level patterns for nr right-hand sides (scratch: grown, never copied)
-static emfa_status_t reserve_rhs(emfa_mlfma* M, int nr)
-{
-    if (nr <= M->rcap) return EMFA_OK;
-    for (auto& ml : M->lv) {
-        const size_t per = sizeof(float2) * 3 * (size_t)ml.nbox * ml.K;
-        EMFA_TRY(ml.up.alloc(M->ctx, per * nr));
-        EMFA_TRY(ml.down.alloc(M->ctx, per * nr));
-    }
-    M->rcap = nr;
-    return EMFA_OK;
-}
+static emfa_status_t reserve_rhs(emfa_mlfma* M, int nr) { return nr <= M->rcap ? EMFA_OK : alloc_patterns(M, nr); }
 
 // shared bytes of k_finish<RB>
 static size_t finish_smem(emfa_mlfma* M, int rb)
@@ -1975,7 +2107,7 @@ emfa_status_t emfa_mlfma_plan(const double* verts_host, int n_vert, const int* r
     *levels = P.L;
     if (level_boxes) {
         if (level_cap < P.L + 1) return EMFA_ERR_INVALID;
-        for (int l = 0; l <= P.L; ++l) level_boxes[l] = (int)P.lb[l].size();
+        for (int l = 0; l <= P.L; ++l) level_boxes[l] = (int)P.lev[l].b.size();
     }
     if (poles)
         for (size_t i = 0; i < P.poles.size(); ++i) poles[i] = P.poles[i];
