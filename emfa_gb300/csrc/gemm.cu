@@ -16,6 +16,9 @@
 #include "gemm.cuh"
 
 #include <algorithm>
+#include <climits>
+
+#include <algorithm>
 
 namespace emfa {
 
@@ -238,9 +241,231 @@ static emfa_status_t cgemv_blocks(Ctx* c, const void* Z, size_t ldz, const void*
     return EMFA_OK;
 }
 
-emfa_status_t cgemv_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)
+// ---------------------------------------------------------------------------
+// FP32 product of a block of right-hand sides on the CUDA cores: a cluster of
+// CTAs per tile of 16 FT rows of Z and 8 RT right-hand sides, each CTA a part
+// of k.  Bound by the FP32 FMAs: a thread keeps FT x RT sums, so FT + RT
+// 8-byte reads of shared memory feed 4 FT RT FMAs.  Both operands are rows
+// along k, copied 16 k at a time (cp.async, CT_STAGES deep) into rows of 17
+// elements: the 16 rows that half a warp reads lie in distinct banks.  The
+// cluster's partial sums meet in distributed shared memory, added in rank
+// order: the parts fill the SMs where n / (16 FT) tiles do not, shorten the
+// sums (and with them their error), and need no scratch.  Up to 40
+// right-hand sides a thread also closes its sums every 64 k: the error at
+// n = 5067, 6.5e-7 -> 2.2e-7.
+// us on GB300 | GEMV (up to 32) or digit planes: 480 x 37, 38 | 57; 1033 x 37,
+// 52 | 68; 2000 x 17, 56 | 67, x 37, 68 | 102, x 80, 96 | 125; 3000 x 37,
+// 102 | 156; 5067 x 16, 123 | 252, x 37, 205 | 350 (FMA rate: 103, 111 with
+// the padding to 40), x 80, 403 | 483.  The 64 x 64 tiles below took 97, 170,
+// 299, 308, 465, 801 and 814 for the ones of 17 and 37.
+// ---------------------------------------------------------------------------
+constexpr int CT_THREADS = 128, CT_BK = 16, CT_LD = CT_BK + 1, CT_STAGES = 3, CT_SPLITS = 8, CT_FLUSH = 4;
+
+constexpr int ct_resident(int rt) { return rt <= 5 ? 4 : 3; }  // CTAs an SM
+
+__device__ __forceinline__ void cp_async8_zfill(void* smem, const void* gmem, bool in)
 {
-    return cgemv_blocks<float>(c, Z, ldz, X, n, nrhs, Y, st);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
+                 "l"(gmem), "r"(in ? 8 : 0)
+                 : "memory");
+}
+
+template <int FT, int RT>
+__global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const float2* __restrict__ Z, size_t ldz,
+                                                      const float2* __restrict__ X, int n, int nrhs, int kper,
+                                                      float2* __restrict__ Y)
+{
+    constexpr int BM = 16 * FT, BN = 8 * RT, STAGE = (BM + BN) * CT_LD;
+    extern __shared__ float2 s_ct[];  // [stage][BM + BN][CT_LD], then the partial sums [BN][BM]
+    const int tid = threadIdx.x, tf = tid & 15, tr = tid >> 4;
+    const int f0 = blockIdx.y * BM, r0 = blockIdx.z * BN;
+    const int rank = blockIdx.x, csize = gridDim.x;
+    const int k0 = rank * kper, k1 = min(n, k0 + kper), steps = k1 > k0 ? (k1 - k0 + CT_BK - 1) / CT_BK : 0;
+    const auto load = [&](int t) {
+        float2* st = s_ct + (t % CT_STAGES) * STAGE;
+        const int k = k0 + t * CT_BK + tf;
+#pragma unroll
+        for (int i = 0; i < BM / 8; ++i) {
+            const int f = tr + 8 * i;
+            const bool in = k < k1 && f0 + f < n;
+            cp_async8_zfill(st + f * CT_LD + tf, Z + (in ? (size_t)(f0 + f) * ldz + k : 0), in);
+        }
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+            const int r = tr + 8 * i;
+            const bool in = k < k1 && r0 + r < nrhs;
+            cp_async8_zfill(st + (BM + r) * CT_LD + tf, X + (in ? (size_t)(r0 + r) * n + k : 0), in);
+        }
+    };
+    constexpr bool TWO = FT * RT <= 20;  // sums of CT_FLUSH steps, and their sum
+    float2 acc[FT][RT], tot[TWO ? FT : 1][TWO ? RT : 1];
+#pragma unroll
+    for (int i = 0; i < FT; ++i)
+#pragma unroll
+        for (int j = 0; j < RT; ++j) {
+            acc[i][j] = make_float2(0.f, 0.f);
+            if constexpr (TWO) tot[i][j] = make_float2(0.f, 0.f);
+        }
+#pragma unroll
+    for (int t = 0; t < CT_STAGES - 1; ++t) {
+        if (t < steps) load(t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int t = 0; t < steps; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(CT_STAGES - 2) : "memory");
+        __syncthreads();  // stage t has landed for every thread, and stage t - 1 has been read
+        if (t + CT_STAGES - 1 < steps) load(t + CT_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float2* A = s_ct + (t % CT_STAGES) * STAGE + tf * CT_LD;
+        const float2* B = s_ct + (t % CT_STAGES) * STAGE + (BM + tr) * CT_LD;
+#pragma unroll 4
+        for (int kk = 0; kk < CT_BK; ++kk) {
+            float2 a[FT], b[RT];
+#pragma unroll
+            for (int i = 0; i < FT; ++i) a[i] = A[16 * i * CT_LD + kk];
+#pragma unroll
+            for (int j = 0; j < RT; ++j) b[j] = B[8 * j * CT_LD + kk];
+#pragma unroll
+            for (int i = 0; i < FT; ++i)
+#pragma unroll
+                for (int j = 0; j < RT; ++j) {
+                    acc[i][j].x = fmaf(a[i].x, b[j].x, acc[i][j].x);
+                    acc[i][j].y = fmaf(a[i].x, b[j].y, acc[i][j].y);
+                    acc[i][j].x = fmaf(-a[i].y, b[j].y, acc[i][j].x);
+                    acc[i][j].y = fmaf(a[i].y, b[j].x, acc[i][j].y);
+                }
+        }
+        if constexpr (TWO)
+            if (t % CT_FLUSH == CT_FLUSH - 1 || t == steps - 1) {
+#pragma unroll
+                for (int i = 0; i < FT; ++i)
+#pragma unroll
+                    for (int j = 0; j < RT; ++j) {
+                        tot[i][j].x += acc[i][j].x;
+                        tot[i][j].y += acc[i][j].y;
+                        acc[i][j] = make_float2(0.f, 0.f);
+                    }
+            }
+    }
+    if constexpr (TWO) {
+#pragma unroll
+        for (int i = 0; i < FT; ++i)
+#pragma unroll
+            for (int j = 0; j < RT; ++j) acc[i][j] = tot[i][j];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (csize == 1) {
+#pragma unroll
+        for (int j = 0; j < RT; ++j)
+#pragma unroll
+            for (int i = 0; i < FT; ++i) {
+                const int f = f0 + tf + 16 * i, r = r0 + tr + 8 * j;
+                if (f < n && r < nrhs) Y[(size_t)r * n + f] = acc[i][j];
+            }
+        return;
+    }
+    __syncthreads();  // the last stages have been read
+#pragma unroll
+    for (int j = 0; j < RT; ++j)
+#pragma unroll
+        for (int i = 0; i < FT; ++i) s_ct[(tr + 8 * j) * BM + tf + 16 * i] = acc[i][j];
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // rank's share of the tile, from every part in rank order
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_ct);
+    for (int q = rank * CT_THREADS + tid; q < BM * BN; q += csize * CT_THREADS) {
+        const int f = f0 + q % BM, r = r0 + q / BM;
+        if (f >= n || r >= nrhs) continue;
+        float2 v[CT_SPLITS], t = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < CT_SPLITS; ++c)
+            if (c < csize) {
+                uint32_t ra;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(base + 8u * q), "r"(c));
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[c].x), "=f"(v[c].y) : "r"(ra) : "memory");
+            }
+#pragma unroll
+        for (int c = 0; c < CT_SPLITS; ++c)
+            if (c < csize) {
+                t.x += v[c].x;
+                t.y += v[c].y;
+            }
+        Y[(size_t)r * n + f] = t;
+    }
+    // no CTA leaves while another may still read its sums
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int FT, int RT>
+static emfa_status_t launch_ctile(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                                  cudaStream_t st)
+{
+    constexpr int BM = 16 * FT, BN = 8 * RT;
+    constexpr size_t stages = sizeof(float2) * CT_STAGES * (BM + BN) * CT_LD, sums = sizeof(float2) * BM * BN;
+    constexpr size_t smem = stages > sums ? stages : sums;
+    EMFA_TRY(ensure_smem(c, k_ctile<FT, RT>, smem));
+    const int ft = (n + BM - 1) / BM, rt = (nrhs + BN - 1) / BN;
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    // parts of k: the fewest steps of the busiest SM, whose CTAs share its
+    // FMAs (below two and a half a SM they wait for their loads instead),
+    // with about four steps a CTA of filling and adding, in one wave
+    int splits = 1;
+    long best = LONG_MAX;
+    for (int q = 1; q <= CT_SPLITS; ++q) {
+        const long per_sm = ((long)ft * rt * q + sms - 1) / sms, steps = (n + q * CT_BK - 1) / (q * CT_BK) + 4;
+        if (q > 1 && per_sm > ct_resident(RT)) break;
+        const long cost = steps * std::max(2 * per_sm, 5L);
+        if (cost < best) {
+            best = cost;
+            splits = q;
+        }
+    }
+    const int kper = ((n + splits - 1) / splits + CT_BK - 1) / CT_BK * CT_BK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)splits, (unsigned)ft, (unsigned)rt);
+    cfg.blockDim = dim3(CT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)splits;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    EMFA_CUDA(c, cudaLaunchKernelEx(&cfg, k_ctile<FT, RT>, (const float2*)Z, ldz, (const float2*)X, n, nrhs, kper,
+                                    (float2*)Y));
+    c->kernel_launches += 1;
+    return EMFA_OK;
+}
+
+static emfa_status_t cgemm_f32_tiles(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                                     cudaStream_t st)
+{
+    // even tiles of up to 80 right-hand sides, eight a step
+    const int blocks = (nrhs + 79) / 80, rt = ((nrhs + blocks - 1) / blocks + 7) / 8;
+    switch (rt) {
+    case 1:
+    case 2: return launch_ctile<4, 2>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 3: return launch_ctile<4, 3>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 4: return launch_ctile<4, 4>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 5: return launch_ctile<4, 5>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 6: return launch_ctile<4, 6>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 7: return launch_ctile<4, 7>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 8: return launch_ctile<4, 8>(c, Z, ldz, X, n, nrhs, Y, st);
+    case 9: return launch_ctile<4, 9>(c, Z, ldz, X, n, nrhs, Y, st);
+    default: return launch_ctile<4, 10>(c, Z, ldz, X, n, nrhs, Y, st);
+    }
+}
+
+// One FP32 product, the kernel chosen (us, GEMV | tiles): the GEMV up to 4
+// right-hand sides (5067 x 3, 102 | 121), below n = 4000 up to 8 (3000 x 8, 74 | 68, x 5,
+// 65 | 68; 5067 x 5, 151 | 121) and below 2500 up to 16 (2000 x 12, 57 | 62;
+// 3000 x 12, 88 | 68; 5067 x 16, 252 | 123).
+emfa_status_t cgemm_f32_block(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                              cudaStream_t st)
+{
+    if (nrhs <= 4 || (nrhs <= 8 && n < 4000) || (nrhs <= 16 && n < 2500)) return cgemv_blocks<float>(c, Z, ldz, X, n, nrhs, Y, st);
+    return cgemm_f32_tiles(c, Z, ldz, X, n, nrhs, Y, st);
 }
 
 emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st)

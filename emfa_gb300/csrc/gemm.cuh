@@ -5,8 +5,11 @@
 namespace emfa {
 
 // Y = Z X on CUDA cores (complex64 / complex128), X and Y RHS-major.
-// cgemm_f32 takes the GEMV up to 16 right-hand sides and 64 x 64 tiles above
-emfa_status_t cgemv_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st);
+// One FP32 product: GEMV or clustered tiles by size; the explicit FP32 product
+// and the solver's operator keep cgemm_f32 and its order of sums: the GEMV up
+// to 16 right-hand sides, 64 x 64 tiles above
+emfa_status_t cgemm_f32_block(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+                              cudaStream_t st);
 emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st);
 emfa_status_t cgemm_f64(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st);
 // Yd (complex128) = Bsub - Z X (Bsub may be null: Yd = Z X), FP32 products,

@@ -604,15 +604,16 @@ bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st)
     return nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
 }
 
-// One FP32 product with its split of Z, above the right-hand sides up to which
-// the GEMV is faster or as fast (us, this | GEMV: n = 480 x 17, 56 | 35, x 33,
-// 56 | 39; 1033 x 33, 68 | 52; 2000 x 17, 97 | 64, x 33, 98 | 102; 3000 x 24, 150 | 98,
-// x 33, 153 | 158; 5067 x 17, 343 | 220, x 24, 346 | 265, x 33, 348 | 360).
-// Errors on normal entries, n = 480 to 5067: this 3e-8, the GEMV, whose lane
-// sums are short, 1.2e-7 to 3.3e-7, 64 x 64 tiles 5.5e-7 to 1.8e-6.
+// One FP32 product with its split of Z, where it beats the CUDA cores' tiles
+// (us, this | tiles: n = 480 x 360, 69 | 56; 1033 x 181, 85 | 72, x 360, 119 | 123;
+// 2000 x 96, 125 | 118, x 128, 129 | 152; 3000 x 80, 202 | 173, x 96, 202 | 183,
+// x 128, 207 | 229; 5067 x 80, 483 | 403, x 96, 488 | 535): above 80 right-hand
+// sides and 200000 results.  Errors on normal entries, n = 480 to 5067: this
+// 3e-8, the tiles 2.1e-7 to 8.1e-7, the GEMV 1.2e-7 to 3.3e-7, 64 x 64 tiles 5.5e-7
+// to 1.8e-6.
 static bool slice_worthwhile_f32(Ctx* c, int n, int nrhs, cudaStream_t st)
 {
-    return slice_allowed(c, sl::Cut<float>::NS, n, st) && nrhs > SLICE_F32_MIN_RHS;
+    return nrhs > 80 && (long)n * nrhs > 200000 && slice_allowed(c, sl::Cut<float>::NS, n, st);
 }
 
 template <typename T>

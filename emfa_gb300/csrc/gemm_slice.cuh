@@ -16,9 +16,6 @@ struct SlicePlanes {
     size_t ldk = 0;
 };
 
-// one FP32 product (automatic choice) takes the planes above this many right-hand sides
-constexpr int SLICE_F32_MIN_RHS = 32;
-
 // FP64: whether a block of nrhs products of n unknowns is worth the planes; built:
 // the planes exist already (a Krylov solve splits Z once).
 bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st);

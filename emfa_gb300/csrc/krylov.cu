@@ -2680,8 +2680,7 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
     bool done = false;
     if (matvec != EMFA_MV_F32) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
     if (done) return EMFA_OK;
-    // above 16 the 64 x 64 tiles stay what an explicit FP32 product runs
-    if (matvec != EMFA_MV_F32 && n_rhs <= SLICE_F32_MIN_RHS) return cgemv_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    if (matvec != EMFA_MV_F32) return cgemm_f32_block(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
     return cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
 }
 

@@ -52,7 +52,7 @@ typedef enum {
                        /* error no larger than an FP64 sum's relative to the row and */
                        /* vector maxima), else FP64 SIMT; F32: EMFA_MV_F16X in solves */
                        /* and residuals, in emfa_matvec FP32 accuracy the same way   */
-                       /* (four digits) above 32 right-hand sides, else FP32 SIMT    */
+                       /* (four digits) for wide blocks (above 80), else FP32 SIMT   */
     EMFA_MV_F64 = 1,   /* FP64 complex product on CUDA cores (plain path)            */
     EMFA_MV_F32 = 2,   /* FP32 complex GEMM on CUDA cores; residual FP32 products    */
                        /* with FP64 chunk sums                                       */
