@@ -411,35 +411,41 @@ __device__ __forceinline__ float2 fsub2_rn(float2 a, float2 b)
 // columns, 5e-6 over the whole row).  Here every k-block (64 real columns)
 // starts a fresh accumulator, the two correction products go first (their
 // partial sums are 2^-11 smaller, so truncating them costs little) and the
-// hi x hi products last; eight epilogue warps drain each k-block into
-// Kahan-compensated FP32 sums in registers (56 columns each) while the next
-// k-block accumulates in the second buffer, and the last step forms
+// hi x hi products last; sixteen epilogue warps drain each k-block into
+// Kahan-compensated FP32 sums in registers (RBN / 4 columns each) while the
+// next k-block accumulates in the second buffer, and the last step forms
 // B - sum / (s t) in FP64.  A drain releases the accumulator as soon as its
-// 56 columns are in registers, before the sums.
+// columns are in registers, before the sums.  Bound by the arrival of the
+// operands (64 bytes a cycle and SM) and the turns between MMAs and drain:
+// at 7680 x 360, five 144-column tiles a row block make two waves, 446 us,
+// seven of 112 three, 525; one right-hand side takes 16 columns (n = 480,
+// 15 -> 12 us).
 // ---------------------------------------------------------------------------
-constexpr int RBN = 112;
 constexpr int REPI = 16;                   // epilogue warps: four per SM sub-partition
-constexpr int RCOLS = RBN * 4 / REPI;      // 28 accumulator columns per epilogue warp
 constexpr int RTHREADS = 32 * (2 + REPI);  // producer, MMA, epilogue
 
+template <int RBN>
 struct RSmem {
+    static constexpr int RCOLS = RBN * 4 / REPI;  // accumulator columns per epilogue warp
     static constexpr int A_BYTES = BM * 128;
     static constexpr int B_BYTES = RBN * 128;
     static constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES);
     static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES;
-    static constexpr int ACC = 128;
-    static constexpr int TMEM_COLS = 256;
+    static constexpr int ACC = RBN <= 16 ? 16 : RBN <= 64 ? 64 : RBN <= 128 ? 128 : 256;
+    static constexpr int TMEM_COLS = 2 * ACC;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 1024 + 256;
 };
 
+template <int RBN>
 __global__ void __launch_bounds__(RTHREADS, 1)
     k_hresid(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
              const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
              const void* __restrict__ Bv, int b_f64, double2* __restrict__ Rout, int M, int R, int kblocks,
              const float* __restrict__ inv_s, const float* __restrict__ inv_t, int* __restrict__ err)
 {
-    using S = RSmem;
+    using S = RSmem<RBN>;
     using namespace tc;
+    constexpr int RCOLS = S::RCOLS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sA = base;                               // [stage][plane]
@@ -549,7 +555,15 @@ __global__ void __launch_bounds__(RTHREADS, 1)
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float v[RCOLS];
-            tmem_ld28(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * S::ACC + col0), v);
+            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * S::ACC + col0);
+            if constexpr (RCOLS == 36)
+                tmem_ld36(ta, v);
+            else if constexpr (RCOLS == 28)
+                tmem_ld28(ta, v);
+            else if constexpr (RCOLS == 16)
+                tmem_ld16(ta, v);
+            else
+                tmem_ld4(ta, v);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + a);
@@ -913,10 +927,33 @@ emfa_status_t hgemm_pack(Ctx* c, const HPlanes& h, const void* X, const HPack& p
     return EMFA_OK;
 }
 
+template <int RBN>
+static emfa_status_t launch_resid(Ctx* c, const HPlanes& h, const __half* bh, const __half* bl, const float* inv_t,
+                                  const void* B, bool b_is_f32, double2* R, int nrhs, int* err, cudaStream_t st)
+{
+    using S = th::RSmem<RBN>;
+    const int n = h.n;
+    CUtensorMap a0, a1, b0, b1;
+    EMFA_TRY(make_map_h(c, &a0, h.zh, 2 * (uint64_t)n, (uint64_t)n, h.ldh, th::BM));
+    EMFA_TRY(make_map_h(c, &a1, h.zl, 2 * (uint64_t)n, (uint64_t)n, h.ldh, th::BM));
+    EMFA_TRY(make_map_h(c, &b0, bh, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, h.ldh, RBN));
+    EMFA_TRY(make_map_h(c, &b1, bl, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, h.ldh, RBN));
+    EMFA_TRY(ensure_smem(c, th::k_hresid<RBN>, S::TOTAL));
+    const dim3 grd((2 * nrhs + RBN - 1) / RBN, (n + th::BM - 1) / th::BM);
+    const int kblocks = (2 * n + th::BKH - 1) / th::BKH;
+    {
+        TimedLaunch tl(c, KT_RESIDUAL, st, 8.0 * n * (double)n * nrhs);
+        th::k_hresid<RBN><<<grd, th::RTHREADS, S::TOTAL, st>>>(a0, a1, b0, b1, B, b_is_f32 ? 0 : 1, R, n, nrhs,
+                                                               kblocks, h.inv_s, inv_t, err);
+    }
+    c->kernel_launches += 1;
+    EMFA_CUDA(c, cudaGetLastError());
+    return EMFA_OK;
+}
+
 emfa_status_t hgemm_residual(Ctx* c, const HPlanes& h, const double2* X, const void* B, bool b_is_f32, double2* R,
                              int nrhs, cudaStream_t st)
 {
-    using S = th::RSmem;
     const int n = h.n;
     const size_t ldh = h.ldh;
     const size_t bplane = Carver::round(sizeof(__half) * ldh * 2 * (size_t)nrhs);
@@ -930,22 +967,19 @@ emfa_status_t hgemm_residual(Ctx* c, const HPlanes& h, const double2* X, const v
     EMFA_TRY(herr(c, &err));
     th::k_hpack_f64<<<nrhs, 256, 0, st>>>(X, n, ldh, bh, bl, inv_t);
     c->kernel_launches += 1;
-    CUtensorMap a0, a1, b0, b1;
-    EMFA_TRY(make_map_h(c, &a0, h.zh, 2 * (uint64_t)n, (uint64_t)n, ldh, th::BM));
-    EMFA_TRY(make_map_h(c, &a1, h.zl, 2 * (uint64_t)n, (uint64_t)n, ldh, th::BM));
-    EMFA_TRY(make_map_h(c, &b0, bh, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ldh, th::RBN));
-    EMFA_TRY(make_map_h(c, &b1, bl, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ldh, th::RBN));
-    EMFA_TRY(ensure_smem(c, th::k_hresid, S::TOTAL));
-    dim3 grd((2 * nrhs + th::RBN - 1) / th::RBN, (n + th::BM - 1) / th::BM);
-    const int kblocks = (2 * n + th::BKH - 1) / th::BKH;
-    {
-        TimedLaunch tl(c, KT_RESIDUAL, st, 8.0 * n * (double)n * nrhs);
-        th::k_hresid<<<grd, th::RTHREADS, S::TOTAL, st>>>(a0, a1, b0, b1, B, b_is_f32 ? 0 : 1, R, n, nrhs, kblocks,
-                                                          h.inv_s, inv_t, err);
-    }
-    c->kernel_launches += 1;
-    EMFA_CUDA(c, cudaGetLastError());
-    return EMFA_OK;
+    // The narrowest tile that holds every column; above 112, the width of 112
+    // and 144 with the shorter time: waves of tiles times a k-block's operands
+    // (a tile is bound by their arrival).
+    const int cols = 2 * nrhs, sms = c->sm_count > 0 ? c->sm_count : 148;
+    const auto cost = [&](int bn) {
+        const long tiles = (long)((cols + bn - 1) / bn) * ((n + th::BM - 1) / th::BM);
+        return (tiles + sms - 1) / sms * (th::BM + bn);
+    };
+    const auto launch = cols <= 16   ? launch_resid<16>
+                        : cols <= 64 ? launch_resid<64>
+                        : cost(144) < cost(112) ? launch_resid<144>
+                                                : launch_resid<112>;
+    return launch(c, h, bh, bl, inv_t, B, b_is_f32, R, nrhs, err, st);
 }
 
 emfa_status_t hgemm_check_error(Ctx* c, cudaStream_t st)

@@ -24,6 +24,23 @@ def test_block_equals_its_columns(ctx, n, r):
         assert torch.equal(y[c], api.matvec(ctx, z, x[c:c + 1].contiguous(), "f16x")[0])
 
 
+@pytest.mark.parametrize("n", [33, 129, 300, 1000])
+@pytest.mark.parametrize("r", [1, 8, 9, 32, 33, 56, 57, 72, 73, 150])
+def test_residual_block_equals_its_columns(ctx, n, r):
+    """The refinement residual at the widths of its column tiles (16, 64, 112 and 144)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + 1000 * r)
+    z = torch.randn(n, n, dtype=torch.complex64, device="cuda", generator=g)
+    b = torch.randn(r, n, dtype=torch.complex64, device="cuda", generator=g)
+    x = torch.randn(r, n, dtype=torch.complex128, device="cuda", generator=g)
+    y = api.residual(ctx, z, x, b, "f16x")
+    for c in sorted({0, r // 2, r - 1}):
+        assert torch.equal(y[c], api.residual(ctx, z, x[c:c + 1].contiguous(), b[c:c + 1].contiguous(), "f16x")[0])
+    # two 11-bit halves a factor: 2^-21 of |z||x| summed, the FP32 rounding of B - Z X, the dropped low-low products
+    bound = 2.0 ** -19 * (x.abs() @ z.abs().to(torch.float64).T) + 2.0 ** -22 * b.abs()
+    assert bool(((y - (b - x @ z.to(torch.complex128).T)).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("n,r", [(31, 1), (512, 1), (513, 2), (1024, 160), (1025, 1), (2500, 40), (4100, 30), (8200, 2)])
 @pytest.mark.parametrize("restart", [2, 32])
 def test_gmres_step_layouts(ctx, n, r, restart):
