@@ -1272,6 +1272,16 @@ __device__ __forceinline__ double2 ld_cluster_d2(const double2* local, int rank)
     return make_double2(x, y);
 }
 
+__device__ __forceinline__ float2 ld_cluster_f2(const float2* local, int rank)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    float x, y;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(ra) : "memory");
+    return make_float2(x, y);
+}
+
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -1500,6 +1510,228 @@ __global__ void __launch_bounds__(AS_ALL, 2)
         cluster_arrive_relaxed();
         cluster_wait();
     }
+}
+
+// ---------------------------------------------------------------------------
+// One Arnoldi step on the FP16 basis in one launch: k_vdots_hw, k_vupdate_h
+// and k_finish_pack on a cluster per right-hand side, a CTA per chunk of
+// VCHUNK elements (so N up to 8 chunks).  Coefficients and norms meet in
+// distributed shared memory, in block order, with the sums of the separate
+// passes: their results bit for bit.  Bound by memory traffic and the
+// latency between its phases, which the other clusters of an SM hide: W is
+// read once from HBM and never written, and the second reading of the basis
+// finds it in L1 or L2.  Dense CFIE jobs, against the three launches: 7680 x 360,
+// 14.89 -> 14.76 ms; 7680 x 91, 9.53 -> 9.37; 3000 x 360, 4.11 -> 3.94;
+// 1920 x 360, 2.58 -> 2.49 (five CTAs an SM 14.67, 9.42, 4.03 and 2.41, six
+// 15.1, 9.5, 4.25 and 2.5).
+// ---------------------------------------------------------------------------
+template <bool ODD>
+__global__ void __launch_bounds__(256, 4)
+    k_arnoldi_h(GmresDev s, int j, const __half* __restrict__ Bh, size_t plane, size_t ldh,
+                const float* __restrict__ inv_tb, const float2* __restrict__ W, int n, int nrhs, HPack pk)
+{
+    __shared__ float sp[8][2 * VW_MAXV];
+    __shared__ float2 hpart[VW_MAXV];     // this chunk's coefficients (read by the cluster)
+    __shared__ float hs0[VW_MAXV], hs1[VW_MAXV], hx[VW_MAXV], hy[VW_MAXV];
+    __shared__ float red[8], redm[8];
+    __shared__ float2 npart;              // this chunk's |w|^2 and max (read by the cluster)
+    __shared__ float sbeta, nscale[2];
+    const int blk = blockIdx.x, nblk = gridDim.x, r = blockIdx.y, nv = j + 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    griddep_wait();
+    griddep_launch();
+    if (blk == 0 && r == 0 && tid == 0) *s.step_next = 0;
+    if (!s.active[r]) {  // the same branch in every CTA of the cluster
+        if (blk == 0 && tid == 0) s.scale[r] = 0.0;
+        return;
+    }
+    const float2* w0 = W + (size_t)r * n;
+    const int k1 = min(n, (blk + 1) * VCHUNK), p0 = (blk * VCHUNK) >> 1, p1 = (k1 + 1) >> 1;
+    // 1. coefficients of the chunk (k_vdots_hw)
+    {
+        const int q0 = p0 + warp * 64 + lane, q1 = q0 + 32;
+        const bool in0 = q0 < p1, in1 = q1 < p1;
+        const float4 x0 = in0 ? ld_wpair<ODD>(w0, q0, n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 x1 = in1 ? ld_wpair<ODD>(w0, q1, n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int g = 0; g < nv; g += 8) {
+            uint2 a[8][2];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const bool ok = g + u < nv;
+                const __half2* row = hrow(Bh, plane, ldh, ok ? g + u : 0, r);
+                a[u][0] = ok && in0 ? ld_bpair<ODD>(row, q0, n) : make_uint2(0u, 0u);
+                a[u][1] = ok && in1 ? ld_bpair<ODD>(row, q1, n) : make_uint2(0u, 0u);
+            }
+            float v[16];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                float re = 0.f, im = 0.f;
+                cmac2(a[u][0], x0, re, im);
+                cmac2(a[u][1], x1, re, im);
+                v[2 * u] = re;
+                v[2 * u + 1] = im;
+            }
+#pragma unroll
+            for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int t = 0; t < h; ++t) {
+                    const float send = up ? v[t] : v[t + h];
+                    const float keep = up ? v[t + h] : v[t];
+                    v[t] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            if ((lane & 1) == 0) sp[warp][2 * g + (lane >> 1)] = v[0];
+        }
+    }
+    __syncthreads();
+    if (tid < nv) {
+        float re = 0.f, im = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            re += sp[q][2 * tid];
+            im += sp[q][2 * tid + 1];
+        }
+        const float st = inv_tb[(size_t)tid * nrhs + r];  // a power of two: exact
+        hpart[tid] = make_float2(re * st, im * st);
+    }
+    cluster_arrive();
+    // W again, by the update's pairs, while the cluster's sums are formed
+    constexpr int EP = VCHUNK / 512, VG = 4;
+    int pc[EP];
+    float4 w[EP];
+#pragma unroll
+    for (int e = 0; e < EP; ++e) {
+        pc[e] = min(p0 + tid + 256 * e, p1 - 1);
+        w[e] = ld_wpair<ODD>(w0, pc[e], n);
+    }
+    cluster_wait();
+    if (tid < nv) {
+        float2 p[AS_MAX_CLUSTER];
+#pragma unroll
+        for (int b = 0; b < AS_MAX_CLUSTER; ++b)
+            if (b < nblk) p[b] = ld_cluster_f2(&hpart[tid], b);
+        float tx = 0.f, ty = 0.f;
+#pragma unroll
+        for (int b = 0; b < AS_MAX_CLUSTER; ++b)
+            if (b < nblk) {
+                tx += p[b].x;
+                ty += p[b].y;
+            }
+        const float st = inv_tb[(size_t)tid * nrhs + r];
+        hx[tid] = tx;
+        hy[tid] = ty;
+        hs0[tid] = tx * st;
+        hs1[tid] = ty * st;
+    }
+    __syncthreads();
+    // 2. w -= V h (k_vupdate_h)
+    float nr = 0.f, mx = 0.f;
+    {
+        float sr[EP][2], si[EP][2];
+#pragma unroll
+        for (int e = 0; e < EP; ++e) sr[e][0] = sr[e][1] = si[e][0] = si[e][1] = 0.f;
+        for (int i = 0; i < nv; i += VG) {
+            uint2 v[VG][EP];
+#pragma unroll
+            for (int u = 0; u < VG; ++u) {
+                const __half2* vi = hrow(Bh, plane, ldh, min(i + u, nv - 1), r);
+#pragma unroll
+                for (int e = 0; e < EP; ++e) v[u][e] = ld_bpair<ODD>(vi, pc[e], n);
+            }
+#pragma unroll
+            for (int u = 0; u < VG; ++u) {
+                const bool ok = i + u < nv;
+                const float hr = ok ? hs0[i + u] : 0.f, hi = ok ? hs1[i + u] : 0.f;
+#pragma unroll
+                for (int e = 0; e < EP; ++e) {
+                    // h v with v = conj(c)
+                    const float2 c0 = h2f(v[u][e].x), c1 = h2f(v[u][e].y);
+                    sr[e][0] += hr * c0.x + hi * c0.y;
+                    si[e][0] += hi * c0.x - hr * c0.y;
+                    sr[e][1] += hr * c1.x + hi * c1.y;
+                    si[e][1] += hi * c1.x - hr * c1.y;
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < EP; ++e) {
+            if (p0 + tid + 256 * e >= p1) continue;
+            w[e].x -= sr[e][0];
+            w[e].y -= si[e][0];
+            w[e].z -= sr[e][1];
+            w[e].w -= si[e][1];  // past the row (odd N): 0 - 0, not stored
+            nr += w[e].x * w[e].x + w[e].y * w[e].y + w[e].z * w[e].z + w[e].w * w[e].w;
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(w[e].x), fabsf(w[e].y)), fmaxf(fabsf(w[e].z), fabsf(w[e].w))));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        nr += __shfl_xor_sync(0xffffffffu, nr, o);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) {
+        red[warp] = nr;
+        redm[warp] = mx;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        float t = 0.f, tm = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            t += red[q];
+            tm = fmaxf(tm, redm[q]);
+        }
+        npart = make_float2(t, tm);
+    }
+    // 3. beta, the column and the packed vector (k_finish_pack)
+    cluster_arrive();
+    ColumnF32 col;
+    const bool column = blk == 0 && warp == 7;
+    if (column)
+        col = column_f32_begin(s, r, j, lane <= j ? make_double2((double)hx[lane], (double)hy[lane]) : make_double2(0.0, 0.0));
+    cluster_wait();
+    if (tid == 0) {
+        float2 p[AS_MAX_CLUSTER];
+#pragma unroll
+        for (int b = 0; b < AS_MAX_CLUSTER; ++b)
+            if (b < nblk) p[b] = ld_cluster_f2(&npart, b);
+        float nr2 = 0.f, wm = 0.f;
+#pragma unroll
+        for (int b = 0; b < AS_MAX_CLUSTER; ++b)
+            if (b < nblk) {
+                nr2 += p[b].x;
+                wm = fmaxf(wm, p[b].y);
+            }
+        const float beta = sqrtf(nr2);
+        const float scale = beta > 0.f ? 1.f / beta : 0.f;
+        const int ex = hpack_exponent_f(wm, scale);
+        sbeta = beta;
+        nscale[0] = scale;
+        nscale[1] = ldexpf(1.f, 14 - ex);
+        if (blk == 0) {
+            s.wmax[r] = wm;
+            pk.inv_t[r] = ldexpf(1.f, ex - 14);
+        }
+    }
+    __syncthreads();
+    cluster_arrive_relaxed();  // this CTA's reads of the others' shared memory are done
+    const float sc = nscale[0], t = nscale[1];
+    uint2* g0 = reinterpret_cast<uint2*>(pk.bh + (size_t)(2 * r) * pk.ldh);
+    uint2* g1 = reinterpret_cast<uint2*>(pk.bh + (size_t)(2 * r + 1) * pk.ldh);
+#pragma unroll
+    for (int e = 0; e < EP; ++e) {
+        const int q = p0 + tid + 256 * e;
+        if (q >= p1) continue;
+        const float4 y = make_float4(w[e].x * sc, w[e].y * sc, w[e].z * sc, w[e].w * sc);
+        const __half re0 = __float2half_rn(t * y.x), im0 = __float2half_rn(t * y.y);
+        const __half re1 = __float2half_rn(t * y.z), im1 = __float2half_rn(t * y.w);
+        g0[q] = make_uint2(h2u(__halves2half2(re0, __hneg(im0))), h2u(__halves2half2(re1, __hneg(im1))));
+        g1[q] = make_uint2(h2u(__halves2half2(im0, re0)), h2u(__halves2half2(im1, re1)));
+    }
+    if (column) column_f32_end<false>(s, r, j, col, sbeta);
+    cluster_wait();  // no CTA leaves while another may still read its shared memory
 }
 
 // out[r] = scale[r] W[r]: grid over (chunks of 1024, RHS).  An FP32 basis is
@@ -1952,7 +2184,25 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                     // the pair kernels by the parity of N (odd N: 8-byte W accesses)
                     const auto finish = n % 2 ? k_finish_pack<true> : k_finish_pack<false>;
                     const dim3 fg((n + FP_CHUNK - 1) / FP_CHUNK, nrhs);
-                    if (hbasis) {
+                    if (hbasis && vblk <= AS_MAX_CLUSTER && sp->orth != 3) {  // one launch (orth 3: the passes)
+                        cudaLaunchConfig_t cfg = {};
+                        cfg.gridDim = vg;
+                        cfg.blockDim = dim3(256);
+                        cfg.stream = st;
+                        cudaLaunchAttribute at[2];
+                        at[0].id = cudaLaunchAttributeClusterDimension;
+                        at[0].val.clusterDim.x = vblk;
+                        at[0].val.clusterDim.y = 1;
+                        at[0].val.clusterDim.z = 1;
+                        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                        at[1].val.programmaticStreamSerializationAllowed = 1;
+                        cfg.attrs = at;
+                        cfg.numAttrs = 2;
+                        EMFA_CUDA(c, cudaLaunchKernelEx(&cfg, n % 2 ? k_arnoldi_h<true> : k_arnoldi_h<false>, s, j,
+                                                        (const __half*)Bh, hplane, pk0.ldh, (const float*)inv_tb,
+                                                        (const float2*)W, n, nrhs, pk));
+                        c->kernel_launches -= 2;  // of the three counted below
+                    } else if (hbasis) {
                         const auto dots = n % 2 ? k_vdots_hw<true> : k_vdots_hw<false>;
                         const auto upd = n % 2 ? k_vupdate_h<true> : k_vupdate_h<false>;
                         EMFA_CUDA(c, launch_dependent(dots, vg, dim3(256), 0, st, (const __half*)Bh, hplane, pk0.ldh,

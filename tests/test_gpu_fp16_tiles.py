@@ -54,3 +54,27 @@ def test_gmres_step_layouts(ctx, n, r, restart):
     res = b.to(torch.complex128) - x @ z.to(torch.complex128).T
     # two roundings of the FP64 residual apart from the solver's own
     assert float((res.norm(dim=1) / b.norm(dim=1)).max()) <= 1e-6 * (1 + 1e-6)
+
+
+@pytest.mark.parametrize("n,r", [(300, 700), (1024, 640), (1500, 320), (1501, 320), (4097, 130), (7680, 80), (8192, 77),
+                                 (8193, 70)])
+def test_one_launch_step_equals_the_passes(ctx, n, r):
+    """A step on the FP16 basis by one cluster a right-hand side (up to eight chunks of 1024) and by the three passes: the
+    same sums in the same order, so the same bits; a zero right-hand side among them is done at once.  Where the blocks are
+    few (at most four CTAs an SM) the automatic choice is the FP32-basis step: the same solution to the tolerance."""
+    import torch
+    few = r * min(8, -(-n // 1024)) <= 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(n + r)
+    z = torch.randn(n, n, dtype=torch.complex64, device="cuda", generator=g)
+    z.diagonal().add_(2.5 * n ** 0.5)
+    b = torch.randn(r, n, dtype=torch.complex64, device="cuda", generator=g)
+    b[r // 2] = 0
+    for restart in (3, 30):
+        x, info = api.solve(ctx, z, b, api.solver_params("gmres", restart=restart, tol=1e-6))
+        y, other = api.solve(ctx, z, b, api.solver_params("gmres", restart=restart, tol=1e-6, orth="cgs1_split"))
+        assert info.converged == r and other.converged == r
+        if few:
+            assert float((x - y).norm() / y.norm()) < 1e-5
+            continue
+        assert (info.iterations, info.cycles) == (other.iterations, other.cycles)
+        assert torch.equal(x, y)
