@@ -933,12 +933,22 @@ __device__ __forceinline__ double2 shfl_d2(double2 v, int src)
 // Arnoldi column j of right-hand side r (one warp): lane i <= j holds the
 // Gram-Schmidt coefficient h_i, beta = ||w||.  Applies the previous
 // rotations, forms the new one, updates g and tests convergence.
-__device__ void arnoldi_column(const GmresDev& s, int r, int j, double2 h, double beta)
+// In two parts: the earlier rotations need the column's coefficients only,
+// the new one needs beta as well.
+struct ColumnF64 {
+    double2 h, ph, gj;  // lane i: the rotated entry i; lane j: entry j over its modulus, and g[j]
+    double aa;          // lane j: the modulus of entry j
+    double thr, small;  // the step's residual target and breakdown bound
+};
+
+__device__ __forceinline__ ColumnF64 column_f64_begin(const GmresDev& s, int r, int j, double2 h)
 {
     const int lane = threadIdx.x & 31, m = s.m;
-    double2* H = s.H + (size_t)r * (m + 1) * m;
-    double* cs = s.cs + (size_t)r * m;
-    double2* sn = s.sn + (size_t)r * m;
+    ColumnF64 q;
+    q.gj = s.g[(size_t)r * (m + 1) + j];
+    const double bn = s.bnorm[r], tr = s.true_res[r];
+    const double* cs = s.cs + (size_t)r * m;
+    const double2* sn = s.sn + (size_t)r * m;
     const double cl = lane < j ? cs[lane] : 0.0;
     const double2 sl = lane < j ? sn[lane] : make_double2(0.0, 0.0);
     // previous rotations: [x; y] <- [c x + s y; -conj(s) x + c y] on entries (i, i + 1)
@@ -951,10 +961,26 @@ __device__ void arnoldi_column(const GmresDev& s, int r, int j, double2 h, doubl
         else if (lane == i + 1)
             h = make_double2(-(sv.x * x.x + sv.y * x.y) + c * y.x, -(sv.x * x.y - sv.y * x.x) + c * y.y);
     }
+    q.h = h;
+    q.aa = hypot(h.x, h.y);
+    q.ph = make_double2(h.x / q.aa, h.y / q.aa);
+    q.thr = fmax(s.inner * (s.tol_abs ? s.tol : s.tol * bn), s.red * tr * bn);
+    q.small = 1e-14 * bn;
+    return q;
+}
+
+// SCALE: the 1 / beta of a vector that another launch normalises
+// seen (optional): a page-locked host word told 1 by a right-hand side that
+// stays active
+template <bool SCALE>
+__device__ __forceinline__ void column_f64_end(const GmresDev& s, int r, int j, const ColumnF64& q, double beta,
+                                               int* seen = nullptr)
+{
+    const int lane = threadIdx.x & 31, m = s.m;
+    double2* H = s.H + (size_t)r * (m + 1) * m;
+    double2 h = q.h;
     if (lane == j) {
-        const double2 a = h;
-        const double b = beta;
-        const double aa = hypot(a.x, a.y);
+        const double b = beta, aa = q.aa;
         const double nu = hypot(aa, b);
         double c;
         double2 sv;
@@ -964,29 +990,27 @@ __device__ void arnoldi_column(const GmresDev& s, int r, int j, double2 h, doubl
             h = make_double2(b, 0.0);
         } else {
             c = aa / nu;
-            const double2 ph = make_double2(a.x / aa, a.y / aa);
-            sv = make_double2(ph.x * b / nu, ph.y * b / nu);
-            h = make_double2(ph.x * nu, ph.y * nu);
+            sv = make_double2(q.ph.x * b / nu, q.ph.y * b / nu);
+            h = make_double2(q.ph.x * nu, q.ph.y * nu);
         }
         H[(j + 1) * m + j] = make_double2(0.0, 0.0);
-        cs[j] = c;
-        sn[j] = sv;
+        s.cs[(size_t)r * m + j] = c;
+        s.sn[(size_t)r * m + j] = sv;
         double2* g = s.g + (size_t)r * (m + 1);
-        const double2 gj = g[j];
-        g[j + 1] = make_double2(-(sv.x * gj.x + sv.y * gj.y), -(sv.x * gj.y - sv.y * gj.x));
+        const double2 gj = q.gj, gn = make_double2(-(sv.x * gj.x + sv.y * gj.y), -(sv.x * gj.y - sv.y * gj.x));
+        g[j + 1] = gn;
         g[j] = make_double2(c * gj.x, c * gj.y);
-        const double res = hypot(g[j + 1].x, g[j + 1].y);
+        const double res = hypot(gn.x, gn.y);
         s.jlen[r] = j + 1;
         s.est[r] = res;
-        const double thr =
-            fmax(s.inner * (s.tol_abs ? s.tol : s.tol * s.bnorm[r]), s.red * s.true_res[r] * s.bnorm[r]);
-        const bool breakdown = beta <= 1e-14 * s.bnorm[r];
-        if (res < thr || breakdown || j + 1 == m) {
+        const bool breakdown = beta <= q.small;
+        if (res < q.thr || breakdown || j + 1 == m) {
             s.active[r] = 0;
             s.scale[r] = 0.0;
         } else {
-            s.scale[r] = 1.0 / beta;
+            if constexpr (SCALE) s.scale[r] = 1.0 / beta;
             atomicAdd(s.step_cnt, 1);
+            if (seen) *(volatile int*)seen = 1;
         }
     }
     if (lane <= j) H[lane * m + j] = h;
@@ -1114,7 +1138,7 @@ __global__ void k_arnoldi_finish_warp(GmresDev s, int j, const double2* __restri
             h.y += b.y;
         }
     }
-    arnoldi_column(s, r, j, h, beta);
+    column_f64_end<true>(s, r, j, column_f64_begin(s, r, j, h), beta);
 }
 
 // Last kernel of the separate-pass CGS1 step (FP32 basis, restarts up to
@@ -1272,6 +1296,15 @@ __device__ __forceinline__ double2 ld_cluster_d2(const double2* local, int rank)
     return make_double2(x, y);
 }
 
+__device__ __forceinline__ double ld_cluster_d(const double* local, int rank)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    double x;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(ra) : "memory");
+    return x;
+}
 __device__ __forceinline__ float2 ld_cluster_f2(const float2* local, int rank)
 {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
@@ -1734,6 +1767,194 @@ __global__ void __launch_bounds__(256, 4)
     cluster_wait();  // no CTA leaves while another may still read its shared memory
 }
 
+// ---------------------------------------------------------------------------
+// One FP64 Arnoldi step (CGS2) in one launch, for grids that leave the
+// separate passes to their latency: a cluster of up to 8 CTAs per right-hand
+// side, CTA `rank` owning elements [rank slice, (rank + 1) slice).  w stays
+// in shared memory and registers; twice over, eight lanes a basis vector form
+// its coefficient over the slice, the cluster adds the slices in rank order,
+// and every thread updates its elements (the basis from L1 and L2).  Then
+// beta, V_{j+1} = w / beta and, on a warp of the first CTA's own, the Givens
+// column: its earlier rotations beside the second update, the new one beside
+// the stores.  Bound by the chain: FP64 products (a warp
+// instruction holds the SM's FP64 pipe 16 cycles), four barriers.  It replaces
+// two passes of coefficients and update, a memset, the column (16 us) and the
+// normalisation.  Jobs to 1e-6: EFIE 480 x 2 (177 steps), 14.3 -> 8.6 ms; CFIE
+// 480 x 1, 3.6 -> 2.5; 1080 x 8, 6.3 -> 5.1.
+// ---------------------------------------------------------------------------
+constexpr int A64_THREADS = 256, A64_ALL = A64_THREADS + 32, A64_MAXV = 32;  // restarts up to 31
+
+template <int E>
+__global__ void __launch_bounds__(A64_ALL)
+    k_arnoldi_step64(GmresDev s, int j, const double2* __restrict__ V, size_t vstride, const double2* __restrict__ W,
+                     int n, int slice, double2* __restrict__ Vout, const int* __restrict__ prev, int* __restrict__ seen_prev,
+                     int* __restrict__ seen)
+{
+    __shared__ double2 sw[A64_THREADS * E];
+    __shared__ double2 hpart[A64_MAXV];    // this CTA's partial coefficients (read by the cluster)
+    __shared__ double2 hs[A64_MAXV];       // the cluster's sums of a pass
+    __shared__ double2 hsum[A64_MAXV];     // of both
+    __shared__ double nred[A64_THREADS / 32];
+    __shared__ double npart;               // this CTA's |w|^2 (read by the cluster)
+    __shared__ double nfin[2];             // beta, 1 / beta
+    const int r = blockIdx.y, rank = blockIdx.x, csize = gridDim.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool colwarp = warp == A64_THREADS / 32;
+    const int nv = j + 1, k0 = rank * slice, len = min(n, k0 + slice) - k0;  // len >= 1 for every rank
+    const double2* Vs = V + (size_t)r * n + k0;
+    griddep_wait();
+    if (rank == 0 && r == 0 && tid == 0) {
+        if (prev && *(volatile const int*)prev == 0) *(volatile int*)seen_prev = 0;  // nobody told 1
+        *s.step_next = 0;
+    }
+    if (!s.active[r]) {  // the same branch in every CTA of the cluster
+        if (rank == 0 && tid == 0) s.scale[r] = 0.0;
+        return;
+    }
+    double2 w[E];
+    if (!colwarp) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int k = tid + e * A64_THREADS;
+            w[e] = k < len ? W[(size_t)r * n + k0 + k] : make_double2(0.0, 0.0);
+            sw[k] = w[e];
+        }
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        __syncthreads();  // w of the slice is in shared memory
+        const int i = tid >> 3, p = tid & 7;
+        if (!colwarp && (i & ~3) < nv) {  // whole warps
+            const double2* vi = Vs + (size_t)min(i, nv - 1) * vstride;
+            double re = 0, im = 0;
+#pragma unroll 4
+            for (int k = p; k < len; k += 8) {
+                const double2 a = vi[k], x = sw[k];
+                re = fma(a.x, x.x, fma(a.y, x.y, re));
+                im = fma(a.x, x.y, fma(-a.y, x.x, im));
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                re += __shfl_xor_sync(0xffffffffu, re, o);
+                im += __shfl_xor_sync(0xffffffffu, im, o);
+            }
+            if (p == 0 && i < nv) hpart[i] = make_double2(re, im);
+        }
+        if (csize > 1) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+        if (tid < nv) {
+            double2 q[AS_MAX_CLUSTER], t = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+                if (c < csize) q[c] = ld_cluster_d2(&hpart[tid], c);
+#pragma unroll
+            for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+                if (c < csize) {
+                    t.x += q[c].x;
+                    t.y += q[c].y;
+                }
+            hs[tid] = t;
+            hsum[tid] = pass == 0 ? t : make_double2(hsum[tid].x + t.x, hsum[tid].y + t.y);
+        }
+        // hpart is read again by nobody once every CTA is here
+        if (pass == 0 && csize > 1) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+        if (!colwarp) {
+            for (int i0 = 0; i0 < nv; i0 += 4) {
+                double2 v[4][E];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int e = 0; e < E; ++e) {
+                        const int k = tid + e * A64_THREADS;
+                        v[u][e] = k < len ? Vs[(size_t)min(i0 + u, nv - 1) * vstride + k] : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (i0 + u >= nv) break;
+                    const double2 h = hs[i0 + u];
+#pragma unroll
+                    for (int e = 0; e < E; ++e)
+                        if (e * A64_THREADS + (warp << 5) < len) {  // whole warps
+                            w[e].x = fma(-h.x, v[u][e].x, fma(h.y, v[u][e].y, w[e].x));
+                            w[e].y = fma(-h.x, v[u][e].y, fma(-h.y, v[u][e].x, w[e].y));
+                        }
+                }
+            }
+            if (pass == 0) {
+#pragma unroll
+                for (int e = 0; e < E; ++e) sw[tid + e * A64_THREADS] = w[e];
+            }
+        }
+    }
+    if (colwarp) {
+        // the column's earlier rotations beside the update, the new one beside the stores
+        if (csize > 1) cluster_arrive();  // of the norm: publishes nothing
+        ColumnF64 col;
+        if (rank == 0) col = column_f64_begin(s, r, j, lane <= j ? hsum[lane] : make_double2(0.0, 0.0));
+        if (csize > 1) cluster_wait();
+        named_sync(2, A64_ALL);  // beta
+        if (rank == 0) {
+            if (lane == 0) s.wmax[r] = 0.0;
+            column_f64_end<false>(s, r, j, col, nfin[0], seen);
+        }
+        if (csize > 1) {
+            cluster_arrive_relaxed();
+            cluster_wait();
+        }
+        return;
+    }
+    double nr = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) nr = fma(w[e].x, w[e].x, fma(w[e].y, w[e].y, nr));  // 0 past the slice
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nr += __shfl_xor_sync(0xffffffffu, nr, o);
+    if (lane == 0) nred[warp] = nr;
+    named_sync(1, A64_THREADS);
+    if (tid == 0) {
+        double t = 0;
+#pragma unroll
+        for (int q = 0; q < A64_THREADS / 32; ++q) t += nred[q];
+        npart = t;
+    }
+    if (csize > 1) {
+        cluster_arrive();
+        cluster_wait();
+    }
+    if (tid == 0) {
+        double q[AS_MAX_CLUSTER], nr2 = 0;
+#pragma unroll
+        for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+            if (c < csize) q[c] = ld_cluster_d(&npart, c);
+#pragma unroll
+        for (int c = 0; c < AS_MAX_CLUSTER; ++c)
+            if (c < csize) nr2 += q[c];
+        const double beta = sqrt(nr2);
+        nfin[0] = beta;
+        nfin[1] = beta > 0.0 ? 1.0 / beta : 0.0;
+    }
+    named_sync(1, A64_THREADS);
+    named_arrive(2, A64_ALL);
+    const double sc = nfin[1];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int k = tid + e * A64_THREADS;
+        if (k < len) Vout[(size_t)r * n + k0 + k] = make_double2(w[e].x * sc, w[e].y * sc);
+    }
+    if (csize > 1) {
+        // no CTA leaves while another may still read its shared memory
+        cluster_arrive_relaxed();
+        cluster_wait();
+    }
+}
+
 // out[r] = scale[r] W[r]: grid over (chunks of 1024, RHS).  An FP32 basis is
 // scaled in FP32 and an FP64 source converted by split_f64 (integer
 // operations): FP64 products and conversions per element would run on
@@ -1966,6 +2187,48 @@ static emfa_status_t launch_arnoldi_step(Ctx* c, const StepShape& sh, int nrhs, 
     return launch_step_e<4>(c, sh, nrhs, st, s, j, V, vstride, W, n, Vout, pk);
 }
 
+// The FP64 step's clusters: as many CTAs a right-hand side as four an SM
+// allow, at least enough for four elements a thread, slices of 32 or more
+// (cs 0: too large).
+struct Step64 {
+    int cs = 0, slice = 0, e = 0;
+};
+static Step64 step64_shape(Ctx* c, int n, int nrhs)
+{
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    Step64 q;
+    const int least = (n + 4 * A64_THREADS - 1) / (4 * A64_THREADS);
+    if (least > AS_MAX_CLUSTER) return q;
+    q.cs = std::max(least, std::min({AS_MAX_CLUSTER, 4 * sms / nrhs, (n + 31) / 32}));
+    q.slice = (n + q.cs - 1) / q.cs;
+    q.cs = (n + q.slice - 1) / q.slice;  // no empty slice
+    const int e = (q.slice + A64_THREADS - 1) / A64_THREADS;
+    q.e = e <= 1 ? 1 : e <= 2 ? 2 : 4;
+    return q;
+}
+
+static emfa_status_t launch_step64(Ctx* c, const Step64& q, int nrhs, cudaStream_t st, const GmresDev& s, int j,
+                                   const double2* V, size_t vstride, const double2* W, int n, double2* Vout,
+                                   const int* prev, int* seen_prev, int* seen)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.cs, nrhs);
+    cfg.blockDim = dim3(A64_ALL);
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = q.cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    const auto kernel = q.e == 1 ? k_arnoldi_step64<1> : q.e == 2 ? k_arnoldi_step64<2> : k_arnoldi_step64<4>;
+    EMFA_CUDA(c, cudaLaunchKernelEx(&cfg, kernel, s, j, V, vstride, W, n, q.slice, Vout, prev, seen_prev, seen));
+    return EMFA_OK;
+}
+
 template <typename T>
 static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2* X, const emfa_solver_params_t* sp,
                              emfa_solve_info_t* info, cudaStream_t st)
@@ -1997,6 +2260,14 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
     // orth 4 takes the fused step whatever the grid size (for measurement)
     const bool fused = std::is_same<T, float>::value && !two_pass && sp->orth != 3 && m <= AS_MAXV && sh.e > 0 &&
                        ((long)nrhs * sh.cs <= 4L * sms || sp->orth == 4);
+    // FP64: the step in one launch (orth 2 keeps the passes) up to 100000
+    // elements of a block, where launches and chains count more than the FP64
+    // pipe.  us a step with its product, one launch | passes: 480 x 1, 45 | 77,
+    // x 16, 67 | 96, x 91, 105 | 118; 1080 x 30, 87 | 112, x 91, 161 | 167;
+    // 750 x 91, 126 | 125; 2430 x 91, 358 | 353; 750 x 360, 346 | 276.
+    const Step64 sh64 = std::is_same<T, double>::value ? step64_shape(c, n, nrhs) : Step64();
+    const bool fused64 = std::is_same<T, double>::value && two_pass && sp->orth == 0 && m <= A64_MAXV - 1 && sh64.cs > 0 &&
+                         (long)n * nrhs <= 100000;
     // separate passes on an FP32 basis with one Gram-Schmidt pass end in
     // k_finish_pack (column, normalisation and packing in one launch)
     const bool finish_pack = std::is_same<T, float>::value && !fused && !two_pass && m <= 32;
@@ -2157,8 +2428,8 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             bool packs = false;
             // the step normalises V_{j+1} itself (fused, or separate passes
             // ending in k_finish_pack); otherwise normalize_apply does
-            const bool normalises = fused || finish_pack;
-            if (normalises) {
+            const bool normalises = fused || finish_pack || fused64;
+            if (normalises && !fused64) {
                 packs = A.pack_target(c, nrhs, &pk);
                 if (!packs) pk = HPack{};
                 if (hbasis) {  // V_{j+1} is plane j + 1
@@ -2168,7 +2439,20 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                 // the next product skips itself if this step leaves nothing active
                 pk.skip = s.step_cnt;
             }
-            if (fused) {
+            if (fused64) {
+                if constexpr (std::is_same<T, double>::value) {
+                    // a step tells the host 1 as soon as a right-hand side
+                    // stays active, the next one 0 if none did; a word a step,
+                    // as the host may be past a step that others still tell of
+                    // (each cycle begins with the stream idle)
+                    const int* prev = j > 0 ? s.counters + 2 + (j - 1) % 3 : nullptr;
+                    slot[2 + j] = -1;
+                    EMFA_TRY(launch_step64(c, sh64, nrhs, st, s, j, (const double2*)V, vec, (const double2*)W, n,
+                                           (double2*)(V + (size_t)(j + 1) * vec), prev,
+                                           const_cast<int*>(slot + 1 + j), const_cast<int*>(slot + 2 + j)));
+                    c->kernel_launches += 1;
+                }
+            } else if (fused) {
                 // V_{j+1} and the next product's operand come out of the step
                 EMFA_TRY(launch_arnoldi_step(c, sh, nrhs, st, s, j, (const float2*)V, vec, (const float2*)W, n,
                                              (float2*)(V + (size_t)(j + 1) * vec), pk));
@@ -2260,7 +2544,8 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
                 }
             }
             const bool told = normalises && packs;
-            if (told) {
+            if (fused64) {
+            } else if (told) {
                 pk.seen = const_cast<int*>(slot + (j & 1));
                 slot[j & 1] = -1;
             } else {
@@ -2275,11 +2560,12 @@ static emfa_status_t gmres_t(Ctx* c, LinOp& A, const void* B, int nrhs, double2*
             }
             ++steps;
             if (j > 0) {
-                if (told)
-                    EMFA_TRY(await_count(slot + ((j - 1) & 1)));
+                volatile int* word = slot + (fused64 ? 1 + j : (j - 1) & 1);
+                if (told || fused64)
+                    EMFA_TRY(await_count(word));
                 else
                     EMFA_CUDA(c, cudaEventSynchronize(sev.e[(j - 1) & 1]));
-                if (slot[(j - 1) & 1] == 0) {  // step j (queued) found nothing active
+                if (*word == 0) {  // step j (queued) found nothing active
                     --steps;
                     break;
                 }

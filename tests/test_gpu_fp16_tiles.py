@@ -1,4 +1,4 @@
-"""The split-FP16 product at the widths where its column tile changes (16, 64 and 144 real columns), the rows where a tile
+"""Steps and tiles of the Krylov solves.  The split-FP16 product at the widths where its column tile changes (16, 64 and 144 real columns), the rows where a tile
 ends, and K shorter and longer than the stages loaded ahead; and GMRES steps whose basis fits the shared memory of a CTA
 that has an SM to itself, or of one of two.
 
@@ -78,3 +78,28 @@ def test_one_launch_step_equals_the_passes(ctx, n, r):
             continue
         assert (info.iterations, info.cycles) == (other.iterations, other.cycles)
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n,r", [(1, 1), (31, 1), (33, 3), (257, 2), (480, 1), (480, 91), (1025, 7), (2049, 48), (4097, 3),
+                                 (8192, 1), (8193, 1)])
+@pytest.mark.parametrize("restart", [1, 7, 31, 32])
+def test_fp64_step_agrees_with_the_passes(ctx, n, r, restart):
+    """The FP64 step in one launch (restarts up to 31, N up to 8192) against the separate passes: FP64 sums in another
+    order, so both meet the target and agree to its rounding (condition below 10)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + r + restart)
+    z = torch.randn(n, n, dtype=torch.complex128, device="cuda", generator=g)
+    z.diagonal().add_(4 * n ** 0.5)
+    b = torch.randn(r, n, dtype=torch.complex128, device="cuda", generator=g)
+    if r > 2:
+        b[1] = 0
+    sols = []
+    for orth in ("auto", "cgs2"):
+        x, info = api.solve(ctx, z, b, api.solver_params("gmres", restart=restart, tol=1e-11, orth=orth, max_iter=3000))
+        assert info.converged == r
+        res = (b - x @ z.T).norm(dim=1) / b.norm(dim=1).clamp_min(1e-300)
+        assert float(res.max()) <= 2e-11
+        sols.append((x, info.iterations, info.cycles))
+    # a step at the target's very edge may fall either way
+    assert abs(sols[0][1] - sols[1][1]) <= max(1, restart) and abs(sols[0][2] - sols[1][2]) <= 1
+    assert float((sols[0][0] - sols[1][0]).norm() / sols[1][0].norm()) <= 20 * 2e-11
