@@ -30,8 +30,8 @@
 // panels 8 to 9 (24 with 64-wide chunks and loads waited for one by one),
 // columns 3.8 and 5.3 (11 and 16), and no gap of more than 1.5 us (a separate
 // packing launch was 9.5 a pair and each crossing of streams 3 to 4).  EFIE
-// jobs of 8 incidences: n = 480, 1.26 -> 0.91 ms; 1470, 3.50 -> 2.38; 3630,
-// 8.85 -> 5.81; 5070, 13.1 -> 8.8.
+// jobs of 8 incidences: n = 480, 1.26 -> 0.88 ms; 1470, 3.50 -> 2.25; 3630,
+// 8.85 -> 5.39; 5070, 13.1 -> 8.2.
 // Rows of the factor are padded to an even number of complex elements
 // (16-byte TMA strides).
 // Solve for many right-hand sides (RHS-major, (r, u) at r n + u): gather by
@@ -896,8 +896,11 @@ constexpr int RC = 8;  // right-hand sides per CTA of a triangular solve
 //   x_k = inv_k acc, stored in Out, then the block's flag is raised
 // Each x_j is read once its flag is up (bounded wait: on timeout, or once
 // any wait has given up, the kernel records an error and stops waiting); the
-// 64 x 64 blocks of A stream through a cp.async double buffer.  RC right-hand
-// sides per CTA (blockIdx.y).  Thread: row i = tid / 4, right-hand sides
+// 64 x 64 blocks of A stream through a cp.async double buffer, the inverse
+// last.  A chain of blocks bounds it: 4.0 -> 2.7 us a block (eight right-hand
+// sides, 228 -> 155 us a sweep on the batch's mean) since the inverse no longer
+// loads on the chain and the error word is polled with every 64th read of a flag
+// only.  RC right-hand sides per CTA (blockIdx.y).  Thread: row i = tid / 4, right-hand sides
 // 2 (tid % 4) and the next.
 constexpr int WLD = NB + 2;  // tile row stride in float2: 16-byte aligned, 8 rows on distinct banks
 
@@ -951,22 +954,30 @@ __global__ void __launch_bounds__(256) k_lu_wave(const float2* __restrict__ A, i
     // the blocks this row block depends on, in the order they are solved
     const int nd = DIR == 0 ? k : nblk - 1 - k;
     auto dep = [&](int s) { return DIR == 0 ? s : nblk - 1 - s; };
-    if (nd > 0) {
-        tile_async(T0, A, n, lda, k0, dep(0) * NB);
+    // the block's inverse is the tile after the last one: in shared memory by
+    // the time the chain reaches it
+    const float2* iv = inv + (size_t)k * NB * NB;
+    auto fetch = [&](float2* T, int s) {
+        if (s < nd)
+            tile_async(T, A, n, lda, k0, dep(s) * NB);
+        else
+            for (int q = tid; q < NB * NB / 2; q += blockDim.x)
+                cp_async16(T + (q / (NB / 2)) * WLD + 2 * (q % (NB / 2)), iv + 2 * q, 16);
         cp_async_commit();
-    }
+    };
+    fetch(T0, 0);
     bool ok = true;
     for (int s = 0; s < nd; ++s) {
         float2* T = (s & 1) ? T1 : T0;
-        if (s + 1 < nd) tile_async((s & 1) ? T0 : T1, A, n, lda, k0, dep(s + 1) * NB);
-        cp_async_commit();
+        fetch((s & 1) ? T0 : T1, s + 1);
         const int j = dep(s), j0 = j * NB, nbj = min(NB, n - j0);
         if (tid == 0) {
             int got = ok;
             if (got) {
                 const long long t0 = clock64();
-                while (*(volatile int*)(fl + j) == 0) {
-                    if (*(volatile int*)err || clock64() - t0 > limit) {
+                for (int spin = 1; *(volatile int*)(fl + j) == 0; ++spin) {
+                    // now and then: a second read would double the time to see the flag
+                    if ((spin & 63) == 0 && (*(volatile int*)err || clock64() - t0 > limit)) {
                         atomicCAS(err, 0, 21);
                         got = 0;
                         break;
@@ -1004,13 +1015,12 @@ __global__ void __launch_bounds__(256) k_lu_wave(const float2* __restrict__ A, i
     // x_k = inv_k acc
 #pragma unroll
     for (int h = 0; h < 2; ++h) xs[i][r + h] = acc[h];
-    const float2* iv = inv + (size_t)k * NB * NB;
-    for (int q = tid; q < NB * NB; q += blockDim.x) T0[(q / NB) * WLD + q % NB] = iv[q];
+    const float2* Ti = (nd & 1) ? T1 : T0;
     __syncthreads();
     float2 x[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll 8
     for (int c = 0; c < NB; ++c) {
-        const float2 m = T0[i * WLD + c];
+        const float2 m = Ti[i * WLD + c];
 #pragma unroll
         for (int h = 0; h < 2; ++h) x[h] = cfma(m, xs[c][r + h], x[h]);
     }
