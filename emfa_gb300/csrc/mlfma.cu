@@ -709,7 +709,11 @@ struct FinishArgs {
     int parts;  // 0 near + far, 1 near, 2 far
     float2* y;
 };
-constexpr int FINISH_WARPS = 4;
+// Eight warps: the phases between the CTA's barriers have a few hundred
+// outputs each and a box a handful of unknowns.  A product in us with 4 | 8 |
+// 12 warps: 122880 x 1, 792 | 780 | 840; 10830 x 4, 282 | 260 | 271; 43320 x 8,
+// 1884 | 1630 | 1700.
+constexpr int FINISH_WARPS = 8;
 
 template <int RB>
 __global__ void __launch_bounds__(32 * FINISH_WARPS) k_finish(const __grid_constant__ FinishArgs A)
@@ -1921,8 +1925,8 @@ static void launch_agg_disagg(emfa_mlfma* M, bool agg, const float2* x, int nr, 
     MLevel& fl = M->lv[nl - 1];
     const int Kf = fl.K, n = M->n;
     const size_t lstride = (size_t)3 * fl.nbox * Kf;
-    if (agg)
-        k_agg_finest<RB><<<dim3(fl.nbox, RB == 1 ? nr : 1), 128, 0, st>>>(x, n, nr, dptr<C2f>(M->rad), dptr<float>(M->tp),
+    if (agg)  // 256 threads cover the samples of a box in one turn (27000 x 2, 412 -> 405 us a product)
+        k_agg_finest<RB><<<dim3(fl.nbox, RB == 1 ? nr : 1), 256, 0, st>>>(x, n, nr, dptr<C2f>(M->rad), dptr<float>(M->tp),
                                                   dptr<int>(M->box_off), dptr<int>(M->box_cnt), Kf,
                                                   dptr<float2>(fl.up), lstride);
     else
