@@ -475,12 +475,15 @@ __global__ void k_upward(const float2* __restrict__ child, int Lc, const int* __
 // Per (source, sibling): one 8-byte shared load and 12 FMA, against an 8-byte
 // table and a 24-byte pattern load through L1 when a thread took one box's far
 // list (5-wavelength sphere, 122,880 unknowns: 518 us for the five levels with
-// the anterpolation, the L1 data path 80 % busy).  Now 290 us,
-// and 107 for the anterpolation above the finest level; still bound by L1
+// the anterpolation, the L1 data path 80 % busy).  Now 290 us
+// with twelve warps, and 107 for the anterpolation above the finest level; still bound by L1
 // wavefronts (71 %), half of them the siblings' table values.  Eight siblings a
 // warp, or two patterns in flight, were no faster (spills; latency).
 constexpr int TRANS_LEVELS = 24;  // octree levels a launch takes
-constexpr int TRANS_WARPS = 12, TRANS_K = 32, TRANS_OFF = 343, TRANS_NC = 4, TRANS_BATCH = 4;
+// sixteen warps, two CTAs an SM by the table: a product in us with 12 | 14 | 16 |
+// 18 warps (64 registers up to 16): 122880 x 1, 778 | 782 | 766 | 808; 43320 x 8,
+// 1635 | 1633 | 1600 | 1619
+constexpr int TRANS_WARPS = 16, TRANS_K = 32, TRANS_OFF = 343, TRANS_NC = 4, TRANS_BATCH = 4;
 constexpr size_t TRANS_SMEM = sizeof(float2) * TRANS_OFF * TRANS_K;
 struct TransGroup {
     int s0, s1, nc, pad;      // sources [s0, s1), multiples of TRANS_BATCH; siblings
@@ -1726,14 +1729,15 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
             series.put(sv[i].kd, kd[i]);
         }
     }
-    // translation work: up to 24 groups a CTA (two a warp and right-hand side, so
-    // that the table's staging is a few percent), fewer where that leaves SMs idle
+    // translation work: up to 48 groups a CTA (three a warp and right-hand side,
+    // so that the table's staging is a few percent; 122880 x 1, us with 24 | 36 | 48 |
+    // 72: 762 | 751 | 739 | 742), fewer where that leaves SMs idle
     {
         std::vector<TransWork> tw;
         size_t tasks = 0;
         for (const MLevel& ml : M->lv) tasks += (size_t)ml.ngrp * ((ml.K + TRANS_K - 1) / TRANS_K);
         const size_t sms = c->sm_count > 0 ? c->sm_count : 148;
-        const int per = (int)std::min<size_t>(24, std::max<size_t>(6, tasks / (8 * sms)));
+        const int per = (int)std::min<size_t>(48, std::max<size_t>(6, tasks / (8 * sms)));
         for (int i = nl - 1; i >= 0; --i) {
             const MLevel& ml = M->lv[i];
             const int parts = std::max(1, (ml.ngrp + per / 2) / per);
