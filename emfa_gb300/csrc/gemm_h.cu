@@ -848,6 +848,21 @@ static emfa_status_t hgemm_run(Ctx* c, const HPlanes& h, const __half* bh, const
     return launch_variant(c, v, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st, true, skip, seen);
 }
 
+emfa_status_t hgemm_planes(Ctx* c, const __half* A, const __half* B, int n, int nrhs, size_t ld, const float* unit,
+                           float2* Y, int* err, cudaStream_t st)
+{
+    CUtensorMap ta, tb[3];
+    const int sms = c->sm_count > 0 ? c->sm_count : 148;
+    EMFA_TRY(make_map_h(c, &ta, A, 2 * (uint64_t)n, (uint64_t)n, ld, th::BM));
+    EMFA_TRY(make_map_h(c, &tb[0], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 64));
+    if (2 * nrhs <= 16) EMFA_TRY(make_map_h(c, &tb[2], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 16));
+    if (2 * nrhs > 64) EMFA_TRY(make_map_h(c, &tb[1], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 144));
+    // 64 columns a tile while they leave SMs idle: a CTA is bound by its operands' arrival
+    const bool narrow = (long)((2 * nrhs + 63) / 64) * ((n + 127) / 128) <= sms;
+    return launch_variant(c, narrow ? HV_64_1 : fixed_variant(n, nrhs, sms), ta, tb, Y, n, nrhs, unit, unit, err, st,
+                          false);
+}
+
 emfa_status_t hgemm_tuned_shape(int device, int n, int nrhs, int* variant, float* ms)
 {
     std::lock_guard<std::mutex> g(g_tune_mu);

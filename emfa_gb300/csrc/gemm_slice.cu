@@ -3,24 +3,35 @@
 // GB300's FP64 pipe runs at 1/64 of the FP32 one, so the CUDA-core FP64 product
 // (gemm.cu) is bound by it from a few right-hand sides on.  Here both operands
 // are cut into eight signed 8-bit digits,
-//     z = 2^(e-62) sum_s d_s 2^(8 (7 - s)),   |d_s| <= 128,
+//     z = 2^(e-63) sum_s d_s 2^(8 (7 - s)),   |d_s| <= 128,
 // with one power of two per row of Z and per right-hand side (the fixed-point
-// form of an FP64 significand: a row's largest entries keep all 53 bits, 62
-// below the row's maximum for the others), and the digits' products run as
-// FP16 MMAs (integers up to 128 are exact in FP16, their products in FP32).
-// Digit pairs (i, j) of one level i + j share an accumulator; levels 0..7 are
-// kept (36 of the 64 pairs: the next level is 2^-70 of the product of the
-// maxima).  128 columns of at most eight pairs add up to at most 2^24, so every
-// FP32 accumulator holds an exact integer, and the sums across those groups are
+// form of an FP64 significand: an entry keeps all 53 bits down to 2^-10 of its
+// row's scale), and the digits' products run as FP16 MMAs (integers up to 128
+// are exact in FP16, their products in FP32).  Digit pairs (i, j) of one level
+// i + j share an accumulator; levels 0..7 are kept (36 of the 64 pairs).  128
+// columns of at most eight pairs add up to at most 2^24, so every FP32
+// accumulator holds an exact integer, and the sums across those groups are
 // exact in 64-bit integers: the result is one rounding of the sum, whatever the
 // order, so K can be split over CTAs freely.
 //
-// Accuracy: relative to (row maximum) x (right-hand side's maximum) x sqrt(n) the
-// error is about 2^-68 before the final rounding, so a row's result is as good
-// as an FP64 sum's or better (measured against extended precision at n = 2430,
-// impedance-like with a dominant diagonal: 9e-17, the CUDA-core sums 3e-15); as with any blockwise scaling,
-// entries of a row below 2^-62 of its largest one count as zero.  A row or a
-// right-hand side with an infinity or NaN takes FP64 arithmetic in k_combine.
+// Accuracy.  In units of the two scales, a real product is off by at most
+// 7 x 2^14 x 2^48 / 2^126 for level 8, 2^-69 for the rest below it, and 2 x 2^-64
+// for the cut of its factors: 2^-60.8, 2n times that a component of the sum.  A
+// floating-point sum's error goes with S = sum |z||x| instead, and S may be far
+// below the scales (columns of Z scaled against x, a large entry that meets a
+// zero).  So S itself is formed, per component, by one more FP16 product of the
+// operands' magnitudes (10 bits each, every nonzero counted; th::k_hgemm, 1/36
+// of the digit products), and k_combine keeps a digit result only where
+//     S >= FLOOR (37/512 in FP64, 161/512 in FP32):
+// there 2n 2^-60.8 <= (2 ceil(n / 32) + 5) 2^-52 S, the first-order bound of the
+// CUDA-core product's own sum (gemm.cu), for every n; FP32, by the same count,
+// 2n 2^-29.7 <= (2 ceil(n / 32) + 5) 2^-23 S.  The other results, and those of a
+// row or right-hand side with an infinity or NaN, are summed in their own type:
+// in FP64 by k_combine's CTA (a term a thread), in FP32 by gemm.cu's tiles.
+// Impedance-like operands have S of 0.04 to 2: of 100 CFIE Krylov products a few
+// hundredths of a percent of the results are summed again.  Measured against
+// extended precision at n = 2430, impedance-like with a dominant diagonal: 9e-17
+// of the result, the CUDA-core sums 3e-15.
 //
 // Kernel k_slice<BN>: one 128 x BN tile and one range of K per CTA, 18 warps:
 //   warp 0      TMA producer, K in blocks of 64 columns (128-byte rows): the
@@ -41,12 +52,15 @@
 // whatever the drain did.  A single thread issuing MMAs with descriptors from
 // its own registers bounded the second (382 us, 86 cycles a MMA); now 301 us,
 // 45 %.
-// On GB300, a product of n unknowns and R right-hand sides, its split of Z
-// included, against the CUDA-core products:
-// 1080 x 91: 4456 -> 100 us;  2430 x 181: 9928 -> 428 us;  5070 x 360: 80.9 -> 2.93 ms
-// FP32 (complex64) operands take four digits, 30 bits below the scale, of which
-// the ten pairs of levels 0..3 are kept (the next is 2^-31 of the product of the
-// maxima): one rounding to FP32 of a sum that is exact to that, against an FP32
+// On GB300, a product of n unknowns and R right-hand sides, its split of Z and
+// the magnitudes' product (10 us and 18 us) included, against 64 x 64 CUDA-core
+// tiles and against the GEMV that sums again where every result needs it:
+// 1080 x 91: 4456, 860 -> 120 us;  2430 x 181: 9928, 7300 -> 450 us.  All results
+// of columns scaled against x by 10^4: 1.66 and 11.5 ms.
+// FP32 (complex64) operands take four digits, 31 bits below the scale, of which
+// the ten pairs of levels 0..3 are kept (a real product is off by at most 3 x 2^14
+// x 2^16 / 2^62 for level 4, 2^-39 below it, 2 x 2^-32 for the cut: 2^-29.7 of the
+// scales): one rounding to FP32 of a sum that is exact to that, against an FP32
 // sum's rounding at every term.
 #include "emfa_internal.cuh"
 #include "emfa_math.cuh"
@@ -67,17 +81,21 @@ constexpr int RING = 4;      // A planes in flight
 constexpr int THREADS = 32 * (2 + 16);
 constexpr int SLICE_NONFINITE = INT_MAX;
 
-// per element type: digits, bits of a scaled value, exponent field, and the
-// lowest kept level's weight in products of two scaled values
+// per element type: digits, bits of a scaled value, the top word's exponent
+// field, and the least S of a digit result (see above)
 template <typename T> struct Cut;
 template <> struct Cut<double> {
-    static constexpr int NS = 8, BITS = 62, FIELD_MAX = 0x7ff, EXP_ONE = 1022;
+    static constexpr int NS = 8, BITS = 63, MANT = 20, FIELD_MAX = 0x7ff, EXP_ONE = 1022;
+    static constexpr float FLOOR = 37.f / 512.f;
     using Word = unsigned long long;
 };
 template <> struct Cut<float> {
-    static constexpr int NS = 4, BITS = 30, FIELD_MAX = 0xff, EXP_ONE = 126;
+    static constexpr int NS = 4, BITS = 31, MANT = 23, FIELD_MAX = 0xff, EXP_ONE = 126;
+    static constexpr float FLOOR = 161.f / 512.f;
     using Word = unsigned;
 };
+// magnitudes are FP16 values of 2^15 times the entry over its scale
+constexpr float MAG_UNIT = 1.f / 32768.f;
 
 // NS digits; the drain's 16 warps: lane quadrant, column part, four levels each
 template <int NS, int BN>
@@ -315,18 +333,26 @@ __global__ void __launch_bounds__(THREADS, 1)
 // ---------------------------------------------------------------------------
 // operand preparation, integers only
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int exponent_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-__device__ __forceinline__ int exponent_field(float x) { return (__float_as_int(x) >> 23) & 0xff; }
+// exponent and leading mantissa bits of |x|: an integer that orders magnitudes
+__device__ __forceinline__ int top_word(double x) { return __double2hiint(x) & 0x7fffffff; }
+__device__ __forceinline__ int top_word(float x) { return __float_as_int(x) & 0x7fffffff; }
 
-// biased digits of x at scale eb (the row's largest exponent field, at least
-// 1): byte s of the result is d_(NS-1-s) + 128
+// scale of a row from its largest top word: the exponent field eb, at least 1,
+// with |x| < 127/128 2^(eb - EXP_ONE), so that the leading digit stays below 128
+template <typename T>
+__device__ __forceinline__ int scale_field(int top)
+{
+    return max(1, (top + (1 << (Cut<T>::MANT - 6))) >> Cut<T>::MANT);
+}
+
+// biased digits of x at scale eb: byte s of the result is d_(NS-1-s) + 128
 __device__ __forceinline__ unsigned long long digits(double x, int eb)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const int ef = (int)((b >> 52) & 0x7ff);
     unsigned long long m = b & 0xFFFFFFFFFFFFFull;
     if (ef) m |= 1ull << 52;
-    const int s = (ef ? ef : 1) - eb + 9;  // 0..9 for the largest
+    const int s = (ef ? ef : 1) - eb + 10;  // 9 or 10 for the largest
     long long v;
     if (s >= 0)
         v = (long long)(m << s);
@@ -341,7 +367,7 @@ __device__ __forceinline__ unsigned digits(float x, int eb)
     const int ef = (int)((b >> 23) & 0xff);
     unsigned m = b & 0x7fffffu;
     if (ef) m |= 1u << 23;
-    const int s = (ef ? ef : 1) - eb + 6;  // 0..6 for the largest
+    const int s = (ef ? ef : 1) - eb + 7;  // 6 or 7 for the largest
     int v;
     if (s >= 0)
         v = (int)(m << s);
@@ -349,6 +375,39 @@ __device__ __forceinline__ unsigned digits(float x, int eb)
         v = s < -25 ? 0 : (int)((m + (1u << (-s - 1))) >> -s);
     if ((int)b < 0) v = -v;
     return ((unsigned)v + 0x00808080u) ^ 0x80000000u;
+}
+
+// |x| 2^15 / 2^(eb - EXP_ONE) as an FP16 value: 10 mantissa bits, cut off; below
+// FP16's range the smallest value, so that only a zero is zero
+template <typename T>
+__device__ __forceinline__ unsigned magnitude(T x, int eb)
+{
+    int ef, m;  // exponent field and 10 mantissa bits
+    bool zero;
+    if constexpr (sizeof(T) == 8) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+        zero = b == 0;
+        ef = (int)(b >> 52);
+        m = (int)(b >> 42) & 0x3ff;
+        if (ef == 0 && !zero) {  // subnormal
+            const int z = __clzll((long long)b) - 11;
+            ef = 1 - z;
+            m = (int)((b << z) >> 42) & 0x3ff;
+        }
+    } else {
+        const unsigned b = (unsigned)__float_as_int(x) & 0x7fffffffu;
+        zero = b == 0;
+        ef = (int)(b >> 23);
+        m = (int)(b >> 13) & 0x3ff;
+        if (ef == 0 && !zero) {
+            const int z = __clz((int)b) - 8;
+            ef = 1 - z;
+            m = (int)((b << z) >> 13) & 0x3ff;
+        }
+    }
+    const int e = ef - eb + 29;
+    const int low = e < -9 ? 1 : max(1, (m | 0x400) >> (1 - min(e, 1)));
+    return zero ? 0u : (unsigned)(e >= 1 ? (e << 10) | m : low);
 }
 
 // digit s of a complex pair as two FP16 integers: the byte under the exponent
@@ -379,8 +438,8 @@ __device__ __forceinline__ int block_max_int(int m, int* red)
     return red[0];
 }
 
-// CTA per row of Z: its scale, then its digits (the row is read twice, the
-// second time from L2)
+// CTA per row of Z: its scale, then its digits and, in the plane after them, its
+// magnitudes (the row is read twice, the second time from L2)
 template <typename T>
 __global__ void __launch_bounds__(256) k_slice_rows(const Cx<T>* __restrict__ Z, size_t ldz, int n, size_t ldk,
                                                     __half* __restrict__ D, int* __restrict__ ex)
@@ -389,48 +448,61 @@ __global__ void __launch_bounds__(256) k_slice_rows(const Cx<T>* __restrict__ Z,
     __shared__ int red[32];
     const int i = blockIdx.x;
     const Cx<T>* z = Z + (size_t)i * ldz;
-    int m = 1;
+    int m = 0;
 #pragma unroll 4
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const Cx<T> v = z[k];
-        m = max(m, max(exponent_field(v.re), exponent_field(v.im)));
+        m = max(m, max(top_word(v.re), top_word(v.im)));
     }
     m = block_max_int(m, red);
-    const bool bad = m == Cut<T>::FIELD_MAX;
-    if (threadIdx.x == 0) ex[i] = bad ? SLICE_NONFINITE : m;
-    const size_t plane = (size_t)n * ldk / 2;
+    const bool bad = m >> Cut<T>::MANT == Cut<T>::FIELD_MAX;
+    const int eb = scale_field<T>(m);
+    if (threadIdx.x == 0) ex[i] = bad ? SLICE_NONFINITE : eb;
+    const size_t plane = (size_t)gridDim.x * ldk / 2;
     unsigned* o = reinterpret_cast<unsigned*>(D) + (size_t)i * (ldk / 2);
     constexpr Word zero = (Word)0x8080808080808080ull;
     // two elements a thread, one 8-byte store a plane (the rows of D are padded
     // to 16 bytes: an odd row's last store ends in the padding)
     for (int k = 2 * threadIdx.x; k < n; k += 2 * blockDim.x) {
         const Cx<T> v = z[k], u = k + 1 < n ? z[k + 1] : cx(T(0), T(0));
-        const Word a = bad ? zero : digits(v.re, m), b = bad ? zero : digits(v.im, m);
-        const Word c = bad ? zero : digits(u.re, m), d = bad ? zero : digits(u.im, m);
+        const Word a = bad ? zero : digits(v.re, eb), b = bad ? zero : digits(v.im, eb);
+        const Word c = bad ? zero : digits(u.re, eb), d = bad ? zero : digits(u.im, eb);
 #pragma unroll
         for (int s = 0; s < Cut<T>::NS; ++s)
             *reinterpret_cast<uint2*>(o + s * plane + k) = make_uint2(pair_digit(a, b, s), pair_digit(c, d, s));
+        *reinterpret_cast<uint2*>(o + Cut<T>::NS * plane + k) =
+            bad ? make_uint2(0u, 0u)
+                : make_uint2(magnitude(v.re, eb) | magnitude(v.im, eb) << 16,
+                             magnitude(u.re, eb) | magnitude(u.im, eb) << 16);
     }
 }
 
-// CTA per right-hand side: B rows 2r = (Re, -Im) and 2r + 1 = (Im, Re)
+// CTA per right-hand side: B rows 2r = (Re, -Im) and 2r + 1 = (Im, Re), of the
+// magnitudes (|Re|, |Im|) and (|Im|, |Re|).  unit[r]: the magnitudes' unit;
+// *again: no result to be summed again so far.
 template <typename T>
 __global__ void __launch_bounds__(256) k_slice_rhs(const Cx<T>* __restrict__ X, int n, int nrhs, size_t ldk,
-                                                   __half* __restrict__ D, int* __restrict__ ex)
+                                                   __half* __restrict__ D, int* __restrict__ ex,
+                                                   float* __restrict__ unit, int* __restrict__ again)
 {
     using Word = typename Cut<T>::Word;
     __shared__ int red[32];
     const int r = blockIdx.x;
     const Cx<T>* x = X + (size_t)r * n;
-    int m = 1;
+    int m = 0;
 #pragma unroll 4
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const Cx<T> v = x[k];
-        m = max(m, max(exponent_field(v.re), exponent_field(v.im)));
+        m = max(m, max(top_word(v.re), top_word(v.im)));
     }
     m = block_max_int(m, red);
-    const bool bad = m == Cut<T>::FIELD_MAX;
-    if (threadIdx.x == 0) ex[r] = bad ? SLICE_NONFINITE : m;
+    const bool bad = m >> Cut<T>::MANT == Cut<T>::FIELD_MAX;
+    const int eb = scale_field<T>(m);
+    if (threadIdx.x == 0) {
+        ex[r] = bad ? SLICE_NONFINITE : eb;
+        unit[r] = MAG_UNIT;
+        if (r == 0) *again = 0;
+    }
     const size_t plane = (size_t)2 * nrhs * ldk / 2;
     unsigned* o0 = reinterpret_cast<unsigned*>(D) + (size_t)(2 * r) * (ldk / 2);
     unsigned* o1 = o0 + ldk / 2;
@@ -438,13 +510,16 @@ __global__ void __launch_bounds__(256) k_slice_rhs(const Cx<T>* __restrict__ X, 
 #pragma unroll 2
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const Cx<T> v = x[k];
-        const Word a = bad ? zero : digits(v.re, m), b = bad ? zero : digits(v.im, m),
-                   nb = bad ? zero : digits(-v.im, m);
+        const Word a = bad ? zero : digits(v.re, eb), b = bad ? zero : digits(v.im, eb),
+                   nb = bad ? zero : digits(-v.im, eb);
 #pragma unroll
         for (int s = 0; s < Cut<T>::NS; ++s) {
             o0[s * plane + k] = pair_digit(a, nb, s);
             o1[s * plane + k] = pair_digit(b, a, s);
         }
+        const unsigned re = bad ? 0u : magnitude(v.re, eb), im = bad ? 0u : magnitude(v.im, eb);
+        o0[Cut<T>::NS * plane + k] = re | im << 16;
+        o1[Cut<T>::NS * plane + k] = im | re << 16;
     }
 }
 
@@ -485,58 +560,102 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int ex)
     return neg ? -v : v;
 }
 
-// Y from the partial sums of all splits.  A row or a right-hand side with an
-// infinity or NaN is summed in T as gemm.cu does; a pipeline that gave up (err)
-// leaves NaN.
+// Y from the partial sums of all splits where the digits are as good as a sum in
+// T (S at least FLOOR, or zero: no product at all); a pipeline that gave up (err)
+// leaves NaN.  The rest is summed in T: FP64 by the CTA, one result after the
+// other, a term a thread (a few results cost a few us, all of them about the
+// GEMV's time); FP32 results are marked in `mask` for gemm.cu's tiles.
 template <typename T>
 __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ part, int splits, int n, int nrhs,
                                                  const int* __restrict__ exz, const int* __restrict__ exx,
-                                                 const Cx<T>* __restrict__ Z, size_t ldz,
+                                                 const float2* __restrict__ S, const Cx<T>* __restrict__ Z, size_t ldz,
                                                  const Cx<T>* __restrict__ X, const int* __restrict__ err,
-                                                 Cx<T>* __restrict__ Y)
+                                                 Cx<T>* __restrict__ Y, unsigned char* __restrict__ mask,
+                                                 int* __restrict__ again)
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-    if (f >= n) return;
-    const int ez = exz[f], ex = exx[r];
-    Cx<T> y;
-    if (*err) {
-        y.re = y.im = (T)__longlong_as_double(0x7ff8000000000000ll);
-    } else if (ez == SLICE_NONFINITE || ex == SLICE_NONFINITE) {
-        const Cx<T>* z = Z + (size_t)f * ldz;
-        const Cx<T>* x = X + (size_t)r * n;
-        T re = 0, im = 0;
-        for (int k = 0; k < n; ++k) {
-            const Cx<T> a = z[k], b = x[k];
-            re = fma(a.re, b.re, re);
-            re = fma(-a.im, b.im, re);
-            im = fma(a.re, b.im, im);
-            im = fma(a.im, b.re, im);
-        }
-        y = cx(re, im);
-    } else {
-        const size_t plane = (size_t)2 * nrhs * n;
-        const long long* p0 = part + (size_t)(2 * r) * n + f;
-        // z = V 2^(e - BITS), e = field - EXP_ONE; the lowest kept level, NS - 1, weighs 2^(8 (NS - 1)) in V V
-        const int e = ez + ex - 2 * (Cut<T>::EXP_ONE + Cut<T>::BITS) + 8 * (Cut<T>::NS - 1);
-        long long s0 = 0, s1 = 0;  // levels 0-3
-        if constexpr (Cut<T>::NS == 8) {
-            long long l0 = 0, l1 = 0;
-            for (int s = 0; s < splits; ++s, p0 += 2 * plane) {
-                s0 += p0[0];
-                s1 += p0[n];
-                l0 += p0[plane];
-                l1 += p0[plane + n];
-            }
-            y = cx((T)to_double(s0, l0, e), (T)to_double(s1, l1, e));
+    const bool live = f < n;
+    bool sum = false;
+    Cx<T> y = cx(T(0), T(0));
+    if (live) {
+        const int ez = exz[f], ex = exx[r];
+        const float2 s = S[(size_t)r * n + f];
+        if (*err) {
+            y.re = y.im = (T)__longlong_as_double(0x7ff8000000000000ll);
+        } else if (ez == SLICE_NONFINITE || ex == SLICE_NONFINITE || (s.x > 0.f && s.x < Cut<T>::FLOOR) ||
+                   (s.y > 0.f && s.y < Cut<T>::FLOOR)) {
+            sum = true;
         } else {
-            for (int s = 0; s < splits; ++s, p0 += plane) {
-                s0 += p0[0];
-                s1 += p0[n];
+            const size_t plane = (size_t)2 * nrhs * n;
+            const long long* p0 = part + (size_t)(2 * r) * n + f;
+            // z = V 2^(e - BITS), e = field - EXP_ONE; the lowest kept level, NS - 1, weighs 2^(8 (NS - 1)) in V V
+            const int e = ez + ex - 2 * (Cut<T>::EXP_ONE + Cut<T>::BITS) + 8 * (Cut<T>::NS - 1);
+            long long s0 = 0, s1 = 0;  // levels 0-3
+            if constexpr (Cut<T>::NS == 8) {
+                long long l0 = 0, l1 = 0;
+                for (int q = 0; q < splits; ++q, p0 += 2 * plane) {
+                    s0 += p0[0];
+                    s1 += p0[n];
+                    l0 += p0[plane];
+                    l1 += p0[plane + n];
+                }
+                y = cx((T)to_double(s0, l0, e), (T)to_double(s1, l1, e));
+            } else {
+                for (int q = 0; q < splits; ++q, p0 += plane) {
+                    s0 += p0[0];
+                    s1 += p0[n];
+                }
+                y = cx((T)to_double(s0 >> 32, s0 & 0xffffffffll, e), (T)to_double(s1 >> 32, s1 & 0xffffffffll, e));
             }
-            y = cx((T)to_double(s0 >> 32, s0 & 0xffffffffll, e), (T)to_double(s1 >> 32, s1 & 0xffffffffll, e));
         }
     }
-    Y[(size_t)r * n + f] = y;
+    if constexpr (Cut<T>::NS == 8) {
+        __shared__ unsigned todo[8];
+        __shared__ Cx<T> red[2][8];
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        const unsigned b = __ballot_sync(0xffffffffu, sum);
+        if (l == 0) todo[w] = b;
+        if (__syncthreads_or(sum)) {  // uniform
+            const Cx<T>* x = X + (size_t)r * n;
+            int turn = 0;
+            for (int q = 0; q < 8; ++q)
+                for (unsigned left = todo[q]; left; left &= left - 1, turn ^= 1) {
+                    const int t = 32 * q + __ffs((int)left) - 1;
+                    const Cx<T>* z = Z + (size_t)(blockIdx.x * blockDim.x + t) * ldz;
+                    T re = 0, im = 0;
+#pragma unroll 4
+                    for (int k = threadIdx.x; k < n; k += 256) {
+                        const Cx<T> a = z[k], v = x[k];
+                        re = fma(a.re, v.re, re);
+                        re = fma(-a.im, v.im, re);
+                        im = fma(a.re, v.im, im);
+                        im = fma(a.im, v.re, im);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        re += __shfl_xor_sync(0xffffffffu, re, o);
+                        im += __shfl_xor_sync(0xffffffffu, im, o);
+                    }
+                    if (l == 0) red[turn][w] = cx(re, im);
+                    __syncthreads();  // the next result's sums go to the other half
+                    if ((int)threadIdx.x == t) {
+                        y = red[turn][0];
+#pragma unroll
+                        for (int i = 1; i < 8; ++i) {
+                            y.re += red[turn][i].re;
+                            y.im += red[turn][i].im;
+                        }
+                    }
+                }
+        }
+        if (live) Y[(size_t)r * n + f] = y;
+    } else if (live) {
+        mask[(size_t)r * n + f] = sum;
+        if (sum)
+            *again = 1;
+        else
+            Y[(size_t)r * n + f] = y;
+    }
 }
 
 }  // namespace sl
@@ -546,9 +665,10 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
 // ---------------------------------------------------------------------------
 static size_t slice_ld(int n) { return ((size_t)2 * n + 7) & ~(size_t)7; }  // 16-byte rows
 
+// ns digits and the magnitudes
 static size_t slice_plane_bytes(int ns, int n)
 {
-    return Carver::round(sizeof(__half) * ns * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
+    return Carver::round(sizeof(__half) * (ns + 1) * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
 }
 
 static emfa_status_t slice_map(Ctx* c, CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, size_t ld,
@@ -597,23 +717,23 @@ static bool slice_allowed(Ctx* c, int ns, int n, cudaStream_t st)
 bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st)
 {
     if (!slice_allowed(c, sl::Cut<double>::NS, n, st)) return false;
-    // Measured (us, a call with its one split of Z | the CUDA-core GEMV): n = 256, 8 right-hand sides 55 | 48,
-    // 16: 59 | 75; 480, 8: 58 | 63; 1080, 4: 81 | 68, 8: 80 | 106; 2430, 4: 182 | 191; 5070, 2: 646 | 438, 4: 647 | 847.
-    // With Z split already, n = 2430, 2: 125 | 110; 5070, 2: 400 | 438.
-    if (built) return nrhs >= (n >= 2000 ? 3 : n >= 1000 ? 4 : n >= 480 ? 8 : 10);
-    return nrhs >= (n >= 2000 ? 4 : n >= 1000 ? 6 : n >= 480 ? 8 : 12);
+    // Measured (us, a call with its one split of Z | the CUDA-core GEMV): n = 256, 24 right-hand sides 63 | 51,
+    // 40: 65 | 68; 480, 12: 67 | 53, 16: 69 | 71; 750, 8: 71 | 91; 1080, 6: 86 | 83, 8: 86 | 118; 2430, 4: 184 | 192;
+    // 5070, 4: 540 | 842.  The split of Z, which a solve makes once, is 8 us of it at n = 480, 15 at 1080, 60 at 2430.
+    if (built) return nrhs >= (n >= 2000 ? 3 : n >= 1000 ? 6 : n >= 600 ? 8 : n >= 480 ? 12 : 32);
+    return nrhs >= (n >= 2000 ? 4 : n >= 600 ? 8 : n >= 480 ? 16 : 32);
 }
 
 // One FP32 product with its split of Z, where it beats the CUDA cores' tiles
-// (us, this | tiles: n = 480 x 360, 69 | 56; 1033 x 181, 85 | 72, x 360, 119 | 123;
-// 2000 x 96, 125 | 118, x 128, 129 | 152; 3000 x 80, 202 | 173, x 96, 202 | 183,
-// x 128, 207 | 229; 5067 x 80, 483 | 403, x 96, 488 | 535): above 80 right-hand
-// sides and 200000 results.  Errors on normal entries, n = 480 to 5067: this
-// 3e-8, the tiles 2.1e-7 to 8.1e-7, the GEMV 1.2e-7 to 3.3e-7, 64 x 64 tiles 5.5e-7
-// to 1.8e-6.
+// (us, this | tiles: n = 1033 x 360, 139 | 98; 1500 x 360, 177 | 191; 2000 x 280, 252 | 241,
+// x 360, 263 | 346; 3000 x 160, 294 | 296, x 240, 359 | 386, x 360, 443 | 689; 5067 x 96, 574 | 529,
+// x 128, 604 | 677, x 360, 1187 | 1621): above 100 right-hand sides and 600000 results.  With every
+// result summed again (columns scaled against x) 5067 x 360 takes 2921; 64 x 64 tiles, 2350.  Errors on
+// normal entries, n = 480 to 5067: this 3e-8, the tiles 2.1e-7 to 8.1e-7, the GEMV 1.2e-7 to 3.3e-7, 64 x 64 tiles
+// 5.5e-7 to 1.8e-6.
 static bool slice_worthwhile_f32(Ctx* c, int n, int nrhs, cudaStream_t st)
 {
-    return nrhs > 80 && (long)n * nrhs > 200000 && slice_allowed(c, sl::Cut<float>::NS, n, st);
+    return nrhs > 100 && (long)n * nrhs > 600000 && slice_allowed(c, sl::Cut<float>::NS, n, st);
 }
 
 template <typename T>
@@ -624,7 +744,7 @@ static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int 
     void* wp = nullptr;
     EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(NS, n) + 512, &wp));
     Carver cv{(char*)wp};
-    __half* d = cv.take<__half>(NS * (size_t)n * ldk);
+    __half* d = cv.take<__half>((NS + 1) * (size_t)n * ldk);
     int* ex = cv.take<int>(n);
     int* err = nullptr;
     EMFA_TRY(slice_err(c, &err));
@@ -706,13 +826,18 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
     const size_t parts = (size_t)smax * 2 * SETS * rmax * n;
     void* wp = nullptr;
     EMFA_TRY(ctx_workspace(c, slot,
-                           Carver::round(sizeof(__half) * NS * brow) + Carver::round(sizeof(int) * (size_t)rmax) +
-                               Carver::round(sizeof(long long) * parts) + 1024,
+                           Carver::round(sizeof(__half) * (NS + 1) * brow) + 2 * Carver::round(sizeof(int) * (size_t)rmax) +
+                               Carver::round(sizeof(long long) * parts) +
+                               Carver::round(sizeof(float2) * (size_t)rmax * n) + Carver::round((size_t)rmax * n) + 2048,
                            &wp));
     Carver cv{(char*)wp};
-    __half* b = cv.take<__half>(NS * brow);
+    __half* b = cv.take<__half>((NS + 1) * brow);
     int* ex = cv.take<int>(rmax);
+    float* unit = cv.take<float>(rmax);
     long long* part = cv.take<long long>(parts);
+    float2* sums = cv.take<float2>((size_t)rmax * n);
+    unsigned char* mask = cv.take<unsigned char>((size_t)rmax * n);
+    int* again = cv.take<int>(1);
     int* err = nullptr;
     EMFA_TRY(slice_err(c, &err));
     CUtensorMap ta, tb;
@@ -722,15 +847,19 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
         const Cx<T>* x = (const Cx<T>*)X + (size_t)r0 * n;
         slice_shape<T>(c, n, nr, &bn, &splits, &per_split);
         EMFA_TRY(slice_map(c, &tb, b, 2 * (uint64_t)n, 2 * (uint64_t)nr, p.ldk, NS, (uint32_t)bn, NS));
-        sl::k_slice_rhs<T><<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex);
+        Cx<T>* y = (Cx<T>*)Y + (size_t)r0 * n;
+        sl::k_slice_rhs<T><<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex, unit, again);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
         EMFA_TRY((bn == NARROW ? launch_slice<NS, NARROW> : launch_slice<NS, WIDE>)(c, ta, tb, n, nr, splits, per_split,
                                                                                   part, err, st));
-        sl::k_combine<T><<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, (const Cx<T>*)p.Z,
-                                                                    p.ldz, x, err, (Cx<T>*)Y + (size_t)r0 * n);
+        EMFA_TRY(hgemm_planes(c, p.d + NS * (size_t)n * p.ldk, b + NS * (size_t)2 * nr * p.ldk, n, nr, p.ldk, unit, sums,
+                              err, st));
+        sl::k_combine<T><<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, sums, (const Cx<T>*)p.Z,
+                                                                    p.ldz, x, err, y, mask, again);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
+        if (NS == 4) EMFA_TRY(cgemm_f32_masked(c, p.Z, p.ldz, x, n, nr, y, mask, again, st));
     }
     return EMFA_OK;
 }

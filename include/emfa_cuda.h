@@ -48,11 +48,14 @@ typedef enum { EMFA_EFIE = 0, EMFA_CFIE = 1 } emfa_kind_t;
 typedef enum { EMFA_GMRES = 0, EMFA_BICGSTAB = 1, EMFA_LU = 2 } emfa_method_t;
 typedef enum {
     EMFA_MV_AUTO = 0,  /* F64: FP64 accuracy on the tensor cores for blocks of right- */
-                       /* hand sides (operands as 8-bit digit planes, exact sums; an */
-                       /* error no larger than an FP64 sum's relative to the row and */
-                       /* vector maxima), else FP64 SIMT; F32: EMFA_MV_F16X in solves */
-                       /* and residuals, in emfa_matvec FP32 accuracy the same way   */
-                       /* (four digits) for wide blocks (above 80), else FP32 SIMT   */
+                       /* hand sides (operands as 8-bit digit planes, exact sums; a  */
+                       /* component whose own products are small against the row's   */
+                       /* and the vector's maxima is summed in FP64 instead, so the  */
+                       /* error stays within an FP64 sum's bound of sum |z||x|),     */
+                       /* else FP64 SIMT; F32: EMFA_MV_F16X in solves and residuals, */
+                       /* in emfa_matvec FP32 accuracy the same way (four digits)    */
+                       /* for wide blocks (above 100, and 600000 results), else FP32 */
+                       /* SIMT                                                       */
     EMFA_MV_F64 = 1,   /* FP64 complex product on CUDA cores (plain path)            */
     EMFA_MV_F32 = 2,   /* FP32 complex GEMM on CUDA cores; residual FP32 products    */
                        /* with FP64 chunk sums                                       */
