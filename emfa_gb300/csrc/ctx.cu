@@ -1,5 +1,6 @@
 // Context, status strings and HBM-budget accounting of libemfa_cuda.
 #include "emfa_internal.cuh"
+#include "gemm_slice.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -216,13 +217,14 @@ emfa_status_t emfa_ctx_create(int device, size_t hbm_budget_bytes, emfa_ctx_t** 
         delete c;
         return EMFA_ERR_CUDA;
     }
-    e = cudaHostAlloc((void**)&c->pinned, 64 * sizeof(int), cudaHostAllocDefault);
+    e = cudaHostAlloc((void**)&c->pinned, Ctx::PINNED * sizeof(int), cudaHostAllocDefault);
     if (e != cudaSuccess) {
         set_global_error(std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
         cudaStreamDestroy(c->stream);
         delete c;
         return EMFA_ERR_CUDA;
     }
+    std::memset(c->pinned, 0, Ctx::PINNED * sizeof(int));
     *out = c;
     return EMFA_OK;
 }
@@ -292,7 +294,7 @@ emfa_status_t emfa_ctx_synchronize(emfa_ctx_t* ctx)
     if (!ctx) return EMFA_ERR_INVALID;
     EMFA_CUDA(ctx, cudaSetDevice(ctx->device));
     EMFA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return EMFA_OK;
+    return slice_report(ctx);
 }
 
 emfa_status_t emfa_device_alloc(emfa_ctx_t* ctx, size_t bytes, void** dev)

@@ -117,6 +117,7 @@ struct Ctx {
     std::string last_error;
     std::mutex mu;
     std::mutex slice_mu;  // launches of one digit-plane product (its workspaces are the context's)
+    bool slice_word_clear = false;  // the single products' error word has been zeroed
     int sm_count = 0;
     long long kernel_launches = 0;  // kernels launched through this context
     bool stream_ordered = false;  // allocations on `stream` (cudaMallocAsync), for lanes of the server
@@ -125,7 +126,10 @@ struct Ctx {
     KernelTimer timers[KT_COUNT];
     DevBuf ws[WS_COUNT];            // declared after mu: destroyed before it
     std::map<void*, size_t> user_bufs;  // emfa_device_alloc'ed buffers
-    int* pinned = nullptr;          // page-locked host words for asynchronous status reads (64 ints)
+    // page-locked host words for asynchronous status reads: the steps' counts,
+    // and the last for a digit-plane product whose pipeline gave up (slice_report)
+    int* pinned = nullptr;
+    static constexpr int PINNED = 64;
 };
 
 emfa_status_t ctx_workspace(Ctx* c, int slot, size_t bytes, void** p);

@@ -560,6 +560,7 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int ex)
     return neg ? -v : v;
 }
 
+// report (optional): a page-locked host word that gets *err.
 // Y from the partial sums of all splits where the digits are as good as a sum in
 // T (S at least FLOOR, or zero: no product at all); a pipeline that gave up (err)
 // leaves NaN.  The rest is summed in T: FP64 by the CTA, one result after the
@@ -571,8 +572,9 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
                                                  const float2* __restrict__ S, const Cx<T>* __restrict__ Z, size_t ldz,
                                                  const Cx<T>* __restrict__ X, const int* __restrict__ err,
                                                  Cx<T>* __restrict__ Y, unsigned char* __restrict__ mask,
-                                                 int* __restrict__ again)
+                                                 int* __restrict__ again, int* __restrict__ report)
 {
+    if (report && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *err) *(volatile int*)report = *err;
     const int f = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
     const bool live = f < n;
     bool sum = false;
@@ -693,13 +695,39 @@ static emfa_status_t slice_map(Ctx* c, CUtensorMap* m, const void* ptr, uint64_t
     return EMFA_OK;
 }
 
-// error word of the sliced product: int 8 of the context's GEMM error slot
-static emfa_status_t slice_err(Ctx* c, int** err)
+// error words of the products: ints 8 (a solve's) and 9 (single products') of
+// the context's GEMM error slot
+static emfa_status_t slice_err(Ctx* c, int word, int** err)
 {
     void* ep = nullptr;
     EMFA_TRY(ctx_workspace(c, WS_GEMM_ERR, 64, &ep));
-    *err = (int*)ep + 8;
+    *err = (int*)ep + word;
     return EMFA_OK;
+}
+
+emfa_status_t slice_word(Ctx* c, int** err, cudaStream_t st)
+{
+    EMFA_TRY(slice_err(c, 9, err));
+    if (!c->slice_word_clear) EMFA_CUDA(c, cudaMemsetAsync(*err, 0, sizeof(int), st));
+    c->slice_word_clear = true;
+    return EMFA_OK;
+}
+
+static emfa_status_t timed_out(Ctx* c, int stage)
+{
+    set_error(c, "digit-plane tensor-core product: a pipeline wait timed out (stage " + std::to_string(stage) + ")");
+    return EMFA_ERR_TIMEOUT;
+}
+
+emfa_status_t slice_report(Ctx* c)
+{
+    std::lock_guard<std::mutex> lk(c->slice_mu);
+    volatile int* told = c->pinned + Ctx::PINNED - 1;
+    const int stage = *told;
+    if (!stage) return EMFA_OK;
+    *told = 0;
+    c->slice_word_clear = false;
+    return timed_out(c, stage);
 }
 
 // The planes take twice the matrix's memory, in workspaces of the context that
@@ -746,9 +774,6 @@ static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int 
     Carver cv{(char*)wp};
     __half* d = cv.take<__half>((NS + 1) * (size_t)n * ldk);
     int* ex = cv.take<int>(n);
-    int* err = nullptr;
-    EMFA_TRY(slice_err(c, &err));
-    EMFA_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), st));
     sl::k_slice_rows<T><<<n, 256, 0, st>>>((const Cx<T>*)Z, ldz, n, ldk, d, ex);
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
@@ -758,6 +783,9 @@ static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int 
 
 emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
 {
+    int* err = nullptr;
+    EMFA_TRY(slice_err(c, 8, &err));
+    EMFA_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), st));
     return prepare_t<double>(c, slot, Z, ldz, n, out, st);
 }
 
@@ -806,7 +834,8 @@ static emfa_status_t launch_slice(Ctx* c, const CUtensorMap& ta, const CUtensorM
 }
 
 template <typename T>
-static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
+static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, int* err,
+                             int* report, cudaStream_t st)
 {
     constexpr int NS = sl::Cut<T>::NS, SETS = NS / 4, NARROW = Tile<T>::NARROW, WIDE = Tile<T>::WIDE;
     const int n = p.n;
@@ -838,8 +867,6 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
     float2* sums = cv.take<float2>((size_t)rmax * n);
     unsigned char* mask = cv.take<unsigned char>((size_t)rmax * n);
     int* again = cv.take<int>(1);
-    int* err = nullptr;
-    EMFA_TRY(slice_err(c, &err));
     CUtensorMap ta, tb;
     EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)n, p.ldk, NS, sl::BM, 1));
     for (int r0 = 0; r0 < nrhs; r0 += RB) {
@@ -856,7 +883,7 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
         EMFA_TRY(hgemm_planes(c, p.d + NS * (size_t)n * p.ldk, b + NS * (size_t)2 * nr * p.ldk, n, nr, p.ldk, unit, sums,
                               err, st));
         sl::k_combine<T><<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, sums, (const Cx<T>*)p.Z,
-                                                                    p.ldz, x, err, y, mask, again);
+                                                                    p.ldz, x, err, y, mask, again, report);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
         if (NS == 4) EMFA_TRY(cgemm_f32_masked(c, p.Z, p.ldz, x, n, nr, y, mask, again, st));
@@ -866,21 +893,19 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
 
 emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st)
 {
-    return apply_t<double>(c, slot, p, X, nrhs, Y, st);
+    int* err = nullptr;
+    EMFA_TRY(slice_err(c, 8, &err));
+    return apply_t<double>(c, slot, p, X, nrhs, Y, err, nullptr, st);
 }
 
 emfa_status_t slice_check(Ctx* c, cudaStream_t st)
 {
     int* err = nullptr;
-    EMFA_TRY(slice_err(c, &err));
+    EMFA_TRY(slice_err(c, 8, &err));
     int h = 0;
     EMFA_CUDA(c, cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     EMFA_CUDA(c, cudaStreamSynchronize(st));
-    if (h) {
-        set_error(c, "digit-plane tensor-core product: a pipeline wait timed out (stage " + std::to_string(h) + ")");
-        return EMFA_ERR_TIMEOUT;
-    }
-    return EMFA_OK;
+    return h ? timed_out(c, h) : EMFA_OK;
 }
 
 template <typename T>
@@ -890,9 +915,11 @@ static emfa_status_t matvec_t(Ctx* c, const void* Z, size_t ldz, const void* X, 
     // the whole sequence of launches at once: another thread's product on this
     // context's stream uses the same workspaces before or after it
     std::lock_guard<std::mutex> lk(c->slice_mu);
+    int* err = nullptr;
+    EMFA_TRY(slice_word(c, &err, st));
     SlicePlanes p;
     emfa_status_t s = prepare_t<T>(c, WS_SLICE_MV, Z, ldz, n, &p, st);
-    if (s == EMFA_OK) s = apply_t<T>(c, WS_SLICE_MV_B, p, X, nrhs, Y, st);
+    if (s == EMFA_OK) s = apply_t<T>(c, WS_SLICE_MV_B, p, X, nrhs, Y, err, c->pinned + Ctx::PINNED - 1, st);
     if (s == EMFA_ERR_OOM) {
         cudaGetLastError();  // no room: the caller's CUDA-core product
         return EMFA_OK;

@@ -23,9 +23,16 @@ bool slice_worthwhile(Ctx* c, int n, int nrhs, bool built, cudaStream_t st);
 // caller takes the CUDA-core product.
 emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st);
 // Y = Z X (complex128, RHS-major) with scratch from workspace `slot`; the error
-// word of the pipeline's bounded waits turns Y into NaN (and slice_check tells)
+// word of the pipeline's bounded waits turns Y into NaN, and slice_check tells
+// (it reads the word of a solve's products, which slice_prepare zeroes)
 emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st);
 emfa_status_t slice_check(Ctx* c, cudaStream_t st);
+// The error word of single products.  It is not read after a product, which
+// would wait for it: the product tells a page-locked word, and the next call
+// that looks (slice_report: emfa_ctx_synchronize, emfa_matvec, emfa_residual)
+// returns EMFA_ERR_TIMEOUT once and has the word zeroed.
+emfa_status_t slice_word(Ctx* c, int** err, cudaStream_t st);
+emfa_status_t slice_report(Ctx* c);
 // one product in precision prec: splits Z, multiplies; false in *done where the
 // CUDA cores are the better path or there is no room
 emfa_status_t slice_matvec(Ctx* c, int prec, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,

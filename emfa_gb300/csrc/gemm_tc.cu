@@ -23,6 +23,7 @@
 // and returns, and the host reports EMFA_ERR_TIMEOUT.
 #include "emfa_internal.cuh"
 #include "gemm.cuh"
+#include "gemm_slice.cuh"
 #include "tcgen05.cuh"
 
 #include <cuda.h>
@@ -310,6 +311,19 @@ emfa_status_t cgemm_tf32_scratch(const void* Z, size_t ldz, const void* X, int n
 }
 
 }  // namespace emfa
+
+extern "C" emfa_status_t emfa_diag_product_timeout(emfa_ctx_t* ctx)
+{
+    using namespace emfa;
+    if (!ctx) return EMFA_ERR_INVALID;
+    EMFA_CUDA(ctx, cudaSetDevice(ctx->device));
+    int* err = nullptr;
+    EMFA_TRY(slice_word(ctx, &err, ctx->stream));
+    tc::k_diag_wait<<<1, 32, 0, ctx->stream>>>(err, 42, 2000000LL);  // about 1 ms
+    ctx->kernel_launches += 1;
+    EMFA_CUDA(ctx, cudaGetLastError());
+    return EMFA_OK;
+}
 
 extern "C" emfa_status_t emfa_diag_wait_timeout(emfa_ctx_t* ctx, int* code_out)
 {

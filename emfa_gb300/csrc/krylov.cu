@@ -3194,6 +3194,7 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
     }
     EMFA_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    EMFA_TRY(slice_report(ctx));  // of an earlier product
     if (prec == EMFA_F64) {
         bool done = false;
         if (matvec != EMFA_MV_F64) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));

@@ -381,6 +381,11 @@ emfa_status_t emfa_diag_sincospi(const float* x_dev, int n, float* s_dev, float*
  * *code_out = 42 (the stage code it recorded); the context stays usable.
  * No counterpart in the reference (it has no device code). */
 emfa_status_t emfa_diag_wait_timeout(emfa_ctx_t* ctx, int* code_out);
+/* Diagnostics: the same wait, recorded where a digit-plane product's pipeline
+ * would record it: the next such product of emfa_matvec leaves NaN, and the next
+ * emfa_ctx_synchronize or emfa_matvec after it has run returns
+ * EMFA_ERR_TIMEOUT, once. */
+emfa_status_t emfa_diag_product_timeout(emfa_ctx_t* ctx);
 
 /* ---- binary dumps ------------------------------------------------------------ */
 /* Versioned binary dump of a matrix or vector (Z, V, I, operator arrays):
