@@ -3231,13 +3231,24 @@ emfa_status_t emfa_residual(emfa_ctx_t* ctx, int prec, int matvec, const void* Z
     }
     EMFA_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    EMFA_TRY(slice_report(ctx));  // of an earlier product
+    if (prec == EMFA_F64) {
+        // a single product: its planes are emfa_matvec's, not a solve's
+        const size_t vec = (size_t)n * n_rhs;
+        bool done = false;
+        if (matvec != EMFA_MV_F64) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, R_dev, st, &done));
+        if (!done) EMFA_TRY(cgemm_f64(ctx, Z_dev, n, X_dev, n, n_rhs, R_dev, st));
+        k_residual<double2><<<grid1(vec), 256, 0, st>>>((const double2*)B_dev, (const double2*)R_dev, (double2*)R_dev, vec);
+        ctx->kernel_launches += 1;
+        EMFA_CUDA(ctx, cudaGetLastError());
+        EMFA_CUDA(ctx, cudaStreamSynchronize(st));
+        return done ? slice_report(ctx) : EMFA_OK;
+    }
     DenseOp A;
     A.n = n;
     A.prec = prec;
     A.Z = Z_dev;
     A.mode = dense_mode(prec, matvec, Z_dev, n);
-    // one product: planes of their own do not pay unless the block is wide
-    A.plain = matvec == EMFA_MV_F64 || !slice_worthwhile(ctx, n, n_rhs, false, st);
     EMFA_TRY(A.prepare(ctx, n_rhs, st));
     DevBuf xt;
     if (A.mode != DenseOp::F16X) EMFA_TRY(xt.alloc(ctx, sizeof(float2) * (size_t)n * n_rhs));
