@@ -270,24 +270,24 @@ __device__ __forceinline__ void cp_async8_zfill(void* smem, const void* gmem, bo
                  : "memory");
 }
 
-// MASKED: only the results that mask (RHS-major bytes) marks are stored, and a
-// tile without any does nothing; *again 0: there are none at all
+// MASKED: Z has `rows` rows; only the results that mask ([nrhs][rows] bytes) marks
+// are stored, and a tile without any does nothing; *again 0: there are none at all
 template <int FT, int RT, bool MASKED>
 __global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const float2* __restrict__ Z, size_t ldz,
                                                       const float2* __restrict__ X, int n, int nrhs, int kper,
-                                                      float2* __restrict__ Y, const unsigned char* __restrict__ mask,
+                                                      float2* __restrict__ Y, int rows, const unsigned char* __restrict__ mask,
                                                       const int* __restrict__ again)
 {
     constexpr int BM = 16 * FT, BN = 8 * RT, STAGE = (BM + BN) * CT_LD;
     extern __shared__ float2 s_ct[];  // [stage][BM + BN][CT_LD], then the partial sums [BN][BM]
     const int tid = threadIdx.x, tf = tid & 15, tr = tid >> 4;
-    const int f0 = blockIdx.y * BM, r0 = blockIdx.z * BN;
+    const int f0 = blockIdx.y * BM, r0 = blockIdx.z * BN, m = MASKED ? rows : n;
     if constexpr (MASKED) {  // the same answer in every CTA of the cluster
         if (*again == 0) return;
         bool any = false;
         for (int q = tid; q < BM * BN; q += CT_THREADS) {
             const int f = f0 + q % BM, r = r0 + q / BM;
-            any |= f < n && r < nrhs && mask[(size_t)r * n + f];
+            any |= f < m && r < nrhs && mask[(size_t)r * m + f];
         }
         if (!__syncthreads_or(any)) return;
     }
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const flo
 #pragma unroll
         for (int i = 0; i < BM / 8; ++i) {
             const int f = tr + 8 * i;
-            const bool in = k < k1 && f0 + f < n;
+            const bool in = k < k1 && f0 + f < m;
             cp_async8_zfill(st + f * CT_LD + tf, Z + (in ? (size_t)(f0 + f) * ldz + k : 0), in);
         }
 #pragma unroll
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const flo
 #pragma unroll
             for (int i = 0; i < FT; ++i) {
                 const int f = f0 + tf + 16 * i, r = r0 + tr + 8 * j;
-                if (f < n && r < nrhs && (!MASKED || mask[(size_t)r * n + f])) Y[(size_t)r * n + f] = acc[i][j];
+                if (f < m && r < nrhs && (!MASKED || mask[(size_t)r * m + f])) Y[(size_t)r * n + f] = acc[i][j];
             }
         return;
     }
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const flo
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_ct);
     for (int q = rank * CT_THREADS + tid; q < BM * BN; q += csize * CT_THREADS) {
         const int f = f0 + q % BM, r = r0 + q / BM;
-        if (f >= n || r >= nrhs || (MASKED && !mask[(size_t)r * n + f])) continue;
+        if (f >= m || r >= nrhs || (MASKED && !mask[(size_t)r * m + f])) continue;
         float2 v[CT_SPLITS], t = make_float2(0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < CT_SPLITS; ++c)
@@ -409,13 +409,13 @@ __global__ void __launch_bounds__(CT_THREADS, ct_resident(RT)) k_ctile(const flo
 
 template <int FT, int RT, bool MASKED = false>
 static emfa_status_t launch_ctile(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
-                                  cudaStream_t st, const unsigned char* mask = nullptr, const int* again = nullptr)
+                                  cudaStream_t st, int rows = 0, const unsigned char* mask = nullptr, const int* again = nullptr)
 {
     constexpr int BM = 16 * FT, BN = 8 * RT;
     constexpr size_t stages = sizeof(float2) * CT_STAGES * (BM + BN) * CT_LD, sums = sizeof(float2) * BM * BN;
     constexpr size_t smem = stages > sums ? stages : sums;
     EMFA_TRY(ensure_smem(c, k_ctile<FT, RT, MASKED>, smem));
-    const int ft = (n + BM - 1) / BM, rt = (nrhs + BN - 1) / BN;
+    const int ft = ((MASKED ? rows : n) + BM - 1) / BM, rt = (nrhs + BN - 1) / BN;
     const int sms = c->sm_count > 0 ? c->sm_count : 148;
     // parts of k: the fewest steps of the busiest SM, whose CTAs share its
     // FMAs (below two and a half a SM they wait for their loads instead),
@@ -445,7 +445,7 @@ static emfa_status_t launch_ctile(Ctx* c, const void* Z, size_t ldz, const void*
     cfg.attrs = at;
     cfg.numAttrs = 1;
     EMFA_CUDA(c, cudaLaunchKernelEx(&cfg, k_ctile<FT, RT, MASKED>, (const float2*)Z, ldz, (const float2*)X, n, nrhs, kper,
-                                    (float2*)Y, mask, again));
+                                    (float2*)Y, rows, mask, again));
     c->kernel_launches += 1;
     return EMFA_OK;
 }
@@ -469,10 +469,10 @@ static emfa_status_t cgemm_f32_tiles(Ctx* c, const void* Z, size_t ldz, const vo
     }
 }
 
-emfa_status_t cgemm_f32_masked(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+emfa_status_t cgemm_f32_masked(Ctx* c, const void* Z, size_t ldz, int rows, const void* X, int n, int nrhs, void* Y,
                                const unsigned char* mask, const int* again, cudaStream_t st)
 {
-    return launch_ctile<4, 10, true>(c, Z, ldz, X, n, nrhs, Y, st, mask, again);
+    return launch_ctile<4, 10, true>(c, Z, ldz, X, n, nrhs, Y, st, rows, mask, again);
 }
 
 // One FP32 product, the kernel chosen (us, GEMV | tiles): the GEMV up to 4

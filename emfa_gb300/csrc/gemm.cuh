@@ -10,8 +10,9 @@ namespace emfa {
 // to 16 right-hand sides, 64 x 64 tiles above
 emfa_status_t cgemm_f32_block(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
                               cudaStream_t st);
-// the results that `mask` (RHS-major bytes) marks, by the clustered tiles; none where *again is 0
-emfa_status_t cgemm_f32_masked(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
+// the results of `rows` rows of Z that `mask` (bytes, [nrhs][rows]) marks, by the
+// clustered tiles, into Y (n apart a right-hand side); none where *again is 0
+emfa_status_t cgemm_f32_masked(Ctx* c, const void* Z, size_t ldz, int rows, const void* X, int n, int nrhs, void* Y,
                                const unsigned char* mask, const int* again, cudaStream_t st);
 emfa_status_t cgemm_f32(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st);
 emfa_status_t cgemm_f64(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y, cudaStream_t st);
@@ -96,11 +97,11 @@ __device__ __forceinline__ int hpack_exponent_f(float wmax, float scale)
 emfa_status_t hgemm_residual(Ctx* c, const HPlanes& h, const double2* X, const void* B, bool b_is_f32, double2* R,
                              int nrhs, cudaStream_t st);
 emfa_status_t hgemm_check_error(Ctx* c, cudaStream_t st);
-// The product of two planes of FP16 rows in the inner product's layout (A: n rows
-// of 2n halves, B: 2 nrhs rows, ld halves apart): Y (float2, RHS-major) times
-// unit[0] unit[r]; err: the caller's error word of the bounded waits
-emfa_status_t hgemm_planes(Ctx* c, const __half* A, const __half* B, int n, int nrhs, size_t ld, const float* unit,
-                           float2* Y, int* err, cudaStream_t st);
+// The product of two planes of FP16 rows in the inner product's layout (A: `rows`
+// rows of 2n halves, B: 2 nrhs rows, ld halves apart): Y (float2, [nrhs][rows])
+// times unit[0] unit[r]; err: the caller's error word of the bounded waits
+emfa_status_t hgemm_planes(Ctx* c, const __half* A, const __half* B, int rows, int n, int nrhs, size_t ld,
+                           const float* unit, float2* Y, int* err, cudaStream_t st);
 // the inner product's tile shapes (BN x MS) and the autotuner's record of a
 // shape bucket: variant -1 if untuned; ms[v] the best of two timed launches
 // of shape v, -1 where v was not a candidate

@@ -652,25 +652,25 @@ static emfa_status_t make_map_h(Ctx* c, CUtensorMap* m, const void* ptr, uint64_
 // timed: bracket the launch with the context's kernel timer (launches that
 // may skip are not timed: their work is not known on the host)
 template <int BN, int MS>
-static emfa_status_t launch_h(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, float2* Y, int n, int nrhs,
+static emfa_status_t launch_h(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, float2* Y, int rows, int n, int nrhs,
                               const float* inv_s, const float* inv_t, int* err, cudaStream_t st, bool timed,
                               const int* skip, int* seen)
 {
     using S = th::Smem<BN, MS>;
     EMFA_TRY(ensure_smem(c, th::k_hgemm<BN, MS>, S::TOTAL));
-    dim3 grd((2 * nrhs + BN - 1) / BN, (n + th::BM * MS - 1) / (th::BM * MS));
+    dim3 grd((2 * nrhs + BN - 1) / BN, (rows + th::BM * MS - 1) / (th::BM * MS));
     const int kblocks = (2 * n + th::BKH - 1) / th::BKH;
     if (timed && !skip) {
         TimedLaunch tl(c, KT_GEMM, st, 8.0 * n * (double)n * nrhs);
-        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, n, nrhs, kblocks, inv_s, inv_t, err,
+        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, rows, nrhs, kblocks, inv_s, inv_t, err,
                                                                   nullptr, nullptr);
     } else if (skip) {
         // the Krylov loop's product: scheduled while the step that packed its
         // operand drains (programmatic dependent launch)
-        EMFA_CUDA(c, launch_dependent(th::k_hgemm<BN, MS>, grd, dim3(th::THREADS), (size_t)S::TOTAL, st, ta, tb, Y, n,
+        EMFA_CUDA(c, launch_dependent(th::k_hgemm<BN, MS>, grd, dim3(th::THREADS), (size_t)S::TOTAL, st, ta, tb, Y, rows,
                                       nrhs, kblocks, inv_s, inv_t, err, skip, seen));
     } else {
-        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, n, nrhs, kblocks, inv_s, inv_t, err, skip,
+        th::k_hgemm<BN, MS><<<grd, th::THREADS, S::TOTAL, st>>>(ta, tb, Y, rows, nrhs, kblocks, inv_s, inv_t, err, skip,
                                                                   nullptr);
     }
     c->kernel_launches += 1;
@@ -757,19 +757,19 @@ static int fixed_variant(int n, int nrhs, int sms)
     return (long)col_tiles * ((n + 255) / 256) >= (long)sms * 9 / 10 ? HV_144_2 : HV_144_1;
 }
 
-static emfa_status_t launch_variant(Ctx* c, int v, const CUtensorMap& ta, const CUtensorMap* tb, float2* Y, int n,
-                                    int nrhs, const float* inv_s, const float* inv_t, int* err, cudaStream_t st,
+static emfa_status_t launch_variant(Ctx* c, int v, const CUtensorMap& ta, const CUtensorMap* tb, float2* Y, int rows,
+                                    int n, int nrhs, const float* inv_s, const float* inv_t, int* err, cudaStream_t st,
                                     bool timed, const int* skip = nullptr, int* seen = nullptr)
 {
     switch (v) {
     case HV_64_1:
-        if (2 * nrhs <= 16) return launch_h<16, 1>(c, ta, tb[2], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
-        return launch_h<64, 1>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        if (2 * nrhs <= 16) return launch_h<16, 1>(c, ta, tb[2], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        return launch_h<64, 1>(c, ta, tb[0], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     case HV_64_2:
-        if (2 * nrhs <= 16) return launch_h<16, 2>(c, ta, tb[2], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
-        return launch_h<64, 2>(c, ta, tb[0], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
-    case HV_144_1: return launch_h<144, 1>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
-    default: return launch_h<144, 2>(c, ta, tb[1], Y, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        if (2 * nrhs <= 16) return launch_h<16, 2>(c, ta, tb[2], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+        return launch_h<64, 2>(c, ta, tb[0], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    case HV_144_1: return launch_h<144, 1>(c, ta, tb[1], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
+    default: return launch_h<144, 2>(c, ta, tb[1], Y, rows, n, nrhs, inv_s, inv_t, err, st, timed, skip, seen);
     }
 }
 
@@ -794,7 +794,7 @@ static emfa_status_t tune_variants(Ctx* c, const TuneKey& key, const CUtensorMap
         float best = 1e30f;
         for (int rep = 0; rep < 2 && st_ == EMFA_OK; ++rep) {
             cudaEventRecord(ev[0], st);
-            st_ = launch_variant(c, cand[i], ta, tb, Y, n, nrhs, inv_s, inv_t, err, st, false);
+            st_ = launch_variant(c, cand[i], ta, tb, Y, n, n, nrhs, inv_s, inv_t, err, st, false);
             cudaEventRecord(ev[1], st);
             if (st_ != EMFA_OK) break;
             if (cudaEventSynchronize(ev[1]) != cudaSuccess) {
@@ -845,22 +845,22 @@ static emfa_status_t hgemm_run(Ctx* c, const HPlanes& h, const __half* bh, const
         if (known < 0 && !skip) return tune_variants(c, key, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st);
         if (known >= 0) v = known;
     }
-    return launch_variant(c, v, ta, tb, (float2*)Y, n, nrhs, h.inv_s, inv_t, err, st, true, skip, seen);
+    return launch_variant(c, v, ta, tb, (float2*)Y, n, n, nrhs, h.inv_s, inv_t, err, st, true, skip, seen);
 }
 
-emfa_status_t hgemm_planes(Ctx* c, const __half* A, const __half* B, int n, int nrhs, size_t ld, const float* unit,
-                           float2* Y, int* err, cudaStream_t st)
+emfa_status_t hgemm_planes(Ctx* c, const __half* A, const __half* B, int rows, int n, int nrhs, size_t ld,
+                           const float* unit, float2* Y, int* err, cudaStream_t st)
 {
     CUtensorMap ta, tb[3];
     const int sms = c->sm_count > 0 ? c->sm_count : 148;
-    EMFA_TRY(make_map_h(c, &ta, A, 2 * (uint64_t)n, (uint64_t)n, ld, th::BM));
+    EMFA_TRY(make_map_h(c, &ta, A, 2 * (uint64_t)n, (uint64_t)rows, ld, th::BM));
     EMFA_TRY(make_map_h(c, &tb[0], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 64));
     if (2 * nrhs <= 16) EMFA_TRY(make_map_h(c, &tb[2], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 16));
     if (2 * nrhs > 64) EMFA_TRY(make_map_h(c, &tb[1], B, 2 * (uint64_t)n, 2 * (uint64_t)nrhs, ld, 144));
     // 64 columns a tile while they leave SMs idle: a CTA is bound by its operands' arrival
-    const bool narrow = (long)((2 * nrhs + 63) / 64) * ((n + 127) / 128) <= sms;
-    return launch_variant(c, narrow ? HV_64_1 : fixed_variant(n, nrhs, sms), ta, tb, Y, n, nrhs, unit, unit, err, st,
-                          false);
+    const bool narrow = (long)((2 * nrhs + 63) / 64) * ((rows + 127) / 128) <= sms;
+    return launch_variant(c, narrow ? HV_64_1 : fixed_variant(rows, nrhs, sms), ta, tb, Y, rows, n, nrhs, unit, unit, err,
+                          st, false);
 }
 
 emfa_status_t hgemm_tuned_shape(int device, int n, int nrhs, int* variant, float* ms)

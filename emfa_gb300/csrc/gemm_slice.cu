@@ -561,13 +561,13 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int ex)
 }
 
 // report (optional): a page-locked host word that gets *err.
-// Y from the partial sums of all splits where the digits are as good as a sum in
+// Y (rows n apart a right-hand side) from the partial sums of all splits where the digits are as good as a sum in
 // T (S at least FLOOR, or zero: no product at all); a pipeline that gave up (err)
 // leaves NaN.  The rest is summed in T: FP64 by the CTA, one result after the
 // other, a term a thread (a few results cost a few us, all of them about the
 // GEMV's time); FP32 results are marked in `mask` for gemm.cu's tiles.
 template <typename T>
-__global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ part, int splits, int n, int nrhs,
+__global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ part, int splits, int rows, int n, int nrhs,
                                                  const int* __restrict__ exz, const int* __restrict__ exx,
                                                  const float2* __restrict__ S, const Cx<T>* __restrict__ Z, size_t ldz,
                                                  const Cx<T>* __restrict__ X, const int* __restrict__ err,
@@ -576,20 +576,20 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
 {
     if (report && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *err) *(volatile int*)report = *err;
     const int f = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-    const bool live = f < n;
+    const bool live = f < rows;
     bool sum = false;
     Cx<T> y = cx(T(0), T(0));
     if (live) {
         const int ez = exz[f], ex = exx[r];
-        const float2 s = S[(size_t)r * n + f];
+        const float2 s = S[(size_t)r * rows + f];
         if (*err) {
             y.re = y.im = (T)__longlong_as_double(0x7ff8000000000000ll);
         } else if (ez == SLICE_NONFINITE || ex == SLICE_NONFINITE || (s.x > 0.f && s.x < Cut<T>::FLOOR) ||
                    (s.y > 0.f && s.y < Cut<T>::FLOOR)) {
             sum = true;
         } else {
-            const size_t plane = (size_t)2 * nrhs * n;
-            const long long* p0 = part + (size_t)(2 * r) * n + f;
+            const size_t plane = (size_t)2 * nrhs * rows;
+            const long long* p0 = part + (size_t)(2 * r) * rows + f;
             // z = V 2^(e - BITS), e = field - EXP_ONE; the lowest kept level, NS - 1, weighs 2^(8 (NS - 1)) in V V
             const int e = ez + ex - 2 * (Cut<T>::EXP_ONE + Cut<T>::BITS) + 8 * (Cut<T>::NS - 1);
             long long s0 = 0, s1 = 0;  // levels 0-3
@@ -597,15 +597,15 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
                 long long l0 = 0, l1 = 0;
                 for (int q = 0; q < splits; ++q, p0 += 2 * plane) {
                     s0 += p0[0];
-                    s1 += p0[n];
+                    s1 += p0[rows];
                     l0 += p0[plane];
-                    l1 += p0[plane + n];
+                    l1 += p0[plane + rows];
                 }
                 y = cx((T)to_double(s0, l0, e), (T)to_double(s1, l1, e));
             } else {
                 for (int q = 0; q < splits; ++q, p0 += plane) {
                     s0 += p0[0];
-                    s1 += p0[n];
+                    s1 += p0[rows];
                 }
                 y = cx((T)to_double(s0 >> 32, s0 & 0xffffffffll, e), (T)to_double(s1 >> 32, s1 & 0xffffffffll, e));
             }
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
         }
         if (live) Y[(size_t)r * n + f] = y;
     } else if (live) {
-        mask[(size_t)r * n + f] = sum;
+        mask[(size_t)r * rows + f] = sum;
         if (sum)
             *again = 1;
         else
@@ -668,9 +668,20 @@ __global__ void __launch_bounds__(256) k_combine(const long long* __restrict__ p
 static size_t slice_ld(int n) { return ((size_t)2 * n + 7) & ~(size_t)7; }  // 16-byte rows
 
 // ns digits and the magnitudes
-static size_t slice_plane_bytes(int ns, int n)
+static size_t slice_plane_bytes(int ns, int n, int rows)
 {
-    return Carver::round(sizeof(__half) * (ns + 1) * (size_t)n * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)n);
+    return Carver::round(sizeof(__half) * (ns + 1) * (size_t)rows * slice_ld(n)) + Carver::round(sizeof(int) * (size_t)rows);
+}
+
+// A context keeps at most this much of planes between calls: a single product
+// splits Z by blocks of rows that fit (the digits of the right-hand sides, formed
+// anew for each block, are about 1 % of a block's time at n = 6000 x 181), and a
+// solve, whose products all read the planes, gives larger ones back at its end.
+constexpr size_t PLANES_KEPT = (size_t)1 << 30;
+static int rows_kept(int ns, int n)
+{
+    const size_t row = sizeof(__half) * (ns + 1) * slice_ld(n);
+    return (int)std::min<size_t>((size_t)n, std::max<size_t>(PLANES_KEPT / row / sl::BM, 1) * sl::BM);
 }
 
 static emfa_status_t slice_map(Ctx* c, CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t rows, size_t ld,
@@ -736,7 +747,7 @@ emfa_status_t slice_report(Ctx* c)
 // planes above 16 GB keep the CUDA-core product, which needs no memory.
 static bool slice_allowed(Ctx* c, int ns, int n, cudaStream_t st)
 {
-    if (n < 128 || c->budget || c->stream_ordered || st != c->stream || slice_plane_bytes(ns, n) > ((size_t)16 << 30))
+    if (n < 128 || c->budget || c->stream_ordered || st != c->stream || slice_plane_bytes(ns - 1, n, n) > ((size_t)16 << 30))
         return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
@@ -765,19 +776,20 @@ static bool slice_worthwhile_f32(Ctx* c, int n, int nrhs, cudaStream_t st)
 }
 
 template <typename T>
-static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int n, SlicePlanes* out, cudaStream_t st)
+static emfa_status_t prepare_t(Ctx* c, int slot, const void* Z, size_t ldz, int n, int rows, SlicePlanes* out,
+                               cudaStream_t st)
 {
     constexpr int NS = sl::Cut<T>::NS;
     const size_t ldk = slice_ld(n);
     void* wp = nullptr;
-    EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(NS, n) + 512, &wp));
+    EMFA_TRY(ctx_workspace(c, slot, slice_plane_bytes(NS, n, rows) + 512, &wp));
     Carver cv{(char*)wp};
-    __half* d = cv.take<__half>((NS + 1) * (size_t)n * ldk);
-    int* ex = cv.take<int>(n);
-    sl::k_slice_rows<T><<<n, 256, 0, st>>>((const Cx<T>*)Z, ldz, n, ldk, d, ex);
+    __half* d = cv.take<__half>((NS + 1) * (size_t)rows * ldk);
+    int* ex = cv.take<int>(rows);
+    sl::k_slice_rows<T><<<rows, 256, 0, st>>>((const Cx<T>*)Z, ldz, n, ldk, d, ex);
     c->kernel_launches += 1;
     EMFA_CUDA(c, cudaGetLastError());
-    *out = SlicePlanes{d, ex, Z, ldz, n, ldk};
+    *out = SlicePlanes{d, ex, Z, ldz, n, rows, ldk};
     return EMFA_OK;
 }
 
@@ -786,7 +798,7 @@ emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, 
     int* err = nullptr;
     EMFA_TRY(slice_err(c, 8, &err));
     EMFA_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), st));
-    return prepare_t<double>(c, slot, Z, ldz, n, out, st);
+    return prepare_t<double>(c, slot, Z, ldz, n, n, out, st);
 }
 
 // Column tile (narrow for few right-hand sides; the wide one fills tensor
@@ -799,12 +811,12 @@ template <> struct Tile<double> { static constexpr int NARROW = 16, WIDE = 64; }
 template <> struct Tile<float> { static constexpr int NARROW = 32, WIDE = 128; };
 
 template <typename T>
-static void slice_shape(Ctx* c, int n, int nrhs, int* bn, int* splits, int* per_split)
+static void slice_shape(Ctx* c, int n, int rows, int nrhs, int* bn, int* splits, int* per_split)
 {
     const int sms = c->sm_count > 0 ? c->sm_count : 148;
     *bn = 2 * nrhs <= Tile<T>::NARROW ? Tile<T>::NARROW : Tile<T>::WIDE;
     const int blocks = (2 * n + sl::BK - 1) / sl::BK, groups = (blocks + sl::GROUP - 1) / sl::GROUP;
-    const long tiles = (long)((n + sl::BM - 1) / sl::BM) * ((2 * nrhs + *bn - 1) / *bn);
+    const long tiles = (long)((rows + sl::BM - 1) / sl::BM) * ((2 * nrhs + *bn - 1) / *bn);
     long best = -1;
     for (int s = 1; s <= std::min(groups, 16); ++s) {
         const int g = (groups + s - 1) / s, used = (groups + g - 1) / g;
@@ -819,13 +831,13 @@ static void slice_shape(Ctx* c, int n, int nrhs, int* bn, int* splits, int* per_
 }
 
 template <int NS, int BN>
-static emfa_status_t launch_slice(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int n, int nrhs, int splits,
+static emfa_status_t launch_slice(Ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int n, int rows, int nrhs, int splits,
                                   int per_split, long long* part, int* err, cudaStream_t st)
 {
     using S = sl::Smem<NS, BN>;
     EMFA_TRY(ensure_smem(c, sl::k_slice<NS, BN>, S::TOTAL));
-    const dim3 grd((2 * nrhs + BN - 1) / BN, (n + sl::BM - 1) / sl::BM, splits);
-    sl::k_slice<NS, BN><<<grd, sl::THREADS, S::TOTAL, st>>>(ta, tb, n, 2 * nrhs, (2 * n + sl::BK - 1) / sl::BK,
+    const dim3 grd((2 * nrhs + BN - 1) / BN, (rows + sl::BM - 1) / sl::BM, splits);
+    sl::k_slice<NS, BN><<<grd, sl::THREADS, S::TOTAL, st>>>(ta, tb, rows, 2 * nrhs, (2 * n + sl::BK - 1) / sl::BK,
                                                             per_split, make_int4(1, 1 << 8, 1 << 16, 1 << 24), part,
                                                             err);
     c->kernel_launches += 1;
@@ -838,55 +850,57 @@ static emfa_status_t apply_t(Ctx* c, int slot, const SlicePlanes& p, const void*
                              int* report, cudaStream_t st)
 {
     constexpr int NS = sl::Cut<T>::NS, SETS = NS / 4, NARROW = Tile<T>::NARROW, WIDE = Tile<T>::WIDE;
-    const int n = p.n;
-    // blocks of right-hand sides bound the scratch (digits and partial sums)
-    constexpr int RB = 512;
+    const int n = p.n, rows = p.rows;
+    // blocks of right-hand sides bound the scratch: 512, fewer above n = 7000
+    // (256 MB of digits)
+    const int RB = (int)std::min<size_t>(512, std::max<size_t>(1, ((size_t)256 << 20) / (sizeof(__half) * (NS + 1) * 2 * 64 * p.ldk)) * 64);
     const int rmax = std::min(nrhs, RB);
     int bn, splits, per_split;
-    slice_shape<T>(c, n, rmax, &bn, &splits, &per_split);
+    slice_shape<T>(c, n, rows, rmax, &bn, &splits, &per_split);
     const size_t brow = (size_t)2 * rmax * p.ldk;
     int smax = splits;
     if (nrhs % RB) {
         int b2, s2, p2;
-        slice_shape<T>(c, n, nrhs % RB, &b2, &s2, &p2);
+        slice_shape<T>(c, n, rows, nrhs % RB, &b2, &s2, &p2);
         // scratch of the last block: fewer columns, perhaps more splits
         smax = std::max(splits, (int)(((long)s2 * (nrhs % RB) + rmax - 1) / rmax));
     }
-    const size_t parts = (size_t)smax * 2 * SETS * rmax * n;
+    const size_t res = (size_t)rmax * rows, parts = (size_t)smax * 2 * SETS * res;
     void* wp = nullptr;
     EMFA_TRY(ctx_workspace(c, slot,
                            Carver::round(sizeof(__half) * (NS + 1) * brow) + 2 * Carver::round(sizeof(int) * (size_t)rmax) +
-                               Carver::round(sizeof(long long) * parts) +
-                               Carver::round(sizeof(float2) * (size_t)rmax * n) + Carver::round((size_t)rmax * n) + 2048,
+                               Carver::round(sizeof(long long) * parts) + Carver::round(sizeof(float2) * res) +
+                               Carver::round(res) + 2048,
                            &wp));
     Carver cv{(char*)wp};
     __half* b = cv.take<__half>((NS + 1) * brow);
     int* ex = cv.take<int>(rmax);
     float* unit = cv.take<float>(rmax);
     long long* part = cv.take<long long>(parts);
-    float2* sums = cv.take<float2>((size_t)rmax * n);
-    unsigned char* mask = cv.take<unsigned char>((size_t)rmax * n);
+    float2* sums = cv.take<float2>(res);
+    unsigned char* mask = cv.take<unsigned char>(res);
     int* again = cv.take<int>(1);
     CUtensorMap ta, tb;
-    EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)n, p.ldk, NS, sl::BM, 1));
+    EMFA_TRY(slice_map(c, &ta, p.d, 2 * (uint64_t)n, (uint64_t)rows, p.ldk, NS, sl::BM, 1));
     for (int r0 = 0; r0 < nrhs; r0 += RB) {
         const int nr = std::min(RB, nrhs - r0);
         const Cx<T>* x = (const Cx<T>*)X + (size_t)r0 * n;
-        slice_shape<T>(c, n, nr, &bn, &splits, &per_split);
+        slice_shape<T>(c, n, rows, nr, &bn, &splits, &per_split);
         EMFA_TRY(slice_map(c, &tb, b, 2 * (uint64_t)n, 2 * (uint64_t)nr, p.ldk, NS, (uint32_t)bn, NS));
         Cx<T>* y = (Cx<T>*)Y + (size_t)r0 * n;
         sl::k_slice_rhs<T><<<nr, 256, 0, st>>>(x, n, nr, p.ldk, b, ex, unit, again);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
-        EMFA_TRY((bn == NARROW ? launch_slice<NS, NARROW> : launch_slice<NS, WIDE>)(c, ta, tb, n, nr, splits, per_split,
-                                                                                  part, err, st));
-        EMFA_TRY(hgemm_planes(c, p.d + NS * (size_t)n * p.ldk, b + NS * (size_t)2 * nr * p.ldk, n, nr, p.ldk, unit, sums,
-                              err, st));
-        sl::k_combine<T><<<dim3((n + 255) / 256, nr), 256, 0, st>>>(part, splits, n, nr, p.ex, ex, sums, (const Cx<T>*)p.Z,
-                                                                    p.ldz, x, err, y, mask, again, report);
+        EMFA_TRY((bn == NARROW ? launch_slice<NS, NARROW> : launch_slice<NS, WIDE>)(c, ta, tb, n, rows, nr, splits,
+                                                                                  per_split, part, err, st));
+        EMFA_TRY(hgemm_planes(c, p.d + NS * (size_t)rows * p.ldk, b + NS * (size_t)2 * nr * p.ldk, rows, n, nr, p.ldk, unit,
+                              sums, err, st));
+        sl::k_combine<T><<<dim3((rows + 255) / 256, nr), 256, 0, st>>>(part, splits, rows, n, nr, p.ex, ex, sums,
+                                                                       (const Cx<T>*)p.Z, p.ldz, x, err, y, mask, again,
+                                                                       report);
         c->kernel_launches += 1;
         EMFA_CUDA(c, cudaGetLastError());
-        if (NS == 4) EMFA_TRY(cgemm_f32_masked(c, p.Z, p.ldz, x, n, nr, y, mask, again, st));
+        if (NS == 4) EMFA_TRY(cgemm_f32_masked(c, p.Z, p.ldz, rows, x, n, nr, y, mask, again, st));
     }
     return EMFA_OK;
 }
@@ -908,6 +922,12 @@ emfa_status_t slice_check(Ctx* c, cudaStream_t st)
     return h ? timed_out(c, h) : EMFA_OK;
 }
 
+void slice_release(Ctx* c)
+{
+    for (int slot : {WS_SLICE_Z, WS_SLICE_B})
+        if (c->ws[slot].bytes > PLANES_KEPT) c->ws[slot].release();
+}
+
 template <typename T>
 static emfa_status_t matvec_t(Ctx* c, const void* Z, size_t ldz, const void* X, int n, int nrhs, void* Y,
                               cudaStream_t st, bool* done)
@@ -917,9 +937,14 @@ static emfa_status_t matvec_t(Ctx* c, const void* Z, size_t ldz, const void* X, 
     std::lock_guard<std::mutex> lk(c->slice_mu);
     int* err = nullptr;
     EMFA_TRY(slice_word(c, &err, st));
-    SlicePlanes p;
-    emfa_status_t s = prepare_t<T>(c, WS_SLICE_MV, Z, ldz, n, &p, st);
-    if (s == EMFA_OK) s = apply_t<T>(c, WS_SLICE_MV_B, p, X, nrhs, Y, err, c->pinned + Ctx::PINNED - 1, st);
+    const int step = rows_kept(sl::Cut<T>::NS, n);
+    emfa_status_t s = EMFA_OK;
+    for (int f0 = 0; f0 < n && s == EMFA_OK; f0 += step) {
+        SlicePlanes p;
+        s = prepare_t<T>(c, WS_SLICE_MV, (const Cx<T>*)Z + (size_t)f0 * ldz, ldz, n, std::min(step, n - f0), &p, st);
+        if (s == EMFA_OK)
+            s = apply_t<T>(c, WS_SLICE_MV_B, p, X, nrhs, (Cx<T>*)Y + f0, err, c->pinned + Ctx::PINNED - 1, st);
+    }
     if (s == EMFA_ERR_OOM) {
         cudaGetLastError();  // no room: the caller's CUDA-core product
         return EMFA_OK;

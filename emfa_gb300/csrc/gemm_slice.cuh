@@ -4,15 +4,15 @@
 
 namespace emfa {
 
-// Z (n x n) as planes of signed 8-bit digits held in FP16 (eight for complex128,
-// four for complex64), each n x 2n (re, im interleaved), rows ldk halves apart,
-// and a power-of-two scale per row.
+// `rows` rows of Z (n columns) as planes of signed 8-bit digits held in FP16
+// (eight for complex128, four for complex64) and one of magnitudes, each rows x
+// 2n (re, im interleaved), rows ldk halves apart, and a power-of-two scale per row.
 struct SlicePlanes {
-    const __half* d = nullptr;   // [planes][n][ldk]
-    const int* ex = nullptr;     // [n] row scales; SLICE_NONFINITE for a row with an infinity or NaN
-    const void* Z = nullptr;     // the matrix itself
+    const __half* d = nullptr;   // [planes][rows][ldk]
+    const int* ex = nullptr;     // [rows] scales; SLICE_NONFINITE for a row with an infinity or NaN
+    const void* Z = nullptr;     // the rows themselves
     size_t ldz = 0;
-    int n = 0;
+    int n = 0, rows = 0;
     size_t ldk = 0;
 };
 
@@ -27,6 +27,8 @@ emfa_status_t slice_prepare(Ctx* c, int slot, const void* Z, size_t ldz, int n, 
 // (it reads the word of a solve's products, which slice_prepare zeroes)
 emfa_status_t slice_apply(Ctx* c, int slot, const SlicePlanes& p, const void* X, int nrhs, void* Y, cudaStream_t st);
 emfa_status_t slice_check(Ctx* c, cudaStream_t st);
+// after a solve: gives its planes and scratch back where they are large
+void slice_release(Ctx* c);
 // The error word of single products.  It is not read after a product, which
 // would wait for it: the product tells a page-locked word, and the next call
 // that looks (slice_report: emfa_ctx_synchronize, emfa_matvec, emfa_residual)

@@ -3161,8 +3161,10 @@ emfa_status_t solve_dense(Ctx* c, int prec, const void* Z, int n, const void* B,
     A.mode = dense_mode(prec, sp->matvec, Z, n);
     A.plain = sp->matvec == EMFA_MV_F64;
     EMFA_TRY(A.prepare(c, nrhs, st));
-    if (sp->method == EMFA_LU) return lu_refined(c, A, Z, B, nrhs, (double2*)X, sp, info, st);
-    return solve_op(c, A, B, nrhs, X, sp, info, st);
+    const emfa_status_t s = sp->method == EMFA_LU ? lu_refined(c, A, Z, B, nrhs, (double2*)X, sp, info, st)
+                                                  : solve_op(c, A, B, nrhs, X, sp, info, st);
+    if (A.sp.d) slice_release(c);
+    return s;
 }
 }  // namespace emfa
 
