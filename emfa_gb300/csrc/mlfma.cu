@@ -194,7 +194,8 @@ struct MLevel {
     // stencils: theta (CSR over this level's theta index: parent theta, weight)
     // and phi (CSR over this level's phi index: parent phi, weight)
     DevView th_ptr, th_src, th_w, ph_ptr, ph_src, ph_w;
-    size_t down_smem = 0;               // shared bytes per CTA (theta-pass rows)
+    size_t down_smem = 0;               // shared bytes per CTA (theta-pass rows, and the shifted rows where
+    bool down_staged = true;            //   they fit beside them)
     DevView down_win;                    // int2 per chunk: parent phi rows its phi stencils read
     DevView up_phase;                    // float2 [8][K]: exp(-j k k.(parent - child)) for the level below
     int up_rows = 0;                    // interpolation from the level below: phi rows per CTA,
@@ -596,31 +597,46 @@ __global__ void __launch_bounds__(32 * TRANS_WARPS, 2) k_translate(const __grid_
 // [w2.x, w2.y) and every theta column tc of the child
 //   h[comp][pp - w2.x][tc] = sum over the transposed theta stencil of
 //                            w * conj(phase(pp, t)) * parent(pp, t)
-// into shared memory.  The parent's samples are shifted first (each serves
-// about three columns), into s_q, then summed.
+// into shared memory.  STAGED: the parent's samples are shifted first (each
+// serves about three columns), into s_q, then summed; else each column shifts
+// the samples that it reads, to the same bits, for rows too long for both.
+template <bool STAGED>
 __device__ __forceinline__ void anterp_theta(const float2* __restrict__ src, const float2* __restrict__ ph, int2 w2,
                                              int L, int Lp, const int* __restrict__ th_ptr,
                                              const int* __restrict__ th_src, const float* __restrict__ th_w,
                                              float2* s_q, float2* s_h)
 {
     const int Kp = 2 * Lp * Lp, base = w2.x * Lp, qsz = (w2.y - w2.x) * Lp, hsz = (w2.y - w2.x) * L;
-    for (int i = threadIdx.x; i < qsz; i += blockDim.x) {
-        const float2 p = ph[base + i], c = make_float2(p.x, -p.y);  // exp(+j k k.(parent - child))
-        s_q[i] = cmulf(c, src[base + i]);
-        s_q[qsz + i] = cmulf(c, src[Kp + base + i]);
-        s_q[2 * qsz + i] = cmulf(c, src[2 * Kp + base + i]);
+    if constexpr (STAGED) {
+        for (int i = threadIdx.x; i < qsz; i += blockDim.x) {
+            const float2 p = ph[base + i], c = make_float2(p.x, -p.y);  // exp(+j k k.(parent - child))
+            s_q[i] = cmulf(c, src[base + i]);
+            s_q[qsz + i] = cmulf(c, src[Kp + base + i]);
+            s_q[2 * qsz + i] = cmulf(c, src[2 * Kp + base + i]);
+        }
+        __syncthreads();
     }
-    __syncthreads();
     for (int i = threadIdx.x; i < hsz; i += blockDim.x) {
         const int r = i / L, tc = i - r * L;
-        const float2* q = s_q + r * Lp;
         float2 sx = make_float2(0, 0), sy = sx, sz = sx;
-        for (int a = th_ptr[tc]; a < th_ptr[tc + 1]; ++a) {
-            const int t = th_src[a];
-            const float w = th_w[a];
-            sx = caddf(sx, cscalef(q[t], w));
-            sy = caddf(sy, cscalef(q[qsz + t], w));
-            sz = caddf(sz, cscalef(q[2 * qsz + t], w));
+        if constexpr (STAGED) {
+            const float2* q = s_q + r * Lp;
+            for (int a = th_ptr[tc]; a < th_ptr[tc + 1]; ++a) {
+                const int t = th_src[a];
+                const float w = th_w[a];
+                sx = caddf(sx, cscalef(q[t], w));
+                sy = caddf(sy, cscalef(q[qsz + t], w));
+                sz = caddf(sz, cscalef(q[2 * qsz + t], w));
+            }
+        } else {
+            for (int a = th_ptr[tc]; a < th_ptr[tc + 1]; ++a) {
+                const int k = base + r * Lp + th_src[a];
+                const float w = th_w[a];
+                const float2 p = ph[k], c = make_float2(p.x, -p.y);
+                sx = caddf(sx, cscalef(cmulf(c, src[k]), w));
+                sy = caddf(sy, cscalef(cmulf(c, src[Kp + k]), w));
+                sz = caddf(sz, cscalef(cmulf(c, src[2 * Kp + k]), w));
+            }
         }
         s_h[i] = sx;
         s_h[hsz + i] = sy;
@@ -646,6 +662,7 @@ __device__ __forceinline__ void anterp_phi(int pc, int tc, int w0, int L, int hs
 // a level's anterpolation, added to its translated pattern: CTA per (box, chunk
 // of phi rows [pc0, pc0 + R)), i.e. the contiguous samples [pc0 L, (pc0 + R) L)
 // of the box (samples k = pc L + tc, phi-major)
+template <bool STAGED>
 __global__ void k_downward(int L, int R, const float2* __restrict__ pdown, int Lp, const int2* __restrict__ win,
                            const int* __restrict__ parent, const int* __restrict__ oct,
                            const float2* __restrict__ pphase, const int* __restrict__ th_ptr,
@@ -653,7 +670,7 @@ __global__ void k_downward(int L, int R, const float2* __restrict__ pdown, int L
                            const int* __restrict__ ph_ptr, const int* __restrict__ ph_src,
                            const float* __restrict__ ph_w, float2* __restrict__ out, size_t ustride, size_t pstride)
 {
-    extern __shared__ float2 s_h[];  // [3][rows of the window][L], then the shifted rows [3][rows][Lp]
+    extern __shared__ float2 s_h[];  // [3][rows of the window][L], then, STAGED, the shifted rows [3][rows][Lp]
     // right-hand side blockIdx.z: strides in complex64 (this level, parent level)
     out += blockIdx.z * ustride;
     pdown += blockIdx.z * pstride;
@@ -664,7 +681,7 @@ __global__ void k_downward(int L, int R, const float2* __restrict__ pdown, int L
     const int2 w2 = win[blockIdx.y];
     const int hsz = (w2.y - w2.x) * L;
     const int Kp = 2 * Lp * Lp;
-    anterp_theta(pdown + (size_t)3 * parent[b] * Kp, pphase + (size_t)oct[b] * Kp, w2, L, Lp, th_ptr, th_src, th_w,
+    anterp_theta<STAGED>(pdown + (size_t)3 * parent[b] * Kp, pphase + (size_t)oct[b] * Kp, w2, L, Lp, th_ptr, th_src, th_w,
                  s_h + 3 * hsz, s_h);
     for (int i = threadIdx.x; i < ns; i += blockDim.x) {
         const int k = pc0 * L + i;
@@ -742,7 +759,7 @@ __global__ void __launch_bounds__(32 * FINISH_WARPS) k_finish(const __grid_const
     if (A.parts != 1)
         for (int r = 0; r < nr; ++r) {
             if (A.pdown)
-                anterp_theta(A.pdown + (r0 + r) * A.pstride + (size_t)3 * A.parent[b] * qsz, A.pphase + (size_t)A.oct[b] * qsz,
+                anterp_theta<true>(A.pdown + (r0 + r) * A.pstride + (size_t)3 * A.parent[b] * qsz, A.pphase + (size_t)A.oct[b] * qsz,
                              make_int2(0, 2 * Lp), L, Lp, A.th_ptr, A.th_src, A.th_w, s_q, s_h);
             const float2* d = A.down + (r0 + r) * A.dstride + (size_t)3 * b * K;
             for (int k = threadIdx.x; k < K; k += blockDim.x) {
@@ -1531,7 +1548,8 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
     }
     // the interpolation and anterpolation passes may use more than the default 48 KB of shared memory
     EMFA_TRY(ensure_smem(c, k_upward, 96 * 1024));
-    EMFA_TRY(ensure_smem(c, k_downward, 200 * 1024));
+    EMFA_TRY(ensure_smem(c, k_downward<true>, 200 * 1024));
+    EMFA_TRY(ensure_smem(c, k_downward<false>, 200 * 1024));
     EMFA_TRY(ensure_smem(c, k_translate, TRANS_SMEM));
     // finest-level lists and tables
     MLevel& fl = M->lv[nl - 1];
@@ -1763,8 +1781,13 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         tables.put(pm.ip_pl, ploc);
         tables.put(pm.ip_pe, pel);
         {
-            // phi-row chunks of about 256 parent samples and the child rows each reads
-            pm.up_rows = down_rows(pm.L);
+            // phi-row chunks of about 256 parent samples, a thread each (two rows
+            // above 181 samples a row, one above 512), and the child rows each reads
+            if (pm.L > 1024) {
+                set_error(c, "mlfma: more than 1024 multipoles (level too large)");
+                return EMFA_ERR_UNSUPPORTED;
+            }
+            pm.up_rows = pm.L > 512 ? 1 : down_rows(pm.L);
             const int nchunk = (2 * pm.L + pm.up_rows - 1) / pm.up_rows;
             std::vector<int2> win(nchunk);
             int most = 0;
@@ -1849,7 +1872,10 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                 dw[ch] = make_int2(lo, hi);
                 most = std::max(most, hi - lo);
             }
+            // both sets of rows up to an extent of about 180 wavelengths
             cm.down_smem = sizeof(float2) * 3 * (size_t)most * (Lc + Lp);
+            cm.down_staged = cm.down_smem <= 200 * 1024;
+            if (!cm.down_staged) cm.down_smem = sizeof(float2) * 3 * (size_t)most * Lc;
             if (cm.down_smem > 200 * 1024) {
                 set_error(c, "mlfma: anterpolation rows exceed shared memory (level too large)");
                 return EMFA_ERR_UNSUPPORTED;
@@ -1986,6 +2012,7 @@ static emfa_status_t mlfma_apply(emfa_mlfma* M, const float2* x, float2* y, int 
             dptr<int2>(pm.up_win), pm.up_batch, dptr<float2>(pm.up_phase), pm.L, R, dptr<float2>(pm.up),
             (size_t)3 * cm.nbox * cm.K, (size_t)3 * pm.nbox * pm.K);
     }
+    EMFA_CUDA(c, cudaGetLastError());
     TransLevels lv;
     for (int i = 0; i < nl; ++i) {
         MLevel& ml = M->lv[i];
@@ -2000,7 +2027,7 @@ static emfa_status_t mlfma_apply(emfa_mlfma* M, const float2* x, float2* y, int 
         const int R = down_rows(ml.L);
         const int bs = std::min(256, 32 * ((R * ml.L + 31) / 32));
         const dim3 grid((unsigned)ml.nbox, (unsigned)((2 * ml.L + R - 1) / R), (unsigned)nr);
-        k_downward<<<grid, bs, ml.down_smem, st>>>(
+        (ml.down_staged ? k_downward<true> : k_downward<false>)<<<grid, bs, ml.down_smem, st>>>(
             ml.L, R, dptr<float2>(pm.down), pm.L, dptr<int2>(ml.down_win), dptr<int>(ml.parent), dptr<int>(ml.oct),
             dptr<float2>(pm.up_phase), dptr<int>(ml.th_ptr), dptr<int>(ml.th_src), dptr<float>(ml.th_w),
             dptr<int>(ml.ph_ptr), dptr<int>(ml.ph_src), dptr<float>(ml.ph_w), dptr<float2>(ml.down),
