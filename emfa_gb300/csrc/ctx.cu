@@ -44,6 +44,8 @@ emfa_status_t ensure_smem_raw(Ctx* c, const void* func, size_t bytes)
     std::lock_guard<std::mutex> g(mu);
     size_t& cur = limit[std::make_pair(func, dev)];
     if (cur >= bytes) return EMFA_OK;
+    // the call below clears the error of a launch before it: report that first
+    EMFA_CUDA(c, cudaGetLastError());
     EMFA_CUDA(c, cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     cur = bytes;
     return EMFA_OK;
