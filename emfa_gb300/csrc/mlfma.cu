@@ -233,6 +233,7 @@ struct emfa_mlfma {
     size_t nnz = 0;
     emfa::DevView trans_work;       // TransWork per CTA of the translation
     int trans_ctas = 0;
+    bool wide = false;             // a level's pattern elements need more than 32 bits (k_translate)
     int max_cols = 0;              // near columns of a box, most
     emfa::DevBuf tmp_in, tmp_out;  // complex64 scratch for residuals
     // SAI preconditioner P (CSR over box-order rows), built when p.precond
@@ -497,7 +498,7 @@ struct TransLevel {
     const float2* up;
     float2* down;
     const float2* trans;
-    const int4* src;          // per two sources: first element of the pattern, row x 32 of its offset
+    const int4* src;          // per two sources: first element of the pattern (WIDE: first plane), row x 32 of its offset
     const TransGroup* grp;
     int K;
     size_t stride;            // complex64 from one right-hand side to the next
@@ -506,7 +507,9 @@ struct TransLevels {
     TransLevel l[TRANS_LEVELS];
 };
 
-template <int NC>
+// WIDE: a level has patterns of more than 2^32 values, whose elements the 32 bits
+// of a source entry do not count (a few percent slower)
+template <int NC, bool WIDE>
 __device__ __forceinline__ void translate_group(const TransGroup& G, const int4* __restrict__ src,
                                                 const float2* __restrict__ tab, const float2* __restrict__ u, int K,
                                                 int k, bool store, float2* __restrict__ down)
@@ -534,7 +537,10 @@ __device__ __forceinline__ void translate_group(const TransGroup& G, const int4*
         }
         C3f v[TRANS_BATCH];
 #pragma unroll
-        for (int j = 0; j < TRANS_BATCH; ++j) v[j] = C3f{u[at[j]], u1[at[j]], u2[at[j]]};
+        for (int j = 0; j < TRANS_BATCH; ++j) {
+            const size_t o = WIDE ? (size_t)at[j] * (unsigned)K : at[j];
+            v[j] = C3f{u[o], u1[o], u2[o]};
+        }
 #pragma unroll
         for (int j = 0; j < TRANS_BATCH; ++j) {
             const C3f w = v[j];
@@ -561,6 +567,7 @@ __device__ __forceinline__ void translate_group(const TransGroup& G, const int4*
     }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(32 * TRANS_WARPS, 2) k_translate(const __grid_constant__ TransLevels lv,
                                                                    const TransWork* __restrict__ work, int nr)
 {
@@ -585,10 +592,10 @@ __global__ void __launch_bounds__(32 * TRANS_WARPS, 2) k_translate(const __grid_
         const float2* u = L.up + r * L.stride + k;
         float2* down = L.down + r * L.stride;
         switch (G.nc) {
-        case 1: translate_group<1>(G, L.src, tab, u, L.K, k, store, down); break;
-        case 2: translate_group<2>(G, L.src, tab, u, L.K, k, store, down); break;
-        case 3: translate_group<3>(G, L.src, tab, u, L.K, k, store, down); break;
-        default: translate_group<4>(G, L.src, tab, u, L.K, k, store, down); break;
+        case 1: translate_group<1, WIDE>(G, L.src, tab, u, L.K, k, store, down); break;
+        case 2: translate_group<2, WIDE>(G, L.src, tab, u, L.K, k, store, down); break;
+        case 3: translate_group<3, WIDE>(G, L.src, tab, u, L.K, k, store, down); break;
+        default: translate_group<4, WIDE>(G, L.src, tab, u, L.K, k, store, down); break;
         }
     }
 }
@@ -1541,16 +1548,14 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         ml.L = P.poles[i];
         ml.K = 2 * ml.L * ml.L;
         ml.len = P.blen[l];
-        if ((size_t)3 * ml.nbox * ml.K > 0xffffffffull) {
-            set_error(c, "mlfma: level patterns exceed 2^32 values");
-            return EMFA_ERR_UNSUPPORTED;
-        }
+        if ((size_t)3 * ml.nbox * ml.K > 0xffffffffull) M->wide = true;
     }
     // the interpolation and anterpolation passes may use more than the default 48 KB of shared memory
     EMFA_TRY(ensure_smem(c, k_upward, 96 * 1024));
     EMFA_TRY(ensure_smem(c, k_downward<true>, 200 * 1024));
     EMFA_TRY(ensure_smem(c, k_downward<false>, 200 * 1024));
-    EMFA_TRY(ensure_smem(c, k_translate, TRANS_SMEM));
+    EMFA_TRY(ensure_smem(c, k_translate<false>, TRANS_SMEM));
+    EMFA_TRY(ensure_smem(c, k_translate<true>, TRANS_SMEM));
     // finest-level lists and tables
     MLevel& fl = M->lv[nl - 1];
     const int Kf = fl.K;
@@ -1668,7 +1673,7 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
                     // from the source box to the parent's first octant, in boxes
                     int off = 0;
                     for (int d = 0; d < 3; ++d) off = 7 * off + (2 * pb.ix[d] - bx[f].ix[d]) + 3;
-                    gsrc.push_back(make_int2((int)(unsigned)((size_t)3 * f * K), off * TRANS_K));
+                    gsrc.push_back(make_int2(M->wide ? 3 * f : (int)(unsigned)((size_t)3 * f * K), off * TRANS_K));
                 }
             }
             // the offset (0, 0, 0) is near for every octant: T = 0
@@ -2019,7 +2024,7 @@ static emfa_status_t mlfma_apply(emfa_mlfma* M, const float2* x, float2* y, int 
         lv.l[i] = TransLevel{dptr<float2>(ml.up),     dptr<float2>(ml.down),      dptr<float2>(ml.trans),
                              dptr<int4>(ml.grp_src), dptr<TransGroup>(ml.grp), ml.K, (size_t)3 * ml.nbox * ml.K};
     }
-    k_translate<<<M->trans_ctas, 32 * TRANS_WARPS, TRANS_SMEM, st>>>(lv, dptr<TransWork>(M->trans_work), nr);
+    (M->wide ? k_translate<true> : k_translate<false>)<<<M->trans_ctas, 32 * TRANS_WARPS, TRANS_SMEM, st>>>(lv, dptr<TransWork>(M->trans_work), nr);
     const bool fused = finish_smem(M, rb) <= FINISH_SMEM_MAX;
     for (int i = 1; i < (fused ? nl - 1 : nl); ++i) {
         MLevel& ml = M->lv[i];
