@@ -3216,11 +3216,12 @@ emfa_status_t emfa_matvec(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_d
         EMFA_TRY(hgemm_apply(ctx, hp, X_dev, Y_dev, n_rhs, st));
         return hgemm_check_error(ctx, st);
     }
+    // the tiles copy whole elements; a complex64 may lie at any float
+    const bool whole = (((uintptr_t)Z_dev | (uintptr_t)X_dev | (uintptr_t)Y_dev) & 7) == 0;
+    if (matvec == EMFA_MV_F32 || !whole) return cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
     bool done = false;
-    if (matvec != EMFA_MV_F32) EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
-    if (done) return EMFA_OK;
-    if (matvec != EMFA_MV_F32) return cgemm_f32_block(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
-    return cgemm_f32(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
+    EMFA_TRY(slice_matvec(ctx, prec, Z_dev, n, X_dev, n, n_rhs, Y_dev, st, &done));
+    return done ? EMFA_OK : cgemm_f32_block(ctx, Z_dev, n, X_dev, n, n_rhs, Y_dev, st);
 }
 
 emfa_status_t emfa_residual(emfa_ctx_t* ctx, int prec, int matvec, const void* Z_dev, int n, const void* X_dev,
