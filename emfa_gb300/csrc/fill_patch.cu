@@ -243,7 +243,8 @@ __device__ __forceinline__ void stage_patch(Staged<T, NP>& s, const PatchArgs& p
 
 // ---------------------------------------------------------------------------
 // EFIE: 3 x 3 points (self pairs from the table) or 7 x 7 points (self and
-// edge-adjacent pairs from the table)
+// edge-adjacent pairs from the table; a triangle lists three neighbours, so on a
+// mesh with more at an edge a pair may be in one direction's table only)
 // ---------------------------------------------------------------------------
 template <typename T, int NP>
 __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __restrict__ rw, FillConst<T> c,
@@ -270,9 +271,8 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
         for (int pr = threadIdx.x; pr < ntf * nts; pr += blockDim.x) {
             const int tf = pr / nts, ts = pr - tf * nts;
             const int idf = sf.id[tf], ids = ss.id[ts];
-            bool table = idf == ids;
-            if (NP == 7 && !table)
-                table = nbr[3 * (size_t)idf] == ids || nbr[3 * (size_t)idf + 1] == ids || nbr[3 * (size_t)idf + 2] == ids;
+            bool table = idf == ids;  // both ways: no regular value is read
+            if (NP == 7 && !table) table = table_slot(nbr, idf, ids) >= 0 && table_slot(nbr, ids, idf) >= 0;
             T sr[3][3], si[3][3];  // S_ij
 #pragma unroll
             for (int i = 0; i < 3; ++i)
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
                 out_t = edm_value(S, F, c);
             }
         } else {
-            T zr = T(0), zi = T(0);
+            T zr = T(0), zi = T(0), yr = T(0), yi = T(0);  // regular part of (f, s) and of (s, f)
             // self terms, of (f, s) and of (s, f): each pair's value formed in FP64 and rounded once to T
             T tr = T(0), ti = T(0), ur = T(0), ui = T(0);
 #pragma unroll
@@ -414,12 +414,13 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
                 const int la = sidef[2 * lf + a] * PS, tf = F.tri[a];
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    const Cx<T> v = val[la + sides[2 * ls + b]];
-                    zr += a == b ? v.re : -v.re;
-                    zi += a == b ? v.im : -v.im;
+                    Cx<T> v = val[la + sides[2 * ls + b]];
+                    if (a != b) v = cx(-v.re, -v.im);
                     const int ts = S.tri[b];
                     const double sgn = a == b ? 1.0 : -1.0;
                     if (NP == 3) {
+                        zr += v.re;
+                        zi += v.im;
                         if (tf != ts) continue;
                         const double2* p = tab + 3 * (9 * (size_t)tf + 3 * F.e[a] + S.e[b]);
                         const double2* q = tab + 3 * (9 * (size_t)ts + 3 * S.e[b] + F.e[a]);
@@ -434,18 +435,28 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
                             const double2 p = tab[36 * (size_t)tf + 9 * sl + 3 * F.e[a] + S.e[b]];
                             tr += (T)(sgn * p.x);
                             ti += (T)(sgn * p.y);
+                        } else {
+                            zr += v.re;
+                            zi += v.im;
                         }
                         if (st >= 0) {
                             const double2 q = tab[36 * (size_t)ts + 9 * st + 3 * S.e[b] + F.e[a]];
                             ur += (T)(sgn * q.x);
                             ui += (T)(sgn * q.y);
+                        } else {
+                            yr += v.re;
+                            yi += v.im;
                         }
                     }
                 }
             }
+            if (NP == 3) {
+                yr = zr;
+                yi = zi;
+            }
             const T kz = (T)c.coef_efie * (F.len * S.len);
             out = cx(-kz * (w2 * zi + ti), kz * (w2 * zr + tr));
-            out_t = cx(-kz * (w2 * zi + ui), kz * (w2 * zr + ur));
+            out_t = cx(-kz * (w2 * yi + ui), kz * (w2 * yr + ur));
         }
         Z[(size_t)f * ldz + s] = out;
         if (bf != bs) Z[(size_t)s * ldz + f] = out_t;
