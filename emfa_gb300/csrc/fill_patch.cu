@@ -407,8 +407,10 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
             }
         } else {
             T zr = T(0), zi = T(0), yr = T(0), yi = T(0);  // regular part of (f, s) and of (s, f)
-            // self terms, of (f, s) and of (s, f): each pair's value formed in FP64 and rounded once to T
-            T tr = T(0), ti = T(0), ur = T(0), ui = T(0);
+            // table terms, of (f, s) and of (s, f), summed in FP64 and rounded once to T
+            // (few entries have any: the sums start, and are rounded, where one does)
+            double tr = 0, ti = 0, ur = 0, ui = 0;
+            bool any = false;
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
                 const int la = sidef[2 * lf + a] * PS, tf = F.tri[a];
@@ -425,24 +427,27 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
                         const double2* p = tab + 3 * (9 * (size_t)tf + 3 * F.e[a] + S.e[b]);
                         const double2* q = tab + 3 * (9 * (size_t)ts + 3 * S.e[b] + F.e[a]);
                         const int var = a == 0 && b == 0 ? 0 : 1;
-                        tr += (T)(sgn * p[var].x + p[2].x);
-                        ti += (T)(sgn * p[var].y + p[2].y);
-                        ur += (T)(sgn * q[var].x + q[2].x);
-                        ui += (T)(sgn * q[var].y + q[2].y);
+                        any = true;
+                        tr += sgn * p[var].x + p[2].x;
+                        ti += sgn * p[var].y + p[2].y;
+                        ur += sgn * q[var].x + q[2].x;
+                        ui += sgn * q[var].y + q[2].y;
                     } else {
                         const int sl = table_slot(nbr, tf, ts), st = table_slot(nbr, ts, tf);
                         if (sl >= 0) {
                             const double2 p = tab[36 * (size_t)tf + 9 * sl + 3 * F.e[a] + S.e[b]];
-                            tr += (T)(sgn * p.x);
-                            ti += (T)(sgn * p.y);
+                            any = true;
+                            tr += sgn * p.x;
+                            ti += sgn * p.y;
                         } else {
                             zr += v.re;
                             zi += v.im;
                         }
                         if (st >= 0) {
                             const double2 q = tab[36 * (size_t)ts + 9 * st + 3 * S.e[b] + F.e[a]];
-                            ur += (T)(sgn * q.x);
-                            ui += (T)(sgn * q.y);
+                            any = true;
+                            ur += sgn * q.x;
+                            ui += sgn * q.y;
                         } else {
                             yr += v.re;
                             yi += v.im;
@@ -455,8 +460,13 @@ __global__ void __launch_bounds__(256) k_fill_patch_efie(const RwgPack<T>* __res
                 yi = zi;
             }
             const T kz = (T)c.coef_efie * (F.len * S.len);
-            out = cx(-kz * (w2 * zi + ti), kz * (w2 * zr + tr));
-            out_t = cx(-kz * (w2 * yi + ui), kz * (w2 * yr + ur));
+            Cx<T> t = cx(T(0), T(0)), u = t;
+            if (any) {
+                t = cx((T)tr, (T)ti);
+                u = cx((T)ur, (T)ui);
+            }
+            out = cx(-kz * (w2 * zi + t.im), kz * (w2 * zr + t.re));
+            out_t = cx(-kz * (w2 * yi + u.im), kz * (w2 * yr + u.re));
         }
         Z[(size_t)f * ldz + s] = out;
         if (bf != bs) Z[(size_t)s * ldz + f] = out_t;

@@ -54,3 +54,24 @@ def test_edges_of_three_triangles(ctx, precision, tol):
         assert (abs(a - b) / np.maximum(abs(b), 1e-3 * abs(b).max())).max() < tol
     else:
         assert np.linalg.norm(a - b) / np.linalg.norm(b) < tol
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("surface", ["sphere", "fins"])
+def test_entries_of_tables_alone(ctx, precision, surface):
+    """A diagonal entry has no regular pair: its FP64 table values are summed in FP64 and rounded once, bit for bit the
+    other kernel's sum (same values, same order, one product after)."""
+    if surface == "fins":
+        m, rows = _finned_sphere()
+        listed = {}  # the neighbours a triangle lists: its first three
+        for r in rows:
+            for t, o in ((r[4], r[5]), (r[5], r[4])):
+                if len(listed.setdefault(t, [])) < 3 and o not in listed[t]:
+                    listed[t].append(o)
+        alone = [u for u, r in enumerate(rows) if r[5] in listed[r[4]] and r[4] in listed[r[5]]]
+    else:
+        m = M.icosphere(2, 0.5)
+        rows = api.build_rwg(m.tris)
+        alone = range(len(rows))
+    a, b = _both(ctx, m, rows, precision)
+    assert len(alone) > 100 and np.array_equal(np.diag(a)[alone], np.diag(b)[alone])
