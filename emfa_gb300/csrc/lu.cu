@@ -1147,8 +1147,11 @@ emfa_status_t lu_factor(Ctx* c, const void* Z, int n, LuFactor& F, cudaStream_t 
     struct Aux {
         cudaStream_t s = nullptr;
         cudaEvent_t panel = nullptr, rest = nullptr;
+        bool open = false;  // work on s that the caller's stream does not wait for yet
         ~Aux()
         {
+            // an error return: the caller frees what that work reads and writes
+            if (open) cudaStreamSynchronize(s);
             if (panel) cudaEventDestroy(panel);
             if (rest) cudaEventDestroy(rest);
             if (s) cudaStreamDestroy(s);
@@ -1211,6 +1214,7 @@ emfa_status_t lu_factor(Ctx* c, const void* Z, int n, LuFactor& F, cudaStream_t 
         return EMFA_OK;
     };
     if (aux.s) EMFA_TRY(wait_for(hs, aux.panel, st));
+    aux.open = aux.s != nullptr;
     EMFA_TRY(diag(0));
     int kb = 0;
     while (kb < F.nblk) {
@@ -1250,6 +1254,7 @@ emfa_status_t lu_factor(Ctx* c, const void* Z, int n, LuFactor& F, cudaStream_t 
         kb += 1;
     }
     if (aux.s) EMFA_TRY(wait_for(st, aux.panel, hs));
+    aux.open = false;
     if (F.nblk > 1) {
         k_lu_rowperm_left<<<dim3((unsigned)(F.nblk - 1) * (NB / 32), (unsigned)F.nblk), 256, 0, st>>>(
             A, n, lda, dptr<int>(F.perm));
