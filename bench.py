@@ -16,9 +16,11 @@ e2e           the same job through the host-buffer C ABI call emfa_dense_rcs
 accuracy      the job's RCS and currents against the reference's own run at
               this size (tests/golden/c2_cfie_sphere_7680.npz: the reference's
               RCS of the exact solution of its FP64 matrix)
-vs_plain_fp64 the same 360-incidence job on the plain FP64 GPU path (FP64
-              fill, FP64 GMRES(30) with two Gram-Schmidt passes): its solves/s
-              and the mixed path's RCS / current difference from it
+vs_plain_fp64 the same 360-incidence job on the FP64 GPU path (FP64 fill, FP64
+              GMRES(30) with two Gram-Schmidt passes, the default FP64
+              products): its solves/s and the mixed path's RCS / current
+              difference from it; vs_plain_fp64_cuda_cores the same with the
+              products on the CUDA cores (matvec "f64")
 c1, mlfma,    the other configurations, a few seconds each: C1 plain FP64 EFIE
 batch, serve  (1,920 RWG, bistatic), C3 MLFMA (122,880 RWG), C4 batched (64
               uneven EFIE problems), C5 served stream (Poisson arrivals)
@@ -202,10 +204,11 @@ def run_emfa(args, workload):
     h2d = m.verts.nbytes + m.tris.nbytes + ang.nbytes + dirs.nbytes
     d2h = out.nbytes
 
-    acc, plain = {}, {}
+    acc, plain, plain_cores = {}, {}, {}
     if args.check and rank == 0:
         acc = accuracy_vs_reference(ang, last["X"], last["rcs"])
-        plain = plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, last["X"], last["rcs"])
+        plain = plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, last["X"], last["rcs"], "auto")
+        plain_cores = plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, last["X"], last["rcs"], "f64")
     torch.cuda.synchronize()
     geo.close()  # geometry before its context, not left to the interpreter's shutdown
     ctx.close()
@@ -216,7 +219,7 @@ def run_emfa(args, workload):
         "stages": {k: statistics.median(v) for k, v in stages.items()}, "infos": infos,
         "launches": launches, "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": int(h2d),
                                       "d2h_bytes_per_step": int(d2h), "ms": statistics.median(e2e_ms)},
-        "clocks": clocks.summary(), "n": n, "n_inc": n_inc, "acc": acc, "plain": plain, "world": world,
+        "clocks": clocks.summary(), "n": n, "n_inc": n_inc, "acc": acc, "plain": plain, "plain_cores": plain_cores, "world": world,
         "rank": rank, "kernels": kernels, "n_tri": int(m.tris.shape[0]),
         "autotune": api.autotune_query(local, n, n_inc),
     }
@@ -239,15 +242,16 @@ def accuracy_vs_reference(ang, X, r):
             "current_max_rel_err": float(max(errs)), "bar_db": 0.1, "bar_current": 1e-4}
 
 
-def plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, X_mixed, r_mixed):
+def plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, X_mixed, r_mixed, matvec):
     """The same 360-incidence job on the plain FP64 GPU path: FP64 fill and
     excitation, FP64 GMRES(30) to 1e-6 with two Gram-Schmidt passes, FP64
-    products on the CUDA cores, RCS.  Timed once end to end on the device
-    (wall clock, device synchronised on both sides)."""
+    products (matvec "auto", the default, or "f64", on the CUDA cores), RCS.
+    Timed once end to end on the device (wall clock, device synchronised on
+    both sides)."""
     import torch
     from emfa_gb300 import api
     fp64 = api.fill_params("cfie", "f64", freq, alpha)
-    sp64 = api.solver_params("gmres", restart=30, max_iter=900, tol=1e-6, matvec="f64")
+    sp64 = api.solver_params("gmres", restart=30, max_iter=900, tol=1e-6, matvec=matvec)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     Z = api.fill_z(geo, fp64)
@@ -264,7 +268,7 @@ def plain_fp64_job(ctx, geo, freq, alpha, ang, dirs, X_mixed, r_mixed):
             "iterations": info.iterations, "converged": info.converged,
             "rcs_max_abs_err_db_mixed_vs_plain": float(np.abs(r_mixed - r).max()),
             "current_max_rel_err_mixed_vs_plain": float(cur),
-            "work": "same job: %d incidences, tol 1e-6, one fill" % len(ang)}
+            "work": "same job: %d incidences, tol 1e-6, one fill" % len(ang), "matvec": matvec}
 
 
 def measured_peaks():
@@ -357,12 +361,12 @@ def run_c1(args):
     dirs = api.bistatic_dirs(0.0, 180.0, 1.0, 0.0, ring=True)
     out = {"workload": "c1_efie_sphere_1920", "n_rwg": geo.n, "directions": int(dirs.shape[0])}
     for name, prec, sp, disc in (
-            ("plain_fp64", "f64", api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000, matvec="f64"), "reference"),
+            ("plain_fp64", "f64", api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000), "reference"),
             ("mixed", "f32", api.solver_params("lu", tol=1e-6, max_iter=50), "reference"),
             # the discretisation the configuration states: 7-point rule,
             # extraction on self and edge-adjacent pairs (no reference run)
             ("plain_fp64_config_discretisation", "f64",
-             api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000, matvec="f64"), "config"),
+             api.solver_params("gmres", restart=30, tol=1e-6, max_iter=20000), "config"),
             ("mixed_config_discretisation", "f32", api.solver_params("lu", tol=1e-6, max_iter=50), "config")):
         fp = api.fill_params("efie", prec, 3e8, 1.0, discretisation=disc)
         times = []
@@ -580,7 +584,7 @@ def run_batch(args):
         geo = api.Geometry(ctx, m)
         fp = api.fill_params("efie", "f64", f, 1.0)
         fp.edm_mode = 2
-        sp = api.solver_params("gmres", restart=250, tol=1e-5, max_iter=5000, matvec="f64")
+        sp = api.solver_params("gmres", restart=250, tol=1e-5, max_iter=5000)
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         Z = api.fill_z(geo, fp)
@@ -742,7 +746,7 @@ def main():
     res = run_emfa(args, args.workload)
     if rank != 0:
         return
-    plain = res["plain"]
+    plain, cores = res["plain"], res["plain_cores"]
     line = {
         "metric": METRIC, "value": round(res["value"], 3), "unit": "solves/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(res["total_ms"] / args.steps, 3),
@@ -762,6 +766,8 @@ def main():
         "clocks": res["clocks"],
         "accuracy": res["acc"],
         "vs_plain_fp64": dict(plain, speedup=round(res["value"] / plain["solves_per_s"], 2)) if plain else None,
+        "vs_plain_fp64_cuda_cores": dict(cores, speedup=round(res["value"] / cores["solves_per_s"], 2)) if cores
+        else None,
         "roofline": roofline(res),
         "fill_roofline": fill_roofline(res),
         "kernels": kernel_table(res),
