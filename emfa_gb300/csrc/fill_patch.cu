@@ -811,9 +811,11 @@ emfa_status_t launch_fill_patch(Ctx* c, Geom* g, const GeomDev<T>& d, const emfa
                                 const FillConst<T>& fc, const double2* tab, void* Z, size_t ldz, cudaStream_t st,
                                 bool* done)
 {
-    EMFA_TRY(patch_plan(c, g, st));
-    *done = g->patch_ok;
-    if (!g->patch_ok) return EMFA_OK;
+    const emfa_status_t plan = patch_plan(c, g, st);
+    *done = plan == EMFA_OK && g->patch_ok;
+    if (plan == EMFA_ERR_OOM) cudaGetLastError();  // no room for the plan: a thread per entry needs none
+    else EMFA_TRY(plan);
+    if (!*done) return EMFA_OK;
     const int nb = g->patch_nb;
     const PatchArgs pa{dptr<int>(g->patch_rwg),           dptr<int>(g->patch_nt),     dptr<int>(g->patch_tri),
                        dptr<unsigned char>(g->patch_slot), dptr<unsigned char>(g->patch_side),

@@ -8,7 +8,8 @@ namespace emfa {
 
 // Fills Z from the self-term table `tab` (the singular table, or the
 // configuration's with the triangles' neighbours in g->nbr).  *done false: the
-// geometry or the parameters are not for this fill, nothing was launched.
+// geometry or the parameters are not for this fill, or there is no room for its
+// plan (24 bytes an RWG); nothing was launched.
 template <typename T>
 emfa_status_t launch_fill_patch(Ctx* c, Geom* g, const GeomDev<T>& d, const emfa_fill_params_t* p,
                                 const FillConst<T>& fc, const double2* tab, void* Z, size_t ldz, cudaStream_t st,
