@@ -1642,6 +1642,9 @@ static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
         c->kernel_launches += 3;
         EMFA_CUDA(c, cudaGetLastError());
     }
+    // under a budget the singular table goes before the level tables come (and
+    // the host waits here for the near field, which it otherwise overlaps)
+    if (c->budget) tab.release();
     // per-level tables
     struct Series {
         DevView hl, rec, minl, kd;

@@ -29,3 +29,22 @@ def test_fill_without_room_for_its_plan(emfa_lib, kind, precision, disc):
         assert np.linalg.norm(z - want) / np.linalg.norm(want) < 2e-5
     geo.close()
     tight.close()
+
+
+def test_mlfma_setup_peak(emfa_lib):
+    """Under a budget the set-up needs the operator and, beside it, at most the singular table of 9 FP64 pairs a triangle."""
+    m = M.icosphere(4, 1.6)
+    c = api.Context(0, 1 << 40)
+    geo = api.Geometry(c, m)
+    op = api.Mlfma(geo, api.mlfma_params(3e8, 0.5, 0.25))
+    used, peak, _ = c.memory()
+    assert peak - used <= 9 * 16 * len(m.tris)
+    need = peak
+    op.close()
+    geo.close()
+    c.close()
+    tight = api.Context(0, need)
+    geo = api.Geometry(tight, m)
+    api.Mlfma(geo, api.mlfma_params(3e8, 0.5, 0.25)).close()
+    geo.close()
+    tight.close()
