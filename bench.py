@@ -326,7 +326,7 @@ def fill_roofline(res):
     mhz = res["clocks"].get("sm_mhz") or 2070.0
     peak = RM.fp32_nominal_tflops(152, mhz)
     achieved = flops / (ms * 1e-3) / 1e12
-    return {"kernel": "k_fill_tile_cfie_sym (CFIE)", "bound": "fp32/mufu issue", "avg_launch_ms": round(ms / n_l, 4),
+    return {"kernel": "k_fill_tile_cfie_sym (CFIE)", "bound": "latency at the phases' barriers (issue 61 %)", "avg_launch_ms": round(ms / n_l, 4),
             "achieved": round(achieved, 2), "unit": "TFLOP/s (model)", "peak": round(peak, 1),
             "frac": round(achieved / peak, 4),
             "peak_source": "nominal FP32 FMA rate at the median SM clock (no measured FP32 figure)"}

@@ -18,8 +18,6 @@
 #include <algorithm>
 #include <climits>
 
-#include <algorithm>
-
 namespace emfa {
 
 template <typename T, bool CHUNKED>

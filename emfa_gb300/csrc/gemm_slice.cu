@@ -50,8 +50,8 @@
 // 64-byte rows: the copies (1536 rows a stage, four cycles each) set its pace,
 // 416 us at n = 2430 x 181 right-hand sides with the tensor pipe 32 % active,
 // whatever the drain did.  A single thread issuing MMAs with descriptors from
-// its own registers bounded the second (382 us, 86 cycles a MMA); now 301 us,
-// 45 %.
+// its own registers bounded the second (382 us, 86 cycles a MMA); now 298 us,
+// 48 %.
 // On GB300, a product of n unknowns and R right-hand sides, its split of Z and
 // the magnitudes' product (10 us and 18 us) included, against 64 x 64 CUDA-core
 // tiles and against the GEMV that sums again where every result needs it:

@@ -477,9 +477,9 @@ __global__ void k_upward(const float2* __restrict__ child, int Lc, const int* __
 // Per (source, sibling): one 8-byte shared load and 12 FMA, against an 8-byte
 // table and a 24-byte pattern load through L1 when a thread took one box's far
 // list (5-wavelength sphere, 122,880 unknowns: 518 us for the five levels with
-// the anterpolation, the L1 data path 80 % busy).  Now 290 us
-// with twelve warps, and 107 for the anterpolation above the finest level; still bound by L1
-// wavefronts (71 %), half of them the siblings' table values.  Eight siblings a
+// the anterpolation, the L1 data path 80 % busy).  Now 248 us, and 109 for the
+// anterpolation above the finest level; still bound by L1 wavefronts (81 %), half
+// of them the siblings' table values.  Eight siblings a
 // warp, or two patterns in flight, were no faster (spills; latency).
 constexpr int TRANS_LEVELS = 24;  // octree levels a launch takes
 // sixteen warps, two CTAs an SM by the table: a product in us with 12 | 14 | 16 |
@@ -711,7 +711,7 @@ __global__ void k_downward(int L, int R, const float2* __restrict__ pdown, int L
 //   2. a warp per unknown: receive pattern times down pattern, then the near row.
 // As two kernels (the anterpolation writing x, y, z patterns that each unknown
 // read and projected again, and gathered its near x itself) this took 252 us on
-// 122,880 unknowns, latency-bound; now 189.
+// 122,880 unknowns, latency-bound; now 181.
 struct FinishArgs {
     const float2* x;
     int n, nr;
@@ -1497,7 +1497,7 @@ static emfa_status_t alloc_patterns(emfa_mlfma* M, int nr)
 // had cost 3 ms more with the first product and the release.  So the
 // singular table runs beside the tree, patterns and near field beside the
 // level tables, and the tables travel as two buffers: 10.6 -> 4.2 ms, with a
-// first product of four right-hand sides and the release 13.4 -> 6.1.
+// first product of four right-hand sides and the release 13.7 -> 6.5.
 static emfa_status_t mlfma_build(emfa_mlfma* M, cudaStream_t st)
 {
     Ctx* c = M->ctx;

@@ -3,8 +3,7 @@ in two; one or several pattern levels; right-hand sides a pass of one, of up to 
 
 The far and near parts are sums of the same FP32 products whatever the pass, so a column of a block is the column alone to
 FP32 rounding of its own sums (a few hundred terms: 1e-5 of the column's norm is far above it), and near + far is the whole.
-Against the dense CFIE matrix the operator is the multilevel approximation; its three-point interpolation keeps it to a few
-percent, which a wrong list, table or phase does not."""
+Against the CFIE entries themselves the multilevel approximation is held in test_gpu_mlfma_extent.py."""
 import pytest
 
 from emfa_gb300 import api
